@@ -11,6 +11,7 @@
 
 #include <algorithm>
 #include <atomic>
+#include <cmath>
 #include <cstdarg>
 #include <cstdio>
 #include <cstring>
@@ -26,7 +27,8 @@
 
 namespace {
 
-constexpr int PJG_KIND_VJP = 2;  // internal kernel kind of pjg_vjp
+constexpr int PJG_KIND_VJP = KIND_VJP;  // internal kernel kind of pjg_vjp
+static_assert(PJG_SPECIES_RATES == KIND_RATES && PJG_JACOBIAN == KIND_JAC, "kernel kinds");
 thread_local char g_err[512] = "";
 // kernel launches issued by this library, and optional per-launch timing of
 // the evaluation kernels (pjg_profile_begin / pjg_profile_end)
@@ -61,16 +63,51 @@ int upload(const std::vector<T>& h, T** d)
     return 0;
 }
 
+// several tables in one device buffer: add() them, then send()
+struct Pack {
+    std::vector<char> bytes;
+    std::vector<std::pair<const void**, size_t>> where;
+    template <class T>
+    void add(const std::vector<T>& h, const T** d)
+    {
+        const size_t at = (bytes.size() + 255) & ~size_t(255);
+        bytes.resize(at + std::max<size_t>(h.size(), 1) * sizeof(T), 0);
+        if (!h.empty()) memcpy(bytes.data() + at, h.data(), h.size() * sizeof(T));
+        where.push_back({(const void**)d, at});
+    }
+    int send(char** buffer)
+    {
+        if (int rc = upload(bytes, buffer)) return rc;
+        for (auto& w : where) *w.first = *buffer + w.second;
+        return 0;
+    }
+};
+
+// tables of one Jacobian output layout
 struct SlotTables {
-    int nslot = 0;
-    int *rxn_slot_off = nullptr, *rxn_slots = nullptr;
-    int *row_off = nullptr, *col_off = nullptr;
-    int2 *row_list = nullptr, *col_list = nullptr;
+    int nslot = 0, n_ns = 0;
+    std::vector<int> slot;  // host: (ns - 1)^2 species-block slots, -1 outside a sparse pattern
+    int *ns_rows = nullptr, *ns_slots = nullptr;
     int *sp_slots = nullptr, *cj_slots = nullptr;
-    int *dchunk_off = nullptr, *dchunk_list = nullptr;
-    int4* dchunk_slots = nullptr;  // sparse output only
+    int* col_off = nullptr;  // with col_list: only where a pattern leaves out a term
+    int2* col_list = nullptr;
     int s00 = 0, s01 = 0, s10 = 0, s11 = 0;
-    size_t bytes = 0;
+};
+
+// the thread-per-state kernel's tables of one (kind, output layout)
+struct WaveHold {
+    WaveTables wt;
+    const PostItem* ns_post = nullptr;
+    int n_ns_post = 0, n_vec = 0;
+    char* buffer = nullptr;
+};
+
+// a tile shape's schedule on the device, with its third-body bath-gas terms (J^T v)
+struct SchedTables {
+    Schedule sc;
+    const PostItem* ns_post = nullptr;
+    int n_ns_post = 0;
+    char* buffer = nullptr;
 };
 
 }  // namespace
@@ -87,12 +124,13 @@ extern "C" int pjg_internal_lu_solve_sparse(const void* p, int64_t n, char order
 
 struct pjg_mech {
     int ns = 0, nr = 0, nn = 0, need_logP = 0, nnz = 0, jac_approx = 0;
-    int nr_e22 = 0;  // leading reactions of the class A + B <=> C + D
     double kc_split_max = 138.0;  // EvalArgs::kc_split_max
-    int ma_off[11] = {};                          // then the mass-action patterns (EvalArgs)
-    int tp_off[4] = {0, 0, 0, 0};                 // then the third-body patterns (EvalArgs)
+    std::vector<int> cls;         // class of each packed record (tile_kernel's switch)
+    int n_m = 0;                  // third-body lists that several reactions share
+    int4* m_lists = nullptr;
+    std::vector<RxnRec> d_rxn;    // host copy of the device records
     int device = 0;
-    PjgRxn* rxn = nullptr;
+    RxnRec* rxn = nullptr;
     double* sp = nullptr;
     int* thd_spec = nullptr;
     double* thd_coef = nullptr;
@@ -103,6 +141,8 @@ struct pjg_mech {
     std::vector<double> h_thd_coef;
     std::vector<int> crs_ptr, crs_ind, ccs_ptr, ccs_ind;
     std::map<int, SlotTables> slots;  // key: (order == 'F') * 2 + sparse
+    std::map<int, SchedTables> scheds;  // key: kind, layout, tile shape
+    std::map<int, WaveHold> waves;      // key: kind * 4 + layout
     std::mutex lock;
     // working buffer shared by device-pointer calls on this mechanism
     double* work = nullptr;
@@ -155,6 +195,20 @@ int slot_of(const pjg_mech* m, bool F, bool sparse, int r, int c)
     return -1;
 }
 
+SchedInput sched_input(const pjg_mech* m, int kind, const std::vector<int>* slot)
+{
+    SchedInput in;
+    in.kind = kind;
+    in.ns = m->ns;
+    in.jac_approx = m->jac_approx;
+    in.rxn = &m->d_rxn;
+    in.cls = &m->cls;
+    in.thd_spec = &m->h_thd_spec;
+    in.thd_coef = &m->h_thd_coef;
+    in.slot = slot;
+    return in;
+}
+
 int build_slots(pjg_mech* m, bool F, bool sparse, SlotTables** out)
 {
     const int key = (F ? 2 : 0) + (sparse ? 1 : 0);
@@ -167,99 +221,61 @@ int build_slots(pjg_mech* m, bool F, bool sparse, SlotTables** out)
     const int ns = m->ns, last = ns - 1, NN = m->nn;
     SlotTables t;
     t.nslot = sparse ? m->nnz : NN * NN;
-    std::vector<int> off(m->nr + 1, 0), list;
-    for (int i = 0; i < m->nr; ++i) {
-        const PjgRxn& R = m->h_rxn[i];
-        const int nsp = R.nspec;
-        off[i] = (int)list.size();
-        for (int a = 0; a < nsp; ++a)
-            for (int b = 0; b < nsp; ++b) {
-                const int k = ent_spec(R.ent[a]), j = ent_spec(R.ent[b]);
-                list.push_back(k == last || j == last ? -1 : slot_of(m, F, sparse, 2 + k, 2 + j));
-            }
-        for (int a = 0; a < nsp; ++a) {
-            const int k = ent_spec(R.ent[a]);
-            list.push_back(k == last ? -1 : slot_of(m, F, sparse, 2 + k, 0));
-            list.push_back(k == last ? -1 : slot_of(m, F, sparse, 2 + k, 1));
-        }
-        for (int l = 0; l < R.thd_cnt; ++l) {
-            const int j = m->h_thd_spec[R.thd_off + l];
-            for (int a = 0; a < nsp; ++a) {
-                const int k = ent_spec(R.ent[a]);
-                list.push_back(k == last || j == last ? -1 : slot_of(m, F, sparse, 2 + k, 2 + j));
-            }
+    t.slot.assign((size_t)last * last, -1);
+    if (!sparse) {
+        for (int r = 0; r < last; ++r)
+            for (int c = 0; c < last; ++c) t.slot[(size_t)r * last + c] = slot_of(m, F, false, 2 + r, 2 + c);
+    } else {
+        const std::vector<int>&ptr = F ? m->ccs_ptr : m->crs_ptr, &ind = F ? m->ccs_ind : m->crs_ind;
+        for (int x = 2; x < NN; ++x)
+            for (int q = ptr[x]; q < ptr[x + 1]; ++q)
+                if (ind[q] >= 2) t.slot[F ? (size_t)(ind[q] - 2) * last + x - 2 : (size_t)(x - 2) * last + ind[q] - 2] = q;
+    }
+    // rows with bath-gas terms: the terms go into every species column
+    std::vector<char> ns_row(ns, 0);
+    for (const PjgRxn& R : m->h_rxn) {
+        const bool ns_terms = (R.flags & RX_HASNS) || (RX_THD(R.flags) && (R.flags & RX_NSLIST));
+        for (int e = 0; e < R.nspec && ns_terms && !m->jac_approx; ++e)
+            if (ent_nur(R.ent[e]) != ent_nuf(R.ent[e]) && ent_spec(R.ent[e]) != last) ns_row[ent_spec(R.ent[e])] = 1;
+    }
+    bool left_out = false;  // a term that is not zero by itself has no entry
+    std::vector<int> ns_rows, ns_slots;
+    for (int k = 0; k < last; ++k) {
+        if (!ns_row[k]) continue;
+        ns_rows.push_back(k);
+        for (int j = 0; j < last; ++j) {
+            const int sl = t.slot[(size_t)k * last + j];
+            if (sl < 0) left_out = true;
+            ns_slots.push_back(sl);
         }
     }
-    off[m->nr] = (int)list.size();
-    std::vector<int> row_off(ns, 0), col_off(ns, 0), sp_slots(2 * std::max(last, 1), -1),
-        cj_slots(2 * std::max(last, 1), -1);
-    std::vector<int2> row_list, col_list;
+    {
+        SchedInput in = sched_input(m, PJG_JACOBIAN, &t.slot);
+        SchedHost sh;
+        sched_build(in, 5, 8, 1, 1 << 10, sh);
+        left_out = left_out || sh.left_out;
+    }
+    std::vector<int> sp_slots(2 * std::max(last, 1), -1), cj_slots(2 * std::max(last, 1), -1), col_off;
+    std::vector<int2> col_list;
     for (int k = 0; k < last; ++k) {
-        row_off[k] = (int)row_list.size();
-        for (int j = 0; j < last; ++j) {
-            const int sl = slot_of(m, F, sparse, 2 + k, 2 + j);
-            if (sl >= 0) row_list.push_back(make_int2(j, sl));
-        }
         sp_slots[2 * k] = slot_of(m, F, sparse, 2 + k, 0);
         sp_slots[2 * k + 1] = slot_of(m, F, sparse, 2 + k, 1);
     }
     for (int j = 0; j < last; ++j) {
-        col_off[j] = (int)col_list.size();
-        for (int k = 0; k < last; ++k) {
-            const int sl = slot_of(m, F, sparse, 2 + k, 2 + j);
-            if (sl >= 0) col_list.push_back(make_int2(k, sl));
-        }
         cj_slots[2 * j] = slot_of(m, F, sparse, 0, 2 + j);
         cj_slots[2 * j + 1] = slot_of(m, F, sparse, 1, 2 + j);
         if (cj_slots[2 * j] < 0 || cj_slots[2 * j + 1] < 0)
             return fail(PJG_ERR_TABLES, "Jacobian pattern lacks entries of rows T/E");
     }
-    row_off[last] = (int)row_list.size();
-    col_off[last] = (int)col_list.size();
-    // the structurally nonzero entries of the species block (the pattern's;
-    // for a dense output also every entry a reaction adds to) in chunks of
-    // PJG_DENSE_COLS columns, the assembly's row lists; a sparse output's
-    // slots of each listed row
-    static_assert(PJG_DENSE_COLS == 4, "one int4 of slots per listed row");
-    std::vector<int> doff, dlist;
-    std::vector<int4> dslots;
-    if (last > 0) {
-        std::vector<char> nz((size_t)last * last, 0);
-        for (int k = 0; k < last; ++k)
-            for (int q = m->crs_ptr[2 + k]; q < m->crs_ptr[3 + k]; ++q) {
-                const int c = m->crs_ind[q] - 2;
-                if (c >= 0 && c < last) nz[(size_t)k * last + c] = 1;
-            }
-        if (!sparse)
-            for (int sl : list) {
-                if (sl < 0) continue;
-                const int r = F ? sl % NN : sl / NN, c = F ? sl / NN : sl % NN;
-                if (r >= 2 && c >= 2) nz[(size_t)(r - 2) * last + (c - 2)] = 1;
-            }
-        for (int j0 = 0; j0 < last; j0 += PJG_DENSE_COLS) {
-            doff.push_back((int)dlist.size());
-            for (int k = 0; k < last; ++k) {
-                int mask = 0, sl[PJG_DENSE_COLS] = {-1, -1, -1, -1};
-                for (int q = 0; q < PJG_DENSE_COLS && j0 + q < last; ++q)
-                    if (nz[(size_t)k * last + j0 + q]) {
-                        mask |= 1 << q;
-                        sl[q] = slot_of(m, F, sparse, 2 + k, 2 + j0 + q);
-                        if (sparse && sl[q] < 0)
-                            return fail(PJG_ERR_TABLES, "Jacobian pattern inconsistent");
-                    }
-                if (mask) {
-                    dlist.push_back(k << 4 | mask);
-                    if (sparse) dslots.push_back(make_int4(sl[0], sl[1], sl[2], sl[3]));
-                }
-            }
+    if (left_out) {
+        for (int j = 0; j < last; ++j) {
+            col_off.push_back((int)col_list.size());
+            for (int k = 0; k < last; ++k)
+                if (t.slot[(size_t)k * last + j] >= 0) col_list.push_back(make_int2(k, t.slot[(size_t)k * last + j]));
         }
-        doff.push_back((int)dlist.size());
-        // a sparse output takes the chunk lists where the pattern fills at
-        // least half of the listed rows' slots (GRI: 1,774 of 2,100); else
-        // its two passes over the pattern (the 500-species mechanism: about a
-        // third, where the lists ran 19 % slower)
-        if (sparse && (size_t)m->nnz * 2 < dlist.size() * PJG_DENSE_COLS) dslots.clear();
+        col_off.push_back((int)col_list.size());
     }
+    t.n_ns = (int)ns_rows.size();
     t.s00 = slot_of(m, F, sparse, 0, 0);
     t.s01 = slot_of(m, F, sparse, 0, 1);
     t.s10 = slot_of(m, F, sparse, 1, 0);
@@ -267,31 +283,17 @@ int build_slots(pjg_mech* m, bool F, bool sparse, SlotTables** out)
     if (t.s00 < 0 || t.s01 < 0 || t.s10 < 0 || t.s11 < 0)
         return fail(PJG_ERR_TABLES, "Jacobian pattern lacks the T/E block");
     int rc;
-    if ((rc = upload(off, &t.rxn_slot_off)) || (rc = upload(list, &t.rxn_slots)) ||
-        (rc = upload(row_off, &t.row_off)) || (rc = upload(row_list, &t.row_list)) ||
-        (rc = upload(col_off, &t.col_off)) || (rc = upload(col_list, &t.col_list)) ||
+    if ((rc = upload(ns_rows, &t.ns_rows)) || (rc = upload(ns_slots, &t.ns_slots)) ||
         (rc = upload(sp_slots, &t.sp_slots)) || (rc = upload(cj_slots, &t.cj_slots)) ||
-        (rc = upload(doff, &t.dchunk_off)) || (rc = upload(dlist, &t.dchunk_list)) ||
-        (!dslots.empty() && (rc = upload(dslots, &t.dchunk_slots))))
+        (left_out && ((rc = upload(col_off, &t.col_off)) || (rc = upload(col_list, &t.col_list)))))
         return rc;
-    t.bytes = (off.size() + list.size() + row_off.size() + col_off.size() + sp_slots.size() +
-               cj_slots.size() + doff.size() + dlist.size()) * sizeof(int) +
-              (row_list.size() + col_list.size()) * sizeof(int2) + dslots.size() * sizeof(int4);
     auto res = m->slots.emplace(key, t);
     *out = &res.first->second;
     return 0;
 }
 
-// per-state bytes of working arrays for one evaluation
-size_t state_bytes(const pjg_mech* m, int kind, bool c_order_jac, int nslot)
-{
-    size_t arrs = kind == PJG_SPECIES_RATES ? ARR_N_RATES : ARR_N_JAC;
-    size_t b = arrs * m->ns * sizeof(double);
-    if (kind == PJG_JACOBIAN && c_order_jac) b += (size_t)nslot * sizeof(double);
-    return b;
-}
-
 constexpr size_t kWorkBudget = size_t(8) << 30;  // bytes of working buffer per call
+constexpr int64_t kStateUnit = 128;              // chunks are multiples of it
 
 // States one launch can take with per_state bytes of working arrays: a whole
 // number of waves of resident blocks within the budget (a launch of a
@@ -309,17 +311,174 @@ int64_t chunk_states(size_t per_state, int64_t n, int64_t wave)
         if (cudaMemGetInfo(&free_b, &total_b) != cudaSuccess) free_b = 0;
         const int64_t fit = (int64_t)(free_b / 2 / per_state);
         c = std::max<int64_t>(c, std::min<int64_t>(fit, wave));
-        c = std::max<int64_t>(PJG_BLOCK, c / PJG_BLOCK * PJG_BLOCK);
+        c = std::max<int64_t>(kStateUnit, c / kStateUnit * kStateUnit);
     }
     return std::min<int64_t>(c, n);
 }
 
-// States of one full wave of the evaluation kernel of `kind` on the mechanism's device.
-int64_t wave_states(const pjg_mech* m, int kind)
+int sm_count(const pjg_mech* m)
 {
     int sms = 1;
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, m->device);
-    return (int64_t)sms * pjg_eval_blocks_per_sm(kind) * PJG_BLOCK;
+    return sms;
+}
+
+// States of one full wave of the thread-per-state kernel (a launch of a
+// fraction of a wave takes more than its share of a whole one).
+int64_t wave_states(const pjg_mech* m, int kind)
+{
+    return (int64_t)sm_count(m) * pjg_wave_blocks_per_sm(kind) * PJG_BLOCK;
+}
+
+constexpr int64_t kNoallocStates = 4096;
+constexpr int kListTerms = 8;  // entries of an unshared third-body list, at most
+
+// The tile shape for n states: the states of a tile and its warps.
+struct Shape {
+    int slog, warps, rounds, buf_terms;
+};
+
+// Shared memory of a block: two blocks of 8 warps per SM where the tile's
+// arrays leave room for a batch's terms in half of it, else the whole.
+constexpr size_t kHalfSmem = ((228u << 10) / 2 - 1024) & ~size_t(127);
+
+bool shape_fits(const pjg_mech* m, int kind, int slog, int warps, Shape* out)
+{
+    const int S = 1 << slog, wpw = 32 / S;
+    // terms of a full batch (10 per reaction is more than most leave), at
+    // least one reaction per warp and the sums kept in the buffers
+    const int per = kind == KIND_RATES ? 1 : kind == KIND_JAC ? PJG_MAXSP + kListTerms + 6 : PJG_MAXSP + kListTerms + 1;
+    const int rounds = kind == KIND_RATES ? 4 : 1;
+    // the buffers also hold the sums over species: 11 and 6 x 8 partial ones,
+    // and three per worker for J^T v
+    const int sums = (72 + (kind == KIND_VJP ? 96 * warps / S : 0) + 1) / 2;
+    const int want = std::max((kind == KIND_RATES ? 1 : 10) * rounds * warps * wpw + 1, sums);
+    const int least = std::max(per + 1, sums);
+    for (size_t limit : {kHalfSmem, (size_t)kTileSmemMax}) {
+        if (warps > 8 && limit != (size_t)kTileSmemMax) continue;
+        const size_t fixed = pjg_tile_smem(kind, m->ns, m->n_m, slog, warps, 0);
+        if (fixed >= limit) continue;
+        const int fit = (int)((limit - fixed) / (2 * S * sizeof(double)));
+        const bool half = limit == kHalfSmem;
+        if (fit < (half ? std::max(least, want / 2) : least)) continue;
+        *out = Shape{slog, warps, rounds, std::min(std::min(fit, want), 65000)};
+        return true;
+    }
+    return false;
+}
+
+int choose_shape(const pjg_mech* m, int kind, int64_t n, Shape* out)
+{
+    const int sms = sm_count(m);
+    bool any = false;
+    for (int slog = 5; slog >= 0; --slog) {
+        const int64_t tiles = (n + (1 << slog) - 1) >> slog;
+        Shape s;
+        if (!shape_fits(m, kind, slog, 8, &s)) continue;
+        *out = s;
+        any = true;
+        if (tiles >= 2 * sms) break;
+    }
+    if (!any) return fail(PJG_ERR_UNSUPPORTED, "mechanism too large for the evaluation kernels");
+    return 0;
+}
+
+int sched_tables(pjg_mech* m, int kind, int layout, const std::vector<int>* slot, const Shape& sh, SchedTables** out)
+{
+    const int key = ((kind * 4 + layout) * 8 + sh.slog) * 32 + sh.warps;
+    std::lock_guard<std::mutex> g(m->lock);
+    auto it = m->scheds.find(key);
+    if (it != m->scheds.end()) {
+        *out = &it->second;
+        return 0;
+    }
+    SchedHost h;
+    if (!sched_build(sched_input(m, kind, slot), sh.slog, sh.warps, sh.rounds, sh.buf_terms, h))
+        return fail(PJG_ERR_UNSUPPORTED, "a reaction's terms pass the evaluation kernel's buffer");
+    SchedTables t;
+    t.sc.slog = h.slog;
+    t.sc.warps = h.warps;
+    t.sc.rounds = h.rounds;
+    t.sc.n_batch = h.n_batch;
+    t.sc.buf_terms = h.buf_terms;
+    t.sc.n_vec = h.n_vec;
+    t.n_ns_post = (int)h.ns_post.size();
+    int rc;
+    Pack pk;
+    pk.add(h.tasks, &t.sc.tasks);
+    pk.add(h.term_off, &t.sc.term_off);
+    pk.add(h.item_off, &t.sc.item_off);
+    pk.add(h.items, &t.sc.items);
+    pk.add(h.post_off, &t.sc.post_off);
+    pk.add(h.post, &t.sc.post);
+    pk.add(h.ns_post, &t.ns_post);
+    if ((rc = pk.send(&t.buffer))) return rc;
+    *out = &m->scheds.emplace(key, t).first->second;
+    return 0;
+}
+
+int wave_tables(pjg_mech* m, int kind, int layout, const std::vector<int>* slot, WaveHold** out)
+{
+    const int key = kind * 4 + layout;
+    std::lock_guard<std::mutex> g(m->lock);
+    auto it = m->waves.find(key);
+    if (it != m->waves.end()) {
+        *out = &it->second;
+        return 0;
+    }
+    SchedHost h;
+    sched_build(sched_input(m, kind, slot), 5, 8, 1, 1 << 10, h);
+    WaveHold t;
+    t.n_vec = h.n_vec;
+    t.wt.n_post = (int)h.wave_post.size();
+    t.wt.n_zero = (int)h.wave_zero.size();
+    t.n_ns_post = (int)h.ns_post.size();
+    int rc;
+    Pack pk;
+    pk.add(h.wave_slot_off, &t.wt.slot_off);
+    pk.add(h.wave_slots, &t.wt.slots);
+    pk.add(h.wave_tb_off, &t.wt.tb_off);
+    pk.add(h.wave_tb, &t.wt.tb);
+    pk.add(h.wave_post, &t.wt.post);
+    pk.add(h.wave_zero, &t.wt.zero);
+    pk.add(h.ns_post, &t.ns_post);
+    if ((rc = pk.send(&t.buffer))) return rc;
+    *out = &m->waves.emplace(key, t).first->second;
+    return 0;
+}
+
+// Per-state bytes of the thread-per-state kernel's arrays.
+size_t wave_state_bytes(const pjg_mech* m, int kind, int n_vec)
+{
+    return ((size_t)tile_arrays(kind) * m->ns + n_vec) * sizeof(double);
+}
+
+// Whether a thread per state evaluates `rest` states, less than a wave, sooner
+// than tiles do.  A launch of part of a wave takes a fixed share of the wave's
+// time (0.55 for the Jacobian, 0.5 for J^T v, 0.35 for the rates) and the rest
+// in proportion, tiles take 1.09 to 1.6 times a wave's time in proportion (2.4
+// where the mechanism's tiles are smaller than 32 states).  Measured on GB300,
+// thread per state / tiles, ms: GRI-Mech 3.0 dense Jacobian F 20,000 states
+// 3.11 / 1.69, 60,000 4.28 / 4.14, 77,824 (a wave) 4.63 / 5.03; H2/O2 30,000
+// 0.301 / 0.279, 77,824 0.455 / 0.598; GRI rates 40,000 1.25 / 1.16, 80,000
+// 1.82 / 2.17; GRI J^T v 20,000 1.71 / 1.59, 30,000 1.78 / 2.23; 500 species,
+// sparse Jacobian, 16,384 59 / 46, rates 8,192 12.2 / 5.8, 32,768 16.4 / 22.3.
+bool wave_sooner(const pjg_mech* m, int kind, int64_t rest)
+{
+    Shape s;
+    bool fits = false;
+    for (int slog = 5; slog >= 0 && !fits; --slog) fits = shape_fits(m, kind, slog, 8, &s);
+    if (!fits) return true;  // no tile of this mechanism fits in shared memory
+    const double share = s.slog < 5 ? 0.25 : kind == PJG_JACOBIAN ? 0.75 : 0.45;
+    return rest >= (int64_t)(share * wave_states(m, kind));
+}
+
+// blocks of a launch over n states
+int grid_of(const pjg_mech* m, int kind, const Schedule& sc, int64_t n)
+{
+    const int64_t tiles = (n + (1 << sc.slog) - 1) >> sc.slog;
+    const int per_sm = pjg_tile_blocks_per_sm(kind, sc.warps, pjg_tile_smem(kind, m->ns, m->n_m, sc.slog, sc.warps, sc.buf_terms));
+    return (int)std::min<int64_t>(tiles, (int64_t)per_sm * sm_count(m));
 }
 
 int ensure_work(pjg_mech* m, size_t bytes)
@@ -356,20 +515,62 @@ void fill_common(const pjg_mech* m, EvalArgs& a)
     a.aux = m->aux;
     a.ns = m->ns;
     a.nr = m->nr;
-    a.nr_e22 = m->nr_e22;
-    for (int q = 0; q <= pjg::kMaPatterns; ++q) a.ma_off[q] = m->ma_off[q];
-    for (int q = 0; q <= pjg::kTpPatterns; ++q) a.tp_off[q] = m->tp_off[q];
+    a.m_lists = m->m_lists;
+    a.n_m = m->n_m;
+    for (int c = 0, i = 0; c < 16; ++c) {
+        while (i < m->nr && m->cls[i] < c) ++i;
+        a.cls_off[c] = i;
+    }
     a.need_logP = m->need_logP;
     a.jac_approx = m->jac_approx;
     a.kc_split_max = m->kc_split_max;
 }
 
-// Per-state bytes of working arrays one evaluation needs.  The Jacobian
-// accumulates in scratch for order 'C' (then transposed); an output of order
-// 'F' is its own accumulator.
-size_t eval_state_bytes(const pjg_mech* m, int kind, bool F, const SlotTables* t)
+// Per-state bytes of the Jacobian accumulator one evaluation needs: order 'C'
+// accumulates state-innermost and is then transposed; an output of order 'F'
+// is its own accumulator.
+size_t eval_state_bytes(int kind, bool F, const SlotTables* t)
 {
-    return state_bytes(m, kind, kind == PJG_JACOBIAN && !F, t ? t->nslot : 0);
+    return kind == PJG_JACOBIAN && !F ? (size_t)t->nslot * sizeof(double) : 0;
+}
+
+// How n states are evaluated: whole waves go to the thread-per-state kernel,
+// what is left to the sooner one, in launches of ch_wave and ch_tile states
+// (most_states at most, or by the budget of the shared working buffer).
+struct Plan {
+    int64_t n_wave = 0, ch_wave = 0, ch_tile = 0;
+    WaveHold* wh = nullptr;
+    SchedTables* sd = nullptr;
+    int grid = 0;
+    size_t need = 0;  // bytes of working buffer
+};
+
+int make_plan(pjg_mech* m, int kind, bool F, bool sparse, const SlotTables* t, int64_t n, int64_t most_states, Plan* p)
+{
+    const size_t per_state = eval_state_bytes(kind, F, t);
+    const int layout = kind == PJG_JACOBIAN ? (F ? 2 : 0) + (sparse ? 1 : 0) : 0;
+    const std::vector<int>* slot = t ? &t->slot : nullptr;
+    const int64_t W = wave_states(m, kind);
+    p->n_wave = wave_sooner(m, kind, n % W) ? n : n / W * W;
+    if (p->n_wave > 0) {
+        if (int rc = wave_tables(m, kind, layout, slot, &p->wh)) return rc;
+        const size_t each = per_state + wave_state_bytes(m, kind, p->wh->n_vec);
+        p->ch_wave = std::min<int64_t>(most_states ? most_states : chunk_states(each, p->n_wave, W), p->n_wave);
+        p->need = each * (size_t)p->ch_wave;
+    }
+    if (p->n_wave < n) {
+        // the accumulator's states, then the blocks' scratch slices
+        p->ch_tile = n - p->n_wave;
+        if (per_state)
+            p->ch_tile = std::min<int64_t>(most_states ? most_states : chunk_states(per_state, p->ch_tile, W), p->ch_tile);
+        Shape sh;
+        if (int rc = choose_shape(m, kind, p->ch_tile, &sh)) return rc;
+        if (int rc = sched_tables(m, kind, layout, slot, sh, &p->sd)) return rc;
+        p->grid = grid_of(m, kind, p->sd->sc, p->ch_tile);
+        p->need = std::max(p->need, per_state * (size_t)p->ch_tile +
+                                        (size_t)p->grid * p->sd->sc.n_vec * sizeof(double) * ((size_t)1 << p->sd->sc.slog));
+    }
+    return 0;
 }
 
 // Evaluate n states.  The per-state working arrays go to ext_work (ext_bytes)
@@ -380,7 +581,7 @@ size_t eval_state_bytes(const pjg_mech* m, int kind, bool F, const SlotTables* t
 int run_eval(pjg_mech* m, int kind, int64_t n, char order, int conp, int jac_format,
              const double* param, const double* phi, double* out, cudaStream_t st,
              const double* v = nullptr, double* ext_work = nullptr, size_t ext_bytes = 0,
-             double* dphi = nullptr)
+             int64_t ext_states = 0, double* dphi = nullptr)
 {
     if (!m) return fail(PJG_ERR_ARG, "null mechanism");
     if (n < 0) return fail(PJG_ERR_ARG, "negative problem size");
@@ -398,23 +599,24 @@ int run_eval(pjg_mech* m, int kind, int64_t n, char order, int conp, int jac_for
         int rc = build_slots(m, F, jac_format == PJG_JAC_SPARSE, &t);
         if (rc) return rc;
     }
-    const size_t per_state = eval_state_bytes(m, kind, F, t);
-    int64_t ch;
+    const size_t per_state = eval_state_bytes(kind, F, t);
+    Plan pl;
+    if (int rc = make_plan(m, kind, F, jac_format == PJG_JAC_SPARSE, t, n, ext_work ? ext_states : 0, &pl)) return rc;
+    const size_t need = pl.need;
+    const int64_t n_wave = pl.n_wave;
+    WaveHold* wh = pl.wh;
+    SchedTables* sd = pl.sd;
     double* work = ext_work;
     if (ext_work) {
-        ch = per_state ? (int64_t)(ext_bytes / per_state) / PJG_BLOCK * PJG_BLOCK : n;
-        if (ch < PJG_BLOCK && ch < n) return fail(PJG_ERR_ARG, "working buffer too small");
-        ch = std::min<int64_t>(std::max<int64_t>(ch, 1), n);
+        if (need > ext_bytes) return fail(PJG_ERR_ARG, "working buffer too small");
     } else {
-        ch = chunk_states(per_state, n, wave_states(m, kind));
-        if (per_state) {
-            int rc = ensure_work(m, per_state * (size_t)ch);
-            if (rc) return rc;
-        }
+        if (int rc = ensure_work(m, need)) return rc;
         work = m->work;
     }
-    for (int64_t off = 0; off < n; off += ch) {
-        const int64_t cnt = std::min<int64_t>(ch, n - off);
+    for (int64_t off = 0, cnt = 0; off < n; off += cnt) {
+        const bool wave = off < n_wave;
+        const int64_t ch = wave ? pl.ch_wave : pl.ch_tile;
+        cnt = std::min<int64_t>(ch, (wave ? n_wave : n) - off);
         EvalArgs a;
         fill_common(m, a);
         a.n = cnt;
@@ -429,7 +631,17 @@ int run_eval(pjg_mech* m, int kind, int64_t n, char order, int conp, int jac_for
             a.phi_ss = NN;
             a.phi_sj = 1;
         }
-        a.scratch = work;
+        if (wave) {
+            a.wt = wh->wt;
+            a.sc.n_vec = wh->n_vec;
+            a.ns_post = wh->ns_post;
+            a.n_ns_post = wh->n_ns_post;
+        } else {
+            a.sc = sd->sc;
+            a.ns_post = sd->ns_post;
+            a.n_ns_post = sd->n_ns_post;
+        }
+        a.scratch = work + per_state / sizeof(double) * (size_t)ch;
         a.sc_ld = ch;
         if (kind == PJG_SPECIES_RATES) {
             a.dphi = F ? out + off : out + off * NN;
@@ -444,40 +656,27 @@ int run_eval(pjg_mech* m, int kind, int64_t n, char order, int conp, int jac_for
                 a.dphi_ss = a.phi_ss;
                 a.dphi_sj = a.phi_sj;
             }
-            a.nslot = t->nslot;
             if (F) {
                 a.acc = out + off;
                 a.acc_ld = n;
             } else {
-                a.acc = work + (size_t)ARR_N_JAC * m->ns * ch;
+                a.acc = work;
                 a.acc_ld = ch;
             }
-            a.rxn_slot_off = t->rxn_slot_off;
-            a.rxn_slots = t->rxn_slots;
-            a.row_off = t->row_off;
-            a.row_list = t->row_list;
+            a.acc_ss = 1;
+            a.ns_rows = t->ns_rows;
+            a.ns_slots = t->ns_slots;
+            a.n_ns = t->n_ns;
             a.col_off = t->col_off;
             a.col_list = t->col_list;
             a.sp_slots = t->sp_slots;
             a.cj_slots = t->cj_slots;
-            a.dchunk_off = t->dchunk_off;
-            a.dchunk_list = t->dchunk_list;
-            a.dchunk_slots = t->dchunk_slots;
             a.s00 = t->s00;
             a.s01 = t->s01;
             a.s10 = t->s10;
             a.s11 = t->s11;
-            if (jac_format != PJG_JAC_SPARSE) {
-                a.dense_rs = F ? 1 : NN;
-                a.dense_cs = F ? NN : 1;
-            }
         }
         int rc = 0;
-        if (kind == PJG_JACOBIAN) {
-            rc = pjg_launch_zero(a.acc, a.acc_ld, cnt, a.nslot, st);
-            if (rc) return fail(PJG_ERR_CUDA, "zero launch failed");
-            g_launches.fetch_add(1);
-        }
         cudaEvent_t e0 = nullptr, e1 = nullptr;
         const bool prof = g_prof_on.load();
         if (prof) {
@@ -485,7 +684,8 @@ int run_eval(pjg_mech* m, int kind, int64_t n, char order, int conp, int jac_for
             cudaEventCreate(&e1);
             cudaEventRecord(e0, st);
         }
-        rc = pjg_launch_eval(a, kind, st);
+        rc = wave ? pjg_launch_wave(a, kind, st)
+                  : pjg_launch_tile(a, kind, (int)std::min<int64_t>(pl.grid, (cnt + (1 << sd->sc.slog) - 1) >> sd->sc.slog), st);
         if (rc) return fail(PJG_ERR_CUDA, "kernel launch failed: %s", pjg_launch_error_string());
         g_launches.fetch_add(1);
         if (prof) {
@@ -753,9 +953,9 @@ void order_reactions(pjg_mech* m)
     Packing pk;
     pack_reactions(m->h_rxn, m->h_thd_spec.data(), m->h_thd_coef.data(), pk);
     m->h_rxn.swap(pk.rx);
-    m->nr_e22 = pk.nr_e22;
-    for (int q = 0; q <= pjg::kMaPatterns; ++q) m->ma_off[q] = pk.ma_off[q];
-    for (int q = 0; q <= pjg::kTpPatterns; ++q) m->tp_off[q] = pk.tp_off[q];
+    m->cls.assign(pk.cls.begin(), pk.cls.end());
+    for (int& c : m->cls)
+        if (c < 0) c = 1 + pjg::kMaPatterns + pjg::kTpPatterns;  // the general code
     // bound on a state's |b_k| under which 1 / Kc is formed from per-species
     // factors: 690 / (largest sum |nu| of a reversible reaction), at most
     // 690 / 5 (every coefficient pattern has sum |nu| <= 5)
@@ -772,11 +972,105 @@ void order_reactions(pjg_mech* m)
     m->kc_split_max = 690.0 / numax;
 }
 
+// The device's reaction records: the packed ones with the row-E weight
+// sum nu_k (1 - W_k / W_ns) (sum nu where mass is conserved, so zero for most
+// reactions: their rounding is dropped) and the number of the [M] list where
+// several reactions share it (its reactions then read [M] from the tile).
+void device_records(pjg_mech* m, const double* species, std::vector<int4>& m_lists)
+{
+    std::map<std::pair<int, double>, int> uses, number;
+    auto key = [](const PjgRxn& R) { return std::make_pair(R.thd_off * 2 + (R.thd_cnt > 0), R.p[P_FLAG]); };
+    for (const PjgRxn& R : m->h_rxn)
+        if (RX_THD(R.flags) != THD_NONE) ++uses[key(R)];
+    // x 2^B / ln 2 as an integer and a rest
+    auto cut = [](long double x, int* n, double* rest) {
+        x = x * 1.4426950408889634073599246810018921L * PJG_EXP_TAB;
+        const long double r = nearbyintl(x);
+        *n = (int)r;
+        *rest = (double)(x - r);
+    };
+    m->d_rxn.clear();
+    for (size_t i = 0; i < m->h_rxn.size(); ++i) {
+        const PjgRxn& H = m->h_rxn[i];
+        RxnRec R{};
+        R.flags = H.flags;
+        R.nspec = H.nspec;
+        R.thd_off = H.thd_off;
+        R.thd_cnt = H.thd_cnt;
+        R.aux = H.aux;
+        R.bint = H.bint;
+        R.fbint = H.fbint;
+        std::copy(H.ent, H.ent + PJG_MAXSP, R.ent);
+        std::copy(H.p, H.p + P_WE, R.p);
+        double w = 0.0, scale = 0.0;
+        int nu_sum = 0;
+        for (int e = 0; e < R.nspec; ++e) {
+            const int nu = ent_nur(R.ent[e]) - ent_nuf(R.ent[e]);
+            nu_sum += nu;
+            if (ent_spec(R.ent[e]) == m->ns - 1) continue;
+            const double om = species[(size_t)ent_spec(R.ent[e]) * PJG_SP_DOUBLES + SP_OMW];
+            w += nu * om;
+            scale += std::abs(nu) * (1.0 + std::abs(om));
+        }
+        R.p[P_WE] = std::abs(w - nu_sum) <= 1e-12 * scale ? (double)nu_sum : w;
+        R.flags &= ~(RX_WE | RX_WEREAL | RX_E22 | RX_RATIO);
+        if (R.p[P_WE] != 0.0) R.flags |= RX_WE;
+        if (R.p[P_WE] != (double)nu_sum) R.flags |= RX_WE | RX_WEREAL;
+        if (m->cls[i] == 0) R.flags |= RX_E22;
+        const int blend = RX_BLEND(R.flags);
+        if (RX_FORM(R.flags) == FORM_ARR) cut(H.p[P_A], &R.bint, &R.p[P_A]);
+        if (blend != BL_NONE && RX_FORM(R.flags) == FORM_ARR && RX_FFORM(R.flags) == FORM_ARR) {
+            const int sg = R.flags & RX_CHEM ? -1 : 1;  // the other rate is k0 in a fall-off
+            cut(sg * ((long double)H.p[P_FA] - H.p[P_A]), &R.fbint, &R.p[P_RA]);
+            R.p[P_RB] = sg * (H.p[P_FB] - H.p[P_B]);
+            R.p[P_RTA] = sg * (H.p[P_FTA] - H.p[P_TA]);
+            R.p[P_RN] = R.fbint;
+            R.flags |= RX_RATIO;
+        } else if (blend != BL_NONE && RX_FFORM(R.flags) == FORM_ARR) {
+            cut(H.p[P_FA], &R.fbint, &R.p[P_FA]);
+        }
+        R.list = -1;
+        // (a long list too: its terms would not fit a tile's buffer)
+        if (RX_THD(R.flags) != THD_NONE && R.thd_cnt > 0 && (uses[key(H)] >= 2 || R.thd_cnt > kListTerms)) {
+            auto it = number.find(key(H));
+            if (it == number.end()) {
+                it = number.emplace(key(H), (int)m_lists.size()).first;
+                m_lists.push_back(make_int4(R.thd_off, R.thd_cnt, R.p[P_FLAG] != 0.0, 0));
+            }
+            R.list = it->second;
+            if ((blend == BL_TROE || blend == BL_SRI) && (R.flags & RX_RATIO)) m_lists[R.list].w = 1;
+        }
+        m->d_rxn.push_back(R);
+    }
+    m->n_m = (int)m_lists.size();
+    // one kind of row-E weight per mechanism (a target's additions are of one kind)
+    bool real = false;
+    for (const RxnRec& R : m->d_rxn) real = real || (R.flags & RX_WEREAL);
+    for (RxnRec& R : m->d_rxn)
+        if (real && (R.flags & RX_WE)) R.flags |= RX_WEREAL;
+}
+
 }  // namespace
 
 // Internal accessors for other translation units of this library.
 int pjg_internal_fail(int code, const char* msg) { return fail(code, "%s", msg); }
-void pjg_internal_fill_args(const pjg_mech* m, EvalArgs* a) { fill_common(m, *a); }
+// The J^T v launch of n states with scratch_doubles of scratch, in tiles of the
+// shape for kNoallocStates states, whose schedule pjg_mech_create has made: the argument
+// block's mechanism and schedule, and the grid.
+int pjg_internal_vjp_args(pjg_mech* m, int64_t n, size_t scratch_doubles, EvalArgs* a, int* grid)
+{
+    Shape sh;
+    SchedTables* sd = nullptr;
+    if (int rc = choose_shape(m, PJG_KIND_VJP, kNoallocStates, &sh)) return rc;
+    if (int rc = sched_tables(m, PJG_KIND_VJP, 0, nullptr, sh, &sd)) return rc;
+    fill_common(m, *a);
+    a->sc = sd->sc;
+    a->ns_post = sd->ns_post;
+    a->n_ns_post = sd->n_ns_post;
+    const size_t slice = (size_t)sd->sc.n_vec << sd->sc.slog;
+    *grid = (int)std::min<size_t>(grid_of(m, PJG_KIND_VJP, sd->sc, n), scratch_doubles / slice);
+    return *grid > 0 ? 0 : fail(PJG_ERR_ARG, "scratch too small for one tile");
+}
 int pjg_internal_mech_ns(const pjg_mech* m) { return m->ns; }
 int pjg_internal_check_device(const pjg_mech* m) { return check_device(m); }
 void pjg_internal_count_launch() { g_launches.fetch_add(1); }
@@ -1020,15 +1314,24 @@ int pjg_mech_create(const pjg_tables* tb, pjg_mech** out)
         delete m;
         return fail(PJG_ERR_TABLES, "pattern pointers inconsistent with nnz");
     }
-    std::vector<PjgRxn> rx(m->h_rxn);
+    std::vector<int4> m_lists;
+    device_records(m, tb->species, m_lists);
     std::vector<double> sp(tb->species, tb->species + (size_t)tb->ns * PJG_SP_DOUBLES);
     std::vector<double> coef(tb->thd_coef, tb->thd_coef + std::max(tb->n_thd, 0));
     std::vector<double> aux(tb->aux ? tb->aux : (const double*)nullptr,
                             tb->aux ? tb->aux + std::max(tb->n_aux, 0) : (const double*)nullptr);
     int rc;
-    if ((rc = upload(rx, &m->rxn)) || (rc = upload(sp, &m->sp)) ||
+    if ((rc = upload(m->d_rxn, &m->rxn)) || (rc = upload(m_lists, &m->m_lists)) || (rc = upload(sp, &m->sp)) ||
         (rc = upload(m->h_thd_spec, &m->thd_spec)) || (rc = upload(coef, &m->thd_coef)) ||
         (rc = upload(aux, &m->aux))) {
+        pjg_mech_destroy(m);
+        return rc;
+    }
+    // pjg_vjp_noalloc may not allocate: its schedule now
+    Shape sh;
+    SchedTables* sd = nullptr;
+    if (!choose_shape(m, PJG_KIND_VJP, kNoallocStates, &sh) &&
+        (rc = sched_tables(m, PJG_KIND_VJP, 0, nullptr, sh, &sd))) {
         pjg_mech_destroy(m);
         return rc;
     }
@@ -1048,18 +1351,16 @@ int pjg_mech_destroy(pjg_mech* m)
     pjg_internal_lu_plan_destroy(m->lu_plan);
     for (auto& kv : m->slots) {
         SlotTables& t = kv.second;
-        cudaFree(t.rxn_slot_off);
-        cudaFree(t.rxn_slots);
-        cudaFree(t.row_off);
-        cudaFree(t.row_list);
+        cudaFree(t.ns_rows);
+        cudaFree(t.ns_slots);
         cudaFree(t.col_off);
         cudaFree(t.col_list);
         cudaFree(t.sp_slots);
         cudaFree(t.cj_slots);
-        cudaFree(t.dchunk_off);
-        cudaFree(t.dchunk_list);
-        cudaFree(t.dchunk_slots);
     }
+    for (auto& kv : m->scheds) cudaFree(kv.second.buffer);
+    for (auto& kv : m->waves) cudaFree(kv.second.buffer);
+    cudaFree(m->m_lists);
     delete m;
     return 0;
 }
@@ -1125,7 +1426,7 @@ int pjg_jacobian_rates(pjg_mech* m, int64_t n, char order, int conp, int jac_for
 {
     if (n > 0 && !dphi) return fail(PJG_ERR_ARG, "null array");
     return run_eval(m, PJG_JACOBIAN, n, order, conp, jac_format, param, phi, jac, (cudaStream_t)stream,
-                    nullptr, nullptr, 0, dphi);
+                    nullptr, nullptr, 0, 0, dphi);
 }
 
 int pjg_eval_chunk(pjg_mech* m, int kind, int64_t n, char order, int jac_format, int64_t* states)
@@ -1141,7 +1442,13 @@ int pjg_eval_chunk(pjg_mech* m, int kind, int64_t n, char order, int jac_format,
         int rc = build_slots(m, order == 'F', jac_format == PJG_JAC_SPARSE, &t);
         if (rc) return rc;
     }
-    *states = chunk_states(eval_state_bytes(m, kind, order == 'F', t), n, wave_states(m, kind));
+    const int layout = kind == PJG_JACOBIAN ? (order == 'F' ? 2 : 0) + (jac_format == PJG_JAC_SPARSE ? 1 : 0) : 0;
+    WaveHold* wh = nullptr;
+    if (int rc = wave_tables(m, kind, layout, t ? &t->slot : nullptr, &wh)) return rc;
+    const size_t per_state = eval_state_bytes(kind, order == 'F', t);
+    const int64_t W = wave_states(m, kind), n_wave = wave_sooner(m, kind, n % W) ? n : n / W * W;
+    *states = n_wave ? chunk_states(per_state + wave_state_bytes(m, kind, wh->n_vec), n_wave, W)
+                     : chunk_states(per_state, n, W);
     return 0;
 }
 
@@ -1236,7 +1543,7 @@ int pjg_ros2_step(pjg_mech* m, int64_t n, char order, int conp, const double* pa
     double* k2 = vec_work + (size_t)n * nn;
     // f(y) comes out of the Jacobian's pass
     int rc = run_eval(m, PJG_JACOBIAN, n, order, conp, PJG_JAC_FULL, param, phi, jac_work, st, nullptr,
-                      nullptr, 0, k1);
+                      nullptr, 0, 0, k1);
     if (!rc) rc = factor();
     if (!rc) rc = solve(k1);
     if (!rc) rc = pjg_internal_ros2_combine(0, nn, n, order, h, h0, phi, k1, nullptr, phi_new, nullptr, st);
@@ -1312,14 +1619,16 @@ int pjg_kernel_resize(pjg_kernel* k, size_t problem_size, size_t work_size)
         if (rc) return rc;
     }
     const size_t nn = m->nn;
-    const size_t per_state = eval_state_bytes(m, k->kind, k->order == 'F', t);
+    const size_t per_state = eval_state_bytes(k->kind, k->order == 'F', t);
     // two waves per chunk; where the ring and working arrays of two waves
     // would pass the kernel object's budget (large mechanisms), as many whole
     // waves as the budget holds, and at least one wave if half the free
     // device memory holds it: a launch of part of a wave takes as long as a
     // whole one (synthetic 500-species sparse C-order Jacobian, 1.37 MB per
     // state: a third-of-a-wave chunk ran end to end at 48 % of the copy floor)
-    const size_t ring_state = kRing * (1 + nn + k->out_per_state) * sizeof(double) + per_state;
+    // (the evaluation's arrays a little above their size, which the tables give)
+    const size_t arrays = (size_t)(tile_arrays(k->kind) + vec_arrays(k->kind) + 2) * m->ns * sizeof(double);
+    const size_t ring_state = kRing * (1 + nn + k->out_per_state) * sizeof(double) + per_state + arrays;
     const int64_t wave = wave_states(m, PJG_JACOBIAN);
     int64_t chunk = std::min<int64_t>((int64_t)problem_size, PJG_CHUNK_WAVES * wave);
     if ((size_t)chunk * ring_state > kKernelBudget) {
@@ -1332,23 +1641,36 @@ int pjg_kernel_resize(pjg_kernel* k, size_t problem_size, size_t work_size)
             c = std::max<int64_t>(c, std::min<int64_t>((int64_t)(free_b / 2 / ring_state), wave));
         }
         chunk = std::min<int64_t>((int64_t)problem_size,
-                                  std::max<int64_t>(PJG_BLOCK, c / PJG_BLOCK * PJG_BLOCK));
+                                  std::max<int64_t>(kStateUnit, c / kStateUnit * kStateUnit));
     }
-    if (chunk == k->chunk && k->d_phi[0]) {
+    if (problem_size == 0) {
+        free_buffers(k);
+        k->problem_size = 0;
+        return 0;
+    }
+    // working buffer of a full chunk and of the last one (which makes the tables
+    // of their launches, too)
+    size_t work_bytes = 8;
+    for (int64_t cnt : {chunk, (int64_t)(problem_size % (size_t)chunk)}) {
+        if (cnt == 0) continue;
+        Plan pl;
+        if (int rc = make_plan(m, k->kind, k->order == 'F', k->jac_format == PJG_JAC_SPARSE, t, cnt, chunk, &pl))
+            return rc;
+        work_bytes = std::max(work_bytes, pl.need);
+    }
+    if (chunk == k->chunk && k->d_phi[0] && work_bytes <= k->work_bytes) {
         k->problem_size = problem_size;
         return 0;
     }
     free_buffers(k);
     k->problem_size = problem_size;
-    if (problem_size == 0) return 0;
     for (int b = 0; b < kRing; ++b) {
         CUDA_TRY(cudaMalloc((void**)&k->d_param[b], chunk * sizeof(double)));
         CUDA_TRY(cudaMalloc((void**)&k->d_phi[b], chunk * nn * sizeof(double)));
         CUDA_TRY(cudaMalloc((void**)&k->d_out[b], chunk * k->out_per_state * sizeof(double)));
     }
-    const int64_t padded = (chunk + PJG_BLOCK - 1) / PJG_BLOCK * PJG_BLOCK;
-    k->work_bytes = per_state * (size_t)padded;
-    if (k->work_bytes) CUDA_TRY(cudaMalloc((void**)&k->work, k->work_bytes));
+    k->work_bytes = work_bytes;
+    CUDA_TRY(cudaMalloc((void**)&k->work, k->work_bytes));
     k->chunk = chunk;
     return 0;
 }
@@ -1381,7 +1703,7 @@ int kernel_stream(pjg_kernel* k, const double* param, const double* phi, double*
         CUDA_TRY(cudaStreamWaitEvent(k->s_comp, k->ev_in[b], 0));
         if (c >= kRing) CUDA_TRY(cudaStreamWaitEvent(k->s_comp, k->ev_out[b], 0));
         int rc = run_eval(k->mech, k->kind, cnt, k->order, k->conp, k->jac_format, k->d_param[b],
-                          k->d_phi[b], k->d_out[b], k->s_comp, nullptr, k->work, k->work_bytes);
+                          k->d_phi[b], k->d_out[b], k->s_comp, nullptr, k->work, k->work_bytes, k->chunk);
         if (rc) return rc;
         CUDA_TRY(cudaEventRecord(k->ev_k[b], k->s_comp));
         CUDA_TRY(cudaStreamWaitEvent(k->s_out, k->ev_k[b], 0));

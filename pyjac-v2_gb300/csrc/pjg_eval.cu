@@ -34,13 +34,25 @@
 // records, Troe's Fcent^(1/(1+(A/B)^2)) is exp(X ln Fcent) with ln Fcent shared
 // with log10 Fcent, fall-off derivative factors are formed once per reaction,
 // stoichiometric multiplications by +-1/+-2 are adds, and d(rop)/dc products
-// skip zero exponents instead of dividing.
+// skip zero exponents instead of dividing.  Rows T and E of the Jacobian are
+// summed per reaction (d R_i / d c_j times the reaction's enthalpy, and times
+// sum nu) instead of over the species block, which is not read back; the
+// exponentials take their integer part on the integer pipe (fexp_s).  FP64
+// instructions per GRI state, ncu: Jacobian 27,817 -> 21,700, rates 11,255 ->
+// 9,830; 1M states dense F 68.5 -> 61.8 ms, rates 21.9 -> 19.0 ms.  What bounds
+// it now: loads of the per-state arrays (L1 hit rate 22 %, half of the warps'
+// stalls; DRAM moves 5.5x the output), at 56 % FP64 pipe for the Jacobian and
+// 74 % for the rates.
 #include <cuda_runtime.h>
+
 #include "pjg_eval.cuh"
 #include "pjg_math.cuh"
 #include "pjg_rxn.cuh"
 
 using namespace pjg;
+
+thread_local cudaError_t pjg_launch_err = cudaSuccess;
+const char* pjg_launch_error_string() { return cudaGetErrorString(pjg_launch_err); }
 
 namespace {
 
@@ -51,6 +63,8 @@ struct SV {
     __device__ __forceinline__ double& operator[](int k) const { return b[(int64_t)k * st]; }
 };
 
+// Registers against warps, 1M GRI states dense F: 3 blocks per SM 75.4 ms, 4
+// 63.0, 5 65.2.
 #ifndef PJG_VJP_MINB
 #define PJG_VJP_MINB 3  // resident 128-thread blocks per SM requested for the J^T v kernel
 #endif
@@ -59,190 +73,79 @@ struct SV {
 #define PJG_JAC_MINB 4  // resident 128-thread blocks per SM requested for the Jacobian kernel
 #endif
 
-// Species-rate kernel: 6 blocks per SM fit its 80 registers without spills.
-// Measured on 1M GRI states (F): 4 blocks 22.35 ms, 5: 22.34, 6: 21.86, 8:
-// 21.75 (64 registers, with spills); the Jacobian at 5 blocks 68.7 against
-// 68.2 ms at 4, J^T v at 4 blocks 13.8 against 13.6 ms at 3.
 #ifndef PJG_RATES_MINB
 #define PJG_RATES_MINB 6  // resident 128-thread blocks per SM requested for the species-rate kernel
 #endif
 
-// Rows T and E of the output and the bath-gas terms of its species block
-// (the assembly step of eval_kernel<1>), out of line so that its registers do
-// not shape the reaction loops' allocation.  One pass over the species block
-// in chunks of kCols columns whose row-T and row-E sums stay in registers,
-// visiting only the rows with a structurally nonzero entry in the chunk
-// (dchunk_list; GRI: 1,774 of 2,704 entries).  A row's entries are loaded
-// together, have the row's bath-gas sum subtracted (stored back only then)
-// and are summed into their columns' sums in increasing row order.  Slots:
-// (2 + k) rs + (2 + j) cs for a dense output, dchunk_slots (one quadruple per
-// listed row) and cj_slots for a sparse one.  Software-pipelined: the next
-// listed row's entries and weights are loaded before this row's are summed.
-// Measured on 1M GRI states (dense F): chunks of 4 columns 92.1 ms, 6: 92.8,
-// 8: 93.3, 10: 96.1, 16: 101.1 (register pressure), against 96.3 ms for two
-// passes (subtract, then sum); loads and stores interleaved entry by entry
-// serialised on possible aliasing (100.4 ms).  Later, with the row lists
-// 70.3 ms against every entry visited, pipelined 68.35 against 69.11 ms, out
-// of line 68.3 against 68.4 ms inlined.
-__device__ __noinline__ void rows_te(bool sparse, double* acc, int64_t ld, int rs, int cs,
-                                     const int* dchunk_off, const int* dchunk_list,
-                                     const int4* dchunk_slots, const int* cj_slots,
-                                     const double* sp, SV nsrow, SV hw, SV cpa, int last,
-                                     double cp_ns, double Tdot, double inv_vcp, double TRf,
-                                     double eTj)
-{
-    constexpr int kCols = PJG_DENSE_COLS;
-    static_assert(kCols == 4, "one int4 of slots per listed row");
-    for (int c = 0, j0 = 0; j0 < last; ++c, j0 += kCols) {
-        double sT[kCols], sE[kCols];
-#pragma unroll
-        for (int q = 0; q < kCols; ++q) {
-            sT[q] = 0.0;
-            sE[q] = 0.0;
-        }
-        auto fetch = [&](int t, int e, double (&J)[kCols], int (&sl)[kCols], double& v_,
-                         double& hw_, double& om_) {
-            const int k = e >> 4, mask = e & 15;
-            if (sparse) {
-                const int4 q4 = __ldg(dchunk_slots + t);
-                sl[0] = q4.x;
-                sl[1] = q4.y;
-                sl[2] = q4.z;
-                sl[3] = q4.w;
-            } else {
-#pragma unroll
-                for (int q = 0; q < kCols; ++q) sl[q] = (2 + k) * rs + (2 + j0 + q) * cs;
-            }
-#pragma unroll
-            for (int q = 0; q < kCols; ++q)
-                J[q] = (mask >> q & 1) ? __ldcg(acc + (int64_t)sl[q] * ld) : 0.0;
-            v_ = __ldcg(&nsrow[k]);
-            hw_ = hw[k];
-            om_ = ldg(sp + (int64_t)k * PJG_SP_DOUBLES + SP_OMW);
-        };
-        int t = __ldg(dchunk_off + c);
-        const int t1 = __ldg(dchunk_off + c + 1);
-        int en = 0;
-        int sln[kCols] = {0, 0, 0, 0};
-        double Jn[kCols], vn = 0.0, hwn = 0.0, omn = 0.0;
-        if (t < t1) {
-            en = __ldg(dchunk_list + t);  // the same for every thread
-            fetch(t, en, Jn, sln, vn, hwn, omn);
-        }
-        for (; t < t1; ++t) {
-            const int mask = en & 15;
-            double Jv[kCols];
-            int sl[kCols];
-#pragma unroll
-            for (int q = 0; q < kCols; ++q) {
-                Jv[q] = Jn[q];
-                sl[q] = sln[q];
-            }
-            const double v = vn, hwk = hwn, omk = omn;
-            if (t + 1 < t1) {
-                en = __ldg(dchunk_list + t + 1);
-                fetch(t + 1, en, Jn, sln, vn, hwn, omn);
-            }
-            if (mask == (1 << kCols) - 1) {
-                if (nonzero(v)) {
-#pragma unroll
-                    for (int q = 0; q < kCols; ++q) {
-                        Jv[q] = Jv[q] - v;
-                        acc[(int64_t)sl[q] * ld] = Jv[q];
-                    }
-                }
-#pragma unroll
-                for (int q = 0; q < kCols; ++q) {
-                    sT[q] = fma(hwk, Jv[q], sT[q]);
-                    sE[q] = fma(omk, Jv[q], sE[q]);
-                }
-            } else {
-                if (nonzero(v)) {
-#pragma unroll
-                    for (int q = 0; q < kCols; ++q) {
-                        if (mask >> q & 1) {
-                            Jv[q] = Jv[q] - v;
-                            acc[(int64_t)sl[q] * ld] = Jv[q];
-                        }
-                    }
-                }
-#pragma unroll
-                for (int q = 0; q < kCols; ++q) {
-                    if (mask >> q & 1) {
-                        sT[q] = fma(hwk, Jv[q], sT[q]);
-                        sE[q] = fma(omk, Jv[q], sE[q]);
-                    }
-                }
-            }
-        }
-#pragma unroll
-        for (int q = 0; q < kCols; ++q) {
-            const int j = j0 + q;
-            if (j < last) {
-                const int s0 = sparse ? __ldg(cj_slots + 2 * j) : (2 + j) * cs;
-                const int s1 = sparse ? __ldg(cj_slots + 2 * j + 1) : rs + (2 + j) * cs;
-                const double J0 = -1.0 * (sT[q] + Tdot * (cpa[j] + -1.0 * cp_ns)) * inv_vcp;
-                acc[(int64_t)s0 * ld] = J0;
-                acc[(int64_t)s1 * ld] = TRf * sE[q] + eTj * J0;
-            }
-        }
-    }
-}
+constexpr int kPostUnroll = 8;
 
-template <int KIND>  // 0 species rates, 1 Jacobian, 2 J^T v
-__global__ void __launch_bounds__(PJG_BLOCK, KIND == 1 ? PJG_JAC_MINB : (KIND == 2 ? PJG_VJP_MINB : PJG_RATES_MINB))
-    eval_kernel(const EvalArgs a)
+// stoichiometry of the elementary class A + B <=> C + D
+struct E22Stoich {
+    __device__ static constexpr int nsp(const RxnHead&) { return 4; }
+    __device__ static constexpr int nuf(const RxnHead&, int e) { return e < 2; }
+    __device__ static constexpr int nur(const RxnHead&, int e) { return e >= 2; }
+};
+
+// One thread per state; the per-state arrays and accumulators live in global
+// scratch (state-innermost, so a warp's accesses are coalesced).
+template <int KIND>  // KIND_RATES, KIND_JAC, KIND_VJP
+__global__ void __launch_bounds__(PJG_BLOCK, KIND == KIND_JAC ? PJG_JAC_MINB : (KIND == KIND_VJP ? PJG_VJP_MINB : PJG_RATES_MINB))
+    wave_kernel(const EvalArgs a)
 {
     __shared__ double etab[PJG_EXP_TAB];
     fill_exp_table(etab);
     __syncthreads();
     const int64_t s = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (s >= a.n) return;  // no block-wide synchronisation below
-    constexpr bool JAC = KIND == 1;
-    constexpr bool VJP = KIND == 2;
-    constexpr bool DER = KIND >= 1;  // derivative terms needed
+    constexpr bool JAC = KIND == KIND_JAC;
+    constexpr bool VJP = KIND == KIND_VJP;
+    constexpr bool DER = JAC || VJP;  // derivative terms needed
+    constexpr int kArr = tile_arrays(KIND);
     const int ns = a.ns, last = ns - 1;
-    auto arr = [&](int which) -> SV {
-        return SV{a.scratch + (int64_t)which * ns * a.sc_ld + s, a.sc_ld};
-    };
-    // ep holds b_k until the state's split is known (then exp(b_k) if it
-    // holds); the per-reaction fallback reads b_k from it as bk
-    SV conc = arr(ARR_CONC), ep = arr(ARR_EP), em = arr(ARR_EM), wdot = arr(ARR_WDOT);
-    const SV& bk = ep;
-    SV db{nullptr, 0}, nsrow{nullptr, 0}, hw{nullptr, 0}, cpa{nullptr, 0}, dcpa{nullptr, 0},
-        ha{nullptr, 0};
-    if (DER) {
-        db = arr(ARR_DB);
-        nsrow = arr(ARR_NSROW);
-        hw = arr(ARR_HW);
-        cpa = arr(ARR_CP);
-        dcpa = arr(ARR_DCP);
-        ha = arr(ARR_H);
-    }
-    // The per-state arrays live in global scratch (state-innermost, so a
-    // warp's accesses are coalesced) and stay in L1/L2: shared memory would
-    // hold too few states per SM to keep the FP64 pipe busy.  Accumulators
-    // take fire-and-forget reductions, performed in L2, and are read back
-    // from L2 after a fence.
+    const int64_t ld = a.sc_ld;
+    auto arr = [&](int which) -> SV { return SV{a.scratch + (int64_t)which * ns * ld + s, ld}; };
+    auto vec = [&](int v) -> SV { return arr(kArr + v); };
+    const SV conc = arr(ARR_CONC), ep = arr(ARR_EP), em = arr(ARR_EM);
+    const SV& bk = ep;  // b_k until the state's split is known (then exp(b_k) if it holds)
+    const SV hk = DER ? arr(ARR_H) : vec(VEC_H), vt = VJP ? arr(ARR_VT) : conc;
+    const SV sums = vec(0);  // by entry of the vector space (third-body sums)
+    const SV wdot = vec(VEC_WDOT), cpa = vec(VEC_CP), dcpa = vec(VEC_DCP), nsrow = vec(VEC_NS);
+    const SV rT = vec(VEC_RT), rE = vec(VEC_RE), cT = vec(VEC_CT), cE = vec(VEC_CE);
+    // Additions are fire-and-forget reductions (red.global.add.f64): the thread
+    // does not wait for the accumulator's old value.  Only this thread updates
+    // its state's entries, and one thread's operations on one address apply in
+    // program order, so every entry sums its reactions in a fixed order; the
+    // sums are read back from L2 after a fence.  The first addition to an entry
+    // of the output is a plain store (marked by the host, which knows the
+    // order), so the output needs no zeroing pass.
     auto accum = [&](const SV& v, int k, double x) { atomicAdd(&v[k], x); };
     auto rd = [&](const SV& v, int k) -> double { return __ldcg(&v[k]); };
+    double* accs = a.acc + s;  // Jacobian only
+    auto add = [&](unsigned sl, double x) {
+        if (sl == TGT_MASK) return;
+        double* p = accs + (int64_t)(sl & TGT_MASK) * a.acc_ld;
+        if (sl & TGT_FIRST) *p = x;
+        else atomicAdd(p, x);
+    };
     const bool conp = a.conp;
     const double* ph = a.phi + s * a.phi_ss;
     const double T = ph[0];
     const double Tc = fmin(10000.0, fmax(100.0, T));
     const double logT = log(Tc), Tinv = 1.0 / Tc;
+    const double lg2T = log2(Tc), tis = kExpScale / Tc;
     const double E = ph[a.phi_sj];
     const double prm = a.param[s];
     const double V = conp ? E : prm;
     const double P = conp ? prm : E;
     const double Vinv = 1.0 / fmax(1e-30, V);
     const double logP = a.need_logP ? log(P) : 0.0;
-    const double Tjinv = DER ? 1.0 / T : 0.0;
+    const double Tjinv = 1.0 / T;
     const double rt_inv = 1.0 / (RU * T);  // unclamped, as the reference's thd concentration
     const double PoRT = P * rt_inv;
     StateVars sv;
     sv.T = T; sv.Tc = Tc; sv.logT = logT; sv.Tinv = Tinv; sv.Tjinv = Tjinv;
     sv.V = V; sv.P = P; sv.PoRT = PoRT; sv.rt_inv = rt_inv; sv.logP = logP; sv.conp = conp;
+    set_scaled<DER>(sv, lg2T, tis);
     sv.etab = etab;
 
     // concentrations (rate_subs.py get_concentrations :597-706)
@@ -251,41 +154,38 @@ __global__ void __launch_bounds__(PJG_BLOCK, KIND == 1 ? PJG_JAC_MINB : (KIND ==
         const double nk = gsmall(ph[(int64_t)(2 + k) * a.phi_sj]);
         nsum = nsum + nk;
         conc[k] = nk * Vinv;
-        wdot[k] = 0.0;
-        if (DER) nsrow[k] = 0.0;
     }
     conc[last] = P / (RU * Tc) + -1.0 * gsmall(nsum) * Vinv;
-    wdot[last] = 0.0;
-
-    // thermo: Gibbs functions for Kc (+ derivatives and cp, h for the Jacobian),
-    // and their exponentials, the factors of 1 / Kc (StateVars::split)
-    double h_ns = 0.0, cp_ns = 0.0, dcp_ns = 0.0;
-    bool split = true;
-    auto gibbs = [&](int k, double b) {
-        ep[k] = b;
-        split = split && abs_le(b, a.kc_split_max);
-    };
-    if (DER) {
-        const Thermo tl = thermo<true>(a.sp + (int64_t)last * PJG_SP_DOUBLES, Tc, logT, Tinv, conp);
-        h_ns = tl.h;
-        cp_ns = tl.cp;
-        dcp_ns = tl.dcp;
-        for (int k = 0; k < ns; ++k) {
-            const double* rec = a.sp + (int64_t)k * PJG_SP_DOUBLES;
-            const Thermo t = k == last ? tl : thermo<true>(rec, Tc, logT, Tinv, conp);
-            gibbs(k, t.b);
-            db[k] = t.db;
-            ha[k] = t.h;
-            if (k < last) {
-                hw[k] = t.h - h_ns * ldg(rec + SP_MW);
-                cpa[k] = t.cp;
-                dcpa[k] = t.dcp;
-            }
+    for (int k = 0; k < ns; ++k) {
+        wdot[k] = 0.0;
+        if (DER) nsrow[k] = 0.0;
+        if (JAC) {
+            rT[k] = 0.0;
+            rE[k] = 0.0;
+            cT[k] = 0.0;
+            cE[k] = 0.0;
         }
-    } else {
-        for (int k = 0; k < ns; ++k)
-            gibbs(k, thermo<false>(a.sp + (int64_t)k * PJG_SP_DOUBLES, Tc, logT, Tinv, conp).b);
     }
+    if (DER)
+        for (int k = vec_arrays(KIND) * ns; k < a.sc.n_vec; ++k) sums[k] = 0.0;
+    if (JAC)
+#pragma unroll 8
+        for (int q = 0; q < a.wt.n_zero; ++q) accs[(int64_t)__ldg(a.wt.zero + q) * a.acc_ld] = 0.0;
+
+    // thermo: Gibbs functions for Kc, cp, h (+ derivatives); the Gibbs functions'
+    // exponentials, the factors of 1 / Kc (StateVars::split)
+    bool split = __double2hiint(conc[last]) >= 0;
+    for (int k = 0; k < ns; ++k) {
+        const Thermo t = thermo<DER>(a.sp + (int64_t)k * PJG_SP_DOUBLES, Tc, logT, Tinv, conp);
+        ep[k] = t.b;
+        split = split && abs_le(t.b, a.kc_split_max);
+        hk[k] = t.h;
+        cpa[k] = t.cp;
+        if (DER) dcpa[k] = t.dcp;
+    }
+    const double h_ns = DER ? hk[last] : 0.0, cp_ns = DER ? cpa[last] : 0.0;
+    sv.h_ns = h_ns;
+    sv.split = split;
     if (split) {
         for (int k = 0; k < ns; ++k) {
             const double b = ep[k];
@@ -293,297 +193,277 @@ __global__ void __launch_bounds__(PJG_BLOCK, KIND == 1 ? PJG_JAC_MINB : (KIND ==
             em[k] = fexp(-b, etab);
         }
     }
-    sv.split = split;
-
     // J^T v: rows T and E of J are linear in the species rows, so v folds into
-    // species weights vt_k = v_k + alpha * hw_k + beta * (1 - W_k/W_ns) known
-    // before the reaction pass (cp_tot needs no rates); vt overwrites hw and the
-    // species part of the product accumulates in nsrow.
+    // species weights vt_k = v_k + alpha * (h_k - h_ns W_k / W_ns)
+    // + beta * (1 - W_k / W_ns) known before the reactions (cp_tot needs no
+    // rates); the species part of the product accumulates in VEC_NS.
     double vt_c0 = 0.0, v1 = 0.0, vout0 = 0.0, vout1 = 0.0, vNS = 0.0, cp_tot_v = 0.0;
     if (VJP) {
         const double* vv = a.v + s * a.phi_ss;
         const double v0 = vv[0];
         v1 = vv[a.phi_sj];
         double ct = 0.0;
-        for (int k = 0; k < last; ++k) ct = fma(conc[k], cpa[k], ct);
-        ct = fma(conc[last], cp_ns, ct);
+        for (int k = 0; k < ns; ++k) ct = fma(conc[k], cpa[k], ct);
         cp_tot_v = ct;
         const double extra = conp ? V : P, fixed = conp ? P : V;
         vt_c0 = v0 + v1 * extra * Tjinv;
         const double alpha = -vt_c0 / (V * ct), beta = v1 * T * RU / fixed;
         for (int k = 0; k < last; ++k) {
-            const double omw = ldg(a.sp + (int64_t)k * PJG_SP_DOUBLES + SP_OMW);
-            hw[k] = vv[(int64_t)(2 + k) * a.phi_sj] + alpha * hw[k] + beta * omw;
+            const double* rec = a.sp + (int64_t)k * PJG_SP_DOUBLES;
+            vt[k] = vv[(int64_t)(2 + k) * a.phi_sj] + alpha * (hk[k] - h_ns * ldg(rec + SP_MW)) +
+                    beta * ldg(rec + SP_OMW);
         }
+        vt[last] = 0.0;
     }
 
-    // ------------------------------------- reactions A + B <=> C + D (packed first)
-    // the next reaction's record and per-state values are loaded while this
-    // one computes
-    E22Head hn;
-    E22Vals vn;
-    if (a.nr_e22 > 0) {
-        load_e22(a.rxn, hn);
-        e22_fetch<DER>(hn, split, conc, ep, em, db, vn);
-    }
-    for (int i = 0; i < a.nr_e22; ++i) {
-        const E22Head h = hn;
-        const E22Vals vv = vn;
-        if (i + 1 < a.nr_e22) {
-            load_e22(a.rxn + i + 1, hn);
-            e22_fetch<DER>(hn, split, conc, ep, em, db, vn);
+    // [M] and log10 [M] of the list of the last third-body reaction that shares
+    // it (such reactions follow one another)
+    MLast ml;
+
+    const bool approx = a.jac_approx;
+    // what one reaction adds; g holds d net / d c_j with the pressure modification
+    auto scatter = [&](auto st_tag, const RxnHead& h, int i, double net, double w_t, const double* g, double d0,
+                       double d1, double gns, double X) {
+        using ST = decltype(st_tag);
+        const int nsp = ST::nsp(h), flags = h.flags, thd = RX_THD(flags);
+        int sp[PJG_MAXSP];
+#pragma unroll
+        for (int e = 0; e < PJG_MAXSP; ++e) {
+            if (e >= nsp) break;
+            sp[e] = ent_spec(h.ent[e]);
+            const int nu = ST::nur(h, e) - ST::nuf(h, e);
+            if (nu) accum(wdot, sp[e], nux(nu, net));
         }
-        E22Terms o;
-        e22_terms_v<DER>(h, vv, last, sv, o);
-        accum(wdot, h.s[0], negi(o.net));
-        accum(wdot, h.s[1], negi(o.net));
-        accum(wdot, h.s[2], o.net);
-        accum(wdot, h.s[3], o.net);
-        if (!DER) continue;
-        const bool hasns = (h.flags & RX_HASNS) && !a.jac_approx;
+        if (!DER) return;
+        const bool hasns = (flags & RX_HASNS) && !approx, has_d1 = rxn_has_d1(flags);
+        const bool listed = thd && h.list >= 0;  // a shared list
+        const int n_l = thd && !listed ? h.thd_cnt : 0;
+        const int* tb = a.wt.tb + (listed ? __ldg(a.wt.tb_off + i) : 0);
         if (VJP) {
             double w = 0.0;
-#pragma unroll
-            for (int ka = 0; ka < 4; ++ka)
-                if (h.s[ka] != last) w = ka < 2 ? w - hw[h.s[ka]] : w + hw[h.s[ka]];
-            if (nonzero(w)) {
-#pragma unroll
-                for (int jb = 0; jb < 4; ++jb)
-                    if (h.s[jb] != last) accum(nsrow, h.s[jb], w * o.g[jb]);
-                if (hasns) vNS = fma(w, o.gns, vNS);
-                vout0 = fma(w, o.d0, vout0);
-                vout1 = fma(w, o.d1, vout1);
-            }
-            continue;
-        }
-        const int* slots = a.rxn_slots + __ldg(a.rxn_slot_off + i);
-        double* accs = a.acc + s;
-#pragma unroll
-        for (int ka = 0; ka < 4; ++ka) {
-            const int k = h.s[ka];
-            if (k == last) continue;
-            // row k gets -v (reactants) or +v (products); reductions as below
-#pragma unroll
-            for (int jb = 0; jb < 6; ++jb) {
-                const int sl = jb < 4 ? __ldg(slots + ka * 4 + jb) : __ldg(slots + 16 + 2 * ka + (jb - 4));
-                const double v = jb < 4 ? o.g[jb] : (jb == 4 ? o.d0 : o.d1);
-                if (sl >= 0) atomicAdd(accs + (int64_t)sl * a.acc_ld, ka < 2 ? negi(v) : v);
-            }
-            if (hasns) accum(nsrow, k, ka < 2 ? negi(o.gns) : o.gns);
-        }
-    }
-
-    // ------------------------- other mass-action reactions in fixed patterns
-    auto ma_range = [&](auto tag, int i0, int i1) {
-        using PT = decltype(tag);
-        constexpr int N = PT::n;
-        for (int i = i0; i < i1; ++i) {
-            RxnHead h;
-            load_head(a.rxn + i, h);
-            MaTerms o;
-            ma_terms<PT, DER>(h, last, sv, conc, bk, ep, em, db, o);
-            int sp[N];
-#pragma unroll
-            for (int e = 0; e < N; ++e) {
-                sp[e] = ent_spec(h.ent[e]);
-                if (PT::nur(e) != PT::nuf(e)) accum(wdot, sp[e], nux(PT::nur(e) - PT::nuf(e), o.net));
-            }
-            if (!DER) continue;
-            const bool hasns = (h.flags & RX_HASNS) && !a.jac_approx;
-            if (VJP) {
-                double w = 0.0;
-#pragma unroll
-                for (int ka = 0; ka < N; ++ka)
-                    if (sp[ka] != last) w = addnu(w, PT::nur(ka) - PT::nuf(ka), hw[sp[ka]]);
-                if (nonzero(w)) {
-#pragma unroll
-                    for (int jb = 0; jb < N; ++jb)
-                        if (sp[jb] != last) accum(nsrow, sp[jb], w * o.g[jb]);
-                    if (hasns) vNS = fma(w, o.gns, vNS);
-                    vout0 = fma(w, o.d0, vout0);
-                    vout1 = fma(w, o.d1, vout1);
-                }
-                continue;
-            }
-            const int* slots = a.rxn_slots + __ldg(a.rxn_slot_off + i);
-            double* accs = a.acc + s;
-#pragma unroll
-            for (int ka = 0; ka < N; ++ka) {
-                const int nuk = PT::nur(ka) - PT::nuf(ka);
-                if (nuk == 0 || sp[ka] == last) continue;
-#pragma unroll
-                for (int jb = 0; jb < N + 2; ++jb) {
-                    const int sl = jb < N ? __ldg(slots + ka * N + jb)
-                                          : __ldg(slots + N * N + 2 * ka + (jb - N));
-                    const double v = jb < N ? o.g[jb] : (jb == N ? o.d0 : o.d1);
-                    if (sl >= 0) atomicAdd(accs + (int64_t)sl * a.acc_ld, nux(nuk, v));
-                }
-                if (hasns) accum(nsrow, sp[ka], nux(nuk, o.gns));
-            }
-        }
-    };
-    ma_range(MaP0{}, a.ma_off[0], a.ma_off[1]);
-    ma_range(MaP1{}, a.ma_off[1], a.ma_off[2]);
-    ma_range(MaP2{}, a.ma_off[2], a.ma_off[3]);
-    ma_range(MaP3{}, a.ma_off[3], a.ma_off[4]);
-    ma_range(MaP4{}, a.ma_off[4], a.ma_off[5]);
-    ma_range(MaP5{}, a.ma_off[5], a.ma_off[6]);
-    ma_range(MaP6{}, a.ma_off[6], a.ma_off[7]);
-    ma_range(MaP7{}, a.ma_off[7], a.ma_off[8]);
-    ma_range(MaP8{}, a.ma_off[8], a.ma_off[9]);
-    ma_range(MaP9{}, a.ma_off[9], a.ma_off[10]);
-
-    // ------------------------------------------------------- other reactions
-    // (the general code; third-body and fall-off reactions of the patterns
-    // TpP0..TpP2 compiled per pattern, the rest reading their coefficients)
-    auto general = [&](auto st_tag, int i0, int i1) {
-        using ST = decltype(st_tag);
-        MCache mc;
-        for (int i = i0; i < i1; ++i) {
-            RxnHead h;
-            load_head(a.rxn + i, h);
-            RxnTerms o;
-            rxn_terms<DER, ST>(h, a.aux, a.thd_spec, a.thd_coef, last, sv, conc, bk, ep, em, db, mc, o);
-            const int flags = h.flags, nsp = ST::nsp(h), thd_off = h.thd_off, thd_cnt = h.thd_cnt;
-            const unsigned* ent = h.ent;
-            const double* p = h.p;
 #pragma unroll
             for (int e = 0; e < PJG_MAXSP; ++e) {
                 if (e >= nsp) break;
                 const int nu = ST::nur(h, e) - ST::nuf(h, e);
-                if (nu != 0) accum(wdot, ent_spec(ent[e]), nux(nu, o.net));
+                if (nu) w = e == 0 ? nux(nu, vt[sp[e]]) : addnu(w, nu, vt[sp[e]]);
             }
-            if (!DER) continue;
-
-            // ------------------------------------------------- Jacobian terms
-            const int* slots = JAC ? a.rxn_slots + __ldg(a.rxn_slot_off + i) : nullptr;
-            const int thd = RX_THD(flags);
-            const bool hasns = flags & RX_HASNS;
-            const double ci_ = o.ci_, X = o.X, d0 = o.d0, d1 = o.d1, gns = o.gns;
-            const double* g = o.g;
-            const double cns = ldg(p + P_CNS);
-            const bool nslist = flags & RX_NSLIST;
-            if (VJP) {
-                // w = sum_k nu_k vt_k over the species rows of this reaction
-                double w = 0.0;
 #pragma unroll
-                for (int ka = 0; ka < PJG_MAXSP; ++ka) {
-                    if (ka >= nsp) break;
-                    const int k = ent_spec(ent[ka]);
-                    if (k == last) continue;
-                    w = addnu(w, ST::nur(h, ka) - ST::nuf(h, ka), hw[k]);
-                }
-                if (nonzero(w)) {
-                    const double wc = w * ci_;
-#pragma unroll
-                    for (int jb = 0; jb < PJG_MAXSP; ++jb) {
-                        if (jb >= nsp) break;
-                        if (ent_spec(ent[jb]) != last) accum(nsrow, ent_spec(ent[jb]), wc * g[jb]);
-                    }
-                    if (hasns && !a.jac_approx) vNS = fma(wc, gns, vNS);
-                    if (thd) {
-                        const double wx = w * X;
-                        for (int l = 0; l < thd_cnt; ++l) {
-                            const int j = __ldg(a.thd_spec + thd_off + l);
-                            if (j != last) accum(nsrow, j, __ldg(a.thd_coef + thd_off + l) * wx);
-                        }
-                        if (nslist && !a.jac_approx) vNS = fma(cns, wx, vNS);
-                    }
-                    vout0 = fma(w, d0, vout0);
-                    vout1 = fma(w, d1, vout1);
-                }
-                continue;
+            for (int e = 0; e < PJG_MAXSP; ++e) {
+                if (e >= nsp) break;
+                if (sp[e] != last) accum(nsrow, sp[e], w * g[e]);
             }
-            // d R / d c_j times the pressure modification, once per reaction (ci is
-            // exactly 1 without a third body)
-            double gci[PJG_MAXSP];
+            if (listed) accum(sums, __ldg(tb), w * X);
+            for (int l = 0; l < n_l; ++l) {
+                const int j = __ldg(a.thd_spec + h.thd_off + l);
+                const double x = __dmul_rn(__ldg(a.thd_coef + h.thd_off + l), w * X);
+                if (j != last) accum(nsrow, j, x);
+                else if (!approx) vNS = vNS + x;
+            }
+            if (hasns) vNS = fma(w, gns, vNS);
+            vout0 = fma(w, d0, vout0);
+            if (has_d1) vout1 = fma(w, d1, vout1);
+            return;
+        }
+        const unsigned* slots = a.wt.slots + __ldg(a.wt.slot_off + i);
+        int nu_sum = 0;
 #pragma unroll
-            for (int e = 0; e < PJG_MAXSP; ++e) gci[e] = e < nsp ? (thd ? g[e] * ci_ : g[e]) : 0.0;
-            // scatter into the species rows of this reaction
+        for (int ka = 0; ka < PJG_MAXSP; ++ka) {
+            if (ka >= nsp) break;
+            const int nu = ST::nur(h, ka) - ST::nuf(h, ka);
+            nu_sum += nu;
+            if (nu == 0 || sp[ka] == last) continue;
+#pragma unroll
+            for (int e = 0; e < PJG_MAXSP; ++e) {
+                if (e >= nsp) break;
+                add(__ldg(slots + ka * (nsp + n_l) + e), nux(nu, g[e]));
+            }
+            accum(cT, sp[ka], nux(nu, d0));
+            if (has_d1) accum(cE, sp[ka], nux(nu, d1));
+            if (hasns) accum(nsrow, sp[ka], nux(nu, gns));
+            if (listed) accum(sums, __ldg(tb + ka), nux(nu, X));
+        }
+        const bool we = flags & RX_WE, real = flags & RX_WEREAL;
+        const double wE = real ? ldg(h.p + P_WE) : 0.0;
+#pragma unroll
+        for (int e = 0; e < PJG_MAXSP; ++e) {
+            if (e >= nsp) break;
+            if (sp[e] == last || (!(flags & RX_REV) && ST::nuf(h, e) == 0)) continue;
+            accum(rT, sp[e], __dmul_rn(w_t, g[e]));
+            if (we) accum(rE, sp[e], real ? __dmul_rn(wE, g[e]) : nux(nu_sum, g[e]));
+        }
+        if (listed) {
+            accum(sums, __ldg(tb + nsp), __dmul_rn(w_t, X));
+            if (we) accum(sums, __ldg(tb + nsp + 1), real ? __dmul_rn(wE, X) : nux(nu_sum, X));
+        }
+        for (int l = 0; l < n_l; ++l) {
+            const int j = __ldg(a.thd_spec + h.thd_off + l);
+            const double x = __dmul_rn(__ldg(a.thd_coef + h.thd_off + l), X);
+            if (j == last && approx) continue;
 #pragma unroll
             for (int ka = 0; ka < PJG_MAXSP; ++ka) {
                 if (ka >= nsp) break;
-                const int k = ent_spec(ent[ka]);
-                if (k == last) continue;
-                const int nuk = ST::nur(h, ka) - ST::nuf(h, ka);
-                if (nuk == 0) continue;
-                // Fire-and-forget reductions (red.global.add.f64): the thread does not
-                // wait for the accumulator's old value.  Only this thread updates its
-                // state's entries, and one thread's operations on one address apply
-                // in program order, so every entry sums its reactions in a fixed order.
-                double* accs = a.acc + s;
-#pragma unroll
-                for (int jb = 0; jb < PJG_MAXSP + 2; ++jb) {
-                    if (jb >= nsp + 2) break;
-                    const int sl = jb < nsp ? __ldg(slots + ka * nsp + jb)
-                                            : __ldg(slots + nsp * nsp + 2 * ka + (jb - nsp));
-                    const double v = jb < nsp ? gci[jb] : (jb == nsp ? d0 : d1);
-                    if (sl >= 0) atomicAdd(accs + (int64_t)sl * a.acc_ld, nux(nuk, v));
-                }
-                double nsacc = 0.0;
-                if (hasns) nsacc = gns * ci_;
-                if (thd && nslist) nsacc = fma(cns, X, nsacc);
-                if ((hasns || (thd && nslist)) && !a.jac_approx) accum(nsrow, k, nux(nuk, nsacc));
+                const int nu = ST::nur(h, ka) - ST::nuf(h, ka);
+                if (nu == 0 || sp[ka] == last) continue;
+                if (j == last) accum(nsrow, sp[ka], nux(nu, x));
+                else add(__ldg(slots + ka * (nsp + n_l) + nsp + l), nux(nu, x));
             }
-            // third-body list columns: coefficient x X formed once per list
-            // entry, then +-it (or twice it) into every row of the reaction
-            // (each entry still takes this reaction's terms after its
-            // species-column terms, the order of the rows' own loops)
-            if (thd) {
-                double* accs = a.acc + s;
-                for (int l = 0; l < thd_cnt; ++l) {
-                    const double cw = __ldg(a.thd_coef + thd_off + l) * X;
-#pragma unroll
-                    for (int ka = 0; ka < PJG_MAXSP; ++ka) {
-                        if (ka >= nsp) break;
-                        if (ent_spec(ent[ka]) == last) continue;
-                        const int nuk = ST::nur(h, ka) - ST::nuf(h, ka);
-                        if (nuk == 0) continue;
-                        const int sl = __ldg(slots + nsp * nsp + 2 * nsp + l * nsp + ka);
-                        if (sl >= 0) atomicAdd(accs + (int64_t)sl * a.acc_ld, nux(nuk, cw));
-                    }
-                }
-            }
+            if (j == last) continue;
+            accum(rT, j, __dmul_rn(w_t, x));
+            if (we) accum(rE, j, real ? __dmul_rn(wE, x) : nux(nu_sum, x));
         }
     };
-    general(PatStoich<TpP0>{}, a.tp_off[0], a.tp_off[1]);
-    general(PatStoich<TpP1>{}, a.tp_off[1], a.tp_off[2]);
-    general(PatStoich<TpP2>{}, a.tp_off[2], a.tp_off[3]);
-    general(RunStoich{}, a.tp_off[kTpPatterns], a.nr);
+
+    // ------------------------------------- reactions A + B <=> C + D (packed first)
+    // the next reaction's record and per-state values are loaded while this
+    // one computes
+    {
+        const int n22 = a.cls_off[1];
+        E22Head hn;
+        E22Vals vn;
+        if (n22 > 0) {
+            load_e22(a.rxn, hn);
+            e22_fetch<DER>(hn, split, conc, ep, em, hk, vn);
+        }
+        for (int i = 0; i < n22; ++i) {
+            const E22Head h = hn;
+            const E22Vals v = vn;
+            if (i + 1 < n22) {
+                load_e22(a.rxn + i + 1, hn);
+                e22_fetch<DER>(hn, split, conc, ep, em, hk, vn);
+            }
+            E22Terms o;
+            e22_terms<DER>(h, v, last, sv, o);
+            RxnHead r;
+            r.flags = h.flags;
+            r.p = h.p;
+            r.thd_cnt = 0;
+            r.list = -1;
+#pragma unroll
+            for (int e = 0; e < 4; ++e) r.ent[e] = (unsigned)h.s[e];
+            scatter(E22Stoich{}, r, i, o.net, o.w, o.g, o.d0, o.d1, o.gns, 0.0);
+        }
+    }
+    // the next reaction's record and values, brought nearer while this one computes
+    auto touch = [&](const void* p) { asm volatile("prefetch.global.L1 [%0];" ::"l"(p)); };
+    auto prefetch = [&](int i) {
+        const RxnRec* R = a.rxn + (i + 1 < a.nr ? i + 1 : i);
+        touch(reinterpret_cast<const char*>(R) + 128);
+        const int n = __ldg(&R->nspec);
+        for (int e = 0; e < n; ++e) {
+            const int k = ent_spec(__ldg(&R->ent[e]));
+            touch(&conc[k]);
+            touch(&ep[k]);
+            touch(&em[k]);
+            if (DER) touch(&hk[k]);
+        }
+    };
+    // ------------------------- other mass-action reactions in fixed patterns
+    auto ma_range = [&](auto tag, int c) {
+        using PT = decltype(tag);
+        for (int i = a.cls_off[c]; i < a.cls_off[c + 1]; ++i) {
+            RxnHead h;
+            load_head(a.rxn + i, h);
+            prefetch(i);
+            MaTerms o;
+            ma_terms<PT, DER>(h, last, sv, conc, bk, ep, em, hk, o);
+            scatter(PatStoich<PT>{}, h, i, o.net, o.w, o.g, o.d0, o.d1, o.gns, 0.0);
+        }
+    };
+    ma_range(MaP0{}, 1);
+    ma_range(MaP1{}, 2);
+    ma_range(MaP2{}, 3);
+    ma_range(MaP3{}, 4);
+    ma_range(MaP4{}, 5);
+    ma_range(MaP5{}, 6);
+    ma_range(MaP6{}, 7);
+    ma_range(MaP7{}, 8);
+    ma_range(MaP8{}, 9);
+    ma_range(MaP9{}, 10);
+    // ------------------------------------------------------- other reactions
+    // (the general code; third-body and fall-off reactions of the patterns
+    // TpP0..TpP2 compiled per pattern, the rest reading their coefficients)
+    auto general = [&](auto st_tag, int c) {
+        using ST = decltype(st_tag);
+        for (int i = a.cls_off[c]; i < a.cls_off[c + 1]; ++i) {
+            RxnHead h;
+            load_head(a.rxn + i, h);
+            prefetch(i);
+            RxnTerms o;
+            rxn_terms<DER, ST>(h, a.aux, a.thd_spec, a.thd_coef, last, sv, conc, bk, ep, em, hk, ml, o);
+            double gci[PJG_MAXSP];
+            if (DER) {
+                const bool thd = RX_THD(h.flags) != THD_NONE;
+#pragma unroll
+                for (int e = 0; e < PJG_MAXSP; ++e)
+                    if (e < ST::nsp(h)) gci[e] = thd ? __dmul_rn(o.g[e], o.ci_) : o.g[e];
+            }
+            scatter(ST{}, h, i, o.net, o.w, gci, o.d0, o.d1, o.gns * o.ci_, o.X);
+        }
+    };
+    general(PatStoich<TpP0>{}, 11);
+    general(PatStoich<TpP1>{}, 12);
+    general(PatStoich<TpP2>{}, 13);
+    general(RunStoich{}, 14);
 
     __threadfence();
 
-    // ------------------------------------------- temperature and E rates
-    double upper = 0.0, lower = 0.0;
+    // ------------------------ third-body columns, temperature and E rates
     if (DER) {
-        for (int k = 0; k < last; ++k) {
-            lower = fma(conc[k], cpa[k], lower);
-            upper = fma(ha[k], rd(wdot, k), upper);
+        for (int q0 = 0; q0 < a.wt.n_post; q0 += kPostUnroll) {
+            int4 it[kPostUnroll];
+            double x[kPostUnroll];
+#pragma unroll
+            for (int e = 0; e < kPostUnroll; ++e)
+                it[e] = __ldg(reinterpret_cast<const int4*>(a.wt.post + (q0 + e < a.wt.n_post ? q0 + e : q0)));
+#pragma unroll
+            for (int e = 0; e < kPostUnroll; ++e) x[e] = rd(sums, it[e].x);
+#pragma unroll
+            for (int e = 0; e < kPostUnroll; ++e) {
+                if (q0 + e >= a.wt.n_post) break;
+                const unsigned tgt = (unsigned)it[e].y;
+                const double y = __dmul_rn(__hiloint2double(it[e].w, it[e].z), x[e]);
+                // J^T v has no output entries among the targets
+                if (!JAC || (tgt & TGT_VEC)) accum(sums, (int)(tgt & TGT_MASK), y);
+                else add(tgt, y);
+            }
         }
-        lower = fma(conc[last], cp_ns, lower);
-        upper = fma(h_ns, rd(wdot, last), upper);
-    } else {
-        for (int k = 0; k < ns; ++k) {
-            const Thermo t = thermo<false>(a.sp + (int64_t)k * PJG_SP_DOUBLES, Tc, logT, Tinv, conp);
-            lower = fma(conc[k], t.cp, lower);
-            upper = fma(t.h, rd(wdot, k), upper);
-        }
+        __threadfence();
     }
-    const double Tdot = 0.0 + -1.0 * upper / lower;
-    double dE = 0.0;
-    for (int k = 0; k < last; ++k)
-        dE = fma(ldg(a.sp + (int64_t)k * PJG_SP_DOUBLES + SP_OMW), rd(wdot, k), dE);
+    // sums over species in partial sums (the order of the tile kernels)
+    const int n_parts = sum_parts(ns);
+    double upper = 0.0, lower = 0.0, dE = 0.0, dTsum = 0.0, dTsum1 = 0.0;
+    for (int w = 0; w < n_parts; ++w) {
+        double pu = 0.0, pl = 0.0, pe = 0.0, pt = 0.0, p1 = 0.0;
+#pragma unroll 4
+        for (int k = w; k < ns; k += n_parts) {
+            const double w_k = rd(wdot, k), cpk = cpa[k], ck = conc[k];
+            pu = fma(hk[k], w_k, pu);
+            pl = fma(ck, cpk, pl);
+            pe = fma(ldg(a.sp + (int64_t)k * PJG_SP_DOUBLES + SP_OMW), w_k, pe);  // omw of the bath gas is 0
+            if (DER) {
+                pt = fma(cp_ns * Tjinv - dcpa[k], ck, pt);
+                p1 = fma(cpk - cp_ns, ck, p1);
+            }
+        }
+        upper = w ? upper + pu : pu;
+        lower = w ? lower + pl : pl;
+        dE = w ? dE + pe : pe;
+        dTsum = w ? dTsum + pt : pt;
+        dTsum1 = w ? dTsum1 + p1 : p1;
+    }
+    const double inv_cp = 1.0 / lower;
+    const double Tdot = -upper * inv_cp;
     const double Vval = fmax(1e-30, V);
-    double Edot;
-    if (conp) {
-        Edot = Vval * Tdot / Tc;
-        Edot = Edot + Vval * dE * Tc * RU / P;
-    } else {
-        Edot = P * Tdot / Tc;
-        Edot = Edot + Tc * RU * dE;
-    }
     if (a.dphi) {
         double* o = a.dphi + s * a.dphi_ss;
+        double Edot;
+        if (conp) {
+            Edot = Vval * Tdot / Tc;
+            Edot = Edot + Vval * dE * Tc * RU / P;
+        } else {
+            Edot = P * Tdot / Tc;
+            Edot = Edot + Tc * RU * dE;
+        }
         o[0] = Tdot;
         o[a.dphi_sj] = Edot;
         for (int k = 0; k < last; ++k) o[(int64_t)(2 + k) * a.dphi_sj] = Vval * rd(wdot, k);
@@ -592,28 +472,27 @@ __global__ void __launch_bounds__(PJG_BLOCK, KIND == 1 ? PJG_JAC_MINB : (KIND ==
         // constant parts of columns T and E (from rows T, E of dTdot_dT :1847,
         // dEdotdT :2001, dTdotdE :1595, dEdotdE :1740) and the species columns'
         // bath-gas and d cp_tot / dn_j terms
-        const double extra = conp ? V : P;
-        double dTsum = (cp_ns * Tjinv - dcp_ns) * conc[last];
-        double wsum = 0.0, omws = 0.0, dTsum1 = 0.0, hws = 0.0;
+        const double extra = conp ? V : P, ct = cp_tot_v;
+        for (int q = 0; q < a.n_ns_post; ++q)
+            vNS = fma(__ldg(&a.ns_post[q].coef), rd(sums, (int)__ldg(&a.ns_post[q].src)), vNS);
+        double wsum = 0.0, omws = 0.0, hws = 0.0, vws = 0.0;
         for (int k = 0; k < last; ++k) {
             const double* rec = a.sp + (int64_t)k * PJG_SP_DOUBLES;
             const double mw = ldg(rec + SP_MW), omw = ldg(rec + SP_OMW);
-            const double wk = rd(wdot, k), ck = conc[k], cpk = cpa[k];
-            dTsum = dTsum + (cp_ns * Tjinv - dcpa[k]) * ck;
-            wsum = wsum + wk * (-cpk + mw * cp_ns);
-            omws = fma(omw, wk, omws);
-            dTsum1 = dTsum1 + (cpk - cp_ns) * ck;
-            hws = fma(ha[k] - h_ns * mw, wk, hws);
+            const double w_k = rd(wdot, k), cpk = cpa[k];
+            wsum = wsum + w_k * (-cpk + mw * cp_ns);
+            omws = fma(omw, w_k, omws);
+            hws = fma(hk[k] - h_ns * mw, w_k, hws);
+            vws = fma(vt[k], w_k, vws);
         }
-        const double ct = cp_tot_v;
-        double C0 = vt_c0 * (Tdot * dTsum + wsum) / ct - v1 * extra * Tdot * Tjinv * Tjinv +
-                    v1 * RU * (conp ? V / P : 1.0) * omws;
-        double C1 = conp ? vt_c0 * (Tdot * dTsum1 + hws) / (ct * V)
-                         : -vt_c0 * Tdot * cp_ns * rt_inv / ct;
+        if (conp) vout1 = vout1 - vws;  // the reactions' -net of column E
+        const double C0 = vt_c0 * (Tdot * dTsum + wsum) / ct - v1 * extra * Tdot * Tjinv * Tjinv +
+                          v1 * RU * (conp ? V / P : 1.0) * omws;
+        double C1 = conp ? vt_c0 * (Tdot * dTsum1 + hws) / (ct * V) : -vt_c0 * Tdot * cp_ns * rt_inv / ct;
         C1 += v1 * Tdot * Tjinv;
         const double gam = -vt_c0 * Tdot / (V * ct);
         double* o = a.vjp + s * a.phi_ss;
-        o[0] = vout0 + C0;
+        o[0] = fma(vout0, V * Tjinv, C0);  // the reactions' terms of column T leave V / T out
         o[a.phi_sj] = vout1 + C1;
         for (int j = 0; j < last; ++j)
             o[(int64_t)(2 + j) * a.phi_sj] = rd(nsrow, j) - vNS + gam * (cpa[j] - cp_ns);
@@ -622,73 +501,84 @@ __global__ void __launch_bounds__(PJG_BLOCK, KIND == 1 ? PJG_JAC_MINB : (KIND ==
     if (!JAC) return;
 
     // ------------------------------------------- assemble rows T and E
-    double* acc = a.acc + s;
-    const int64_t ld = a.acc_ld;
-    // the reductions are performed in L2: read the accumulator there
-    __threadfence();
-    auto accr = [&](int64_t sl) { return __ldcg(acc + sl * ld); };
-    const double cp_tot = lower;
+    // Both rows are linear in the species rows, so each reaction has added its
+    // share (w_i d R_i / d c_j, with w_i = sum_k nu_ki hw_k for row T and
+    // sum_k nu_ki (1 - W_k / W_ns) = sum nu for row E); the bath-gas terms, the
+    // same for every species column, take one sum per state.
+    const int64_t ald = a.acc_ld;
     const double fixed = conp ? P : V, extra = conp ? V : P;
-    const double inv_vcp = 1.0 / (V * cp_tot);
-    const double TRf = T * RU / fixed, eTj = extra * Tjinv;
-    if (a.dense_rs || a.dchunk_slots) {
-        rows_te(a.dense_rs == 0, acc, ld, a.dense_rs, a.dense_cs, a.dchunk_off, a.dchunk_list,
-                a.dchunk_slots, a.cj_slots, a.sp, nsrow, hw, cpa, last, cp_ns, Tdot, inv_vcp, TRf,
-                eTj);
-    } else {
-        // sparse output whose pattern fills under half of the chunk lists' slots
-        // (dchunk_slots null; large sparse mechanisms): the bath-gas terms (per-row
-        // sums subtracted from every species column of the pattern), then the
-        // column sums of rows T and E, two passes over the pattern
-        for (int k = 0; k < last; ++k) {
-            const double v = rd(nsrow, k);
-            if (!nonzero(v)) continue;
-            const int r0 = __ldg(a.row_off + k), r1 = __ldg(a.row_off + k + 1);
-            for (int q = r0; q < r1; ++q) {
-                const int2 e = __ldg(a.row_list + q);
-                acc[(int64_t)e.y * ld] = accr(e.y) - v;
-            }
-        }
+    const double Vjinv = V >= 1e-30 ? Vinv : 1.0 / V;
+    const double inv_vcp = Vjinv * inv_cp;
+    const double eTj = extra * Tjinv, VTj = V * Tjinv, TRf = T * RU / fixed;
+    for (int q = 0; q < a.n_ns; ++q) {
+        const double mv = negi(rd(nsrow, __ldg(a.ns_rows + q)));
+        if (!nonzero(mv)) continue;
+        const int* sl = a.ns_slots + q * last;
+#pragma unroll 8
         for (int j = 0; j < last; ++j) {
-            double sum = 0.0, sumE = 0.0;
+            const int t = __ldg(sl + j);
+            if (t >= 0) atomicAdd(accs + (int64_t)t * ald, mv);
+        }
+    }
+    // T column of rows T, E and E column of rows T, E; column E of a species
+    // row: at constant pressure the terms leave out -net of each reaction, in
+    // sum -wdot_k
+    double rate_sum = 0.0, sumT = 0.0, spec1 = 0.0, sumE1 = 0.0, nsT = 0.0, nsE = 0.0;
+    for (int w = 0; w < n_parts; ++w) {
+        double pr = 0.0, pt = 0.0, ps = 0.0, pe = 0.0, pnt = 0.0, pne = 0.0;
+#pragma unroll 2
+        for (int k = w; k < last; k += n_parts) {
+            const double* rec = a.sp + (int64_t)k * PJG_SP_DOUBLES;
+            const double mw = ldg(rec + SP_MW), omw = ldg(rec + SP_OMW);
+            const int sl0 = __ldg(a.sp_slots + 2 * k), sl1 = __ldg(a.sp_slots + 2 * k + 1);
+            const double w_k = rd(wdot, k), cpk = cpa[k], hwk = fma(-h_ns, mw, hk[k]);
+            const double ct = rd(cT, k), ce = rd(cE, k), ek = conp ? ce - w_k : ce;
+            if (sl0 >= 0) accs[(int64_t)sl0 * ald] = ct * VTj;
+            if (sl1 >= 0) accs[(int64_t)sl1 * ald] = ek;
+            const double vk = sl0 >= 0 ? ct * Tjinv : 0.0;  // J_kT / V
+            const double Jk1 = sl1 >= 0 ? ek : 0.0;
+            pr = fma(-vk, hwk, pr);
+            pr = fma(w_k, fma(mw, cp_ns, -cpk), pr);
+            pt = fma(omw, conp ? fma(Tjinv, w_k, vk) : fma(T, vk, w_k), pt);
+            ps = fma(hwk, conp ? Jk1 - w_k : Jk1, ps);
+            pe = fma(omw, Jk1, pe);
+        }
+        for (int q = w; q < a.n_ns; q += n_parts) {
+            const int k = __ldg(a.ns_rows + q);
+            const double v = rd(nsrow, k);
+            pnt = fma(fma(-h_ns, ldg(a.sp + (int64_t)k * PJG_SP_DOUBLES + SP_MW), hk[k]), v, pnt);
+            pne = fma(ldg(a.sp + (int64_t)k * PJG_SP_DOUBLES + SP_OMW), v, pne);
+        }
+        rate_sum = w ? rate_sum + pr : pr;
+        sumT = w ? sumT + pt : pt;
+        spec1 = w ? spec1 + ps : ps;
+        sumE1 = w ? sumE1 + pe : pe;
+        nsT = w ? nsT + pnt : pnt;
+        nsE = w ? nsE + pne : pne;
+    }
+    const bool summed = a.col_list == nullptr;
+    if (!summed) __threadfence();  // the species block is read back below
+#pragma unroll 2
+    for (int j = 0; j < last; ++j) {
+        double sT, sE;
+        if (summed) {
+            sT = rd(rT, j) - nsT;
+            sE = rd(rE, j) - nsE;
+        } else {
+            sT = 0.0;
+            sE = 0.0;
             const int c0 = __ldg(a.col_off + j), c1 = __ldg(a.col_off + j + 1);
             for (int q = c0; q < c1; ++q) {
                 const int2 e = __ldg(a.col_list + q);
-                const double Jkj = accr(e.y);
-                sum = fma(hw[e.x], Jkj, sum);
-                sumE = fma(ldg(a.sp + (int64_t)e.x * PJG_SP_DOUBLES + SP_OMW), Jkj, sumE);
+                const double Jkj = __ldcg(accs + (int64_t)e.y * ald);
+                sT = fma(fma(-h_ns, ldg(a.sp + (int64_t)e.x * PJG_SP_DOUBLES + SP_MW), hk[e.x]), Jkj, sT);
+                sE = fma(ldg(a.sp + (int64_t)e.x * PJG_SP_DOUBLES + SP_OMW), Jkj, sE);
             }
-            const double J0 = -1.0 * (sum + Tdot * (cpa[j] + -1.0 * cp_ns)) * inv_vcp;
-            acc[(int64_t)__ldg(a.cj_slots + 2 * j) * ld] = J0;
-            acc[(int64_t)__ldg(a.cj_slots + 2 * j + 1) * ld] = TRf * sumE + eTj * J0;
         }
+        const double J0 = -1.0 * (sT + Tdot * (cpa[j] + -1.0 * cp_ns)) * inv_vcp;
+        accs[(int64_t)__ldg(a.cj_slots + 2 * j) * ald] = J0;
+        accs[(int64_t)__ldg(a.cj_slots + 2 * j + 1) * ald] = TRf * sE + eTj * J0;
     }
-
-    // T column of rows T, E and E column of rows T, E
-    double dTsum = (cp_ns * Tjinv - dcp_ns) * conc[last];
-    double rate_sum = 0.0, sumT = 0.0, sumE1 = 0.0, spec1 = 0.0, dTsum1 = 0.0;
-    const double Vjinv = 1.0 / V;
-    for (int k = 0; k < last; ++k) {
-        const double* rec = a.sp + (int64_t)k * PJG_SP_DOUBLES;
-        const double mw = ldg(rec + SP_MW), omw = ldg(rec + SP_OMW);
-        const int sl0 = __ldg(a.sp_slots + 2 * k), sl1 = __ldg(a.sp_slots + 2 * k + 1);
-        const double Jk0 = sl0 >= 0 ? accr(sl0) : 0.0;
-        const double Jk1 = sl1 >= 0 ? accr(sl1) : 0.0;
-        const double wk = rd(wdot, k), ck = conc[k], cpk = cpa[k], hwk = hw[k];
-        rate_sum = rate_sum + Vjinv * Jk0 * (-1.0 * hwk);
-        rate_sum = rate_sum + wk * (-cpk + mw * cp_ns);
-        dTsum = dTsum + (cp_ns * Tjinv - dcpa[k]) * ck;
-        if (conp) {
-            sumT = sumT + omw * (Vjinv * Jk0 + Tjinv * wk);
-            spec1 = spec1 + hwk * (Jk1 - wk);
-            dTsum1 = dTsum1 + (cpk - cp_ns) * ck;
-        } else {
-            sumT = sumT + omw * (Jk0 * (T * Vjinv) + wk);
-            spec1 = spec1 + hwk * Jk1;
-        }
-        sumE1 = fma(omw, Jk1, sumE1);
-    }
-    const double inv_cp = 1.0 / cp_tot;
     const double J00 = (Tdot * dTsum + rate_sum) * inv_cp;
     double J10;
     if (conp) {
@@ -707,17 +597,19 @@ __global__ void __launch_bounds__(PJG_BLOCK, KIND == 1 ? PJG_JAC_MINB : (KIND ==
     }
     double J11 = TRf * sumE1;
     J11 = J11 + (extra * J01 + Tdot) * Tjinv;
-    acc[(int64_t)a.s00 * ld] = J00;
-    acc[(int64_t)a.s10 * ld] = J10;
-    acc[(int64_t)a.s01 * ld] = J01;
-    acc[(int64_t)a.s11 * ld] = J11;
+    accs[(int64_t)a.s00 * ald] = J00;
+    accs[(int64_t)a.s10 * ald] = J10;
+    accs[(int64_t)a.s01 * ald] = J01;
+    accs[(int64_t)a.s11 * ald] = J11;
 }
+
+constexpr int kChemBlock = 128;
 
 // Species thermo of the chem_utils kernel type (rate_subs.py write_chem_utils
 // :3391-3444, polyfit_kernel_gen :3281-3388): at the guarded temperature,
 // cp (cv), h (u) and the Gibbs function b of every species.  Entry (s, k) of
 // each output at out[s * out_ss + k * out_sk].
-__global__ void __launch_bounds__(PJG_BLOCK) chem_utils_kernel(const double* __restrict__ sp, int ns,
+__global__ void __launch_bounds__(kChemBlock) chem_utils_kernel(const double* __restrict__ sp, int ns,
                                                                int64_t n, int conp,
                                                                const double* __restrict__ phi,
                                                                int64_t phi_ss, double* cp, double* h,
@@ -744,48 +636,37 @@ int pjg_launch_chem_utils(const double* sp, int ns, int64_t n, int conp, const d
                           int64_t out_sk, void* stream)
 {
     if (n <= 0) return 0;
-    chem_utils_kernel<<<(unsigned)((n + PJG_BLOCK - 1) / PJG_BLOCK), PJG_BLOCK, 0, (cudaStream_t)stream>>>(
+    chem_utils_kernel<<<(unsigned)((n + kChemBlock - 1) / kChemBlock), kChemBlock, 0, (cudaStream_t)stream>>>(
         sp, ns, n, conp, phi, phi_ss, cp, h, b, out_ss, out_sk);
     return cudaGetLastError() == cudaSuccess ? 0 : -2;
 }
 
+
 namespace {
 
-template <int KIND>
-void launch(const EvalArgs& a, unsigned grid, cudaStream_t st)
+const void* wave_of(int kind)
 {
-    eval_kernel<KIND><<<grid, PJG_BLOCK, 0, st>>>(a);
+    return kind == KIND_JAC ? (const void*)wave_kernel<KIND_JAC>
+           : kind == KIND_VJP ? (const void*)wave_kernel<KIND_VJP> : (const void*)wave_kernel<KIND_RATES>;
 }
 
 }  // namespace
 
-int pjg_eval_blocks_per_sm(int kind)
+int pjg_wave_blocks_per_sm(int kind)
 {
     int b = 0;
-    cudaError_t e;
-    if (kind == 1)
-        e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, eval_kernel<1>, PJG_BLOCK, 0);
-    else if (kind == 2)
-        e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, eval_kernel<2>, PJG_BLOCK, 0);
-    else
-        e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, eval_kernel<0>, PJG_BLOCK, 0);
+    const cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, wave_of(kind), PJG_BLOCK, 0);
     return e == cudaSuccess && b > 0 ? b : 1;
 }
 
-namespace {
-thread_local cudaError_t g_launch_err = cudaSuccess;  // of this thread's last evaluation launch
-}
-
-const char* pjg_launch_error_string() { return cudaGetErrorString(g_launch_err); }
-
-int pjg_launch_eval(const EvalArgs& a, int kind, void* stream)
+int pjg_launch_wave(const EvalArgs& a, int kind, void* stream)
 {
     if (a.n <= 0) return 0;
-    cudaStream_t st = (cudaStream_t)stream;
+    const cudaStream_t st = (cudaStream_t)stream;
     const unsigned grid = (unsigned)((a.n + PJG_BLOCK - 1) / PJG_BLOCK);
-    if (kind == 1) launch<1>(a, grid, st);
-    else if (kind == 2) launch<2>(a, grid, st);
-    else launch<0>(a, grid, st);
-    g_launch_err = cudaGetLastError();
-    return g_launch_err == cudaSuccess ? 0 : -2;
+    if (kind == KIND_JAC) wave_kernel<KIND_JAC><<<grid, PJG_BLOCK, 0, st>>>(a);
+    else if (kind == KIND_VJP) wave_kernel<KIND_VJP><<<grid, PJG_BLOCK, 0, st>>>(a);
+    else wave_kernel<KIND_RATES><<<grid, PJG_BLOCK, 0, st>>>(a);
+    pjg_launch_err = cudaGetLastError();
+    return pjg_launch_err == cudaSuccess ? 0 : -2;
 }

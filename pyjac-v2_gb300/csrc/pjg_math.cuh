@@ -143,6 +143,51 @@ __device__ __forceinline__ double fexp(double x, const double* tab)
     return __longlong_as_double(__double_as_longlong(y) + ((long long)(n >> PJG_EXP_BITS) << 52));
 }
 
+// exp of (xs + n0) ln 2 / 2^B, the argument scaled by the caller (its products
+// with 2^B / ln 2 are folded into per-state values and stored constants) and n0
+// an integer.  The nearest integer to xs comes from its bits on the integer
+// pipe, so that of fexp's eight FP64 instructions five remain: xs - n, two for
+// the polynomial (in units of the table step), and two for the result.  The
+// rest xs - n is exact.  Values whose exponent leaves the normal range, the
+// reference's clamp at exp(690.775...), infinities and NaN take fexp's way.
+#if PJG_EXP_BITS < 10
+#error "fexp_s takes the degree-3 polynomial of the tables with 1,024 entries and more"
+#endif
+constexpr double kExpStep = 0.6931471805599453 * (1.0 / PJG_EXP_TAB);    // ln 2 / 2^B
+constexpr double kExpScale = 1.4426950408889634 * PJG_EXP_TAB;           // 2^B / ln 2
+
+static __device__ __noinline__ double fexp_far(double xs, int n0)
+{
+    const double x = (xs + (double)n0) * kExpStep;
+    return exp(x < EXP_MAX ? x : (x >= EXP_MAX ? EXP_MAX : x));
+}
+
+__device__ __forceinline__ double fexp_s(double xs, int n0, const double* tab)
+{
+    const int hi = __double2hiint(xs), ah = hi & 0x7fffffff;
+    const int e = (ah >> 20) - 1023;  // |xs| = 1.m 2^e
+    const int ec = e < 0 ? 0 : e;
+    // round |xs| to an integer: add a half, clear the fraction (all in the high
+    // word for |xs| < 2^20); below 1/2 it is 0, from 1/2 to 1 it is 1
+    int r = ah + (0x100000 >> (e < 0 ? 0 : e + 1));
+    r &= (int)0xfff00000 >> ec;
+    r = e < -1 ? 0 : r;
+    const int sh = 20 - ((r >> 20) - 1023);
+    int n = ((r & 0xfffff) | 0x100000) >> (sh & 31);
+    n = e < -1 ? 0 : n;
+    n = (hi < 0 ? -n : n) + n0;
+    const int m = n >> PJG_EXP_BITS;
+    if (ah >= 0x41300000 || (unsigned)(m + 1020) > 2015u) return fexp_far(xs, n0);
+    const double f = __dsub_rn(xs, __hiloint2double(r | (hi & 0x80000000), 0));
+    constexpr double c1 = kExpStep, c2 = PJG_EXP_C2 * kExpStep * kExpStep,
+                     c3 = PJG_EXP_C3 * kExpStep * kExpStep * kExpStep;
+    double q = fma(f, c3, c2);
+    q = fma(q, f, c1);
+    const double tj = tab[n & (PJG_EXP_TAB - 1)];
+    const double y = fma(tj, __dmul_rn(f, q), tj);
+    return __hiloint2double(__double2hiint(y) + (m << 20), __double2loint(y));
+}
+
 // min(c, x) for a positive constant c on the integer pipe (GB300's FP64 pipe
 // is the kernels' bound): as signed 64-bit integers, doubles order like
 // their values against a positive c, negative values having the sign bit set.
@@ -176,27 +221,20 @@ __device__ __forceinline__ double gsmall(double x)
     return __longlong_as_double(b > s ? b : s);
 }
 
-// Arrhenius forms of rate_subs.py get_simple_arrhenius_rates (:2642-3023)
-__device__ __forceinline__ double arrhenius(int form, double A, double b, double Ta, int bint,
-                                            double Tc, double logT, double Tinv, const double* tab)
-{
-    if (form == FORM_A) return A;
-    // fast_powi of a negative exponent inverts its base first
-    if (form == FORM_AT) return A * (bint < 0 ? powi(Tinv, -bint) : powi(Tc, bint));
-    return gexp(A + logT * b + -1.0 * Ta * Tinv, tab);
-}
-
-// the same, also giving ln k (the clamped exponent) for the exponential form
-// (has_ln false for the forms A and A T^b)
-__device__ __forceinline__ double arrhenius_ln(int form, double A, double b, double Ta, int bint,
-                                               double Tc, double logT, double Tinv,
-                                               const double* tab, double& lnk, bool& has_ln)
+// Arrhenius forms of rate_subs.py get_simple_arrhenius_rates (:2642-3023).  ls
+// is ln T and tis 1 / T, both times 2^B / ln 2; A and its integer n as RxnRec
+// holds them.  lns is the exponent's part besides n (has_ln false for the
+// forms A and A T^b).
+__device__ __forceinline__ double arrhenius(int form, double A, int n, double b, double Ta, double Tc,
+                                            double Tinv, double ls, double tis, const double* tab,
+                                            double& lns, bool& has_ln)
 {
     has_ln = form > FORM_AT;
     if (form == FORM_A) return A;
-    if (form == FORM_AT) return A * (bint < 0 ? powi(Tinv, -bint) : powi(Tc, bint));
-    lnk = min_pos(EXP_MAX, A + logT * b + -1.0 * Ta * Tinv);
-    return fexp(lnk, tab);
+    // fast_powi of a negative exponent inverts its base first
+    if (form == FORM_AT) return __dmul_rn(A, n < 0 ? powi(Tinv, -n) : powi(Tc, n));
+    lns = fma(-Ta, tis, fma(b, ls, A));
+    return fexp_s(lns, n, tab);
 }
 
 // PLOG: ln kf interpolated linearly in ln P between bracketing pressures,
@@ -300,7 +338,7 @@ __device__ inline double cheb_log10k(const double* blk, double Tinv, double logP
 
 // NASA-7 properties of one species at T (rate_subs.py polyfit_kernel_gen :3335-3356)
 struct Thermo {
-    double cp, h, b, db, dcp;
+    double cp, h, b, dcp;
 };
 
 template <bool DERIV>
@@ -326,11 +364,8 @@ __device__ __forceinline__ Thermo thermo(const double* rec, double Tc, double lo
     t.b = Tc * (Tc * (Tc * (Tc * ldg(c + TH_R + 3) + ldg(c + TH_R + 2)) + ldg(c + TH_R + 1)) +
                 ldg(c + TH_R)) + ldg(c + TH_A0M1) * logT + ldg(c + TH_A6MA0) + -1.0 * a5 * Tinv;
     if (DERIV) {
-        t.db = Tc * (Tc * (Tc * ldg(c + TH_Q + 3) + ldg(c + TH_Q + 2)) + ldg(c + TH_Q + 1)) +
-               ldg(c + TH_Q) + Tinv * (ldg(c + TH_A0M1) + a5 * Tinv);
         t.dcp = RU * (Tc * (Tc * (Tc * ldg(c + TH_S + 2) + ldg(c + TH_S + 1)) + ldg(c + TH_S)) + a1);
     } else {
-        t.db = 0.0;
         t.dcp = 0.0;
     }
     return t;

@@ -12,12 +12,10 @@
 // routine.
 //
 // The scratch array is kScratchDoubles doubles (16 MiB) on every device that
-// loads the library, held until the process exits.  It holds the kernel's
-// per-state working arrays (10 * Ns doubles per state, 4,240 bytes for
-// GRI-Mech 3.0), so one launch covers up to floor(16 MiB / (80 Ns bytes))
-// states rounded down to a multiple of 128 (3,840 for GRI-Mech 3.0); larger
-// problems run as several launches in order on the caller's stream.  A
-// mechanism whose 128-state block does not fit (more than 1,638 species) is
+// loads the library, held until the process exits.  It holds the blocks'
+// scratch slices (about 5 Ns doubles per state of a tile); the grid is cut to
+// as many blocks as have a slice, whatever the problem's size.  A mechanism
+// of which 128 states at 10 Ns doubles do not fit (more than 1,638 species) is
 // rejected with PJG_ERR_ARG.
 //
 // Set-up: the first call on each device, with that device current, takes the
@@ -40,7 +38,7 @@
 #include "pjg_eval.cuh"
 
 int pjg_internal_fail(int code, const char* msg);
-void pjg_internal_fill_args(const pjg_mech* m, EvalArgs* a);
+int pjg_internal_vjp_args(pjg_mech* m, int64_t n, size_t scratch_doubles, EvalArgs* a, int* grid);
 int pjg_internal_mech_ns(const pjg_mech* m);
 int pjg_internal_check_device(const pjg_mech* m);
 void pjg_internal_count_launch();
@@ -86,13 +84,12 @@ extern "C" int pjg_vjp_noalloc(pjg_mech* mech, int64_t n, char order, int conp, 
     if (n == 0) return 0;
     if (!param || !phi || !v || !out) return pjg_internal_fail(PJG_ERR_ARG, "null array");
     const int ns = pjg_internal_mech_ns(mech);
-    const size_t per_state = (size_t)ARR_N_JAC * ns;  // doubles
-    int64_t chunk = (int64_t)(kScratchDoubles / per_state) / PJG_BLOCK * PJG_BLOCK;
-    if (chunk < PJG_BLOCK) {
+    const size_t need = (size_t)10 * ns * 128;  // doubles
+    if (need > kScratchDoubles) {
         char msg[256];
         snprintf(msg, sizeof(msg),
                  "pjg_vjp_noalloc: %d species need %zu bytes of scratch per 128 states, more than "
-                 "the fixed %zu-byte array", ns, per_state * 8 * PJG_BLOCK, kScratchDoubles * 8);
+                 "the fixed %zu-byte array", ns, need * 8, kScratchDoubles * 8);
         return pjg_internal_fail(PJG_ERR_ARG, msg);
     }
     // the scratch address below is the current device's: the mechanism's
@@ -102,39 +99,26 @@ extern "C" int pjg_vjp_noalloc(pjg_mech* mech, int64_t n, char order, int conp, 
     double* scratch = nullptr;
     rc = scratch_for_current_device(&scratch);
     if (rc) return rc;
-    if (chunk > n) chunk = n;
-    const bool F = order == 'F';
     const int NN = ns + 1;
-    for (int64_t off = 0; off < n; off += chunk) {
-        const int64_t cnt = n - off < chunk ? n - off : chunk;
-        EvalArgs a;
-        pjg_internal_fill_args(mech, &a);
-        a.n = cnt;
-        a.conp = conp;
-        a.param = param + off;
-        if (F) {
-            a.phi = phi + off;
-            a.phi_ss = 1;
-            a.phi_sj = n;
-            a.v = v + off;
-            a.vjp = out + off;
-        } else {
-            a.phi = phi + off * NN;
-            a.phi_ss = NN;
-            a.phi_sj = 1;
-            a.v = v + off * NN;
-            a.vjp = out + off * NN;
-        }
-        a.scratch = scratch;
-        a.sc_ld = chunk;
-        rc = pjg_launch_eval(a, 2, stream);
-        if (rc) {
-            char msg[256];
-            snprintf(msg, sizeof(msg), "pjg_vjp_noalloc: kernel launch failed: %s",
-                     pjg_launch_error_string());
-            return pjg_internal_fail(PJG_ERR_CUDA, msg);
-        }
-        pjg_internal_count_launch();
+    EvalArgs a;
+    int grid = 0;
+    rc = pjg_internal_vjp_args(mech, n, kScratchDoubles, &a, &grid);
+    if (rc) return rc;
+    a.n = n;
+    a.conp = conp;
+    a.param = param;
+    a.phi = phi;
+    a.phi_ss = order == 'F' ? 1 : NN;
+    a.phi_sj = order == 'F' ? n : 1;
+    a.v = v;
+    a.vjp = out;
+    a.scratch = scratch;
+    rc = pjg_launch_tile(a, KIND_VJP, grid, stream);
+    if (rc) {
+        char msg[256];
+        snprintf(msg, sizeof(msg), "pjg_vjp_noalloc: kernel launch failed: %s", pjg_launch_error_string());
+        return pjg_internal_fail(PJG_ERR_CUDA, msg);
     }
+    pjg_internal_count_launch();
     return 0;
 }

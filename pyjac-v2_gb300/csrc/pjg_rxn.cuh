@@ -10,10 +10,16 @@
 // dRopidE :1458-1594, dci_*_dT :2117-2588, dci_*_dE :362-880).
 //
 // The caller owns the accumulation: species rates get nu_k * net, species row
-// k of the Jacobian gets nu_k * (g_j ci) in column j, nu_k * d0 in column T,
-// nu_k * d1 in column E, nu_k * coef_l * X in the columns of the third-body
-// list, and nu_k * (gns ci + cns X) in every species column (the bath-gas
-// terms, gathered per row).
+// k of the Jacobian gets nu_k * (g_j ci) in column j, nu_k * d0 (times V / T) in
+// column T, nu_k * (d1 - net) (constant pressure; else nu_k * d1) in column E,
+// nu_k * coef_l * X in the columns of the third-body list, and
+// nu_k * (gns ci + cns X) in every species column (the bath-gas terms, gathered
+// per row).
+//
+// The temperature derivative of a reaction's Gibbs sum needs no array of its
+// own: d b_k / dT = (h_k / (R T) - 1) / T, so sum nu_k d b_k / dT follows from
+// the reaction's enthalpy dH = sum nu_k h_k (at constant volume, with energies,
+// the -1 drops out), which is also its weight in row T of the Jacobian.
 //
 // Per-state arrays are read through an accessor with operator[] (a strided
 // view of global memory, or a shared-memory pointer).
@@ -61,29 +67,43 @@ struct StateVars {
     double T;       // temperature (unclamped: explicit factors of the Jacobian)
     double Tc;      // T clamped to [100, 10000] K (rate evaluation)
     double logT, Tinv;  // of Tc
+    double ls, tis;     // the same in units of the exponential's table step
     double Tjinv;   // 1 / T
     double V, P;
     double PoRT;    // P / (R T)
     double rt_inv;  // 1 / (R T)
+    double kB, kC;  // T sum nu d b / dT = dH kB - (sum nu) kC
+    double h_ns;    // enthalpy (energy) of the bath gas
     double logP;    // ln P (PLOG / Chebyshev mechanisms only)
     bool conp;
     // every |b_k| <= EvalArgs::kc_split_max = 690 / (the mechanism's largest
-    // sum |nu| of a reversible reaction): 1 / Kc is the product of the
-    // participants' exp(+-b_k) (no partial product past e^690, so the
-    // reference's clamp of sum nu b at 690.78 never acts); else
-    // exp(-sum nu b) per reaction from b_k
+    // sum |nu| of a reversible reaction) and the bath gas's concentration is
+    // not negative: 1 / Kc is the product of the participants' exp(+-b_k) (no
+    // partial product past e^690, so the reference's clamp of sum nu b at
+    // 690.78 never acts); else exp(-sum nu b) per reaction from b_k
     bool split;
     const double* etab;  // fexp table (shared memory)
 };
 
+// the values derived from T, Tc, Tinv and conp; ls is log2(Tc) times a power of
+// two and tis one quotient, so that neither is rounded twice
+template <bool DER>
+__device__ __forceinline__ void set_scaled(StateVars& sv, double lg2T, double tis)
+{
+    sv.ls = __dmul_rn(lg2T, (double)PJG_EXP_TAB);
+    sv.tis = tis;
+    sv.kC = sv.conp ? __dmul_rn(sv.T, sv.Tinv) : 0.0;
+    sv.kB = DER ? __dmul_rn(__dmul_rn(__dmul_rn(sv.T, sv.Tinv), sv.Tinv), 1.0 / RU) : 0.0;
+}
+
 // decoded reaction header
 struct RxnHead {
-    int flags, nsp, thd_off, thd_cnt, auxo, bint, fbint;
+    int flags, nsp, thd_off, thd_cnt, auxo, list, bint, fbint;
     unsigned ent[PJG_MAXSP];
     const double* p;
 };
 
-__device__ __forceinline__ void load_head(const PjgRxn* R, RxnHead& h)
+__device__ __forceinline__ void load_head(const RxnRec* R, RxnHead& h)
 {
     const int4 h0 = __ldg(reinterpret_cast<const int4*>(R));
     const int4 h1 = __ldg(reinterpret_cast<const int4*>(R) + 1);
@@ -92,6 +112,7 @@ __device__ __forceinline__ void load_head(const PjgRxn* R, RxnHead& h)
     h.thd_off = h0.z;
     h.thd_cnt = h0.w;
     h.auxo = h1.x;
+    h.list = h1.y;
     h.bint = h1.z;
     h.fbint = h1.w;
     const uint4 e0 = __ldg(reinterpret_cast<const uint4*>(R) + 2);
@@ -103,12 +124,30 @@ __device__ __forceinline__ void load_head(const PjgRxn* R, RxnHead& h)
 
 struct RxnTerms {
     double net;              // pressure-modified net rate of progress
-    double g[PJG_MAXSP];          // d (rf - rr) / d c_j for participant j
+    double w;                // sum nu_k hw_k, the weight in row T
+    double g[PJG_MAXSP];     // d (rf - rr) / d c_j for participant j
     double gns;              // the same for the bath gas (0 if absent)
     double ci_;              // pressure modification (1 without third body)
-    double d0, d1;           // temperature and extra-variable column terms
+    // temperature column (times V / T) and extra-variable column terms; at
+    // constant pressure the latter without -net, which sums to -wdot over a
+    // row's reactions
+    double d0, d1;
     double X;                // third-body column factor, Rnet d ci / d [M]
 };
+
+// the weight in row T from the reaction's enthalpy: sum over the species rows
+// of nu_k (h_k - h_ns W_k / W_ns), which is sum nu_k h_k where mass is conserved
+__device__ __forceinline__ double row_t_weight(int flags, const double* p, double dH, int nu_sum, double h_ns)
+{
+    return (flags & RX_WEREAL) ? fma(-h_ns, (double)nu_sum - ldg(p + P_WE), dH) : dH;
+}
+
+// T sum nu_k d b_k / dT
+__device__ __forceinline__ double gibbs_slope(const StateVars& sv, double dH, int nu_sum)
+{
+    const double x = __dmul_rn(dH, sv.kB);
+    return nu_sum ? addnu(x, -nu_sum, sv.kC) : x;
+}
 
 // mulpow with rounded products: the rates of progress must not depend on
 // how the compiler contracts them into later FMAs, which differs between the
@@ -161,58 +200,94 @@ __device__ __forceinline__ double inv_kc_split(const RxnHead& h, const ARR& ep, 
     return r;
 }
 
-// [M] of the last third-body reaction evaluated and ln [M] of the last
-// fall-off reaction that formed it: the packing makes reactions with the
-// same [M] adjacent and marks the repeats (RX_SAMEM, RX_SAMELNM)
-struct MCache {
-    double M = 0.0, logM = 0.0;
+// [M] and log10 [M] of the third-body lists that several reactions share
+// (pjg_capi.cu numbers them): from the tile's arrays, formed once per state, ...
+template <class ARR>
+struct MLists {
+    ARR m;
+    int n;
+    template <class FORM>
+    __device__ __forceinline__ double conc(int l, FORM&&)
+    {
+        return m[l];
+    }
+    __device__ __forceinline__ double log10(int l, double) { return m[n + l]; }
+};
+// ... or kept from the last reaction (the packing lets them follow one another)
+struct MLast {
+    int list = -1, list_log = -1;
+    double M = 0.0, lgM = 0.0;
+    template <class FORM>
+    __device__ __forceinline__ double conc(int l, FORM&& form)
+    {
+        if (l != list) {
+            M = form();
+            list = l;
+        }
+        return M;
+    }
+    __device__ __forceinline__ double log10(int l, double m)
+    {
+        if (l != list_log) {
+            lgM = __dmul_rn(log(m), INV_LN10);
+            list_log = l;
+        }
+        return lgM;
+    }
 };
 
 struct FallState {
     double Pr, Fi, A, B, Fc, lnFc, X, lnQ, kratio, logPr;
+    double inv1, ci0, rabs;  // 1 / (1 + Pr), Fi / (1 + Pr), Troe 1 / (A^2 + B^2)
     double e1, e2, e3;  // Troe exponentials at the clamped temperature
 };
 
-template <bool DER, class ST = RunStoich, class ARR>
+template <bool DER, class ST = RunStoich, class ARR, class ML>
 __device__ __forceinline__ void rxn_terms(const RxnHead& h, const double* aux,
                                           const int* thd_spec, const double* thd_coef, int last,
                                           const StateVars& sv, const ARR& conc, const ARR& bk,
-                                          const ARR& ep, const ARR& em, const ARR& db, MCache& mc,
-                                          RxnTerms& o)
+                                          const ARR& ep, const ARR& em, const ARR& hk,
+                                          ML& ml, RxnTerms& o)
 {
     const int flags = h.flags, nsp = ST::nsp(h);
     const double* p = h.p;
     const int form = RX_FORM(flags);
     const bool rev = flags & RX_REV;
-    const double Tc = sv.Tc, logT = sv.logT, Tinv = sv.Tinv, Tjinv = sv.Tjinv;
+    const double Tc = sv.Tc, Tjinv = sv.Tjinv;
     const double* et = sv.etab;
 
-    // forward rate constant and its log-derivatives
-    double kf, dlnkf_dT = 0.0, dlnkf_dlnP = 0.0, lnkf = 0.0;
+    // forward rate constant and its log-derivatives (dl: T d ln kf / dT)
+    double kf, dl = 0.0, dlnkf_dlnP = 0.0, lnkf = 0.0;
     bool has_lnkf = false;
     if (form <= FORM_ARR) {
-        kf = arrhenius_ln(form, ldg(p + P_A), ldg(p + P_B), ldg(p + P_TA), h.bint, Tc, logT, Tinv,
-                          et, lnkf, has_lnkf);
-        if (DER) dlnkf_dT = (ldg(p + P_B) + ldg(p + P_TA) * Tjinv) * Tjinv;
+        kf = arrhenius(form, ldg(p + P_A), h.bint, ldg(p + P_B), ldg(p + P_TA), Tc, sv.Tinv, sv.ls, sv.tis,
+                       et, lnkf, has_lnkf);
+        if (DER) dl = fma(ldg(p + P_TA), Tjinv, ldg(p + P_B));
     } else if (form == FORM_PLOG) {
-        kf = gexp(plog_logk(aux + h.auxo, logT, Tinv, sv.logP, Tjinv, &dlnkf_dT, &dlnkf_dlnP), et);
+        kf = gexp(plog_logk(aux + h.auxo, sv.logT, sv.Tinv, sv.logP, Tjinv, &dl, &dlnkf_dlnP), et);
+        dl *= sv.T;
     } else {
-        const double l10 = cheb_log10k(aux + h.auxo, Tinv, sv.logP, Tjinv, &dlnkf_dT, &dlnkf_dlnP);
+        const double l10 = cheb_log10k(aux + h.auxo, sv.Tinv, sv.logP, Tjinv, &dl, &dlnkf_dlnP);
         kf = fexp(LN10 * min_pos(EXP_MAX, l10), et);
-        dlnkf_dT *= LN10;
+        dl *= LN10 * sv.T;
         dlnkf_dlnP *= LN10;
     }
-    // reverse rate: kr = kf / Kc, Kc = (P_atm/R)^nu_sum exp(sum nu b)
-    double kr = 0.0, dB = 0.0;
-    if (rev) {
-        if (DER) {
+    // reaction enthalpy; reverse rate: kr = kf / Kc, Kc = (P_atm/R)^nu_sum exp(sum nu b)
+    int nu_sum = 0;
+    double dH = 0.0;
+    if (DER) {
 #pragma unroll
-            for (int e = 0; e < PJG_MAXSP; ++e) {
-                if (e >= nsp) break;
-                const int nu = ST::nur(h, e) - ST::nuf(h, e);
-                if (nu != 0) dB = addnu(dB, nu, db[ent_spec(h.ent[e])]);
-            }
+        for (int e = 0; e < PJG_MAXSP; ++e) {
+            if (e >= nsp) break;
+            const int nu = ST::nur(h, e) - ST::nuf(h, e);
+            if (nu == 0) continue;
+            nu_sum += nu;
+            dH = addnu(dH, nu, hk[ent_spec(h.ent[e])]);
         }
+        o.w = row_t_weight(flags, p, dH, nu_sum, sv.h_ns);
+    }
+    double kr = 0.0;
+    if (rev) {
         double ikc;
         if (sv.split) {
             ikc = inv_kc_split<ST>(h, ep, em);
@@ -226,7 +301,7 @@ __device__ __forceinline__ void rxn_terms(const RxnHead& h, const double* aux,
             }
             ikc = fexp(-min_pos(EXP_MAX, Bsum), et);
         }
-        kr = kf * ldg(p + P_PSUM) * ikc;
+        kr = __dmul_rn(__dmul_rn(kf, ldg(p + P_PSUM)), ikc);
     }
     // rates of progress (mass action on raw concentrations)
     double rf = kf, rr = kr;
@@ -245,82 +320,86 @@ __device__ __forceinline__ void rxn_terms(const RxnHead& h, const double* aux,
     FallState fs;
     fs.Pr = 0.0; fs.Fi = 1.0; fs.A = 0.0; fs.B = 0.0; fs.Fc = 1.0; fs.lnFc = 0.0; fs.X = 0.0;
     fs.lnQ = 0.0; fs.kratio = 0.0; fs.e1 = 0.0; fs.e2 = 0.0; fs.e3 = 0.0; fs.logPr = 0.0;
+    fs.inv1 = 0.0; fs.ci0 = 0.0; fs.rabs = 0.0;
     if (thd) {
-        if (flags & RX_SAMEM) {
-            M = mc.M;
-        } else {
-            M = sv.PoRT * ldg(p + P_FLAG);
+        auto form_m = [&]() -> double {
+            double m = sv.PoRT * ldg(p + P_FLAG);
             for (int l = 0; l < h.thd_cnt; ++l)
-                M = fma(__ldg(thd_coef + h.thd_off + l), conc[__ldg(thd_spec + h.thd_off + l)], M);
-            mc.M = M;
-        }
+                m = fma(__ldg(thd_coef + h.thd_off + l), conc[__ldg(thd_spec + h.thd_off + l)], m);
+            return m;
+        };
+        M = h.list >= 0 ? ml.conc(h.list, form_m) : form_m();
         if (blend == BL_NONE) {
             ci = M;
         } else {
-            double lnkfall = 0.0;
-            bool has_lnkfall = false;
-            const double kfall = arrhenius_ln(RX_FFORM(flags), ldg(p + P_FA), ldg(p + P_FB),
-                                              ldg(p + P_FTA), h.fbint, Tc, logT, Tinv, et,
-                                              lnkfall, has_lnkfall);
-            fs.kratio = chem ? kf / kfall : kfall / kf;  // k0 / kinf
-            fs.Pr = M * fs.kratio;
-            // log10 Pr: ln [M] (formed once per run of reactions sharing [M])
-            // + ln k0 - ln kinf where both rate constants are exponentials
-            // (the packing's rule for RX_SAMELNM) and Pr >= 1e-300; else the
-            // logarithm of the guarded Pr
+            // k0 / kinf, in one exponential where both are, and its logarithm
+            double lnr = 0.0;
+            bool has_lnr = flags & RX_RATIO;
+            if (has_lnr) {
+                lnr = fma(-ldg(p + P_RTA), sv.tis, fma(ldg(p + P_RB), sv.ls, ldg(p + P_RA)));
+                fs.kratio = fexp_s(lnr, h.fbint, et);
+                lnr = __dadd_rn(lnr, ldg(p + P_RN));
+            } else {
+                double lnkfall = 0.0;
+                bool has_lnkfall = false;
+                const double kfall = arrhenius(RX_FFORM(flags), ldg(p + P_FA), h.fbint, ldg(p + P_FB),
+                                               ldg(p + P_FTA), Tc, sv.Tinv, sv.ls, sv.tis, et, lnkfall, has_lnkfall);
+                fs.kratio = chem ? kf / kfall : kfall / kf;
+            }
+            fs.Pr = __dmul_rn(M, fs.kratio);
+            fs.inv1 = 1.0 / __dadd_rn(1.0, fs.Pr);
+            // log10 Pr from the logarithms where k0 / kinf is one exponential and
+            // Pr >= 1e-300; else the logarithm of the guarded Pr
             if (blend == BL_TROE || blend == BL_SRI) {
-                double lnPr;
-                if (has_lnkf && has_lnkfall) {
-                    if (!(flags & RX_SAMELNM)) mc.logM = log(M);
-                    lnPr = __double_as_longlong(fs.Pr) >= __double_as_longlong(SMALL)
-                               ? mc.logM + (chem ? lnkf - lnkfall : lnkfall - lnkf)
-                               : log(SMALL);
+                if (has_lnr && __double_as_longlong(fs.Pr) >= __double_as_longlong(SMALL)) {
+                    const double lgM = h.list >= 0 ? ml.log10(h.list, M) : __dmul_rn(log(M), INV_LN10);
+                    fs.logPr = fma(lnr, kExpStep * INV_LN10, lgM);
                 } else {
-                    lnPr = log(gsmall(fs.Pr));
+                    fs.logPr = __dmul_rn(log(gsmall(fs.Pr)), INV_LN10);
                 }
-                fs.logPr = lnPr * INV_LN10;
             }
             if (blend == BL_TROE) {
                 const double logPr = fs.logPr;
-                const double ta = ldg(p + P_F0);
-                fs.e1 = gexp(-1.0 * Tc * ldg(p + P_F1), et);
-                fs.e3 = gexp(-1.0 * Tc * ldg(p + P_F3), et);
-                double Fc = ta * fs.e1 + (1.0 + -1.0 * ta) * fs.e3;
+                const double ta = ldg(p + P_F0), tcs = -(Tc * kExpScale);
+                fs.e1 = fexp_s(__dmul_rn(tcs, ldg(p + P_F1)), 0, et);
+                fs.e3 = fexp_s(__dmul_rn(tcs, ldg(p + P_F3)), 0, et);
+                double Fc = fma(ta, fs.e1, __dmul_rn(1.0 - ta, fs.e3));
                 if (flags & RX_T2) {
-                    fs.e2 = gexp(-1.0 * ldg(p + P_F2) * Tinv, et);
-                    Fc = Fc + fs.e2;
+                    fs.e2 = fexp_s(__dmul_rn(-ldg(p + P_F2), sv.tis), 0, et);
+                    Fc = __dadd_rn(Fc, fs.e2);
                 }
                 fs.lnFc = log(gsmall(Fc));
-                const double logFc = fs.lnFc * INV_LN10;
-                fs.B = -1.1762 * logFc + -0.14 * logPr + 0.806;
-                fs.A = -0.67 * logFc + logPr + -0.4;
+                const double logFc = __dmul_rn(fs.lnFc, INV_LN10);
+                fs.B = fma(-1.1762, logFc, fma(-0.14, logPr, 0.806));
+                fs.A = fma(-0.67, logFc, __dsub_rn(logPr, 0.4));
                 fs.Fc = Fc;
-                const double B2 = fs.B * fs.B;
-                fs.Fi = fexp(B2 / (fs.A * fs.A + B2) * fs.lnFc, et);
+                const double B2 = __dmul_rn(fs.B, fs.B);
+                fs.rabs = 1.0 / fma(fs.A, fs.A, B2);
+                fs.Fi = fexp_s(__dmul_rn(__dmul_rn(B2, fs.rabs), __dmul_rn(fs.lnFc, kExpScale)), 0, et);
             } else if (blend == BL_SRI) {
                 const double logPr = fs.logPr;
-                fs.X = 1.0 / (logPr * logPr + 1.0);
-                fs.e1 = gexp(-ldg(p + P_F1) * Tinv, et);
+                fs.X = 1.0 / fma(logPr, logPr, 1.0);
+                fs.e1 = fexp_s(__dmul_rn(-ldg(p + P_F1), sv.tis), 0, et);
                 fs.e3 = gexp(-Tc / ldg(p + P_F2), et);
-                const double Q = ldg(p + P_F0) * fs.e1 + fs.e3;
+                const double Q = fma(ldg(p + P_F0), fs.e1, fs.e3);
                 fs.lnQ = log(Q);
-                double Fi = fexp(fs.X * fs.lnQ, et);
-                if (flags & RX_SRID) Fi = Fi * ldg(p + P_F3);
+                double Fi = fexp(__dmul_rn(fs.X, fs.lnQ), et);
+                if (flags & RX_SRID) Fi = __dmul_rn(Fi, ldg(p + P_F3));
                 if (flags & RX_SRIE) {
                     const double e = ldg(p + P_F4);
                     const int ie = (int)e;
-                    Fi = Fi * ((flags & RX_SRIEINT) ? (ie < 0 ? powi(Tinv, -ie) : powi(Tc, ie))
-                                                    : pow(Tc, e));
+                    Fi = __dmul_rn(Fi, (flags & RX_SRIEINT) ? (ie < 0 ? powi(sv.Tinv, -ie) : powi(Tc, ie))
+                                                            : pow(Tc, e));
                 }
                 fs.Fi = Fi;
             }
-            ci = fs.Fi / (1.0 + fs.Pr);
-            if (!chem) ci = ci * fs.Pr;
+            fs.ci0 = __dmul_rn(fs.Fi, fs.inv1);
+            ci = chem ? fs.ci0 : __dmul_rn(fs.ci0, fs.Pr);
         }
     }
     double Rnet = rf;
     if (rev) Rnet = __dsub_rn(Rnet, rr);
-    o.net = thd ? Rnet * ci : Rnet;
+    o.net = thd ? __dmul_rn(Rnet, ci) : Rnet;
     if (!DER) return;
 
     const double T = sv.T, V = sv.V, P = sv.P, PoRT = sv.PoRT, rt_inv = sv.rt_inv;
@@ -360,38 +439,33 @@ __device__ __forceinline__ void rxn_terms(const RxnHead& h, const double* aux,
     o.gns = gns;
     const double ci_ = thd ? ci : 1.0;
     o.ci_ = ci_;
-    // fall-off derivative pieces shared by the n, T and E columns
-    double inv1 = 0.0, dlnFi_dPr = 0.0;
-    if (thd && blend != BL_NONE) {
-        inv1 = 1.0 / (fs.Pr + 1.0);
-        if (blend == BL_TROE) {
-            const double absq = fs.A * fs.A + fs.B * fs.B;
-            dlnFi_dPr = -2.0 * fs.A * fs.B * fs.lnFc * (0.14 * fs.A + fs.B) /
-                        (gsmall(fs.Pr) * absq * absq * LN10);
-        } else if (blend == BL_SRI) {
-            dlnFi_dPr = -2.0 * fs.X * fs.X * fs.logPr / (gsmall(fs.Pr) * LN10) * fs.lnQ;
-        }
-    }
-    // d ci / dx given d Pr / dx = Pr theta + theta_n and the direct part of d ln Fi / dx
-    auto dci = [&](double theta, double theta_n, double direct) -> double {
-        const double dPr = fs.Pr * theta + theta_n;
-        double d = ci * (dlnFi_dPr * dPr + direct - dPr * inv1);
-        if (!chem) d = d + theta * ci + fs.Fi * theta_n * inv1;
-        return d;
+    // Fall-off derivative shared by the n, T and E columns: d ci / dx given
+    // d Pr / dx and the direct part of d ln Fi / dx.  With dlnF = d ln Fi / d ln Pr
+    // and ci = Fi Pr / (1 + Pr), d ci = Fi / (1 + Pr) (d Pr (1 / (1 + Pr) + dlnF)
+    // + Pr direct); chemically activated, ci = Fi / (1 + Pr).
+    double dlnF = 0.0;
+    const bool fall = thd && blend != BL_NONE;
+    if (blend == BL_TROE)
+        dlnF = -2.0 * fs.A * fs.B * fs.lnFc * fma(0.14, fs.A, fs.B) * INV_LN10 * (fs.rabs * fs.rabs);
+    else if (blend == BL_SRI)
+        dlnF = -2.0 * INV_LN10 * fs.X * fs.X * fs.logPr * fs.lnQ;
+    const double slope = chem ? dlnF / gsmall(fs.Pr) - fs.inv1 : dlnF + fs.inv1;
+    auto dci = [&](double dPr, double direct) -> double {
+        return fs.ci0 * fma(dPr, slope, chem ? direct : fs.Pr * direct);
     };
-    const double dMfac = (thd && blend != BL_NONE) ? dci(0.0, fs.kratio, 0.0) : 1.0;
+    const double dMfac = fall ? fs.ci0 * (fs.kratio * slope) : 1.0;
     o.X = Rnet * dMfac;
     const double mod = ldg(p + P_MOD);
     const bool hasns = flags & RX_HASNS;
-    // temperature column (dRopi_dT :2589-3108, dci_*_dT :2117-2588)
-    // rf dlnkf - rr (dlnkf - dB) = Rnet dlnkf + rr dB
-    double d0 = rev ? fma(rr, dB, Rnet * dlnkf_dT) : rf * dlnkf_dT;
-    d0 = d0 * ci_ * V;
-    if (hasns) d0 += -gns * V * ci_ * PoRT * Tjinv;
+    // temperature column times T / V (dRopi_dT :2589-3108, dci_*_dT :2117-2588):
+    // rf dl - rr (dl - T dB) = Rnet dl + rr T dB
+    double d0 = rev ? fma(rr, gibbs_slope(sv, dH, nu_sum), Rnet * dl) : rf * dl;
+    d0 = d0 * ci_;
+    if (hasns) d0 = fma(-gns * ci_, PoRT, d0);
     // extra-variable column (dRopi_dE :1458-1594, dci_*_dE :362-880)
     double d1 = 0.0;
     if (conp) {
-        int nuf = -1, nur = -1;
+        int nuf = -2, nur = -2;
 #pragma unroll
         for (int e = 0; e < PJG_MAXSP; ++e) {
             if (e >= nsp) break;
@@ -402,52 +476,54 @@ __device__ __forceinline__ void rxn_terms(const RxnHead& h, const double* aux,
     } else if (form >= FORM_PLOG) {
         d1 = V * ci_ * Rnet * dlnkf_dlnP / P;
     }
-    if (hasns) d1 += gns * ci_ * (conp ? PoRT : V * rt_inv);
+    if (hasns) d1 = fma(__dmul_rn(gns, ci_), conp ? PoRT : __dmul_rn(V, rt_inv), d1);
     if (thd) {
-        const double dM = -1.0 * PoRT * mod * Tjinv;
+        const double dM = -PoRT * mod;  // T d [M] / dT
         if (blend == BL_NONE) {
-            d0 += dM * V * Rnet;
+            d0 = fma(dM, Rnet, d0);
             if (conp) {
-                if (thd != THD_UNITY) d1 += (mod * PoRT + -1.0 * M) * Rnet;
+                if (thd != THD_UNITY) d1 = fma(fma(mod, PoRT, -M), Rnet, d1);
             } else {
-                d1 += V * Rnet * mod * rt_inv;
+                d1 = fma(__dmul_rn(V, Rnet), __dmul_rn(mod, rt_inv), d1);
             }
         } else {
-            double b0, binf, Ta0, Tainf;
-            if (!chem) {
-                binf = ldg(p + P_B); Tainf = ldg(p + P_TA);
-                b0 = ldg(p + P_FB); Ta0 = ldg(p + P_FTA);
+            double Rb, RTa;
+            if (flags & RX_RATIO) {
+                Rb = ldg(p + P_RB);
+                RTa = ldg(p + P_RTA);
             } else {
-                b0 = ldg(p + P_B); Ta0 = ldg(p + P_TA);
-                binf = ldg(p + P_FB); Tainf = ldg(p + P_FTA);
+                Rb = ldg(p + P_FB) - ldg(p + P_B);
+                RTa = ldg(p + P_FTA) - ldg(p + P_TA);
+                if (chem) {
+                    Rb = -Rb;
+                    RTa = -RTa;
+                }
             }
-            const double theta = Tjinv * (b0 + -1.0 * binf + (Ta0 + -1.0 * Tainf) * Tjinv);
-            const double theta_n = dM * fs.kratio;
-            double direct = 0.0;
+            const double theta = fma(RTa, Tjinv, Rb);  // T d ln (k0 / kinf) / dT
+            double direct = 0.0;  // T times the explicit part
             if (blend == BL_TROE) {
-                const double absq = fs.A * fs.A + fs.B * fs.B;
+                const double absq = fma(fs.A, fs.A, fs.B * fs.B);
                 const double ta = ldg(p + P_F0), t1 = ldg(p + P_F1), t2 = ldg(p + P_F2),
                              t3 = ldg(p + P_F3);
                 // the explicit T derivative uses the unclamped T, as the reference
                 const bool same = T == Tc;
                 const double x1 = same ? fs.e1 : gexp(-1.0 * T * t1, et);
                 const double x3 = same ? fs.e3 : gexp(-1.0 * T * t3, et);
-                double dFc = -1.0 * ta * t1 * x1 + (ta + -1.0) * t3 * x3;
-                if (flags & RX_T2)
-                    dFc += t2 * Tjinv * Tjinv * (same ? fs.e2 : gexp(-1.0 * t2 * Tjinv, et));
+                double dFc = T * ((ta - 1.0) * t3 * x3 - ta * t1 * x1);
+                if (flags & RX_T2) dFc = fma(t2 * Tjinv, same ? fs.e2 : gexp(-1.0 * t2 * Tjinv, et), dFc);
                 direct = -fs.B * dFc *
-                         (2.0 * fs.A * (1.1762 * fs.A + -0.67 * fs.B) * fs.lnFc - fs.B * absq * LN10) /
-                         (fs.Fc * absq * absq * LN10);
+                         (2.0 * fs.A * (1.1762 * fs.A + -0.67 * fs.B) * fs.lnFc - fs.B * absq * LN10) *
+                         (fs.rabs * fs.rabs * INV_LN10) / fs.Fc;
             } else if (blend == BL_SRI) {
                 const double sa = ldg(p + P_F0), sb = ldg(p + P_F1), sc = ldg(p + P_F2);
-                const double Q = sa * fs.e1 + fs.e3;
-                const double dQ = sa * sb * Tjinv * Tjinv * fs.e1 - fs.e3 / sc;
-                direct = fs.X * dQ / Q + ldg(p + P_F4) * Tjinv;
+                const double Q = fma(sa, fs.e1, fs.e3);
+                const double dQ = sa * sb * Tjinv * fs.e1 - T * fs.e3 / sc;
+                direct = fs.X * dQ / Q + ldg(p + P_F4);
             }
-            d0 += dci(theta, theta_n, direct) * V * Rnet;
+            d0 = fma(dci(fma(fs.Pr, theta, dM * fs.kratio), direct), Rnet, d0);
             const double modp = (conp ? (thd == THD_UNITY ? 0.0 : mod) * PoRT : mod * rt_inv) * fs.kratio;
-            const double th = conp ? -1.0 * (thd != THD_UNITY) : 0.0;
-            d1 += dci(th, modp, 0.0) * (conp ? 1.0 : V) * Rnet;
+            const double dPr = conp && thd != THD_UNITY ? modp - fs.Pr : modp;
+            d1 = fma(dci(dPr, 0.0) * (conp ? 1.0 : V), Rnet, d1);
         }
     }
     o.d0 = d0;
@@ -467,7 +543,7 @@ struct E22Head {
     const double* p;
 };
 
-__device__ __forceinline__ void load_e22(const PjgRxn* R, E22Head& h)
+__device__ __forceinline__ void load_e22(const RxnRec* R, E22Head& h)
 {
     const int4 h0 = __ldg(reinterpret_cast<const int4*>(R));
     const int4 h1 = __ldg(reinterpret_cast<const int4*>(R) + 1);
@@ -483,72 +559,81 @@ __device__ __forceinline__ void load_e22(const PjgRxn* R, E22Head& h)
 
 struct E22Terms {
     double net;   // rate of progress
+    double w;     // weight in row T
     double g[4];  // d net / d c_j of the four participants
     double gns;   // the same for the bath gas (0 if it does not take part)
     double d0, d1;
 };
 
-// the per-state values one elementary reaction reads (loaded ahead of use):
-// concentrations, the 1 / Kc factors exp(b) of the reactants and exp(-b) of
-// the products (in a split state; else the four b), d b / dT
+// the per-state values an elementary reaction reads: concentrations, the 1 / Kc
+// factors exp(b) of the reactants and exp(-b) of the products (where the state
+// is not split, the four b), enthalpies
 struct E22Vals {
-    double c[4], x[4], db[4];
+    double c[4], x[4], h[4];
 };
 
 template <bool DER, class ARR>
-__device__ __forceinline__ void e22_fetch(const E22Head& h, bool split, const ARR& conc,
-                                          const ARR& ep, const ARR& em, const ARR& db, E22Vals& v)
+__device__ __forceinline__ void e22_fetch(const E22Head& h, bool split, const ARR& conc, const ARR& ep,
+                                          const ARR& em, const ARR& hk, E22Vals& v)
 {
 #pragma unroll
     for (int q = 0; q < 4; ++q) {
         v.c[q] = conc[h.s[q]];
         v.x[q] = (q < 2 || !split) ? ep[h.s[q]] : em[h.s[q]];  // ep holds b if !split
-        if (DER) v.db[q] = db[h.s[q]];
+        if (DER) v.h[q] = hk[h.s[q]];
     }
 }
 
+// The derivatives by one participant are the partial products of the rates of
+// progress.  Rounded products and one FMA for the difference, the same in every
+// kernel kind: the Jacobian's rates equal the rates kernel's bit for bit.
 template <bool DER>
-__device__ __forceinline__ void e22_terms_v(const E22Head& h, const E22Vals& vv, int last,
-                                            const StateVars& sv, E22Terms& o)
+__device__ __forceinline__ void e22_terms(const E22Head& h, const E22Vals& v, int last, const StateVars& sv,
+                                          E22Terms& o)
 {
     const double* p = h.p;
     const double b = ldg(p + P_B), Ta = ldg(p + P_TA);
-    const double kf = arrhenius(RX_FORM(h.flags), ldg(p + P_A), b, Ta, h.bint, sv.Tc, sv.logT,
-                                sv.Tinv, sv.etab);
+    double lnk;
+    bool has_ln;
+    const double kf = arrhenius(RX_FORM(h.flags), ldg(p + P_A), h.bint, b, Ta, sv.Tc, sv.Tinv, sv.ls, sv.tis,
+                                sv.etab, lnk, has_ln);
     double ikc;  // 1 / Kc = exp(-sum nu b)
     if (sv.split) {
-        ikc = __dmul_rn(__dmul_rn(vv.x[0], vv.x[1]), __dmul_rn(vv.x[2], vv.x[3]));
+        ikc = __dmul_rn(__dmul_rn(v.x[0], v.x[1]), __dmul_rn(v.x[2], v.x[3]));
     } else {
-        const double Bsum = (vv.x[2] + vv.x[3]) - (vv.x[0] + vv.x[1]);
+        const double Bsum = (v.x[2] + v.x[3]) - (v.x[0] + v.x[1]);
         ikc = fexp(-min_pos(EXP_MAX, Bsum), sv.etab);
     }
-    const double kr = kf * ikc;
-    const double c0 = vv.c[0], c1 = vv.c[1], c2 = vv.c[2], c3 = vv.c[3];
-    // rounded products and difference (no contraction into an FMA): the rate
-    // of progress must be the same in every kernel kind, whatever else uses
-    // rf and rr (the Jacobian's rates equal the rates kernel's bit for bit)
-    const double rf = __dmul_rn(__dmul_rn(kf, c0), c1), rr = __dmul_rn(__dmul_rn(kr, c2), c3);
-    o.net = __dsub_rn(rf, rr);
+    const double kr = __dmul_rn(kf, ikc);
+    const double f1 = __dmul_rn(kf, v.c[0]), f2 = __dmul_rn(kr, v.c[2]);
+    const double rr = __dmul_rn(f2, v.c[3]);
+    o.net = fma(f1, v.c[1], negi(rr));
     if (!DER) return;
-    const double dlnkf_dT = (b + Ta * sv.Tjinv) * sv.Tjinv;
-    const double dB = (vv.db[2] + vv.db[3]) - (vv.db[0] + vv.db[1]);
-    o.g[0] = kf * gsmall(c1);
-    o.g[1] = kf * gsmall(c0);
-    o.g[2] = -(kr * gsmall(c3));
-    o.g[3] = -(kr * gsmall(c2));
+    if (sv.split) {
+        o.g[0] = __dmul_rn(kf, v.c[1]);
+        o.g[1] = f1;
+        o.g[2] = negi(__dmul_rn(kr, v.c[3]));
+        o.g[3] = negi(f2);
+    } else {  // a concentration may be negative here
+        o.g[0] = __dmul_rn(kf, gsmall(v.c[1]));
+        o.g[1] = __dmul_rn(kf, gsmall(v.c[0]));
+        o.g[2] = negi(__dmul_rn(kr, gsmall(v.c[3])));
+        o.g[3] = negi(__dmul_rn(kr, gsmall(v.c[2])));
+    }
+    const double dH = (v.h[2] + v.h[3]) - (v.h[0] + v.h[1]);
+    o.w = row_t_weight(h.flags, p, dH, 0, sv.h_ns);
     double gns = 0.0;
 #pragma unroll
     for (int j = 0; j < 4; ++j)
         if (h.s[j] == last) gns = o.g[j];
     o.gns = gns;
-    const bool hasns = h.flags & RX_HASNS;
-    // rf dlnkf - rr (dlnkf - dB) = net dlnkf + rr dB
-    double d0 = fma(rr, dB, o.net * dlnkf_dT) * sv.V;
-    if (hasns) d0 += -gns * sv.V * sv.PoRT * sv.Tjinv;
-    double d1 = sv.conp ? -rf + rr : 0.0;
-    if (hasns) d1 += gns * (sv.conp ? sv.PoRT : sv.V * sv.rt_inv);
-    o.d0 = d0;
-    o.d1 = d1;
+    // rf dl - rr (dl - T dB) = net dl + rr T dB
+    o.d0 = fma(rr, __dmul_rn(dH, sv.kB), __dmul_rn(o.net, fma(Ta, sv.Tjinv, b)));
+    o.d1 = 0.0;
+    if (h.flags & RX_HASNS) {
+        o.d0 = fma(negi(gns), sv.PoRT, o.d0);
+        o.d1 = __dmul_rn(gns, sv.conp ? sv.PoRT : __dmul_rn(sv.V, sv.rt_inv));
+    }
 }
 
 // ------------------------------------------------------------------------
@@ -606,7 +691,7 @@ __device__ __forceinline__ double mulpow_rn(double acc, double v)
 }
 
 struct MaTerms {
-    double net;
+    double net, w;
     double g[5];
     double gns;
     double d0, d1;
@@ -615,13 +700,15 @@ struct MaTerms {
 template <class PT, bool DER, class ARR>
 __device__ __forceinline__ void ma_terms(const RxnHead& h, int last, const StateVars& sv,
                                          const ARR& conc, const ARR& bk, const ARR& ep,
-                                         const ARR& em, const ARR& db, MaTerms& o)
+                                         const ARR& em, const ARR& hk, MaTerms& o)
 {
     constexpr int N = PT::n;
     const double* p = h.p;
     const double b = ldg(p + P_B), Ta = ldg(p + P_TA);
-    const double kf = arrhenius(RX_FORM(h.flags), ldg(p + P_A), b, Ta, h.bint, sv.Tc, sv.logT,
-                                sv.Tinv, sv.etab);
+    double lnk;
+    bool has_ln;
+    const double kf = arrhenius(RX_FORM(h.flags), ldg(p + P_A), h.bint, b, Ta, sv.Tc, sv.Tinv, sv.ls, sv.tis,
+                                sv.etab, lnk, has_ln);
     int sp[N];
     double c[N];
 #pragma unroll
@@ -629,23 +716,27 @@ __device__ __forceinline__ void ma_terms(const RxnHead& h, int last, const State
         sp[e] = ent_spec(h.ent[e]);
         c[e] = conc[sp[e]];
     }
-    double kr = 0.0, dB = 0.0;
-    if (PT::rev) {
-        // the first term starts the sums (no addition to zero)
-        bool first = true;
+    constexpr int nu_sum = PT::sumr() - PT::sumf();
+    double dH = 0.0;
+    if (DER) {
+        bool first = true;  // the first term starts the sum
 #pragma unroll
         for (int e = 0; e < N; ++e) {
             const int nu = PT::nur(e) - PT::nuf(e);
-            if (nu == 0 || !DER) continue;
-            dB = first ? nux(nu, db[sp[e]]) : addnu(dB, nu, db[sp[e]]);
+            if (nu == 0) continue;
+            dH = first ? nux(nu, hk[sp[e]]) : addnu(dH, nu, hk[sp[e]]);
             first = false;
         }
+        o.w = row_t_weight(h.flags, p, dH, nu_sum, sv.h_ns);
+    }
+    double kr = 0.0;
+    if (PT::rev) {
         double ikc;
         if (sv.split) {
             ikc = inv_kc_split<PatStoich<PT>>(h, ep, em);
         } else {
             double Bsum = 0.0;
-            first = true;
+            bool first = true;
 #pragma unroll
             for (int e = 0; e < N; ++e) {
                 const int nu = PT::nur(e) - PT::nuf(e);
@@ -655,7 +746,7 @@ __device__ __forceinline__ void ma_terms(const RxnHead& h, int last, const State
             }
             ikc = fexp(-min_pos(EXP_MAX, Bsum), sv.etab);
         }
-        kr = kf * ldg(p + P_PSUM) * ikc;
+        kr = __dmul_rn(__dmul_rn(kf, ldg(p + P_PSUM)), ikc);
     }
     // rounded products and difference: the rate of progress is the same in
     // every kernel kind (see e22_terms)
@@ -669,7 +760,7 @@ __device__ __forceinline__ void ma_terms(const RxnHead& h, int last, const State
     }
     o.net = PT::rev ? __dsub_rn(rf, rr) : rf;
     if (!DER) return;
-    const double dlnkf_dT = (b + Ta * sv.Tjinv) * sv.Tjinv;
+    const double dl = fma(Ta, sv.Tjinv, b);
     double cg[N];
 #pragma unroll
     for (int e = 0; e < N; ++e) cg[e] = gsmall(c[e]);
@@ -702,12 +793,12 @@ __device__ __forceinline__ void ma_terms(const RxnHead& h, int last, const State
     }
     o.gns = gns;
     const bool hasns = h.flags & RX_HASNS;
-    // rf dlnkf - rr (dlnkf - dB) = net dlnkf + rr dB
-    double d0 = (PT::rev ? fma(rr, dB, o.net * dlnkf_dT) : rf * dlnkf_dT) * sv.V;
-    if (hasns) d0 += -gns * sv.V * sv.PoRT * sv.Tjinv;
+    // rf dl - rr (dl - T dB) = net dl + rr T dB
+    double d0 = PT::rev ? fma(rr, gibbs_slope(sv, dH, nu_sum), o.net * dl) : rf * dl;
+    if (hasns) d0 = fma(negi(gns), sv.PoRT, d0);
     double d1 = 0.0;
-    if (sv.conp) d1 = -nux(PT::sumf() - 1, rf) + (PT::rev ? nux(PT::sumr() - 1, rr) : 0.0);
-    if (hasns) d1 += gns * (sv.conp ? sv.PoRT : sv.V * sv.rt_inv);
+    if (sv.conp) d1 = -nux(PT::sumf() - 2, rf) + (PT::rev ? nux(PT::sumr() - 2, rr) : 0.0);
+    if (hasns) d1 = fma(gns, sv.conp ? sv.PoRT : __dmul_rn(sv.V, sv.rt_inv), d1);
     o.d0 = d0;
     o.d1 = d1;
 }

@@ -53,6 +53,11 @@
 // set by the library's packing (pjg_capi.cu), clear in the tables it is given:
 #define RX_SAMEM (1 << 20)    // [M] equals the previous packed reaction's (same group)
 #define RX_SAMELNM (1 << 21)  // and ln [M] was formed by an earlier reaction of that run
+// device records (RxnRec) only:
+#define RX_E22 (1 << 22)      // of the elementary class A + B <=> C + D
+#define RX_WE (1 << 23)       // the weight in row E, sum nu_k (1 - W_k / W_ns), is not zero
+#define RX_WEREAL (1 << 24)   // and not sum nu (mass not conserved): it is P_WE
+#define RX_RATIO (1 << 25)    // k0 / kinf is one exponential (P_RA..): both are FORM_ARR
 
 #define RX_FORM(f) ((f) & RX_FORM_MASK)
 #define RX_THD(f) (((f) >> RX_THD_SHIFT) & 3)
@@ -87,6 +92,22 @@ struct __align__(16) PjgRxn {
     double p[16];
 };
 static_assert(sizeof(PjgRxn) == PJG_RXN_BYTES, "reaction record size");
+
+// The record as the kernels read it, formed by the library (pjg_capi.cu).
+// Exponents are in units of ln 2 / 1024 (the exponential's table step) and cut
+// into an integer and a rest of at most 1/2, which keeps ln A exact: for
+// FORM_ARR, ln A = (bint + p[P_A]) ln 2 / 1024.
+#define P_WE 15    // sum nu_k (1 - W_k / W_ns)
+#define P_RA 16    // RX_RATIO: rest of ln (A0 / Ainf), its integer in fbint
+#define P_RB 17    // b0 - binf
+#define P_RTA 18   // Ta0 - Tainf
+#define P_RN 19    // the integer of ln (A0 / Ainf) as a double
+struct __align__(16) RxnRec {
+    int flags, nspec, thd_off, thd_cnt;
+    int aux, list, bint, fbint;  // list: number of the shared [M] list, -1 none
+    unsigned ent[PJG_MAXSP];
+    double p[20];
+};
 
 // Species record (48 doubles): T_mid, W_k / W_ns, 1 - W_k / W_ns, padding, then
 // one 20-double block per temperature range (low at SP_LO, high at SP_HI):

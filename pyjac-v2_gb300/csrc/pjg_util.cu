@@ -1,4 +1,4 @@
-// Auxiliary kernels: accumulator zeroing, state-innermost -> 'C' transpose,
+// Auxiliary kernels: state-innermost -> 'C' transpose,
 // and the FP64 throughput probe used as the FP64 roofline denominator.
 #include <cuda_runtime.h>
 #include "pjg_eval.cuh"
@@ -13,13 +13,6 @@ __global__ void fexp_kernel(const double* x, double* y, int64_t n)
     __syncthreads();
     const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i < n) y[i] = pjg::fexp(x[i], tab);
-}
-
-__global__ void zero_acc(double* acc, int64_t ld, int64_t n, int nslot)
-{
-    const int64_t s = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (s >= n) return;
-    for (int q = 0; q < nslot; ++q) acc[(int64_t)q * ld + s] = 0.0;
 }
 
 // dst[s * nslot + q] = src[q * ld + s] through 32 x 32 shared-memory tiles.
@@ -60,14 +53,6 @@ __global__ void dfma_probe(double* out, int iters, double a, double b)
 int pjg_fp64_probe(int blocks, int threads, int iters, double* out, void* stream)
 {
     dfma_probe<<<blocks, threads, 0, (cudaStream_t)stream>>>(out, iters, 0.999999, 1e-7);
-    return cudaGetLastError() == cudaSuccess ? 0 : -2;
-}
-
-int pjg_launch_zero(double* acc, int64_t ld, int64_t n, int nslot, void* stream)
-{
-    if (n <= 0) return 0;
-    const unsigned grid = (unsigned)((n + PJG_BLOCK - 1) / PJG_BLOCK);
-    zero_acc<<<grid, PJG_BLOCK, 0, (cudaStream_t)stream>>>(acc, ld, n, nslot);
     return cudaGetLastError() == cudaSuccess ? 0 : -2;
 }
 
