@@ -43,6 +43,7 @@ struct RowsArgs {
     int act;           // 1: SiLU
     const bf16* zp;    // dgrad: multiply by SiLU'(zp)
     int64_t ldzp;
+    int zvec;          // zp's rows start on 16-byte boundaries
     bf16* Y;
     int64_t ldy;
     bf16* YT;          // transposed copy YT[n * ldyt + m]
@@ -52,6 +53,8 @@ struct RowsArgs {
     float* Y32;        // FP32 output
     int64_t ldy32;
     float* colsum;     // += column sums of the output
+    int NT;            // columns of one CTA (N, or its half)
+    int stages;        // tiles of A in shared memory
 };
 
 // logistic sigmoid with the fast division intrinsic (2 ulp in FP32; results are
@@ -69,74 +72,100 @@ __device__ __forceinline__ float tanh_approx(float x)
 }
 __device__ __forceinline__ float sigmoidf_(float x) { return fmaf(0.5f, tanh_approx(0.5f * x), 0.5f); }
 
-__global__ void __launch_bounds__(128, 1) umma_rows_kernel(const RowsArgs g)
+// One CTA keeps a slice of NT columns of B in shared memory (all of them, or a
+// half where that lets two tiles of A fit beside it) and walks the 128-row
+// tiles of A.  Two stages: while the tensor core multiplies tile i, the 8 warps
+// read tile i - 1's accumulator (two TMEM buffers) and write its outputs, and
+// tile i + 1 is copied into the stage that tile i - 1 left.  Bound by the
+// outputs' bytes; with one stage, four warps and element-wise reads of zp (2
+// bytes per lane and row) it was bound by latency.  49,152 rows, K = N = 256, on
+// GB300: forward with Y, Z, Y^T 87 -> 48 us, input gradient with Y, Y^T and
+// column sums 268 -> 53 us.
+constexpr int kRowsThreads = 256;
+
+template <bool ZP>
+__global__ void __launch_bounds__(kRowsThreads, 1) umma_rows_kernel(const RowsArgs g)
 {
     extern __shared__ __align__(1024) uint8_t smem[];
-    __shared__ uint64_t mbar;
+    __shared__ uint64_t mbar[2];
     __shared__ uint32_t tmem_s;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int kc = g.K >> 3;  // 16-byte chunks per row
+    const int NT = g.NT, halves = g.N / NT, n0 = (int)(blockIdx.x % halves) * NT;
     uint8_t* sB = smem;
-    uint8_t* sA = smem + (size_t)g.N * g.K * 2;
-    const uint32_t ncols = g.N <= 32 ? 32u : (g.N <= 64 ? 64u : (g.N <= 128 ? 128u : 256u));
+    uint8_t* sA = smem + (size_t)NT * g.K * 2;
+    const uint32_t stage_bytes = 128u * g.K * 2, stages = g.stages;
+    uint32_t ncols = 64;  // two accumulators
+    while (ncols < 2u * NT) ncols *= 2;
+    const uint32_t acc = ncols / 2;
     if (warp == 0) {
         umma::tmem_alloc(&tmem_s, ncols);
         umma::tmem_relinquish();
     }
-    if (tid == 0) umma::mbar_init(&mbar, 1);
-    for (int idx = tid; idx < g.N * kc; idx += 128) {
-        const int n = idx / kc, c = idx - n * kc;
-        umma::cp_async16(sB + ((size_t)(n >> 3) * kc + c) * 128 + (n & 7) * 16, g.B + (int64_t)n * g.ldb + c * 8, 16);
+    if (tid == 0) {
+        umma::mbar_init(&mbar[0], 1);
+        umma::mbar_init(&mbar[1], 1);
     }
+    for (int idx = tid; idx < NT * kc; idx += kRowsThreads) {
+        const int n = idx / kc, c = idx - n * kc;
+        umma::cp_async16(sB + ((size_t)(n >> 3) * kc + c) * 128 + (n & 7) * 16,
+                         g.B + (int64_t)(n0 + n) * g.ldb + c * 8, 16);
+    }
+    auto load_a = [&](int64_t t, uint32_t stage) {
+        const int64_t row0 = t * 128;
+        uint8_t* dst = sA + stage * stage_bytes;
+        for (int idx = tid; idx < 128 * kc; idx += kRowsThreads) {
+            const int r = idx / kc, c = idx - r * kc;
+            const int64_t grow = row0 + r;
+            const bool ok = grow < g.M;
+            umma::cp_async16(dst + ((size_t)(r >> 3) * kc + c) * 128 + (r & 7) * 16,
+                             g.A + (ok ? grow : 0) * g.lda + c * 8, ok ? 16u : 0u);
+        }
+    };
+    const int64_t ntiles = (g.M + 127) / 128, step = gridDim.x / halves, t0 = blockIdx.x / halves;
+    if (t0 < ntiles) load_a(t0, 0);
     umma::fence_before();
     __syncthreads();
     umma::fence_after();
     const uint32_t tmem = tmem_s;
-    const uint32_t idesc = umma::idesc_bf16(128, g.N);
+    const uint32_t idesc = umma::idesc_bf16(128, NT);
     const uint32_t sAu = umma::smem_u32(sA), sBu = umma::smem_u32(sB);
     const uint32_t sbo = (uint32_t)kc * 128;
-    uint32_t phase = 0;
-    const int64_t ntiles = (g.M + 127) / 128;
-    for (int64_t t = blockIdx.x; t < ntiles; t += gridDim.x) {
-        const int64_t row0 = t * 128;
-        for (int idx = tid; idx < 128 * kc; idx += 128) {
-            const int r = idx / kc, c = idx - r * kc;
-            const int64_t grow = row0 + r;
-            const bool ok = grow < g.M;
-            umma::cp_async16(sA + ((size_t)(r >> 3) * kc + c) * 128 + (r & 7) * 16,
-                             g.A + (ok ? grow : 0) * g.lda + c * 8, ok ? 16u : 0u);
-        }
-        umma::cp_async_wait_all();
-        umma::fence_proxy_async();
-        __syncthreads();
-        if (tid == 0) {
-            umma::fence_after();
-            for (int ks = 0; ks < (g.K >> 4); ++ks) {
-                const uint64_t ad = umma::sdesc(sAu + ks * 256, 128, sbo);
-                const uint64_t bd = umma::sdesc(sBu + ks * 256, 128, sbo);
-                umma::mma_bf16(tmem, ad, bd, idesc, ks > 0 ? 1u : 0u);
-            }
-            umma::mma_commit(&mbar);
-        }
-        if (!umma::mbar_wait(&mbar, phase) && lane == 0) atomicExch(&g_umma_err, 1);
-        phase ^= 1;
-        umma::fence_after();
-        const int m = warp * 32 + lane;
-        const int64_t grow = row0 + m;
+    const int quarter = warp & 3, chalf = warp >> 2;  // TMEM lanes 32 * quarter.., every other 32 columns
+    const int m = quarter * 32 + lane;
+    float csum[4] = {0.0f, 0.0f, 0.0f, 0.0f};  // column sums: lane's column of this warp's chunks
+
+    auto epilogue = [&](int64_t t, uint32_t buf) {
+        const int64_t grow = t * 128 + m;
         const bool ok = grow < g.M;
-        for (int c0 = 0; c0 < g.N; c0 += 32) {
+        const uint32_t trow = tmem + buf * acc + ((uint32_t)(quarter * 32) << 16);
+        int ci = 0;
+#pragma unroll 1
+        for (int c0 = 32 * chalf; c0 < NT; c0 += 64, ++ci) {
+            const int n = n0 + c0;  // first column of this chunk
+            alignas(16) bf16 zp[32];
+            if (ZP) {
+                const bf16* src = g.zp + (ok ? grow : 0) * g.ldzp + n;
+                if (g.zvec) {
+                    uint4* d = reinterpret_cast<uint4*>(zp);
+#pragma unroll
+                    for (int q = 0; q < 4; ++q) d[q] = *reinterpret_cast<const uint4*>(src + 8 * q);
+                } else {
+#pragma unroll
+                    for (int j = 0; j < 32; ++j) zp[j] = src[j];
+                }
+            }
             float v[32];
-            umma::tmem_ld32(tmem + ((uint32_t)(warp * 32) << 16) + (uint32_t)c0, v);
+            umma::tmem_ld32(trow + (uint32_t)c0, v);
             alignas(16) bf16 yb[32];
             alignas(16) bf16 zb[32];
 #pragma unroll
             for (int j = 0; j < 32; ++j) {
-                const int n = c0 + j;
                 float x = v[j];
-                if (g.bias) x += __ldg(g.bias + n);
+                if (g.bias) x += __ldg(g.bias + n + j);
                 zb[j] = __float2bfloat16(x);
-                if (g.zp) {
-                    const float z = ok ? __bfloat162float(g.zp[grow * g.ldzp + n]) : 0.0f;
+                if (ZP) {
+                    const float z = ok ? __bfloat162float(zp[j]) : 0.0f;
                     const float sg = sigmoidf_(z);
                     x *= sg * (1.0f + z * (1.0f - sg));
                 }
@@ -146,43 +175,91 @@ __global__ void __launch_bounds__(128, 1) umma_rows_kernel(const RowsArgs g)
             }
             if (ok) {
                 if (g.Y) {
-                    uint4* d = reinterpret_cast<uint4*>(g.Y + grow * g.ldy + c0);
+                    uint4* d = reinterpret_cast<uint4*>(g.Y + grow * g.ldy + n);
                     const uint4* s = reinterpret_cast<const uint4*>(yb);
 #pragma unroll
                     for (int q = 0; q < 4; ++q) d[q] = s[q];
                 }
                 if (g.Z) {
-                    uint4* d = reinterpret_cast<uint4*>(g.Z + grow * g.ldz + c0);
+                    uint4* d = reinterpret_cast<uint4*>(g.Z + grow * g.ldz + n);
                     const uint4* s = reinterpret_cast<const uint4*>(zb);
 #pragma unroll
                     for (int q = 0; q < 4; ++q) d[q] = s[q];
                 }
                 if (g.YT) {
+                    bf16* yt = g.YT + (int64_t)n * g.ldyt + grow;
 #pragma unroll
-                    for (int j = 0; j < 32; ++j) g.YT[(int64_t)(c0 + j) * g.ldyt + grow] = yb[j];
+                    for (int j = 0; j < 32; ++j, yt += g.ldyt) *yt = yb[j];
                 }
                 if (g.Y32) {
-                    float4* d = reinterpret_cast<float4*>(g.Y32 + grow * g.ldy32 + c0);
+                    float4* d = reinterpret_cast<float4*>(g.Y32 + grow * g.ldy32 + n);
 #pragma unroll
                     for (int q = 0; q < 8; ++q)
                         d[q] = make_float4(v[4 * q], v[4 * q + 1], v[4 * q + 2], v[4 * q + 3]);
                 }
             }
             if (g.colsum) {
+                // 32 columns over 32 lanes in 31 exchanges: each step folds the
+                // halves of the columns onto the halves of the lanes; lane l ends
+                // with the sum of column l
 #pragma unroll
-                for (int j = 0; j < 32; ++j) {
-                    float sv = ok ? v[j] : 0.0f;
+                for (int j = 0; j < 32; ++j)
+                    if (!ok) v[j] = 0.0f;
 #pragma unroll
-                    for (int o = 16; o > 0; o >>= 1) sv += __shfl_xor_sync(0xffffffffu, sv, o);
-                    if (lane == 0) atomicAdd(g.colsum + c0 + j, sv);
+                for (int h = 16; h > 0; h >>= 1) {
+                    const bool up = lane & h;
+#pragma unroll
+                    for (int j = 0; j < 16; ++j) {
+                        if (j >= h) break;
+                        const float send = up ? v[j] : v[j + h], keep = up ? v[j + h] : v[j];
+                        v[j] = keep + __shfl_xor_sync(0xffffffffu, send, h);
+                    }
                 }
+                if (ci < 4) csum[ci] += v[0];
             }
         }
+    };
+
+    bool timeout = false;
+    int64_t i = 0;
+    for (int64_t t = t0; t < ntiles; t += step, ++i) {
+        const uint32_t buf = (uint32_t)i & 1u, stage = stages == 2 ? buf : 0u;
+        umma::cp_async_wait_all();
+        umma::fence_proxy_async();
         umma::fence_before();
         __syncthreads();
+        if (tid == 0) {
+            umma::fence_after();
+            for (int ks = 0; ks < (g.K >> 4); ++ks) {
+                const uint64_t ad = umma::sdesc(sAu + stage * stage_bytes + ks * 256, 128, sbo);
+                const uint64_t bd = umma::sdesc(sBu + ks * 256, 128, sbo);
+                umma::mma_bf16(tmem + buf * acc, ad, bd, idesc, ks > 0 ? 1u : 0u);
+            }
+            umma::mma_commit(&mbar[buf]);
+        }
+        if (stages == 2) {
+            // tile i - 1 is multiplied (waited for below): its stage takes tile i + 1
+            if (t + step < ntiles) load_a(t + step, buf ^ 1u);
+            if (i > 0) epilogue(t - step, buf ^ 1u);
+            if (!umma::mbar_wait(&mbar[buf], (uint32_t)(i >> 1) & 1u)) timeout = true;
+            umma::fence_after();
+        } else {
+            if (!umma::mbar_wait(&mbar[buf], (uint32_t)(i >> 1) & 1u)) timeout = true;
+            umma::fence_after();
+            if (t + step < ntiles) load_a(t + step, 0);
+            epilogue(t, buf);
+        }
     }
-    umma::fence_after();
+    if (stages == 2 && i > 0) epilogue(t0 + (i - 1) * step, (uint32_t)(i - 1) & 1u);
+    if (timeout && lane == 0) atomicExch(&g_umma_err, 1);
+    if (g.colsum) {
+        int ci = 0;
+        for (int c0 = 32 * chalf; c0 < NT; c0 += 64, ++ci)
+            if (ci < 4 && i > 0) atomicAdd(g.colsum + n0 + c0 + lane, csum[ci]);
+    }
+    umma::fence_before();
     __syncthreads();
+    umma::fence_after();
     if (warp == 0) umma::tmem_dealloc(tmem, ncols);
 }
 
@@ -195,76 +272,107 @@ struct WgradArgs {
     int64_t Kb, kchunk;
     float* C;        // [Mo x No] += A B^T
     int64_t ldc;
+    int vec;         // C and ldc allow 16-byte reductions
 };
 
 constexpr int WK = 64;  // reduction block staged per step
 
-__global__ void __launch_bounds__(128, 1) umma_wgrad_kernel(const WgradArgs g)
+// The reduction blocks pass through a ring of kWStages shared-memory stages:
+// the copies of the next ones run while the tensor core multiplies.  The FP32
+// partial result is added to C four columns per reduction.  256 x 256 over
+// 49,152 states on GB300: 69 us with one stage and one column per reduction,
+// 31 us
+// here.
+constexpr int kWThreads = 256, kWStages = 4;
+
+__global__ void __launch_bounds__(kWThreads, 1) umma_wgrad_kernel(const WgradArgs g)
 {
     extern __shared__ __align__(1024) uint8_t smem[];
-    __shared__ uint64_t mbar;
+    __shared__ uint64_t mbar[kWStages];
     __shared__ uint32_t tmem_s;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     constexpr int kc = WK / 8;
-    uint8_t* sA = smem;                       // 128 x WK
-    uint8_t* sB = smem + 128 * WK * 2;        // No x WK
+    const uint32_t a_bytes = 128u * WK * 2, stage_bytes = (128u + (uint32_t)g.No) * WK * 2;
     const uint32_t ncols = g.No <= 32 ? 32u : (g.No <= 64 ? 64u : (g.No <= 128 ? 128u : 256u));
     if (warp == 0) {
         umma::tmem_alloc(&tmem_s, ncols);
         umma::tmem_relinquish();
     }
-    if (tid == 0) umma::mbar_init(&mbar, 1);
+    if (tid == 0)
+        for (int q = 0; q < kWStages; ++q) umma::mbar_init(&mbar[q], 1);
     umma::fence_before();
     __syncthreads();
     umma::fence_after();
     const uint32_t tmem = tmem_s;
     const uint32_t idesc = umma::idesc_bf16(128, g.No);
-    const uint32_t sAu = umma::smem_u32(sA), sBu = umma::smem_u32(sB);
+    const uint32_t su = umma::smem_u32(smem);
     const int mrow0 = blockIdx.x * 128;
     const int64_t k0 = (int64_t)blockIdx.y * g.kchunk;
     const int64_t k1 = k0 + g.kchunk < g.Kb ? k0 + g.kchunk : g.Kb;
-    uint32_t phase = 0;
-    bool first = true;
-    for (int64_t kb = k0; kb < k1; kb += WK) {
-        for (int idx = tid; idx < 128 * kc; idx += 128) {
-            const int r = idx / kc, c = idx - r * kc;
-            const bool ok = mrow0 + r < g.Mo;
-            umma::cp_async16(sA + ((size_t)(r >> 3) * kc + c) * 128 + (r & 7) * 16,
-                             g.A + (int64_t)(ok ? mrow0 + r : 0) * g.lda + kb + c * 8, ok ? 16u : 0u);
+    const int steps = k1 > k0 ? (int)((k1 - k0) / WK) : 0;
+    auto load = [&](int s) {
+        if (s < steps) {
+            uint8_t* sA = smem + (size_t)(s % kWStages) * stage_bytes;
+            uint8_t* sB = sA + a_bytes;
+            const int64_t kb = k0 + (int64_t)s * WK;
+            for (int idx = tid; idx < 128 * kc; idx += kWThreads) {
+                const int r = idx / kc, c = idx - r * kc;
+                const bool ok = mrow0 + r < g.Mo;
+                umma::cp_async16(sA + ((size_t)(r >> 3) * kc + c) * 128 + (r & 7) * 16,
+                                 g.A + (int64_t)(ok ? mrow0 + r : 0) * g.lda + kb + c * 8, ok ? 16u : 0u);
+            }
+            for (int idx = tid; idx < g.No * kc; idx += kWThreads) {
+                const int n = idx / kc, c = idx - n * kc;
+                umma::cp_async16(sB + ((size_t)(n >> 3) * kc + c) * 128 + (n & 7) * 16,
+                                 g.B + (int64_t)n * g.ldb + kb + c * 8, 16u);
+            }
         }
-        for (int idx = tid; idx < g.No * kc; idx += 128) {
-            const int n = idx / kc, c = idx - n * kc;
-            umma::cp_async16(sB + ((size_t)(n >> 3) * kc + c) * 128 + (n & 7) * 16,
-                             g.B + (int64_t)n * g.ldb + kb + c * 8, 16u);
-        }
-        umma::cp_async_wait_all();
+        umma::cp_async_commit();
+    };
+    for (int s = 0; s < kWStages - 1; ++s) load(s);
+    bool timeout = false;
+    for (int s = 0; s < steps; ++s) {
+        umma::cp_async_wait<kWStages - 2>();
         umma::fence_proxy_async();
         __syncthreads();
         if (tid == 0) {
             umma::fence_after();
+            const uint32_t sAu = su + (uint32_t)(s % kWStages) * stage_bytes, sBu = sAu + a_bytes;
 #pragma unroll
             for (int ks = 0; ks < WK / 16; ++ks) {
                 const uint64_t ad = umma::sdesc(sAu + ks * 256, 128, kc * 128);
                 const uint64_t bd = umma::sdesc(sBu + ks * 256, 128, kc * 128);
-                umma::mma_bf16(tmem, ad, bd, idesc, (first && ks == 0) ? 0u : 1u);
+                umma::mma_bf16(tmem, ad, bd, idesc, (s == 0 && ks == 0) ? 0u : 1u);
             }
-            umma::mma_commit(&mbar);
+            umma::mma_commit(&mbar[s % kWStages]);
         }
-        first = false;
-        if (!umma::mbar_wait(&mbar, phase) && lane == 0) atomicExch(&g_umma_err, 1);
-        phase ^= 1;
+        // the stage of step s - 1, once multiplied, takes step s + kWStages - 1
+        if (s > 0 && !umma::mbar_wait(&mbar[(s - 1) % kWStages], (uint32_t)((s - 1) / kWStages) & 1u)) timeout = true;
+        load(s + kWStages - 1);
+    }
+    if (steps > 0) {
+        if (!umma::mbar_wait(&mbar[(steps - 1) % kWStages], (uint32_t)((steps - 1) / kWStages) & 1u)) timeout = true;
         umma::fence_after();
-        __syncthreads();
-    }
-    if (k1 > k0) {
-        const int m = mrow0 + warp * 32 + lane;
-        for (int c0 = 0; c0 < g.No; c0 += 32) {
+        const int quarter = warp & 3;
+        const int m = mrow0 + quarter * 32 + lane;
+        for (int c0 = 32 * (warp >> 2); c0 < g.No; c0 += 64) {
             float v[32];
-            umma::tmem_ld32(tmem + ((uint32_t)(warp * 32) << 16) + (uint32_t)c0, v);
-            if (m < g.Mo)
-                for (int j = 0; j < 32; ++j) atomicAdd(g.C + (int64_t)m * g.ldc + c0 + j, v[j]);
+            umma::tmem_ld32(tmem + ((uint32_t)(quarter * 32) << 16) + (uint32_t)c0, v);
+            if (m < g.Mo) {
+                float* c = g.C + (int64_t)m * g.ldc + c0;
+                if (g.vec) {
+#pragma unroll
+                    for (int j = 0; j < 32; j += 4)
+                        asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(__cvta_generic_to_global(c + j)),
+                                     "f"(v[j]), "f"(v[j + 1]), "f"(v[j + 2]), "f"(v[j + 3]) : "memory");
+                } else {
+                    for (int j = 0; j < 32; ++j) atomicAdd(c + j, v[j]);
+                }
+            }
         }
     }
+    if (timeout && lane == 0) atomicExch(&g_umma_err, 1);
+    umma::cp_async_wait_all();
     umma::fence_before();
     __syncthreads();
     umma::fence_after();
@@ -559,6 +667,7 @@ int sm_count()
     return n;
 }
 
+constexpr size_t kRowsSmemMax = (227 << 10) - 1024;  // less the kernel's static shared memory
 bool aligned16(const void* p) { return ((uintptr_t)p & 15) == 0; }
 
 }  // namespace
@@ -581,11 +690,31 @@ int mlp_launch_rows(const void* A, int64_t lda, const void* B, int64_t ldb, int6
     g.zp = (const bf16*)zp; g.ldzp = ldzp;
     g.Y = (bf16*)Y; g.ldy = ldy; g.YT = (bf16*)YT; g.ldyt = ldyt; g.Z = (bf16*)Z; g.ldz = ldz;
     g.Y32 = Y32; g.ldy32 = ldy32; g.colsum = colsum;
-    const size_t smem = (size_t)(N + 128) * K * 2;
-    cudaFuncSetAttribute(umma_rows_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    g.zvec = zp && ldzp % 8 == 0 && aligned16(zp);
+    // half of the columns per CTA where that lets a second tile of A fit (A is
+    // then read twice, from L2), as for N = K = 256; an output that overlaps A
+    // keeps whole rows in one CTA, which reads a tile before it writes it
+    g.NT = N;
+    g.stages = 2;
+    auto smem_of = [&](int nt, int st) { return ((size_t)nt + 128 * st) * K * 2; };
+    auto meets_a = [&](const void* p, int64_t ld, int bytes) {
+        const uintptr_t a0 = (uintptr_t)A, a1 = a0 + ((M - 1) * lda + K) * 2;
+        const uintptr_t p0 = (uintptr_t)p, p1 = p0 + ((M - 1) * ld + N) * bytes;
+        return p && p0 < a1 && a0 < p1;
+    };
+    if (smem_of(N, 2) > kRowsSmemMax) {
+        const bool split = N % 64 == 0 && smem_of(N / 2, 2) <= kRowsSmemMax &&
+                           !meets_a(Y, ldy, 2) && !meets_a(Z, ldz, 2) && !meets_a(Y32, ldy32, 4);
+        if (split) g.NT = N / 2;
+        else g.stages = 1;
+    }
+    const size_t smem = smem_of(g.NT, g.stages);
+    auto kern = zp ? umma_rows_kernel<true> : umma_rows_kernel<false>;
+    cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     const int64_t ntiles = (M + 127) / 128;
-    const int grid = (int)(ntiles < sm_count() ? ntiles : sm_count());
-    umma_rows_kernel<<<grid, 128, smem, (cudaStream_t)stream>>>(g);
+    const int halves = N / g.NT, per = sm_count() > halves ? sm_count() / halves : 1;
+    const int grid = (int)(ntiles < per ? ntiles : per) * halves;
+    kern<<<grid, kRowsThreads, smem, (cudaStream_t)stream>>>(g);
     return cudaGetLastError() == cudaSuccess ? 0 : -2;
 }
 
@@ -604,9 +733,10 @@ int mlp_launch_wgrad(const void* A, int64_t lda, const void* B, int64_t ldb, int
     chunk = (chunk + WK - 1) / WK * WK;
     splits = (int)((Kb + chunk - 1) / chunk);
     g.kchunk = chunk;
-    const size_t smem = (size_t)(128 + No) * WK * 2;
+    g.vec = ldc % 4 == 0 && aligned16(C);
+    const size_t smem = (size_t)kWStages * (128 + No) * WK * 2;
     cudaFuncSetAttribute(umma_wgrad_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    umma_wgrad_kernel<<<dim3(mt, splits), 128, smem, (cudaStream_t)stream>>>(g);
+    umma_wgrad_kernel<<<dim3(mt, splits), kWThreads, smem, (cudaStream_t)stream>>>(g);
     return cudaGetLastError() == cudaSuccess ? 0 : -2;
 }
 

@@ -133,6 +133,12 @@ __device__ __forceinline__ void cp_async16(void* dst, const void* src, uint32_t 
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;"
                  :: "r"(smem_u32(dst)), "l"(src), "r"(src_bytes) : "memory");
 }
+__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+template <int N>  // all but the last N groups
+__device__ __forceinline__ void cp_async_wait()
+{
+    asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory");
+}
 __device__ __forceinline__ void cp_async_wait_all()
 {
     asm volatile("cp.async.wait_all;" ::: "memory");
