@@ -48,6 +48,7 @@ struct RowsArgs {
     int64_t ldy;
     bf16* YT;          // transposed copy YT[n * ldyt + m]
     int64_t ldyt;
+    int ytvec;         // pairs of YT's columns start on 4-byte boundaries
     bf16* Z;           // pre-activation copy
     int64_t ldz;
     float* Y32;        // FP32 output
@@ -74,14 +75,54 @@ __device__ __forceinline__ float sigmoidf_(float x) { return fmaf(0.5f, tanh_app
 
 // One CTA keeps a slice of NT columns of B in shared memory (all of them, or a
 // half where that lets two tiles of A fit beside it) and walks the 128-row
-// tiles of A.  Two stages: while the tensor core multiplies tile i, the 8 warps
+// tiles of A.  Two stages: while the tensor core multiplies tile i, the 16 warps
 // read tile i - 1's accumulator (two TMEM buffers) and write its outputs, and
 // tile i + 1 is copied into the stage that tile i - 1 left.  Bound by the
 // outputs' bytes; with one stage, four warps and element-wise reads of zp (2
 // bytes per lane and row) it was bound by latency.  49,152 rows, K = N = 256, on
-// GB300: forward with Y, Z, Y^T 87 -> 48 us, input gradient with Y, Y^T and
-// column sums 268 -> 53 us.
-constexpr int kRowsThreads = 256;
+// GB300: forward with Y, Z, Y^T 87 -> 38 us (48 with 8 warps and a row per
+// lane), input gradient with Y, Y^T and column sums 268 -> 48 us (53).  L2 and
+// L1 run at 30 to 40 % of their rates; what is left is latency between barriers.
+constexpr int kRowsThreads = 512, kRowsParts = kRowsThreads / 128;
+
+// Lane p of a quad holds r[0..3]; afterwards r[q] is what lane q held in r[p].
+// The epilogues read and write a row's 64 bytes with the four lanes of a quad
+// (8 rows per instruction, whole sectors) instead of one lane (32 rows).
+__device__ __forceinline__ void quad_transpose(uint4 (&r)[4], int lane)
+{
+    auto swap = [&](uint4& lo, uint4& hi, bool up, int h) {
+        const uint4 send = up ? lo : hi;
+        uint4 recv;
+        recv.x = __shfl_xor_sync(0xffffffffu, send.x, h);
+        recv.y = __shfl_xor_sync(0xffffffffu, send.y, h);
+        recv.z = __shfl_xor_sync(0xffffffffu, send.z, h);
+        recv.w = __shfl_xor_sync(0xffffffffu, send.w, h);
+        if (up) lo = recv;
+        else hi = recv;
+    };
+    swap(r[0], r[2], lane & 2, 2);
+    swap(r[1], r[3], lane & 2, 2);
+    swap(r[0], r[1], lane & 1, 1);
+    swap(r[2], r[3], lane & 1, 1);
+}
+
+// rows m0 .. m0 + 31 (one per lane, 64 bytes of each in r) to base + row * ld bytes
+__device__ __forceinline__ void store_rows64(uint8_t* base, int64_t ld, int64_t m0, int64_t M, uint4 (&r)[4], int lane)
+{
+    quad_transpose(r, lane);
+    const int64_t row = m0 + (lane & ~3);
+    uint8_t* d = base + row * ld + (lane & 3) * 16;
+#pragma unroll
+    for (int q = 0; q < 4; ++q)
+        if (row + q < M) *reinterpret_cast<uint4*>(d + q * ld) = r[q];
+}
+
+__device__ __forceinline__ uint32_t pack_bf16x2(float a, float b)
+{
+    const uint32_t lo = __bfloat16_as_ushort(__float2bfloat16(a));
+    const uint32_t hi = __bfloat16_as_ushort(__float2bfloat16(b));
+    return lo | (hi << 16);
+}
 
 template <bool ZP>
 __global__ void __launch_bounds__(kRowsThreads, 1) umma_rows_kernel(const RowsArgs g)
@@ -89,6 +130,7 @@ __global__ void __launch_bounds__(kRowsThreads, 1) umma_rows_kernel(const RowsAr
     extern __shared__ __align__(1024) uint8_t smem[];
     __shared__ uint64_t mbar[2];
     __shared__ uint32_t tmem_s;
+    __shared__ __align__(16) float sbias[256];
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int kc = g.K >> 3;  // 16-byte chunks per row
     const int NT = g.NT, halves = g.N / NT, n0 = (int)(blockIdx.x % halves) * NT;
@@ -106,6 +148,9 @@ __global__ void __launch_bounds__(kRowsThreads, 1) umma_rows_kernel(const RowsAr
         umma::mbar_init(&mbar[0], 1);
         umma::mbar_init(&mbar[1], 1);
     }
+    if (g.bias)
+        for (int j = tid; j < NT; j += kRowsThreads) sbias[j] = g.bias[n0 + j];
+    const int lr = tid / kc, lc = tid % kc, dr = kRowsThreads / kc, dc = kRowsThreads % kc;
     for (int idx = tid; idx < NT * kc; idx += kRowsThreads) {
         const int n = idx / kc, c = idx - n * kc;
         umma::cp_async16(sB + ((size_t)(n >> 3) * kc + c) * 128 + (n & 7) * 16,
@@ -114,12 +159,17 @@ __global__ void __launch_bounds__(kRowsThreads, 1) umma_rows_kernel(const RowsAr
     auto load_a = [&](int64_t t, uint32_t stage) {
         const int64_t row0 = t * 128;
         uint8_t* dst = sA + stage * stage_bytes;
-        for (int idx = tid; idx < 128 * kc; idx += kRowsThreads) {
-            const int r = idx / kc, c = idx - r * kc;
+        for (int r = lr, c = lc; r < 128;) {
             const int64_t grow = row0 + r;
             const bool ok = grow < g.M;
             umma::cp_async16(dst + ((size_t)(r >> 3) * kc + c) * 128 + (r & 7) * 16,
                              g.A + (ok ? grow : 0) * g.lda + c * 8, ok ? 16u : 0u);
+            r += dr;
+            c += dc;
+            if (c >= kc) {
+                c -= kc;
+                ++r;
+            }
         }
     };
     const int64_t ntiles = (g.M + 127) / 128, step = gridDim.x / halves, t0 = blockIdx.x / halves;
@@ -131,71 +181,91 @@ __global__ void __launch_bounds__(kRowsThreads, 1) umma_rows_kernel(const RowsAr
     const uint32_t idesc = umma::idesc_bf16(128, NT);
     const uint32_t sAu = umma::smem_u32(sA), sBu = umma::smem_u32(sB);
     const uint32_t sbo = (uint32_t)kc * 128;
-    const int quarter = warp & 3, chalf = warp >> 2;  // TMEM lanes 32 * quarter.., every other 32 columns
+    const int quarter = warp & 3, part = warp >> 2;  // TMEM lanes 32 * quarter.., every kRowsParts-th 32 columns
     const int m = quarter * 32 + lane;
-    float csum[4] = {0.0f, 0.0f, 0.0f, 0.0f};  // column sums: lane's column of this warp's chunks
+    float csum[8 / kRowsParts] = {};  // column sums: lane's column of this warp's chunks
 
     auto epilogue = [&](int64_t t, uint32_t buf) {
         const int64_t grow = t * 128 + m;
         const bool ok = grow < g.M;
         const uint32_t trow = tmem + buf * acc + ((uint32_t)(quarter * 32) << 16);
-        int ci = 0;
-#pragma unroll 1
-        for (int c0 = 32 * chalf; c0 < NT; c0 += 64, ++ci) {
+        const int64_t m0 = t * 128 + quarter * 32;
+#pragma unroll
+        for (int ci = 0; ci < 8 / kRowsParts; ++ci) {
+            const int c0 = 32 * (part + ci * kRowsParts);
+            if (c0 >= NT) break;
             const int n = n0 + c0;  // first column of this chunk
-            alignas(16) bf16 zp[32];
+            uint4 zq[4];
             if (ZP) {
-                const bf16* src = g.zp + (ok ? grow : 0) * g.ldzp + n;
                 if (g.zvec) {
-                    uint4* d = reinterpret_cast<uint4*>(zp);
+                    const int64_t row = m0 + (lane & ~3);
+                    const bf16* src = g.zp + row * g.ldzp + n + (lane & 3) * 8;
 #pragma unroll
-                    for (int q = 0; q < 4; ++q) d[q] = *reinterpret_cast<const uint4*>(src + 8 * q);
+                    for (int q = 0; q < 4; ++q)
+                        zq[q] = row + q < g.M ? *reinterpret_cast<const uint4*>(src + q * g.ldzp) : make_uint4(0, 0, 0, 0);
+                    quad_transpose(zq, lane);
                 } else {
+                    const bf16* src = g.zp + (ok ? grow : 0) * g.ldzp + n;
+                    bf16* d = reinterpret_cast<bf16*>(zq);
 #pragma unroll
-                    for (int j = 0; j < 32; ++j) zp[j] = src[j];
+                    for (int j = 0; j < 32; ++j) d[j] = src[j];
                 }
             }
             float v[32];
             umma::tmem_ld32(trow + (uint32_t)c0, v);
-            alignas(16) bf16 yb[32];
-            alignas(16) bf16 zb[32];
+            uint4 yq[4];
+            uint32_t* yw = reinterpret_cast<uint32_t*>(yq);
+            if (g.bias) {
+#pragma unroll
+                for (int j = 0; j < 32; j += 4) {
+                    const float4 b = *reinterpret_cast<const float4*>(sbias + c0 + j);
+                    v[j] += b.x;
+                    v[j + 1] += b.y;
+                    v[j + 2] += b.z;
+                    v[j + 3] += b.w;
+                }
+            }
+            if (g.Z) {
+#pragma unroll
+                for (int j = 0; j < 16; ++j) yw[j] = pack_bf16x2(v[2 * j], v[2 * j + 1]);
+                store_rows64(reinterpret_cast<uint8_t*>(g.Z + n), g.ldz * 2, m0, g.M, yq, lane);
+            }
 #pragma unroll
             for (int j = 0; j < 32; ++j) {
                 float x = v[j];
-                if (g.bias) x += __ldg(g.bias + n + j);
-                zb[j] = __float2bfloat16(x);
                 if (ZP) {
-                    const float z = ok ? __bfloat162float(zp[j]) : 0.0f;
+                    const float z = ok ? __bfloat162float(reinterpret_cast<const bf16*>(zq)[j]) : 0.0f;
                     const float sg = sigmoidf_(z);
                     x *= sg * (1.0f + z * (1.0f - sg));
                 }
-                const float y = g.act ? x * sigmoidf_(x) : x;
-                v[j] = y;
-                yb[j] = __float2bfloat16(y);
+                v[j] = g.act ? x * sigmoidf_(x) : x;
             }
-            if (ok) {
-                if (g.Y) {
-                    uint4* d = reinterpret_cast<uint4*>(g.Y + grow * g.ldy + n);
-                    const uint4* s = reinterpret_cast<const uint4*>(yb);
 #pragma unroll
-                    for (int q = 0; q < 4; ++q) d[q] = s[q];
+            for (int j = 0; j < 16; ++j) yw[j] = pack_bf16x2(v[2 * j], v[2 * j + 1]);
+            if (g.YT) {
+                // two rows of one column per lane: the even lane takes column 2k, the odd one 2k + 1
+                const int odd = lane & 1;
+                const int64_t row = grow - odd;
+                bf16* yt = g.YT + (int64_t)(n + odd) * g.ldyt + row;
+#pragma unroll
+                for (int k = 0; k < 16; ++k, yt += 2 * g.ldyt) {
+                    const uint32_t other = __shfl_xor_sync(0xffffffffu, yw[k], 1);
+                    const uint32_t two = odd ? __byte_perm(other, yw[k], 0x7632) : __byte_perm(yw[k], other, 0x5410);
+                    if (g.ytvec && row + 1 < g.M) {
+                        *reinterpret_cast<uint32_t*>(yt) = two;
+                    } else {
+                        if (row < g.M) yt[0] = __ushort_as_bfloat16((unsigned short)two);
+                        if (row + 1 < g.M) yt[1] = __ushort_as_bfloat16((unsigned short)(two >> 16));
+                    }
                 }
-                if (g.Z) {
-                    uint4* d = reinterpret_cast<uint4*>(g.Z + grow * g.ldz + n);
-                    const uint4* s = reinterpret_cast<const uint4*>(zb);
+            }
+            if (g.Y) store_rows64(reinterpret_cast<uint8_t*>(g.Y + n), g.ldy * 2, m0, g.M, yq, lane);
+            if (g.Y32) {
 #pragma unroll
-                    for (int q = 0; q < 4; ++q) d[q] = s[q];
-                }
-                if (g.YT) {
-                    bf16* yt = g.YT + (int64_t)n * g.ldyt + grow;
+                for (int h = 0; h < 2; ++h) {
 #pragma unroll
-                    for (int j = 0; j < 32; ++j, yt += g.ldyt) *yt = yb[j];
-                }
-                if (g.Y32) {
-                    float4* d = reinterpret_cast<float4*>(g.Y32 + grow * g.ldy32 + n);
-#pragma unroll
-                    for (int q = 0; q < 8; ++q)
-                        d[q] = make_float4(v[4 * q], v[4 * q + 1], v[4 * q + 2], v[4 * q + 3]);
+                    for (int j = 0; j < 16; ++j) yw[j] = __float_as_uint(v[16 * h + j]);
+                    store_rows64(reinterpret_cast<uint8_t*>(g.Y32 + n + 16 * h), g.ldy32 * 4, m0, g.M, yq, lane);
                 }
             }
             if (g.colsum) {
@@ -215,7 +285,7 @@ __global__ void __launch_bounds__(kRowsThreads, 1) umma_rows_kernel(const RowsAr
                         v[j] = keep + __shfl_xor_sync(0xffffffffu, send, h);
                     }
                 }
-                if (ci < 4) csum[ci] += v[0];
+                csum[ci] += v[0];
             }
         }
     };
@@ -253,9 +323,11 @@ __global__ void __launch_bounds__(kRowsThreads, 1) umma_rows_kernel(const RowsAr
     if (stages == 2 && i > 0) epilogue(t0 + (i - 1) * step, (uint32_t)(i - 1) & 1u);
     if (timeout && lane == 0) atomicExch(&g_umma_err, 1);
     if (g.colsum) {
-        int ci = 0;
-        for (int c0 = 32 * chalf; c0 < NT; c0 += 64, ++ci)
-            if (ci < 4 && i > 0) atomicAdd(g.colsum + n0 + c0 + lane, csum[ci]);
+#pragma unroll
+        for (int ci = 0; ci < 8 / kRowsParts; ++ci) {
+            const int c0 = 32 * (part + ci * kRowsParts);
+            if (c0 < NT && i > 0) atomicAdd(g.colsum + n0 + c0 + lane, csum[ci]);
+        }
     }
     umma::fence_before();
     __syncthreads();
@@ -281,8 +353,8 @@ constexpr int WK = 64;  // reduction block staged per step
 // the copies of the next ones run while the tensor core multiplies.  The FP32
 // partial result is added to C four columns per reduction.  256 x 256 over
 // 49,152 states on GB300: 69 us with one stage and one column per reduction,
-// 31 us
-// here.
+// 26 us here
+// (31 without the quad transpose before the reductions).
 constexpr int kWThreads = 256, kWStages = 4;
 
 __global__ void __launch_bounds__(kWThreads, 1) umma_wgrad_kernel(const WgradArgs g)
@@ -358,16 +430,28 @@ __global__ void __launch_bounds__(kWThreads, 1) umma_wgrad_kernel(const WgradArg
         for (int c0 = 32 * (warp >> 2); c0 < g.No; c0 += 64) {
             float v[32];
             umma::tmem_ld32(tmem + ((uint32_t)(quarter * 32) << 16) + (uint32_t)c0, v);
-            if (m < g.Mo) {
-                float* c = g.C + (int64_t)m * g.ldc + c0;
-                if (g.vec) {
+            if (g.vec) {
+                // the quad transpose of the layer kernels: 64 bytes of a row per quad
 #pragma unroll
-                    for (int j = 0; j < 32; j += 4)
-                        asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(__cvta_generic_to_global(c + j)),
-                                     "f"(v[j]), "f"(v[j + 1]), "f"(v[j + 2]), "f"(v[j + 3]) : "memory");
-                } else {
-                    for (int j = 0; j < 32; ++j) atomicAdd(c + j, v[j]);
+                for (int h = 0; h < 2; ++h) {
+                    uint4 r[4];
+                    uint32_t* w = reinterpret_cast<uint32_t*>(r);
+#pragma unroll
+                    for (int j = 0; j < 16; ++j) w[j] = __float_as_uint(v[16 * h + j]);
+                    quad_transpose(r, lane);
+                    const int row = m & ~3;
+                    float* c = g.C + (int64_t)row * g.ldc + c0 + 16 * h + 4 * (lane & 3);
+#pragma unroll
+                    for (int q = 0; q < 4; ++q)
+                        if (row + q < g.Mo)
+                            asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};"
+                                         :: "l"(__cvta_generic_to_global(c + q * g.ldc)),
+                                            "f"(__uint_as_float(r[q].x)), "f"(__uint_as_float(r[q].y)),
+                                            "f"(__uint_as_float(r[q].z)), "f"(__uint_as_float(r[q].w)) : "memory");
                 }
+            } else if (m < g.Mo) {
+                float* c = g.C + (int64_t)m * g.ldc + c0;
+                for (int j = 0; j < 32; ++j) atomicAdd(c + j, v[j]);
             }
         }
     }
@@ -403,13 +487,6 @@ struct FusedArgs {
 
 constexpr uint32_t FUSED_SLOT = 64 * 1024;
 constexpr size_t FUSED_SMEM = 3 * (size_t)FUSED_SLOT;  // activation tile + two weight slots
-
-__device__ __forceinline__ uint32_t pack_bf16x2(float a, float b)
-{
-    const uint32_t lo = __bfloat16_as_ushort(__float2bfloat16(a));
-    const uint32_t hi = __bfloat16_as_ushort(__float2bfloat16(b));
-    return lo | (hi << 16);
-}
 
 // SiLU of the fused inference epilogue, the same expression as the layer kernels'
 __device__ __forceinline__ float silu_fast(float x) { return x * sigmoidf_(x); }
@@ -667,7 +744,7 @@ int sm_count()
     return n;
 }
 
-constexpr size_t kRowsSmemMax = (227 << 10) - 1024;  // less the kernel's static shared memory
+constexpr size_t kRowsSmemMax = (227 << 10) - 2048;  // less the kernel's static shared memory
 bool aligned16(const void* p) { return ((uintptr_t)p & 15) == 0; }
 
 }  // namespace
@@ -690,6 +767,7 @@ int mlp_launch_rows(const void* A, int64_t lda, const void* B, int64_t ldb, int6
     g.zp = (const bf16*)zp; g.ldzp = ldzp;
     g.Y = (bf16*)Y; g.ldy = ldy; g.YT = (bf16*)YT; g.ldyt = ldyt; g.Z = (bf16*)Z; g.ldz = ldz;
     g.Y32 = Y32; g.ldy32 = ldy32; g.colsum = colsum;
+    g.ytvec = YT && ldyt % 2 == 0 && ((uintptr_t)YT & 3) == 0;
     g.zvec = zp && ldzp % 8 == 0 && aligned16(zp);
     // half of the columns per CTA where that lets a second tile of A fit (A is
     // then read twice, from L2), as for N = K = 256; an output that overlaps A
