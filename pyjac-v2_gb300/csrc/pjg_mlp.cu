@@ -19,6 +19,7 @@
 //
 // Waits on mbarriers are bounded; on timeout the kernel records an error
 // (pjg_mlp_status) and finishes without hanging.
+#include <cuda.h>
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
 
@@ -467,201 +468,264 @@ __global__ void __launch_bounds__(kWThreads, 1) umma_wgrad_kernel(const WgradArg
 // ---------------------------------------------------------------------------
 // Fused forward pass of the whole network, 64 -> 256 -> 256 -> 256 -> 256 -> 64
 // (SiLU on the hidden layers), for inference.  A persistent CTA takes 128-row
-// tiles; a tile's activations stay in shared memory from layer to layer (the
-// epilogue of layer l writes the BF16 A operand of layer l + 1), so only the
-// features are read from and the FP32 outputs written to global memory.  The
-// weights stream from L2 through a two-slot ring of 64 KB: each chunk (W0,
-// each 128-row half of W1..W3, W4) is pre-packed in the no-swizzle core-matrix
-// layout, so one 1-D bulk copy moves it, completing on the slot's mbarrier.
-// Thread 0 issues the copies and the MMAs; the copies of the next layer's
-// weights run while 16 warps (four per TMEM lane quarter, each a quarter of
-// the columns) read the accumulator from TMEM and apply bias and SiLU.
+// tiles two at a time; a tile's activations stay in shared memory from layer to
+// layer (the epilogue of layer l writes the BF16 A operand of layer l + 1), so
+// only the features are read from and the FP32 outputs written to global memory.
+// The two tiles take turns: while one warp multiplies one (tcgen05, half of
+// TMEM each), 16 warps (four per TMEM lane quarter, each a quarter of the
+// columns) read the other's accumulator from TMEM and apply bias and SiLU.  The
+// weights stream from L2 through a ring of 16 KB slots, a slice of K = 32 of all
+// 256 columns each (K = 64 of the last layer's 64), one tensor copy per slice:
+// the packed weights are rows of core matrices to the tensor map, 8 columns each.
+// Bound by the hardware tanh (half the rate of the other special functions:
+// 452 us of 1,048,576 rows on GB300).  1022 us with one tile at a time, whose
+// layers multiplied, then applied SiLU; 1088 us with two tiles while one warp
+// copied and multiplied (its own instructions per slice cost more than the
+// slice); 745 us with a warp for each; 606 us with the biases in shared memory.
 struct FusedArgs {
+    CUtensorMap W[5];    // packed weights: 256x64, 256x256 (x3), 64x256
     const bf16* X;       // [M x 64] features
     int64_t ldx, M;
-    const uint8_t* W[5]; // packed weights: 256x64, 256x256 (x3), 64x256
     const float* b[5];
     float* Y;            // [M x 64] outputs
     int64_t ldy;
 };
 
-constexpr uint32_t FUSED_SLOT = 64 * 1024;
-constexpr size_t FUSED_SMEM = 3 * (size_t)FUSED_SLOT;  // activation tile + two weight slots
+constexpr uint32_t FUSED_SLOT = 16 * 1024;
+constexpr uint32_t FUSED_ACT = 64 * 1024;                 // activation tile
+constexpr int FUSED_SLOTS = 5;
+constexpr size_t FUSED_SMEM = 2 * (size_t)FUSED_ACT + FUSED_SLOTS * (size_t)FUSED_SLOT;
 
 // SiLU of the fused inference epilogue, the same expression as the layer kernels'
 __device__ __forceinline__ float silu_fast(float x) { return x * sigmoidf_(x); }
 
-constexpr int FUSED_THREADS = 512;  // 16 warps: four per TMEM lane quarter, each a quarter of the columns
+constexpr int FUSED_EPI = 512, FUSED_THREADS = FUSED_EPI + 64;  // 16 warps: four per TMEM lane quarter, each a quarter of the columns
 
-__global__ void __launch_bounds__(FUSED_THREADS, 1) mlp_fused_kernel(const FusedArgs g)
+template <int N>
+struct IntC {
+    static constexpr int value = N;
+};
+
+// bounded wait that also ends when another warp gave up
+__device__ __forceinline__ bool wait_or_abort(uint64_t* bar, uint32_t phase, volatile int* stop)
+{
+    bool ok = false;
+    for (uint32_t it = 0; it < (1u << 26); ++it) {
+        ok = umma::mbar_try_wait(bar, phase);
+        if (ok || ((it & 1023u) == 1023u && *stop)) break;
+    }
+    if (!ok) *stop = 1;
+    return ok;
+}
+
+__global__ void __launch_bounds__(FUSED_THREADS, 1) mlp_fused_kernel(const __grid_constant__ FusedArgs g)
 {
     extern __shared__ __align__(1024) uint8_t smem[];
-    __shared__ uint64_t full[2];
-    __shared__ uint64_t mmab;
+    __shared__ uint64_t full[FUSED_SLOTS], empty[FUSED_SLOTS];  // a slot's slice has arrived, is multiplied
+    __shared__ uint64_t ready[2], accum[2], drain;              // a tile's operand is written, is multiplied
     __shared__ uint32_t tmem_s;
     __shared__ int s_abort;
-    __shared__ float sbias[4 * 256 + 64];
+    __shared__ __align__(16) float sbias[4 * 256 + 64];
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const int quarter = warp & 3, part = warp >> 2;  // TMEM lanes 32 * quarter.., column quarter
-    uint8_t* sA = smem;
-    uint8_t* sW[2] = {smem + FUSED_SLOT, smem + 2 * FUSED_SLOT};
+    for (int i = tid; i < 4 * 256 + 64; i += FUSED_THREADS)
+        sbias[i] = i < 1024 ? g.b[i >> 8][i & 255] : g.b[4][i - 1024];
     if (warp == 0) {
-        umma::tmem_alloc(&tmem_s, 256);
+        umma::tmem_alloc(&tmem_s, 512);
         umma::tmem_relinquish();
     }
     if (tid == 0) {
-        umma::mbar_init(&full[0], 1);
-        umma::mbar_init(&full[1], 1);
-        umma::mbar_init(&mmab, 1);
+        for (int q = 0; q < FUSED_SLOTS; ++q) {
+            umma::mbar_init(&full[q], 1);
+            umma::mbar_init(&empty[q], 1);
+        }
+        for (int q = 0; q < 2; ++q) {
+            umma::mbar_init(&ready[q], FUSED_EPI / 32);
+            umma::mbar_init(&accum[q], 1);
+        }
+        umma::mbar_init(&drain, 1);
         s_abort = 0;
     }
-    for (int i = tid; i < 4 * 256 + 64; i += FUSED_THREADS)
-        sbias[i] = i < 1024 ? __ldg(g.b[i >> 8] + (i & 255)) : __ldg(g.b[4] + (i - 1024));
     umma::fence_before();
     __syncthreads();
     umma::fence_after();
     const uint32_t tmem = tmem_s;
-    const uint32_t sAu = umma::smem_u32(sA);
-    const uint32_t sWu[2] = {umma::smem_u32(sW[0]), umma::smem_u32(sW[1])};
-    // thread 0's copy bookkeeping: expected parity and copies in flight per slot
-    uint32_t fphase[2] = {0u, 0u}, mphase = 0u;
-    bool pending[2] = {false, false};
-    bool mma_late = false;  // an MMA whose completion wait ran out
-    auto issue = [&](int slot, const uint8_t* src, uint32_t bytes) {
-        umma::mbar_expect_tx(&full[slot], bytes);
-        umma::bulk_g2s(sW[slot], src, bytes, &full[slot]);
-        pending[slot] = true;
-    };
-    auto take = [&](int slot) -> bool {
-        const bool ok = umma::mbar_wait(&full[slot], fphase[slot]);
-        fphase[slot] ^= 1u;
-        pending[slot] = false;
-        return ok;
-    };
     const int64_t ntiles = (g.M + 127) / 128;
-    if (tid == 0 && blockIdx.x < ntiles) {
-        issue(0, g.W[0], 32 * 1024);
-        issue(1, g.W[1], FUSED_SLOT);
-    }
-    bool aborted = false;
-    for (int64_t t = blockIdx.x; t < ntiles && !aborted; t += gridDim.x) {
-        const int64_t row0 = t * 128;
-        const bool more = t + gridDim.x < ntiles;
-        // features -> A operand of layer 0 (K = 64: 8 chunks of 16 bytes per row)
-        for (int idx = tid; idx < 128 * 8; idx += FUSED_THREADS) {
-            const int r = idx >> 3, c = idx & 7;
-            const int64_t grow = row0 + r;
-            const bool ok = grow < g.M;
-            umma::cp_async16(sA + ((size_t)(r >> 3) * 8 + c) * 128 + (r & 7) * 16,
-                             g.X + (ok ? grow : 0) * g.ldx + c * 8, ok ? 16u : 0u);
-        }
-        umma::cp_async_wait_all();
-        umma::fence_proxy_async();
-        __syncthreads();
-        for (int l = 0; l < 5; ++l) {
-            if (tid == 0) {
-                umma::fence_after();
-                bool ok = true;
-                if (l == 0) {
-                    ok = take(0);
-                    const uint32_t id = umma::idesc_bf16(128, 256);
-                    for (int ks = 0; ks < 4; ++ks)
-                        umma::mma_bf16(tmem, umma::sdesc(sAu + ks * 256, 128, 8 * 128),
-                                       umma::sdesc(sWu[0] + ks * 256, 128, 8 * 128), id, ks ? 1u : 0u);
-                } else if (l < 4) {
-                    ok = take(1) & take(0);
-                    const uint32_t id = umma::idesc_bf16(128, 128);
-                    for (int h = 0; h < 2; ++h)  // half 0 (rows 0..127 of W) in slot 1, half 1 in slot 0
-                        for (int ks = 0; ks < 16; ++ks)
-                            umma::mma_bf16(tmem + 128u * h, umma::sdesc(sAu + ks * 256, 128, 32 * 128),
-                                           umma::sdesc(sWu[1 - h] + ks * 256, 128, 32 * 128), id,
-                                           ks ? 1u : 0u);
-                } else {
-                    ok = take(1);
-                    const uint32_t id = umma::idesc_bf16(128, 64);
-                    for (int ks = 0; ks < 16; ++ks)
-                        umma::mma_bf16(tmem, umma::sdesc(sAu + ks * 256, 128, 32 * 128),
-                                       umma::sdesc(sWu[1] + ks * 256, 128, 32 * 128), id, ks ? 1u : 0u);
-                }
-                umma::mma_commit(&mmab);
-                if (!ok) s_abort = 1;
-            }
-            const bool mok = umma::mbar_wait(&mmab, mphase);
-            if (!mok) {
-                if (lane == 0) s_abort = 1;
-                if (tid == 0) mma_late = true;
-            } else {
-                mphase ^= 1u;
-            }
-            umma::fence_after();
-            if (tid == 0) {
-                // the weights of the next layer (or the next tile's first layers)
-                if (l == 0) {
-                    issue(0, g.W[1] + FUSED_SLOT, FUSED_SLOT);
-                } else if (l < 3) {
-                    issue(1, g.W[l + 1], FUSED_SLOT);
-                    issue(0, g.W[l + 1] + FUSED_SLOT, FUSED_SLOT);
-                } else if (l == 3) {
-                    issue(1, g.W[4], 32 * 1024);
-                    if (more) issue(0, g.W[0], 32 * 1024);
-                } else if (more) {
-                    issue(1, g.W[1], FUSED_SLOT);
-                }
-            }
-            const int m = quarter * 32 + lane;
-            const int64_t grow = row0 + m;
-            const uint32_t trow = tmem + ((uint32_t)(quarter * 32) << 16);
-            if (l < 4) {
-                const float* bias = sbias + 256 * l;
-                for (int c0 = 64 * part; c0 < 64 * part + 64; c0 += 32) {
-                    float v[32];
-                    umma::tmem_ld32(trow + (uint32_t)c0, v);
+    const int mine = (int)((ntiles - blockIdx.x + gridDim.x - 1) / gridDim.x);  // grid <= ntiles
+    auto row_of = [&](int i) { return ((int64_t)blockIdx.x + (int64_t)i * gridDim.x) * 128; };
+    bool ok = true;
+    uint32_t phases = 0u;  // a bit per tile: of ready (the multiplying warp) or accum (the epilogue)
+
+    if (warp == FUSED_EPI / 32) {
+        // multiplies; one thread, with descriptors that only add to a word, because
+        // each instruction before an MMA delays it
+        if (lane == 0) {
+            const uint32_t a0 = umma::smem_u32(smem) >> 4, w0 = a0 + (2 * FUSED_ACT >> 4);
+            const uint32_t lbo = (128u >> 4) << 16;
+            auto desc = [&](uint32_t lo, uint32_t sbo) {
+                return ((uint64_t)((1u << 14) | (sbo >> 4)) << 32) | (lo | lbo);
+            };
+            int slot = 0;
+            uint32_t sphase = 0u;
+            auto step = [&](int b, int nch, auto nks_c, uint32_t asbo, uint32_t bsbo, uint32_t id) {
+                constexpr int nks = decltype(nks_c)::value;
+                ok = wait_or_abort(&ready[b], phases >> b & 1u, &s_abort);
+                phases ^= 1u << b;
+                uint64_t ad = desc(a0 + b * (FUSED_ACT >> 4), asbo);
+                uint32_t acc = 0u;
+                for (int c = 0; c < nch && ok; ++c, ad += nks * 16) {
+                    ok = wait_or_abort(&full[slot], sphase, &s_abort);
+                    if (!ok) break;
+                    umma::fence_after();
+                    const uint64_t bd = desc(w0 + slot * (FUSED_SLOT >> 4), bsbo);
 #pragma unroll
-                    for (int q = 0; q < 4; ++q) {
-                        uint32_t w[4];
-#pragma unroll
-                        for (int e = 0; e < 4; ++e)
-                            w[e] = pack_bf16x2(silu_fast(v[8 * q + 2 * e] + bias[c0 + 8 * q + 2 * e]),
-                                               silu_fast(v[8 * q + 2 * e + 1] + bias[c0 + 8 * q + 2 * e + 1]));
-                        const int c = (c0 >> 3) + q;
-                        *reinterpret_cast<uint4*>(sA + ((size_t)(m >> 3) * 32 + c) * 128 + (m & 7) * 16) =
-                            make_uint4(w[0], w[1], w[2], w[3]);
+                    for (int ks = 0; ks < nks; ++ks) {
+                        umma::mma_bf16(tmem + 256u * b, ad + ks * 16, bd + ks * 16, id, acc);
+                        acc = 1u;
+                    }
+                    umma::mma_commit(&empty[slot]);
+                    if (++slot == FUSED_SLOTS) {
+                        slot = 0;
+                        sphase ^= 1u;
                     }
                 }
-            } else if (part < 2) {
-                const float* bias = sbias + 1024;
-                const int c0 = 32 * part;
-                float v[32];
-                umma::tmem_ld32(trow + (uint32_t)c0, v);
-                if (grow < g.M) {
-                    float4* d = reinterpret_cast<float4*>(g.Y + grow * g.ldy + c0);
-#pragma unroll
-                    for (int q = 0; q < 8; ++q)
-                        d[q] = make_float4(v[4 * q] + bias[c0 + 4 * q], v[4 * q + 1] + bias[c0 + 4 * q + 1],
-                                           v[4 * q + 2] + bias[c0 + 4 * q + 2],
-                                           v[4 * q + 3] + bias[c0 + 4 * q + 3]);
-                }
+                if (ok) umma::mma_commit(&accum[b]);
+            };
+            for (int p = 0; 2 * p < mine && ok; ++p) {
+                const int nb = 2 * p + 1 < mine ? 2 : 1;
+                for (int b = 0; b < nb && ok; ++b)
+                    step(b, 2, IntC<2>{}, 8 * 128, 512, umma::idesc_bf16(128, 256));
+                for (int l = 1; l < 4; ++l)
+                    for (int b = 0; b < nb && ok; ++b)
+                        step(b, 8, IntC<2>{}, 32 * 128, 512, umma::idesc_bf16(128, 256));
+                for (int b = 0; b < nb && ok; ++b)
+                    step(b, 4, IntC<4>{}, 32 * 128, 1024, umma::idesc_bf16(128, 64));
             }
-            umma::fence_before();
-            umma::fence_proxy_async();
-            __syncthreads();
-            if (s_abort) {
-                aborted = true;
-                break;
+            // no MMA may still be reading or writing this CTA's memory when it exits
+            umma::mma_commit(&drain);
+            umma::mbar_wait(&drain, 0u);
+            if (!ok) atomicExch(&g_umma_err, 1);
+        }
+        __syncwarp();
+    } else if (warp == FUSED_EPI / 32 + 1) {
+        // copies the slices, layer by layer and a pair's tiles in turn
+        if (lane == 0) {
+            int slot = 0, n = 0;
+            uint32_t ephase = 1u, fphase = 0u;  // a slot's first use waits for nothing
+            for (int p = 0; 2 * p < mine && ok; ++p)
+                for (int l = 0; l < 5; ++l)
+                    for (int b = 0; b < 2 && 2 * p + b < mine && ok; ++b) {
+                        const int nch = l == 0 ? 2 : (l < 4 ? 8 : 4), width = l < 4 ? 128 : 256;
+                        for (int c = 0; c < nch && ok; ++c) {
+                            if (n >= FUSED_SLOTS) ok = wait_or_abort(&empty[slot], ephase, &s_abort);
+                            if (!ok) break;
+                            umma::mbar_expect_tx(&full[slot], l < 4 ? FUSED_SLOT : FUSED_SLOT / 2);
+                            umma::tensor_g2s_2d(smem + 2 * FUSED_ACT + slot * FUSED_SLOT, &g.W[l], c * width, 0, &full[slot]);
+                            ++n;
+                            if (++slot == FUSED_SLOTS) {
+                                slot = 0;
+                                ephase ^= 1u;
+                                fphase ^= 1u;
+                            }
+                        }
+                    }
+            // nor may a copy: the last use of every slot has arrived
+            for (int q = 0; q < FUSED_SLOTS && q < n; ++q) {
+                if (slot-- == 0) {
+                    slot = FUSED_SLOTS - 1;
+                    fphase ^= 1u;
+                }
+                umma::mbar_wait(&full[slot], fphase);
             }
         }
-    }
-    if (tid == 0) {
-        if (aborted) atomicExch(&g_umma_err, 1);
-        // no copy or MMA may still be writing this CTA's memory when it exits
-        for (int slot = 0; slot < 2; ++slot)
-            if (pending[slot]) take(slot);
-        if (mma_late) umma::mbar_wait(&mmab, mphase);
+        __syncwarp();
+    } else {
+        const int quarter = warp & 3, part = warp >> 2;  // TMEM lanes 32 * quarter.., column quarter
+        const int m = quarter * 32 + lane;
+        // this thread's two 16-byte pieces of a tile's features (8 per row), and
+        // their places in the A operand of layer 0
+        uint4 f[2];
+        auto load_x = [&](int i) {
+#pragma unroll
+            for (int q = 0; q < 2; ++q) {
+                const int idx = tid + q * FUSED_EPI;
+                const int64_t row = row_of(i) + (idx >> 3);
+                f[q] = row < g.M ? *reinterpret_cast<const uint4*>(g.X + row * g.ldx + (idx & 7) * 8)
+                                 : make_uint4(0, 0, 0, 0);
+            }
+        };
+        auto put_x = [&](int b) {
+#pragma unroll
+            for (int q = 0; q < 2; ++q) {
+                const int idx = tid + q * FUSED_EPI, r = idx >> 3, c = idx & 7;
+                *reinterpret_cast<uint4*>(smem + b * FUSED_ACT + ((r >> 3) * 8 + c) * 128 + (r & 7) * 16) = f[q];
+            }
+        };
+        auto publish = [&](int b) {  // this warp's share of a tile's operand is written, its accumulator read
+            umma::fence_before();
+            umma::fence_proxy_async();
+            __syncwarp();
+            if (lane == 0) umma::mbar_arrive(&ready[b]);
+        };
+        for (int b = 0; b < 2 && b < mine; ++b) {
+            load_x(b);
+            put_x(b);
+            publish(b);
+        }
+        for (int p = 0; 2 * p < mine && ok; ++p)
+            for (int l = 0; l < 5 && ok; ++l)
+                for (int b = 0; b < 2 && 2 * p + b < mine && ok; ++b) {
+                    const bool more = 2 * (p + 1) + b < mine;
+                    if (l == 4 && more) load_x(2 * (p + 1) + b);
+                    ok = __all_sync(0xffffffffu, wait_or_abort(&accum[b], phases >> b & 1u, &s_abort));
+                    if (!ok) break;
+                    phases ^= 1u << b;
+                    umma::fence_after();
+                    const uint32_t trow = tmem + 256u * b + ((uint32_t)(quarter * 32) << 16);
+                    if (l < 4) {
+                        const float* bias = sbias + 256 * l;
+                        uint8_t* dst = smem + b * FUSED_ACT + ((m >> 3) * 32) * 128 + (m & 7) * 16;
+#pragma unroll
+                        for (int h = 0; h < 2; ++h) {
+                            const int c0 = 64 * part + 32 * h;
+                            float v[32];
+                            umma::tmem_ld32(trow + (uint32_t)c0, v);
+#pragma unroll
+                            for (int q = 0; q < 4; ++q) {
+                                alignas(16) float bb[8];
+                                *reinterpret_cast<float4*>(bb) = *reinterpret_cast<const float4*>(bias + c0 + 8 * q);
+                                *reinterpret_cast<float4*>(bb + 4) = *reinterpret_cast<const float4*>(bias + c0 + 8 * q + 4);
+                                uint32_t w[4];
+#pragma unroll
+                                for (int e = 0; e < 4; ++e)
+                                    w[e] = pack_bf16x2(silu_fast(v[8 * q + 2 * e] + bb[2 * e]),
+                                                       silu_fast(v[8 * q + 2 * e + 1] + bb[2 * e + 1]));
+                                *reinterpret_cast<uint4*>(dst + ((c0 >> 3) + q) * 128) = make_uint4(w[0], w[1], w[2], w[3]);
+                            }
+                        }
+                        publish(b);
+                    } else {
+                        const int c0 = 16 * part;
+                        float v[16];
+                        umma::tmem_ld16(trow + (uint32_t)c0, v);
+                        if (more) put_x(b);
+                        publish(b);
+                        uint4 r[4];
+#pragma unroll
+                        for (int q = 0; q < 4; ++q) {
+                            const float4 bb = *reinterpret_cast<const float4*>(sbias + 1024 + c0 + 4 * q);
+                            r[q] = make_uint4(__float_as_uint(v[4 * q] + bb.x), __float_as_uint(v[4 * q + 1] + bb.y),
+                                              __float_as_uint(v[4 * q + 2] + bb.z), __float_as_uint(v[4 * q + 3] + bb.w));
+                        }
+                        store_rows64(reinterpret_cast<uint8_t*>(g.Y + c0), g.ldy * 4,
+                                     row_of(2 * p + b) + quarter * 32, g.M, r, lane);
+                    }
+                }
+        if (!ok && lane == 0) atomicExch(&g_umma_err, 1);
     }
     umma::fence_before();
     __syncthreads();
     umma::fence_after();
-    if (warp == 0) umma::tmem_dealloc(tmem, 256);
+    if (warp == 0) umma::tmem_dealloc(tmem, 512);
 }
 
 // ---------------------------------------------------------------------------
@@ -745,6 +809,23 @@ int sm_count()
 }
 
 constexpr size_t kRowsSmemMax = (227 << 10) - 2048;  // less the kernel's static shared memory
+// cuTensorMapEncodeTiled of the loaded driver (the library does not link libcuda)
+using EncodeTiled = CUresult (*)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*, const cuuint64_t*,
+                                 const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave, CUtensorMapSwizzle,
+                                 CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
+EncodeTiled tensor_map_encoder()
+{
+    static const EncodeTiled fn = [] {
+        void* p = nullptr;
+        cudaDriverEntryPointQueryResult found;
+        if (cudaGetDriverEntryPointByVersion("cuTensorMapEncodeTiled", &p, 12000, cudaEnableDefault, &found) != cudaSuccess ||
+            found != cudaDriverEntryPointSuccess)
+            p = nullptr;
+        return reinterpret_cast<EncodeTiled>(p);
+    }();
+    return fn;
+}
+
 bool aligned16(const void* p) { return ((uintptr_t)p & 15) == 0; }
 
 }  // namespace
@@ -824,14 +905,23 @@ int mlp_launch_fused(const void* X, int64_t ldx, int64_t M, const void* const* W
     if (M <= 0) return 0;
     if (!X || !Y || ldx % 8 || ldy % 4 || ldx < 64 || ldy < 64 || !aligned16(X) || !aligned16(Y))
         return -1;
+    const auto encode = tensor_map_encoder();
+    if (!encode) return -2;
     FusedArgs g;
     g.X = (const bf16*)X;
     g.ldx = ldx;
     g.M = M;
     for (int l = 0; l < 5; ++l) {
         if (!W[l] || !b[l] || !aligned16(W[l])) return -1;
-        g.W[l] = (const uint8_t*)W[l];
         g.b[l] = b[l];
+        // rows of 8 columns' core matrices, as 32-bit words; a slice is K = 32 (the last layer: 64) of every row
+        const cuuint64_t dims[2] = {(cuuint64_t)(l ? 1024 : 256), (cuuint64_t)(l < 4 ? 32 : 8)};
+        const cuuint64_t pitch[1] = {dims[0] * 4};
+        const cuuint32_t box[2] = {l < 4 ? 128u : 256u, (cuuint32_t)dims[1]}, ones[2] = {1, 1};
+        if (encode(&g.W[l], CU_TENSOR_MAP_DATA_TYPE_UINT32, 2, const_cast<void*>(W[l]), dims, pitch, box, ones,
+                   CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+                   CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
+            return -2;
     }
     g.Y = Y;
     g.ldy = ldy;

@@ -75,3 +75,29 @@ def test_wgrad_ring(cuda_device, Mo, No, Kb, cpad):
     ops.wgrad(A, B, C)
     assert ops.status() == 0
     assert rel(C, 1 + A.double() @ B.double().t()) < 5e-5
+
+
+@pytest.mark.parametrize("M", [1, 129, 152 * 128, 152 * 128 + 1, 304 * 128 + 1, 100001])
+@pytest.mark.parametrize("off", [0, 1])
+def test_fused_forward_ring(cuda_device, M, off):
+    """One and two CTAs per SM, one and several tiles per CTA, unaligned biases;
+    the layers one by one give the same roundings, so 1e-2 only allows for a
+    few activations that round the other way."""
+    import torch
+    ops = pkg("mlp_ops")
+    torch.manual_seed(M)
+    dims = [(256, 64)] + [(256, 256)] * 3 + [(64, 256)]
+    W = [(torch.randn(n, k, device=cuda_device) / k ** 0.5).bfloat16() for n, k in dims]
+    b = [torch.randn(n + off, device=cuda_device)[off:] for n, _ in dims]
+    a = X = torch.randn(M, 64, device=cuda_device).bfloat16()
+    Y = torch.full((M + 1, 64), 7.0, device=cuda_device)
+    ops.forward_fused(X, [ops.pack_core(w) for w in W], b, Y=Y[:M])
+    for l in range(4):
+        n = torch.empty(M, 256, device=cuda_device, dtype=torch.bfloat16)
+        ops.linear(a, W[l], bias=b[l], act=True, Y=n)
+        a = n
+    ref = torch.empty(M, 64, device=cuda_device)
+    ops.linear(a, W[4], bias=b[4], Y32=ref)
+    assert ops.status() == 0
+    assert rel(Y[:M], ref.double()) < 1e-2
+    assert bool((Y[M] == 7.0).all())
