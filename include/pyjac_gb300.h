@@ -174,6 +174,10 @@ int pjg_mlp_linear(const void* X, int64_t ldx, const void* W, int64_t ldw, int64
                    float* colsum, void* stream);
 int pjg_mlp_wgrad(const void* A, int64_t lda, const void* B, int64_t ldb, int Mo, int No,
                   int64_t Kb, float* C, int64_t ldc, void* stream);
+/* dY [M x 64] (FP32) -> Z = BF16(dY), ZT = Z^T (ZT[n * ldzt + m]) and colsum +=
+ * column sums of dY: the operands of the last layer's gradients. */
+int pjg_mlp_head_grad(const float* dY, int64_t ldy, int64_t M, void* Z, int64_t ldz, void* ZT,
+                      int64_t ldzt, float* colsum, void* stream);
 int pjg_mlp_status(int clear);
 /* The whole surrogate forward pass in one launch: Y [M x 64] (FP32) =
  * L4(SiLU(L3(SiLU(L2(SiLU(L1(SiLU(L0(X)))))))) for X [M x 64] BF16, where

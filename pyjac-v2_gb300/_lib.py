@@ -53,6 +53,8 @@ SIGNATURES = [
     ("pjg_mlp_wgrad", ctypes.c_int,
      [_VP, ctypes.c_int64, _VP, ctypes.c_int64, ctypes.c_int, ctypes.c_int, ctypes.c_int64, _VP,
       ctypes.c_int64, _VP]),
+    ("pjg_mlp_head_grad", ctypes.c_int,
+     [_VP, ctypes.c_int64, ctypes.c_int64, _VP, ctypes.c_int64, _VP, ctypes.c_int64, _VP, _VP]),
     ("pjg_mlp_status", ctypes.c_int, [ctypes.c_int]),
     ("pjg_surrogate_features", ctypes.c_int,
      [ctypes.c_int64, ctypes.c_int32, _VP, _VP, _VP, _VP, ctypes.c_double, _VP]),

@@ -1114,6 +1114,17 @@ int pjg_mlp_wgrad(const void* A, int64_t lda, const void* B, int64_t ldb, int Mo
     return 0;
 }
 
+int pjg_mlp_head_grad(const float* dY, int64_t ldy, int64_t M, void* Z, int64_t ldz, void* ZT, int64_t ldzt,
+                      float* colsum, void* stream)
+{
+    const int rc = mlp_launch_head(dY, ldy, M, Z, ldz, ZT, ldzt, colsum, stream);
+    if (rc == -1)
+        return fail(PJG_ERR_ARG, "pjg_mlp_head_grad: null or misaligned operand (leading dims %% 4)");
+    if (rc) return fail(PJG_ERR_CUDA, "pjg_mlp_head_grad launch failed: %s", cudaGetErrorString(cudaGetLastError()));
+    g_launches.fetch_add(1);
+    return 0;
+}
+
 int pjg_mlp_status(int clear) { return mlp_error_flag(clear); }
 
 int pjg_surrogate_features(int64_t n, int32_t nn, const double* phi, const double* param,

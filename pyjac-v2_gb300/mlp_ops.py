@@ -65,6 +65,20 @@ def wgrad(A, B, C):
     return C
 
 
+def head_grad(dY, Z, ZT, colsum):
+    """Z = bf16(dY), ZT = Z^T and colsum += dY.sum(0), in one pass over dY [M, 64] fp32."""
+    lib = _lib.load()
+    _check(dY, torch.float32, "dY")
+    _check(Z, torch.bfloat16, "Z")
+    _check(ZT, torch.bfloat16, "ZT")
+    if dY.shape[1] != 64:
+        raise ValueError("dY must be [M, 64]")
+    st = torch.cuda.current_stream(dY.device).cuda_stream
+    _lib.check("pjg_mlp_head_grad", lib.pjg_mlp_head_grad(
+        _ptr(dY), _ld(dY), dY.shape[0], _ptr(Z), _ld(Z), _ptr(ZT), _ld(ZT), _ptr(colsum), st))
+    return Z, ZT
+
+
 def pack_core(W):
     """BF16 [N, K] -> the core-matrix layout of pjg_mlp_forward (N, K multiples of 8):
     8-row x 16-byte blocks, row-group major, then K."""

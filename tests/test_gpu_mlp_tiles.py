@@ -101,3 +101,36 @@ def test_fused_forward_ring(cuda_device, M, off):
     assert ops.status() == 0
     assert rel(Y[:M], ref.double()) < 1e-2
     assert bool((Y[M] == 7.0).all())
+
+
+@pytest.mark.parametrize("M", [1, 63, 64, 1000, 152 * 64 * 4 + 65])
+def test_head_grad(cuda_device, M):
+    """Column sums: FP32 over M rows in partial sums, 1e-5 of the sum of magnitudes."""
+    import torch
+    ops = pkg("mlp_ops")
+    torch.manual_seed(M)
+    dY = torch.randn(M, 64, device=cuda_device)
+    Z = torch.empty(M, 64, device=cuda_device, dtype=torch.bfloat16)
+    ZT = torch.empty(64, M, device=cuda_device, dtype=torch.bfloat16)
+    cs = torch.ones(64, device=cuda_device)
+    ops.head_grad(dY, Z, ZT, cs)
+    assert torch.equal(Z, dY.bfloat16()) and torch.equal(ZT, dY.bfloat16().t())
+    d = (cs.double() - 1 - dY.double().sum(0)).abs().max()
+    assert float(d) < 1e-5 * float(1 + dY.double().abs().sum(0).max())
+
+
+def test_backward_takes_any_layout_of_its_gradient(cuda_device):
+    import torch
+    net = pkg("surrogate").MLP(torch.device(cuda_device))
+    X = torch.randn(128, 64, device=cuda_device).bfloat16()
+    XT = X.t().contiguous()
+    dY = torch.randn(128, 64, device=cuda_device)
+    out = []
+    for d in (dY, dY.t().contiguous().t(), torch.cat([dY, dY], 1)[:, :64]):
+        net.forward(X, keep=True)
+        gW, gb = net.backward(XT, d)
+        out.append(gW + gb)
+    for o in out[1:]:
+        for a, b in zip(out[0], o):
+            assert a.shape == b.shape and a.dtype == b.dtype
+            assert float((a - b).abs().max()) <= 1e-5 * float(b.abs().max()) + 1e-30
