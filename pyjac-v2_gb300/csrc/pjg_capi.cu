@@ -469,7 +469,12 @@ bool wave_sooner(const pjg_mech* m, int kind, int64_t rest)
     bool fits = false;
     for (int slog = 5; slog >= 0 && !fits; --slog) fits = shape_fits(m, kind, slog, 8, &s);
     if (!fits) return true;  // no tile of this mechanism fits in shared memory
-    const double share = s.slog < 5 ? 0.25 : kind == PJG_JACOBIAN ? 0.75 : 0.45;
+    // short item lists keep a tile's warps waiting on its barriers, so a small
+    // mechanism's tiles gain less; sum_parts draws the same line.  H2/O2 C, us,
+    // thread per state / tiles: Jacobian 32,000 states 300 / 318, 50,000 361 / 487;
+    // rates 27,000 114 / 100, 38,000 115 / 142, 50,000 146 / 180.
+    const bool small = sum_parts(m->ns) == 1;
+    const double share = s.slog < 5 ? 0.25 : kind == PJG_JACOBIAN ? (small ? 0.375 : 0.75) : kind == PJG_KIND_VJP ? 0.45 : small ? 0.25 : 0.45;
     return rest >= (int64_t)(share * wave_states(m, kind));
 }
 
