@@ -49,9 +49,9 @@ METRIC = "GRI-30 FP64 Jacobians/s"
 UNIT = "Jacobians/s"
 # per --kernel: metric, unit, evaluation kernel
 KERNELS = {
-    "jacobian": (METRIC, UNIT, "eval_kernel<1> (fused Jacobian)"),
-    "rates": ("GRI-30 FP64 species-rate evaluations/s", "states/s", "eval_kernel<0> (species rates)"),
-    "vjp": ("GRI-30 FP64 J^T v products/s", "states/s", "eval_kernel<2> (J^T v)"),
+    "jacobian": (METRIC, UNIT, "wave_kernel<1> (fused Jacobian)"),
+    "rates": ("GRI-30 FP64 species-rate evaluations/s", "states/s", "wave_kernel<0> (species rates)"),
+    "vjp": ("GRI-30 FP64 J^T v products/s", "states/s", "wave_kernel<2> (J^T v)"),
 }
 KIND = {"rates": 0, "jacobian": 1, "vjp": 2}
 # executed FP64 instruction / DRAM counts per state (ncu captures, profiles/)
