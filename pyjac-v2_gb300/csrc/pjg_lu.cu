@@ -366,6 +366,32 @@ __global__ void __launch_bounds__(32 * S * kWarpsPerState) lu_sparse_kernel(long
     }
 }
 
+// y_r - sum over a row's pattern entries of lu_rc y_c, one FMA each in order.
+// The factor entries come kAhead at a time: taken one by one, each waited for
+// memory before the next was asked for.  A ROS2 step with the sparse solves on GB300:
+// GRI F 100 states 1.43 -> 0.87 ms, 20,000 6.28 -> 5.16, 70,000 14.5 -> 13.5;
+// C 20,000 5.63 -> 5.21.
+constexpr int kAhead = 8;
+
+template <bool F>
+__device__ __forceinline__ double row_dot(int nn, long long n, long long i, int r, int q0, int q1,
+                                          const int* __restrict__ idx, const double* __restrict__ lu, const double* y)
+{
+    double acc = y[r];
+    for (int q = q0; q < q1; q += kAhead) {
+        double v[kAhead];
+        int c[kAhead];
+#pragma unroll
+        for (int j = 0; j < kAhead; ++j) c[j] = __ldg(idx + (q + j < q1 ? q + j : q));
+#pragma unroll
+        for (int j = 0; j < kAhead; ++j) v[j] = __ldg(lu + mat_idx(F, i, n, nn, r, c[j]));
+#pragma unroll
+        for (int j = 0; j < kAhead; ++j)
+            if (q + j < q1) acc = fma(-v[j], y[c[j]], acc);
+    }
+    return acc;
+}
+
 // one thread per state: y = P b, L y = y and U x = y over the filled pattern
 // only (row-oriented FMA dot products in increasing column order), x back to
 // the variables' order
@@ -379,19 +405,10 @@ __global__ void __launch_bounds__(128) lu_sparse_solve_kernel(long long n, const
     double y[kSolveNMax];
     for (int r = 0; r < nn; ++r) y[r] = b[vec_idx(F, i, n, nn, __ldg(pl.perm + r))];
     for (int r = 1; r < nn; ++r) {
-        double acc = y[r];
-        for (int q = __ldg(pl.loff + r); q < __ldg(pl.loff + r + 1); ++q) {
-            const int c = __ldg(pl.lidx + q);
-            acc = fma(-__ldg(lu + mat_idx(F, i, n, nn, r, c)), y[c], acc);
-        }
-        y[r] = acc;
+        y[r] = row_dot<F>(nn, n, i, r, __ldg(pl.loff + r), __ldg(pl.loff + r + 1), pl.lidx, lu, y);
     }
     for (int r = nn - 1; r >= 0; --r) {
-        double acc = y[r];
-        for (int q = __ldg(pl.uoff + r); q < __ldg(pl.uoff + r + 1); ++q) {
-            const int c = __ldg(pl.uidx + q);
-            acc = fma(-__ldg(lu + mat_idx(F, i, n, nn, r, c)), y[c], acc);
-        }
+        const double acc = row_dot<F>(nn, n, i, r, __ldg(pl.uoff + r), __ldg(pl.uoff + r + 1), pl.uidx, lu, y);
         y[r] = acc / __ldg(lu + mat_idx(F, i, n, nn, r, r));
     }
     for (int r = 0; r < nn; ++r) b[vec_idx(F, i, n, nn, __ldg(pl.perm + r))] = y[r];
