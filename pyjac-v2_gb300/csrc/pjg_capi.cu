@@ -987,9 +987,14 @@ void device_records(pjg_mech* m, const double* species, std::vector<int4>& m_lis
     auto key = [](const PjgRxn& R) { return std::make_pair(R.thd_off * 2 + (R.thd_cnt > 0), R.p[P_FLAG]); };
     for (const PjgRxn& R : m->h_rxn)
         if (RX_THD(R.flags) != THD_NONE) ++uses[key(R)];
-    // x 2^B / ln 2 as an integer and a rest
+    // x 2^B / ln 2 as an integer and a rest; infinities (ln A of A = 0) stay whole
     auto cut = [](long double x, int* n, double* rest) {
         x = x * 1.4426950408889634073599246810018921L * PJG_EXP_TAB;
+        if (!(std::abs(x) < 1e9L)) {
+            *n = 0;
+            *rest = (double)x;
+            return;
+        }
         const long double r = nearbyintl(x);
         *n = (int)r;
         *rest = (double)(x - r);
@@ -1024,7 +1029,9 @@ void device_records(pjg_mech* m, const double* species, std::vector<int4>& m_lis
         if (m->cls[i] == 0) R.flags |= RX_E22;
         const int blend = RX_BLEND(R.flags);
         if (RX_FORM(R.flags) == FORM_ARR) cut(H.p[P_A], &R.bint, &R.p[P_A]);
-        if (blend != BL_NONE && RX_FORM(R.flags) == FORM_ARR && RX_FFORM(R.flags) == FORM_ARR) {
+        // (k0 / kinf is not one exponential where either is zero)
+        if (blend != BL_NONE && RX_FORM(R.flags) == FORM_ARR && RX_FFORM(R.flags) == FORM_ARR &&
+            std::isfinite(H.p[P_A]) && std::isfinite(H.p[P_FA])) {
             const int sg = R.flags & RX_CHEM ? -1 : 1;  // the other rate is k0 in a fall-off
             cut(sg * ((long double)H.p[P_FA] - H.p[P_A]), &R.fbint, &R.p[P_RA]);
             R.p[P_RB] = sg * (H.p[P_FB] - H.p[P_B]);
@@ -1032,6 +1039,7 @@ void device_records(pjg_mech* m, const double* species, std::vector<int4>& m_lis
             R.p[P_RN] = R.fbint;
             R.flags |= RX_RATIO;
         } else if (blend != BL_NONE && RX_FFORM(R.flags) == FORM_ARR) {
+            // (also where ln A0 or ln Ainf is infinite)
             cut(H.p[P_FA], &R.fbint, &R.p[P_FA]);
         }
         R.list = -1;

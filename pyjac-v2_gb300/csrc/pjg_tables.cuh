@@ -57,7 +57,7 @@
 #define RX_E22 (1 << 22)      // of the elementary class A + B <=> C + D
 #define RX_WE (1 << 23)       // the weight in row E, sum nu_k (1 - W_k / W_ns), is not zero
 #define RX_WEREAL (1 << 24)   // and not sum nu (mass not conserved): it is P_WE
-#define RX_RATIO (1 << 25)    // k0 / kinf is one exponential (P_RA..): both are FORM_ARR
+#define RX_RATIO (1 << 25)    // k0 / kinf is one exponential (P_RA..): both are FORM_ARR, neither zero
 
 #define RX_FORM(f) ((f) & RX_FORM_MASK)
 #define RX_THD(f) (((f) >> RX_THD_SHIFT) & 3)
