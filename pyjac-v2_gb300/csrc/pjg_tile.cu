@@ -67,6 +67,8 @@ __global__ void __launch_bounds__(KIND == KIND_RATES ? 256 : 512, KIND == KIND_R
     const int slog = a.sc.slog, S = 1 << slog, wpw = 32 >> slog;  // states, workers per warp
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int st = lane & (S - 1), grp = lane >> slog, wk = warp * wpw + grp, G = a.sc.warps * wpw;
+    // the worker's lanes: they share its items, so they refill them together
+    const unsigned own_lanes = ((slog == 5 ? 0u : 1u << S) - 1u) << (grp << slog);
     constexpr int kArr = tile_arrays(KIND);
     const int cap = item_stage(slog);
     uint2* stage = reinterpret_cast<uint2*>(smem + kTileStatic / sizeof(double)) + wk * cap;
@@ -405,11 +407,10 @@ __global__ void __launch_bounds__(KIND == KIND_RATES ? 256 : 512, KIND == KIND_R
 #pragma unroll 1
                 for (; q < q1; q += kItemUnroll) {
                     if (q == limit) {  // the next items of a long batch
-                        const unsigned lanes = __activemask();
-                        __syncwarp(lanes);
+                        __syncwarp(own_lanes);
                         fill(q);
                         asm volatile("cp.async.wait_all;" ::: "memory");
-                        __syncwarp(lanes);
+                        __syncwarp(own_lanes);
                         limit = q + cap;
                     }
                     uint2 it[kItemUnroll];
