@@ -48,13 +48,13 @@ class MLP(object):
         for din, dout in self.dims:
             w = torch.randn(dout, din, generator=g, dtype=torch.float64) * math.sqrt(1.7 / din)
             self.W.append(w.float().to(device))
-            self.b.append(torch.zeros(dout, device=device))
+            self.b.append(torch.zeros(dout, dtype=torch.float32, device=device))
         self.W[0][:, NIN:] = 0.0
         self.W[-1][ERR + 1:, :] = 0.0
         self.W[-1] *= 0.3
-        self.mask_in = torch.zeros(HID, NIN_P, device=device)
+        self.mask_in = torch.zeros(HID, NIN_P, dtype=torch.float32, device=device)
         self.mask_in[:, :NIN] = 1.0
-        self.mask_out = torch.zeros(NOUT_P, HID, device=device)
+        self.mask_out = torch.zeros(NOUT_P, HID, dtype=torch.float32, device=device)
         self.mask_out[:ERR + 1] = 1.0
         self.m = [torch.zeros_like(w) for w in self.W] + [torch.zeros_like(b) for b in self.b]
         self.v = [torch.zeros_like(w) for w in self.W] + [torch.zeros_like(b) for b in self.b]
@@ -106,7 +106,7 @@ class MLP(object):
         L = self.depth
         # the accumulated gradients are pieces of one zeroed buffer
         params = self.W + self.b
-        flat = torch.zeros(sum(p.numel() for p in params), device=self.device)
+        flat = torch.zeros(sum(p.numel() for p in params), dtype=torch.float32, device=self.device)
         g = [x.view(p.shape) for x, p in zip(flat.split([p.numel() for p in params]), params)]
         gW, gb = g[:L + 1], g[L + 1:]
         if (type(dY) is torch.Tensor and dY.is_cuda and dY.dtype == torch.float32 and dY.dim() == 2
