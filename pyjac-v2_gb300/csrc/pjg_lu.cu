@@ -1101,10 +1101,12 @@ extern "C" int pjg_internal_lu_solve(int32_t nn, int64_t n, char order, const do
             else lu_solve_lane_kernel<false><<<grid, 128, 0, st>>>(nn, n, lu, piv, b);
         } else {
             auto kern = order == 'F' ? lu_solve_kernel<true> : lu_solve_kernel<false>;
-            const size_t smem = solve_smem(nn);
-            if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
+            // always the largest size: the attribute is the kernel's, and another
+            // thread may be about to launch it for a larger nn
+            if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)solve_smem(kSolveNMax)) !=
+                cudaSuccess)
                 return pjg_internal_fail(PJG_ERR_CUDA, "cannot reserve shared memory for the LU solve kernel");
-            kern<<<(unsigned)((n + 31) / 32), 32 * kSolveWarps, smem, st>>>(nn, n, lu, piv, b);
+            kern<<<(unsigned)((n + 31) / 32), 32 * kSolveWarps, solve_smem(nn), st>>>(nn, n, lu, piv, b);
         }
     }
     pjg_internal_count_launch();
