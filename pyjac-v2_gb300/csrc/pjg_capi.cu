@@ -99,7 +99,7 @@ struct WaveHold {
     WaveTables wt;
     const PostItem* ns_post = nullptr;
     int n_ns_post = 0, n_vec = 0;
-    char* buffer = nullptr;
+    bool made = false;
 };
 
 // a tile shape's schedule on the device, with its third-body bath-gas terms (J^T v)
@@ -107,7 +107,17 @@ struct SchedTables {
     Schedule sc;
     const PostItem* ns_post = nullptr;
     int n_ns_post = 0;
-    char* buffer = nullptr;
+    int resident = 0;  // blocks that the device holds at a time
+    bool made = false;
+};
+
+// the evaluation kernels' tables of one (kind, output layout)
+struct KindTables {
+    bool listed = false;
+    SchedAdds adds;
+    WaveHold wave;
+    SchedTables tile[6];  // by log2 of the tile's states
+    std::vector<char*> buffers;
 };
 
 }  // namespace
@@ -141,8 +151,7 @@ struct pjg_mech {
     std::vector<double> h_thd_coef;
     std::vector<int> crs_ptr, crs_ind, ccs_ptr, ccs_ind;
     std::map<int, SlotTables> slots;  // key: (order == 'F') * 2 + sparse
-    std::map<int, SchedTables> scheds;  // key: kind, layout, tile shape
-    std::map<int, WaveHold> waves;      // key: kind * 4 + layout
+    std::map<int, KindTables> tables;  // key: kind * 4 + layout
     std::mutex lock;
     // working buffer shared by device-pointer calls on this mechanism
     double* work = nullptr;
@@ -195,8 +204,12 @@ int slot_of(const pjg_mech* m, bool F, bool sparse, int r, int c)
     return -1;
 }
 
-SchedInput sched_input(const pjg_mech* m, int kind, const std::vector<int>* slot)
+// The additions of a kind and layout (slot: the Jacobian's species-block
+// slots).  Called with the mechanism's lock held.
+KindTables& kind_tables(pjg_mech* m, int kind, int layout, const std::vector<int>* slot)
 {
+    KindTables& kt = m->tables[kind * 4 + layout];
+    if (kt.listed) return kt;
     SchedInput in;
     in.kind = kind;
     in.ns = m->ns;
@@ -206,7 +219,9 @@ SchedInput sched_input(const pjg_mech* m, int kind, const std::vector<int>* slot
     in.thd_spec = &m->h_thd_spec;
     in.thd_coef = &m->h_thd_coef;
     in.slot = slot;
-    return in;
+    sched_adds(in, kt.adds);
+    kt.listed = true;
+    return kt;
 }
 
 int build_slots(pjg_mech* m, bool F, bool sparse, SlotTables** out)
@@ -249,12 +264,7 @@ int build_slots(pjg_mech* m, bool F, bool sparse, SlotTables** out)
             ns_slots.push_back(sl);
         }
     }
-    {
-        SchedInput in = sched_input(m, PJG_JACOBIAN, &t.slot);
-        SchedHost sh;
-        sched_build(in, 5, 8, 1, 1 << 10, sh);
-        left_out = left_out || sh.left_out;
-    }
+    left_out = left_out || kind_tables(m, PJG_JACOBIAN, key, &t.slot).adds.left_out;
     std::vector<int> sp_slots(2 * std::max(last, 1), -1), cj_slots(2 * std::max(last, 1), -1), col_off;
     std::vector<int2> col_list;
     for (int k = 0; k < last; ++k) {
@@ -367,83 +377,75 @@ bool shape_fits(const pjg_mech* m, int kind, int slog, int warps, Shape* out)
     return false;
 }
 
-int choose_shape(const pjg_mech* m, int kind, int64_t n, Shape* out)
+// The tile shape for n states (log2 of a tile's states), or -1.
+int choose_shape(const pjg_mech* m, int kind, int64_t n)
 {
     const int sms = sm_count(m);
-    bool any = false;
+    int found = -1;
     for (int slog = 5; slog >= 0; --slog) {
-        const int64_t tiles = (n + (1 << slog) - 1) >> slog;
         Shape s;
         if (!shape_fits(m, kind, slog, 8, &s)) continue;
-        *out = s;
-        any = true;
-        if (tiles >= 2 * sms) break;
+        found = slog;
+        if ((n + (1 << slog) - 1) >> slog >= 2 * sms) break;
     }
-    if (!any) return fail(PJG_ERR_UNSUPPORTED, "mechanism too large for the evaluation kernels");
-    return 0;
+    return found;
 }
 
-int sched_tables(pjg_mech* m, int kind, int layout, const std::vector<int>* slot, const Shape& sh, SchedTables** out)
+// The tables of a kind and layout that are not there yet: the shapes from ..
+// to (those that fit), and with `wave` the thread-per-state kernel's.
+int make_tables(pjg_mech* m, int kind, int layout, const std::vector<int>* slot, int from, int to, bool wave,
+                KindTables** out)
 {
-    const int key = ((kind * 4 + layout) * 8 + sh.slog) * 32 + sh.warps;
     std::lock_guard<std::mutex> g(m->lock);
-    auto it = m->scheds.find(key);
-    if (it != m->scheds.end()) {
-        *out = &it->second;
-        return 0;
-    }
-    SchedHost h;
-    if (!sched_build(sched_input(m, kind, slot), sh.slog, sh.warps, sh.rounds, sh.buf_terms, h))
-        return fail(PJG_ERR_UNSUPPORTED, "a reaction's terms pass the evaluation kernel's buffer");
-    SchedTables t;
-    t.sc.slog = h.slog;
-    t.sc.warps = h.warps;
-    t.sc.rounds = h.rounds;
-    t.sc.n_batch = h.n_batch;
-    t.sc.buf_terms = h.buf_terms;
-    t.sc.n_vec = h.n_vec;
-    t.n_ns_post = (int)h.ns_post.size();
-    int rc;
+    KindTables& kt = kind_tables(m, kind, layout, slot);
+    const SchedAdds& ad = kt.adds;
+    *out = &kt;
     Pack pk;
-    pk.add(h.tasks, &t.sc.tasks);
-    pk.add(h.term_off, &t.sc.term_off);
-    pk.add(h.item_off, &t.sc.item_off);
-    pk.add(h.items, &t.sc.items);
-    pk.add(h.post_off, &t.sc.post_off);
-    pk.add(h.post, &t.sc.post);
-    pk.add(h.ns_post, &t.ns_post);
-    if ((rc = pk.send(&t.buffer))) return rc;
-    *out = &m->scheds.emplace(key, t).first->second;
-    return 0;
-}
-
-int wave_tables(pjg_mech* m, int kind, int layout, const std::vector<int>* slot, WaveHold** out)
-{
-    const int key = kind * 4 + layout;
-    std::lock_guard<std::mutex> g(m->lock);
-    auto it = m->waves.find(key);
-    if (it != m->waves.end()) {
-        *out = &it->second;
-        return 0;
+    std::vector<bool*> made;
+    for (int slog = from; slog <= to; ++slog) {
+        SchedTables& t = kt.tile[slog];
+        Shape sh;
+        if (t.made || !shape_fits(m, kind, slog, 8, &sh)) continue;
+        SchedHost h;
+        if (!sched_build(ad, slog, sh.warps, sh.rounds, sh.buf_terms, h))
+            return fail(PJG_ERR_UNSUPPORTED, "a reaction's terms pass the evaluation kernel's buffer");
+        t.sc.slog = slog;
+        t.sc.warps = sh.warps;
+        t.sc.rounds = sh.rounds;
+        t.sc.n_batch = h.n_batch;
+        t.sc.buf_terms = sh.buf_terms;
+        t.sc.n_vec = ad.n_vec;
+        t.n_ns_post = (int)ad.ns_post.size();
+        t.resident = sm_count(m) * pjg_tile_blocks_per_sm(kind, sh.warps, pjg_tile_smem(kind, m->ns, m->n_m, slog, sh.warps, sh.buf_terms));
+        pk.add(h.tasks, &t.sc.tasks);
+        pk.add(h.term_off, &t.sc.term_off);
+        pk.add(h.item_off, &t.sc.item_off);
+        pk.add(h.items, &t.sc.items);
+        pk.add(h.post_off, &t.sc.post_off);
+        pk.add(h.post, &t.sc.post);
+        pk.add(ad.ns_post, &t.ns_post);
+        made.push_back(&t.made);
     }
-    SchedHost h;
-    sched_build(sched_input(m, kind, slot), 5, 8, 1, 1 << 10, h);
-    WaveHold t;
-    t.n_vec = h.n_vec;
-    t.wt.n_post = (int)h.wave_post.size();
-    t.wt.n_zero = (int)h.wave_zero.size();
-    t.n_ns_post = (int)h.ns_post.size();
-    int rc;
-    Pack pk;
-    pk.add(h.wave_slot_off, &t.wt.slot_off);
-    pk.add(h.wave_slots, &t.wt.slots);
-    pk.add(h.wave_tb_off, &t.wt.tb_off);
-    pk.add(h.wave_tb, &t.wt.tb);
-    pk.add(h.wave_post, &t.wt.post);
-    pk.add(h.wave_zero, &t.wt.zero);
-    pk.add(h.ns_post, &t.ns_post);
-    if ((rc = pk.send(&t.buffer))) return rc;
-    *out = &m->waves.emplace(key, t).first->second;
+    if (wave && !kt.wave.made) {
+        WaveHold& t = kt.wave;
+        t.n_vec = ad.n_vec;
+        t.wt.n_post = (int)ad.post.size();
+        t.wt.n_zero = (int)ad.wave_zero.size();
+        t.n_ns_post = (int)ad.ns_post.size();
+        pk.add(ad.wave_slot_off, &t.wt.slot_off);
+        pk.add(ad.wave_slots, &t.wt.slots);
+        pk.add(ad.wave_tb_off, &t.wt.tb_off);
+        pk.add(ad.wave_tb, &t.wt.tb);
+        pk.add(ad.post, &t.wt.post);
+        pk.add(ad.wave_zero, &t.wt.zero);
+        pk.add(ad.ns_post, &t.ns_post);
+        made.push_back(&t.made);
+    }
+    if (made.empty()) return 0;
+    char* buffer = nullptr;
+    if (int rc = pk.send(&buffer)) return rc;
+    kt.buffers.push_back(buffer);
+    for (bool* b : made) *b = true;
     return 0;
 }
 
@@ -479,11 +481,15 @@ bool wave_sooner(const pjg_mech* m, int kind, int64_t rest)
 }
 
 // blocks of a launch over n states
-int grid_of(const pjg_mech* m, int kind, const Schedule& sc, int64_t n)
+int grid_of(const SchedTables& t, int64_t n)
 {
-    const int64_t tiles = (n + (1 << sc.slog) - 1) >> sc.slog;
-    const int per_sm = pjg_tile_blocks_per_sm(kind, sc.warps, pjg_tile_smem(kind, m->ns, m->n_m, sc.slog, sc.warps, sc.buf_terms));
-    return (int)std::min<int64_t>(tiles, (int64_t)per_sm * sm_count(m));
+    return (int)std::min<int64_t>((n + (1 << t.sc.slog) - 1) >> t.sc.slog, t.resident);
+}
+
+// bytes of the blocks' scratch slices
+size_t slice_bytes(const SchedTables& t, int64_t n)
+{
+    return ((size_t)grid_of(t, n) * t.sc.n_vec * sizeof(double)) << t.sc.slog;
 }
 
 int ensure_work(pjg_mech* m, size_t bytes)
@@ -556,9 +562,11 @@ int make_plan(pjg_mech* m, int kind, bool F, bool sparse, const SlotTables* t, i
     const int layout = kind == PJG_JACOBIAN ? (F ? 2 : 0) + (sparse ? 1 : 0) : 0;
     const std::vector<int>* slot = t ? &t->slot : nullptr;
     const int64_t W = wave_states(m, kind);
+    KindTables* kt = nullptr;
     p->n_wave = wave_sooner(m, kind, n % W) ? n : n / W * W;
     if (p->n_wave > 0) {
-        if (int rc = wave_tables(m, kind, layout, slot, &p->wh)) return rc;
+        if (int rc = make_tables(m, kind, layout, slot, 0, -1, true, &kt)) return rc;
+        p->wh = &kt->wave;
         const size_t each = per_state + wave_state_bytes(m, kind, p->wh->n_vec);
         p->ch_wave = std::min<int64_t>(most_states ? most_states : chunk_states(each, p->n_wave, W), p->n_wave);
         p->need = each * (size_t)p->ch_wave;
@@ -568,12 +576,12 @@ int make_plan(pjg_mech* m, int kind, bool F, bool sparse, const SlotTables* t, i
         p->ch_tile = n - p->n_wave;
         if (per_state)
             p->ch_tile = std::min<int64_t>(most_states ? most_states : chunk_states(per_state, p->ch_tile, W), p->ch_tile);
-        Shape sh;
-        if (int rc = choose_shape(m, kind, p->ch_tile, &sh)) return rc;
-        if (int rc = sched_tables(m, kind, layout, slot, sh, &p->sd)) return rc;
-        p->grid = grid_of(m, kind, p->sd->sc, p->ch_tile);
-        p->need = std::max(p->need, per_state * (size_t)p->ch_tile +
-                                        (size_t)p->grid * p->sd->sc.n_vec * sizeof(double) * ((size_t)1 << p->sd->sc.slog));
+        const int slog = choose_shape(m, kind, p->ch_tile);
+        if (slog < 0) return fail(PJG_ERR_UNSUPPORTED, "mechanism too large for the evaluation kernels");
+        if (int rc = make_tables(m, kind, layout, slot, slog, slog, false, &kt)) return rc;
+        p->sd = &kt->tile[slog];
+        p->grid = grid_of(*p->sd, p->ch_tile);
+        p->need = std::max(p->need, per_state * (size_t)p->ch_tile + slice_bytes(*p->sd, p->ch_tile));
     }
     return 0;
 }
@@ -1072,16 +1080,17 @@ int pjg_internal_fail(int code, const char* msg) { return fail(code, "%s", msg);
 // block's mechanism and schedule, and the grid.
 int pjg_internal_vjp_args(pjg_mech* m, int64_t n, size_t scratch_doubles, EvalArgs* a, int* grid)
 {
-    Shape sh;
-    SchedTables* sd = nullptr;
-    if (int rc = choose_shape(m, PJG_KIND_VJP, kNoallocStates, &sh)) return rc;
-    if (int rc = sched_tables(m, PJG_KIND_VJP, 0, nullptr, sh, &sd)) return rc;
+    KindTables* kt = nullptr;
+    const int slog = choose_shape(m, PJG_KIND_VJP, kNoallocStates);
+    if (slog < 0) return fail(PJG_ERR_UNSUPPORTED, "mechanism too large for the evaluation kernels");
+    if (int rc = make_tables(m, PJG_KIND_VJP, 0, nullptr, slog, slog, false, &kt)) return rc;
+    const SchedTables& sd = kt->tile[slog];
     fill_common(m, *a);
-    a->sc = sd->sc;
-    a->ns_post = sd->ns_post;
-    a->n_ns_post = sd->n_ns_post;
-    const size_t slice = (size_t)sd->sc.n_vec << sd->sc.slog;
-    *grid = (int)std::min<size_t>(grid_of(m, PJG_KIND_VJP, sd->sc, n), scratch_doubles / slice);
+    a->sc = sd.sc;
+    a->ns_post = sd.ns_post;
+    a->n_ns_post = sd.n_ns_post;
+    const size_t slice = (size_t)sd.sc.n_vec << slog;
+    *grid = (int)std::min<size_t>(grid_of(sd, n), scratch_doubles / slice);
     return *grid > 0 ? 0 : fail(PJG_ERR_ARG, "scratch too small for one tile");
 }
 int pjg_internal_mech_ns(const pjg_mech* m) { return m->ns; }
@@ -1352,10 +1361,9 @@ int pjg_mech_create(const pjg_tables* tb, pjg_mech** out)
         return rc;
     }
     // pjg_vjp_noalloc may not allocate: its schedule now
-    Shape sh;
-    SchedTables* sd = nullptr;
-    if (!choose_shape(m, PJG_KIND_VJP, kNoallocStates, &sh) &&
-        (rc = sched_tables(m, PJG_KIND_VJP, 0, nullptr, sh, &sd))) {
+    KindTables* kt = nullptr;
+    const int slog = choose_shape(m, PJG_KIND_VJP, kNoallocStates);
+    if (slog >= 0 && (rc = make_tables(m, PJG_KIND_VJP, 0, nullptr, slog, slog, false, &kt))) {
         pjg_mech_destroy(m);
         return rc;
     }
@@ -1382,8 +1390,8 @@ int pjg_mech_destroy(pjg_mech* m)
         cudaFree(t.sp_slots);
         cudaFree(t.cj_slots);
     }
-    for (auto& kv : m->scheds) cudaFree(kv.second.buffer);
-    for (auto& kv : m->waves) cudaFree(kv.second.buffer);
+    for (auto& kv : m->tables)
+        for (char* b : kv.second.buffers) cudaFree(b);
     cudaFree(m->m_lists);
     delete m;
     return 0;
@@ -1467,11 +1475,11 @@ int pjg_eval_chunk(pjg_mech* m, int kind, int64_t n, char order, int jac_format,
         if (rc) return rc;
     }
     const int layout = kind == PJG_JACOBIAN ? (order == 'F' ? 2 : 0) + (jac_format == PJG_JAC_SPARSE ? 1 : 0) : 0;
-    WaveHold* wh = nullptr;
-    if (int rc = wave_tables(m, kind, layout, t ? &t->slot : nullptr, &wh)) return rc;
+    KindTables* kt = nullptr;
+    if (int rc = make_tables(m, kind, layout, t ? &t->slot : nullptr, 0, -1, true, &kt)) return rc;
     const size_t per_state = eval_state_bytes(kind, order == 'F', t);
     const int64_t W = wave_states(m, kind), n_wave = wave_sooner(m, kind, n % W) ? n : n / W * W;
-    *states = n_wave ? chunk_states(per_state + wave_state_bytes(m, kind, wh->n_vec), n_wave, W)
+    *states = n_wave ? chunk_states(per_state + wave_state_bytes(m, kind, kt->wave.n_vec), n_wave, W)
                      : chunk_states(per_state, n, W);
     return 0;
 }

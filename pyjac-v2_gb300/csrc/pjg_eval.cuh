@@ -178,7 +178,6 @@ struct EvalArgs {
     double* vjp;      // same layout
 };
 
-// reaction classes of a packed record list, in packed order (pjg_capi.cu)
 struct SchedInput {
     int kind = 0, ns = 0, jac_approx = 0;
     const std::vector<RxnRec>* rxn = nullptr;  // device records
@@ -187,19 +186,37 @@ struct SchedInput {
     const std::vector<double>* thd_coef = nullptr;
     const std::vector<int>* slot = nullptr;    // (ns-1)^2 species-block slots, -1 none (Jacobian)
 };
-struct SchedHost {  // a schedule's tables before upload
-    int slog = 5, warps = 8, rounds = 1, n_batch = 0, buf_terms = 0, n_vec = 0;
+// The additions of one (kind, output layout), whatever the tile's shape, and
+// the tables of the thread-per-state kernel (WaveTables).
+struct SchedAdds {
+    struct Item {
+        unsigned target;
+        int t, q;  // term of the reaction; factor, or the second term's distance
+        bool prod;
+    };
+    int kind = 0, n_slot = 0, n_vec = 0;
+    unsigned unread = 0;
+    bool left_out = false;           // a term of the species block has no slot
+    std::vector<int> cls, terms, item_off;  // per reaction: class, terms left in the buffer, items
+    std::vector<Item> items;
+    std::vector<unsigned> zeros;     // targets that nothing is added to
+    std::vector<char> general;       // targets with a factor other than 1 and -1 (empty: none)
+    std::vector<int> count, order;   // additions per target; targets, longest first
+    std::vector<PostItem> post, ns_post;
+    std::vector<int> wave_slot_off, wave_tb_off, wave_tb;
+    std::vector<unsigned> wave_slots, wave_zero;
+    int dense(unsigned t) const { return (int)(t & TGT_MASK) + ((t & TGT_VEC) ? n_slot : 0); }
+};
+struct SchedHost {  // one shape's tables before upload
+    int n_batch = 0;
     std::vector<int4> tasks;
     std::vector<int> term_off, item_off, post_off;
     std::vector<uint2> items;
-    std::vector<PostItem> post, ns_post;
-    bool left_out = false;
-    // of the thread-per-state kernel (WaveTables)
-    std::vector<int> wave_slot_off, wave_tb_off, wave_tb;
-    std::vector<unsigned> wave_slots, wave_zero;
-    std::vector<PostItem> wave_post;
+    std::vector<PostItem> post;
 };
-bool sched_build(const SchedInput& in, int slog, int warps, int rounds, int buf_terms, SchedHost& out);
+void sched_adds(const SchedInput& in, SchedAdds& out);
+// false: a reaction's terms pass the buffer
+bool sched_build(const SchedAdds& in, int slog, int warps, int rounds, int buf_terms, SchedHost& out);
 
 // host launchers: pjg_tile.cu
 constexpr size_t kTileStatic = 8192 + 256;  // exp table and flags, bytes

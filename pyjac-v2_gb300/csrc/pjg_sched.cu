@@ -8,54 +8,74 @@
 // one target stay with one worker, in reaction order, so that every sum has
 // that order whatever the tile's shape; the targets go to the least-loaded
 // worker, longest first.
+//
+// The additions themselves do not depend on the tile's shape: sched_adds lists
+// them once per kind and output layout (the thread-per-state kernel's tables
+// among them), sched_build deals them out for one shape.  Both in one cost the
+// first Jacobian call of GRI-Mech 3.0 2.1 ms on the host and each further shape
+// 0.9, with the 500-species mechanism 137 and 75 (dense; sparse 46 and 20); now
+// 0.7 and 0.3, 25 and 12 (sparse 8 and 3.5).
 #include <algorithm>
 #include <cmath>
 #include <map>
 #include <queue>
-#include <set>
 
 #include "pjg_eval.cuh"
 
 namespace {
 
-struct Item {
-    unsigned target;
-    int t, q;   // term; factor, or the second term's distance
-    bool prod;
-};
-
-// workers of targets (dense numbers) by their numbers of additions
-void deal(const std::vector<int>& count, int G, std::vector<int>& owner)
+// Workers of targets (dense numbers) by their numbers of additions, `order`
+// holding the targets longest first: the least-loaded worker, the lowest of
+// several.  Where only single additions are left, that is filling level by
+// level.
+void deal(const std::vector<int>& count, const std::vector<int>& order, int G, std::vector<int>& owner)
 {
-    std::vector<std::pair<int, int>> by;
-    for (int t = 0; t < (int)count.size(); ++t)
-        if (count[t]) by.push_back({-count[t], t});
-    std::sort(by.begin(), by.end());
-    std::priority_queue<std::pair<int, int>, std::vector<std::pair<int, int>>, std::greater<std::pair<int, int>>> load;
-    for (int g = 0; g < G; ++g) load.push({0, g});
+    std::priority_queue<std::pair<int, int>, std::vector<std::pair<int, int>>, std::greater<std::pair<int, int>>> heap;
+    for (int g = 0; g < G; ++g) heap.push({0, g});
     owner.assign(count.size(), 0);
-    for (auto& x : by) {
-        auto [n, g] = load.top();
-        load.pop();
-        owner[x.second] = g;
-        load.push({n - x.first, g});
+    size_t x = 0;
+    for (; x < order.size() && count[order[x]] > 1; ++x) {
+        auto [n, g] = heap.top();
+        heap.pop();
+        owner[order[x]] = g;
+        heap.push({n + count[order[x]], g});
     }
+    std::vector<int> load(G);
+    int level = heap.top().first;
+    for (; !heap.empty(); heap.pop()) load[heap.top().second] = heap.top().first;
+    for (; x < order.size(); ++level)
+        for (int g = 0; g < G && x < order.size(); ++g)
+            if (load[g] == level) {
+                ++load[g];
+                owner[order[x++]] = g;
+            }
+}
+
+// the targets that something is added to, longest first
+std::vector<int> longest_first(const std::vector<int>& count)
+{
+    int top = 0;
+    for (int c : count) top = std::max(top, c);
+    std::vector<size_t> at(top + 2, 0);
+    for (int c : count) ++at[top - c + 1];
+    for (int q = 0; q <= top; ++q) at[q + 1] += at[q];
+    std::vector<int> order(at[top]);  // of count >= 1
+    for (int t = 0; t < (int)count.size(); ++t)
+        if (count[t]) order[at[top - count[t]]++] = t;
+    return order;
 }
 
 }  // namespace
 
-bool sched_build(const SchedInput& in, int slog, int warps, int rounds, int buf_terms, SchedHost& o)
+void sched_adds(const SchedInput& in, SchedAdds& o)
 {
-    const int S = 1 << slog, wpw = 32 / S, G = warps * wpw;
     const int ns = in.ns, last = ns - 1, kind = in.kind;
     const std::vector<RxnRec>& rx = *in.rxn;
     const int nr = (int)rx.size();
     const bool jac = kind == KIND_JAC, vjp = kind == KIND_VJP;
-    o.slog = slog;
-    o.warps = warps;
-    o.rounds = rounds;
-    o.buf_terms = buf_terms;
+    o.kind = kind;
     o.n_vec = vec_arrays(kind) * ns;
+    o.cls = *in.cls;
 
     // third-body sums: one per (list, species row) and two per list (Jacobian:
     // rows T and E), one per list (J^T v)
@@ -65,13 +85,10 @@ bool sched_build(const SchedInput& in, int slog, int warps, int rounds, int buf_
         if (it != sum_of.end()) return it->second;
         return sum_of[{list, row}] = (unsigned)o.n_vec++;
     };
-    std::vector<char> seen_vec;  // marks of scratch entries added to
-    std::vector<char> seen_slot;
-    if (jac) {
-        int top = 0;
-        for (int sl : *in.slot) top = std::max(top, sl + 1);
-        seen_slot.assign(top, 0);
-    }
+    o.n_slot = 0;
+    if (jac)
+        for (int sl : *in.slot) o.n_slot = std::max(o.n_slot, sl + 1);
+    std::vector<char> seen_vec, seen_slot(o.n_slot, 0);  // marks of targets added to
     auto first = [&](unsigned t) -> unsigned {
         std::vector<char>& seen = (t & TGT_VEC) ? seen_vec : seen_slot;
         const unsigned i = t & TGT_MASK;
@@ -82,162 +99,115 @@ bool sched_build(const SchedInput& in, int slog, int warps, int rounds, int buf_
     };
     auto vec_t = [&](int v, int k) -> unsigned { return TGT_VEC | (unsigned)(v * ns + k); };
     auto slot_of = [&](int k, int j) -> int { return (*in.slot)[(size_t)k * last + j]; };
-
     auto has_ns = [&](const RxnRec& R) { return (R.flags & RX_HASNS) && !in.jac_approx; };
-    auto terms_of = [&](const RxnRec& R) {
-        if (vjp) return 1 + R.nspec + rxn_x_terms(R);
-        if (!jac) return 1;
-        return 3 + R.nspec + (has_ns(R) ? 1 : 0) + (rxn_has_d1(R.flags) ? 1 : 0) + rxn_x_terms(R) +
-               ((R.flags & RX_WEREAL) ? 1 : 0);
-    };
 
-    o.term_off.assign(std::max(nr, 1), 0);
-    std::vector<std::vector<Item>> batches;
-    const int n_slot = jac ? (int)seen_slot.size() : 0;
-    auto dense = [&](unsigned t) { return (int)(t & TGT_MASK) + ((t & TGT_VEC) ? n_slot : 0); };
-    std::set<unsigned> general;  // targets with a factor other than 1 and -1
-    int i = 0;
-    while (i < nr) {
-        // one batch
-        int terms = 1, b0 = i;  // term 0 is zero
-        std::vector<int4> tasks;
-        while (i < nr && (int)tasks.size() < warps * rounds) {
-            const int cl = (*in.cls)[i];
-            int cnt = 0, t = 0;
-            while (cnt < wpw && i + cnt < nr && (*in.cls)[i + cnt] == cl) {
-                const int q = terms_of(rx[i + cnt]);
-                if (terms + t + q > buf_terms) break;
-                t += q;
-                ++cnt;
-            }
-            if (!cnt) break;
-            int off = terms;
-            for (int e = 0; e < cnt; ++e) {
-                o.term_off[i + e] = off;
-                off += terms_of(rx[i + e]);
-            }
-            tasks.push_back(make_int4(cl, i, cnt, 0));
-            terms = off;
-            i += cnt;
+    std::vector<unsigned> general;  // targets with a factor other than 1 and -1
+    auto scaled = [&](unsigned target, int t, int q) {
+        o.items.push_back({first(target), t, q, false});
+        if (q != 1 && q != -1) general.push_back(target);
+    };
+    auto product = [&](unsigned target, int t, int t2) {
+        o.items.push_back({first(target), t, t - t2, true});
+    };
+    auto add_slot = [&](int sl, int t, int q, unsigned& wave) {
+        if (sl < 0) {
+            o.left_out = true;
+            return;
         }
-        if (tasks.empty()) return false;  // one reaction's terms pass the buffer
-        while ((int)tasks.size() < warps * rounds) tasks.push_back(make_int4(0, 0, 0, 0));
-        o.tasks.insert(o.tasks.end(), tasks.begin(), tasks.end());
-        ++o.n_batch;
-        // its additions
-        std::vector<Item> items;
-        auto scaled = [&](unsigned target, int t, int q) {
-            items.push_back({target, t, q, false});
-            if (q != 1 && q != -1) general.insert(target);
-        };
-        auto product = [&](unsigned target, int t, int t2) {
-            items.push_back({target, t, t - t2, true});
-        };
-        for (int r = b0; r < i; ++r) {
-            const RxnRec& R = rx[r];
-            const int n = R.nspec, base = o.term_off[r];
-            const int n_x = rxn_x_terms(R);  // 1: summed per list; else one per entry of the list
-            const bool thd = n_x > 0, summed = R.list >= 0;
-            const int t_net = jac ? base + 1 : base, t_g = jac ? base + 3 : base + 1;
-            int sp[PJG_MAXSP], nu[PJG_MAXSP], nu_sum = 0;
-            bool zero[PJG_MAXSP];  // d net / d c_j is zero by itself
-            for (int e = 0; e < n; ++e) {
-                sp[e] = ent_spec(R.ent[e]);
-                nu[e] = ent_nur(R.ent[e]) - ent_nuf(R.ent[e]);
-                nu_sum += nu[e];
-                zero[e] = !(R.flags & RX_REV) && ent_nuf(R.ent[e]) == 0;
-                if (nu[e]) scaled(vec_t(VEC_WDOT, sp[e]), t_net, nu[e]);
-            }
-            o.wave_slot_off.push_back((int)o.wave_slots.size());
-            o.wave_tb_off.push_back((int)o.wave_tb.size());
-            if (vjp) {
-                if (summed) o.wave_tb.push_back((int)tb_sum(R.thd_off, 0));
-                for (int e = 0; e < n; ++e)
-                    if (sp[e] != last && !zero[e]) scaled(vec_t(VEC_NS, sp[e]), t_g + e, 1);
-                if (summed) scaled(TGT_VEC | tb_sum(R.thd_off, 0), t_g + n, 1);
-                else
-                    for (int l = 0; l < n_x; ++l)
-                        if ((*in.thd_spec)[R.thd_off + l] != last && (*in.thd_coef)[R.thd_off + l] != 0.0)
-                            scaled(vec_t(VEC_NS, (*in.thd_spec)[R.thd_off + l]), t_g + n + l, 1);
-            }
-            if (!jac) continue;
-            int t = t_g + n;
-            const int t_ns = has_ns(R) ? t++ : -1, t_d1 = rxn_has_d1(R.flags) ? t++ : -1,
-                      t_x = t, t_we = t + n_x;
-            const bool we_term = R.flags & RX_WEREAL;
-            if (summed) {
-                for (int a = 0; a < n; ++a)
-                    o.wave_tb.push_back(sp[a] == last || !nu[a] ? -1 : (int)tb_sum(R.thd_off, sp[a]));
-                o.wave_tb.push_back((int)tb_sum(R.thd_off, ns));
-                o.wave_tb.push_back(R.flags & RX_WE ? (int)tb_sum(R.thd_off, ns + 1) : -1);
-            }
-            // the thread-per-state kernel's slots: per participant, one per
-            // participant and one per entry of an unshared third-body list
-            const int n_l = summed ? 0 : n_x, row = n + n_l;
-            o.wave_slots.resize(o.wave_slots.size() + n * row, TGT_MASK);
-            unsigned* wave = o.wave_slots.data() + o.wave_slots.size() - n * row;
-            for (int a = 0; a < n; ++a) {
-                if (sp[a] == last || !nu[a]) continue;
-                for (int e = 0; e < n; ++e) {
-                    if (sp[e] == last || zero[e]) continue;
-                    if (slot_of(sp[a], sp[e]) >= 0) wave[a * row + e] = (unsigned)slot_of(sp[a], sp[e]);
-                    const int sl = slot_of(sp[a], sp[e]);
-                    if (sl < 0) o.left_out = true;
-                    else scaled((unsigned)sl, t_g + e, nu[a]);
-                }
-                scaled(vec_t(VEC_CT, sp[a]), base + 2, nu[a]);
-                if (t_d1 >= 0) scaled(vec_t(VEC_CE, sp[a]), t_d1, nu[a]);
-                if (t_ns >= 0) scaled(vec_t(VEC_NS, sp[a]), t_ns, nu[a]);
-                if (summed) scaled(TGT_VEC | tb_sum(R.thd_off, sp[a]), t_x, nu[a]);
-                for (int l = 0; l < n_l; ++l) {
-                    const int j = (*in.thd_spec)[R.thd_off + l];
-                    if ((*in.thd_coef)[R.thd_off + l] == 0.0) continue;
-                    if (j == last) {
-                        if (!in.jac_approx) scaled(vec_t(VEC_NS, sp[a]), t_x + l, nu[a]);
-                        continue;
-                    }
-                    const int sl = slot_of(sp[a], j);
-                    if (sl < 0) o.left_out = true;
-                    else scaled((unsigned)sl, t_x + l, nu[a]);
-                    if (sl >= 0) wave[a * row + n + l] = (unsigned)sl;
-                }
-            }
-            auto row_e = [&](unsigned target, int src) {
-                if (!(R.flags & RX_WE)) return;
-                if (we_term) product(target, src, t_we);
-                else scaled(target, src, nu_sum);
-            };
+        scaled((unsigned)sl, t, q);
+        wave = o.items.back().target;
+    };
+    for (int r = 0; r < nr; ++r) {
+        const RxnRec& R = rx[r];
+        const int n = R.nspec;
+        const int n_x = rxn_x_terms(R);  // 1: summed per list; else one per entry of the list
+        const bool summed = R.list >= 0;
+        const int t_net = jac ? 1 : 0, t_g = jac ? 3 : 1;
+        o.terms.push_back(vjp ? 1 + n + n_x
+                          : !jac ? 1
+                                 : 3 + n + (has_ns(R) ? 1 : 0) + (rxn_has_d1(R.flags) ? 1 : 0) + n_x +
+                                       ((R.flags & RX_WEREAL) ? 1 : 0));
+        o.item_off.push_back((int)o.items.size());
+        int sp[PJG_MAXSP], nu[PJG_MAXSP], nu_sum = 0;
+        bool zero[PJG_MAXSP];  // d net / d c_j is zero by itself
+        for (int e = 0; e < n; ++e) {
+            sp[e] = ent_spec(R.ent[e]);
+            nu[e] = ent_nur(R.ent[e]) - ent_nuf(R.ent[e]);
+            nu_sum += nu[e];
+            zero[e] = !(R.flags & RX_REV) && ent_nuf(R.ent[e]) == 0;
+            if (nu[e]) scaled(vec_t(VEC_WDOT, sp[e]), t_net, nu[e]);
+        }
+        o.wave_slot_off.push_back((int)o.wave_slots.size());
+        o.wave_tb_off.push_back((int)o.wave_tb.size());
+        if (vjp) {
+            if (summed) o.wave_tb.push_back((int)tb_sum(R.thd_off, 0));
+            for (int e = 0; e < n; ++e)
+                if (sp[e] != last && !zero[e]) scaled(vec_t(VEC_NS, sp[e]), t_g + e, 1);
+            if (summed) scaled(TGT_VEC | tb_sum(R.thd_off, 0), t_g + n, 1);
+            else
+                for (int l = 0; l < n_x; ++l)
+                    if ((*in.thd_spec)[R.thd_off + l] != last && (*in.thd_coef)[R.thd_off + l] != 0.0)
+                        scaled(vec_t(VEC_NS, (*in.thd_spec)[R.thd_off + l]), t_g + n + l, 1);
+        }
+        if (!jac) continue;
+        int t = t_g + n;
+        const int t_ns = has_ns(R) ? t++ : -1, t_d1 = rxn_has_d1(R.flags) ? t++ : -1,
+                  t_x = t, t_we = t + n_x;
+        const bool we_term = R.flags & RX_WEREAL;
+        if (summed) {
+            for (int a = 0; a < n; ++a)
+                o.wave_tb.push_back(sp[a] == last || !nu[a] ? -1 : (int)tb_sum(R.thd_off, sp[a]));
+            o.wave_tb.push_back((int)tb_sum(R.thd_off, ns));
+            o.wave_tb.push_back(R.flags & RX_WE ? (int)tb_sum(R.thd_off, ns + 1) : -1);
+        }
+        // the thread-per-state kernel's slots: per participant, one per
+        // participant and one per entry of an unshared third-body list
+        const int n_l = summed ? 0 : n_x, row = n + n_l;
+        o.wave_slots.resize(o.wave_slots.size() + n * row, TGT_MASK);
+        unsigned* wave = o.wave_slots.data() + o.wave_slots.size() - n * row;
+        for (int a = 0; a < n; ++a) {
+            if (sp[a] == last || !nu[a]) continue;
             for (int e = 0; e < n; ++e) {
                 if (sp[e] == last || zero[e]) continue;
-                product(vec_t(VEC_RT, sp[e]), t_g + e, base);
-                row_e(vec_t(VEC_RE, sp[e]), t_g + e);
+                add_slot(slot_of(sp[a], sp[e]), t_g + e, nu[a], wave[a * row + e]);
             }
-            if (summed) {
-                product(TGT_VEC | tb_sum(R.thd_off, ns), t_x, base);
-                if (R.flags & RX_WE) row_e(TGT_VEC | tb_sum(R.thd_off, ns + 1), t_x);
-            }
+            scaled(vec_t(VEC_CT, sp[a]), 2, nu[a]);
+            if (t_d1 >= 0) scaled(vec_t(VEC_CE, sp[a]), t_d1, nu[a]);
+            if (t_ns >= 0) scaled(vec_t(VEC_NS, sp[a]), t_ns, nu[a]);
+            if (summed) scaled(TGT_VEC | tb_sum(R.thd_off, sp[a]), t_x, nu[a]);
             for (int l = 0; l < n_l; ++l) {
                 const int j = (*in.thd_spec)[R.thd_off + l];
-                if ((*in.thd_coef)[R.thd_off + l] == 0.0 || j == last) continue;
-                product(vec_t(VEC_RT, j), t_x + l, base);
-                row_e(vec_t(VEC_RE, j), t_x + l);
+                if ((*in.thd_coef)[R.thd_off + l] == 0.0) continue;
+                if (j == last) {
+                    if (!in.jac_approx) scaled(vec_t(VEC_NS, sp[a]), t_x + l, nu[a]);
+                    continue;
+                }
+                add_slot(slot_of(sp[a], j), t_x + l, nu[a], wave[a * row + n + l]);
             }
         }
-        for (Item& x : items) x.target = first(x.target);
-        if (jac) {  // the same marks in the thread-per-state kernel's slots
-            size_t q = 0;
-            for (int r = b0; r < i; ++r)
-                for (int e = o.wave_slot_off[r]; e < (r + 1 < (int)o.wave_slot_off.size() ? o.wave_slot_off[r + 1] : (int)o.wave_slots.size()); ++e) {
-                    unsigned& sl = o.wave_slots[e];
-                    if (sl == TGT_MASK) continue;
-                    while (items[q].prod || (items[q].target & TGT_VEC) || (items[q].target & TGT_MASK) != sl) ++q;
-                    sl = items[q++].target;
-                }
+        auto row_e = [&](unsigned target, int src) {
+            if (!(R.flags & RX_WE)) return;
+            if (we_term) product(target, src, t_we);
+            else scaled(target, src, nu_sum);
+        };
+        for (int e = 0; e < n; ++e) {
+            if (sp[e] == last || zero[e]) continue;
+            product(vec_t(VEC_RT, sp[e]), t_g + e, 0);
+            row_e(vec_t(VEC_RE, sp[e]), t_g + e);
         }
-        batches.push_back(std::move(items));
+        if (summed) {
+            product(TGT_VEC | tb_sum(R.thd_off, ns), t_x, 0);
+            if (R.flags & RX_WE) row_e(TGT_VEC | tb_sum(R.thd_off, ns + 1), t_x);
+        }
+        for (int l = 0; l < n_l; ++l) {
+            const int j = (*in.thd_spec)[R.thd_off + l];
+            if ((*in.thd_coef)[R.thd_off + l] == 0.0 || j == last) continue;
+            product(vec_t(VEC_RT, j), t_x + l, 0);
+            row_e(vec_t(VEC_RE, j), t_x + l);
+        }
     }
+    o.item_off.push_back((int)o.items.size());
     // the third-body columns, after the reactions: coefficient x sum
-    std::vector<PostItem> post;
     std::map<int, int> lists;  // offset -> reaction with that list
     for (int r = 0; r < nr; ++r)
         if (rx[r].list >= 0) lists.emplace(rx[r].thd_off, r);
@@ -251,33 +221,24 @@ bool sched_build(const SchedInput& in, int slog, int warps, int rounds, int buf_
             if (j == last) {
                 if (in.jac_approx) continue;
                 if (vjp) o.ns_post.push_back({kv.second, 0u, c});
-                else if (row < last) post.push_back({kv.second, vec_t(VEC_NS, row), c});
+                else if (row < last) o.post.push_back({kv.second, vec_t(VEC_NS, row), c});
                 continue;
             }
             if (vjp) {
-                post.push_back({kv.second, vec_t(VEC_NS, j), c});
+                o.post.push_back({kv.second, vec_t(VEC_NS, j), c});
             } else if (row < last) {
                 const int sl = slot_of(row, j);
                 if (sl < 0) o.left_out = true;
-                else post.push_back({kv.second, (unsigned)sl, c});
+                else o.post.push_back({kv.second, (unsigned)sl, c});
             } else if (row >= ns) {
-                post.push_back({kv.second, vec_t(row == ns ? VEC_RT : VEC_RE, j), c});
+                o.post.push_back({kv.second, vec_t(row == ns ? VEC_RT : VEC_RE, j), c});
             }
         }
     }
-    for (PostItem& x : post) x.target = first(x.target);
-    o.wave_post = post;
-    // what nothing is added to is set to zero by items of term 0, spread over
-    // the batches
-    if (batches.empty()) {
-        batches.emplace_back();
-        o.tasks.assign(warps * rounds, make_int4(0, 0, 0, 0));
-        o.n_batch = 1;
-    }
-    size_t next_batch = 0;
+    for (PostItem& x : o.post) x.target = first(x.target);
+    // what nothing is added to is set to zero
     auto zero = [&](unsigned target) {
-        if (!(first(target) & TGT_FIRST)) return;
-        batches[next_batch++ % batches.size()].push_back({target | TGT_FIRST, 0, 1, false});
+        if (first(target) & TGT_FIRST) o.zeros.push_back(target);
     };
     std::vector<int> vecs = {VEC_WDOT};
     if (vjp) vecs.push_back(VEC_NS);
@@ -290,40 +251,82 @@ bool sched_build(const SchedInput& in, int slog, int warps, int rounds, int buf_
                 if (!seen_slot[sl]) o.wave_zero.push_back((unsigned)sl);
                 zero((unsigned)sl);
             }
-    std::vector<int> count(n_slot + o.n_vec, 0), owner;
-    size_t n_items = 0;
-    for (const auto& items : batches) {
-        for (const Item& x : items) ++count[dense(x.target)];
-        n_items += items.size();
+    o.general.assign(general.empty() ? 0 : o.n_slot + o.n_vec, 0);
+    for (unsigned t : general) o.general[o.dense(t)] = 1;
+    o.count.assign(o.n_slot + o.n_vec, 0);
+    for (const SchedAdds::Item& x : o.items) ++o.count[o.dense(x.target)];
+    for (unsigned t : o.zeros) ++o.count[o.dense(t)];
+    o.order = longest_first(o.count);
+    o.unread = (unsigned)o.n_vec++;  // the slice's last entry
+}
+
+bool sched_build(const SchedAdds& in, int slog, int warps, int rounds, int buf_terms, SchedHost& o)
+{
+    const int S = 1 << slog, wpw = 32 / S, G = warps * wpw;
+    const int nr = (int)in.terms.size();
+    o.n_batch = 0;
+    // batches of tasks
+    o.term_off.assign(std::max(nr, 1), 0);
+    std::vector<int> batch_r = {0};  // first reactions of the batches
+    for (int i = 0; i < nr;) {
+        int terms = 1, n_tasks = 0;  // term 0 is zero
+        while (i < nr && n_tasks < warps * rounds) {
+            const int cl = in.cls[i], i0 = i;
+            while (i < nr && i - i0 < wpw && in.cls[i] == cl && terms + in.terms[i] <= buf_terms) {
+                o.term_off[i] = terms;
+                terms += in.terms[i++];
+            }
+            if (i == i0) break;
+            o.tasks.push_back(make_int4(cl, i0, i - i0, 0));
+            ++n_tasks;
+        }
+        if (!n_tasks) return false;  // one reaction's terms pass the buffer
+        o.tasks.resize(o.tasks.size() + warps * rounds - n_tasks, make_int4(0, 0, 0, 0));
+        ++o.n_batch;
+        batch_r.push_back(i);
     }
-    deal(count, G, owner);
-    const unsigned unread = (unsigned)o.n_vec++;  // the slice's last entry
-    // a batch's items by worker and run, each run in order (a counting sort)
+    if (!nr) {  // one empty batch, for the zeros
+        o.tasks.assign(warps * rounds, make_int4(0, 0, 0, 0));
+        o.n_batch = 1;
+        batch_r.push_back(0);
+    }
+    std::vector<int> owner;
+    deal(in.count, in.order, G, owner);
+    // a batch's items by worker and run, each run in order (a counting sort);
+    // the zeros are items of term 0, spread over the batches
     o.item_off.assign(1, 0);
-    o.items.reserve(n_items * 5 / 4 + 64);
-    std::vector<int> at(G * RUN_N + 1), key;
-    std::vector<int> sorted;
-    for (const auto& items : batches) {
+    o.items.reserve((in.items.size() + in.zeros.size()) * 5 / 4 + 64);
+    std::vector<int> at(G * RUN_N + 1), put, key;
+    std::vector<SchedAdds::Item> items, sorted;
+    for (int b = 0; b < o.n_batch; ++b) {
+        items.clear();
+        for (int r = batch_r[b]; r < batch_r[b + 1]; ++r)
+            for (int q = in.item_off[r]; q < in.item_off[r + 1]; ++q) {
+                items.push_back(in.items[q]);
+                items.back().t += o.term_off[r];
+            }
+        for (size_t q = b; q < in.zeros.size(); q += o.n_batch) items.push_back({in.zeros[q] | TGT_FIRST, 0, 1, false});
         key.resize(items.size());
         sorted.resize(items.size());
         std::fill(at.begin(), at.end(), 0);
         for (size_t i = 0; i < items.size(); ++i) {
-            const Item& x = items[i];
+            const SchedAdds::Item& x = items[i];
             const bool fi = x.target & TGT_FIRST, vec = x.target & TGT_VEC;
+            const int d = in.dense(x.target);
             const int run = x.prod ? (fi ? RUN_PROD_FIRST : RUN_PROD)
-                            : !general.empty() && general.count(x.target & ~TGT_FIRST) ? RUN_GENERAL
+                            : !in.general.empty() && in.general[d] ? RUN_GENERAL
                             : vec ? (fi ? RUN_VEC_FIRST : RUN_VEC) : (fi ? RUN_SLOT_FIRST : RUN_SLOT);
-            key[i] = owner[dense(x.target)] * RUN_N + run;
+            key[i] = owner[d] * RUN_N + run;
             ++at[key[i] + 1];
         }
         for (size_t q = 1; q < at.size(); ++q) at[q] += at[q - 1];
-        std::vector<int> put(at.begin(), at.end() - 1);
-        for (size_t i = 0; i < items.size(); ++i) sorted[put[key[i]]++] = (int)i;
+        put.assign(at.begin(), at.end() - 1);
+        for (size_t i = 0; i < items.size(); ++i) sorted[put[key[i]]++] = items[i];
         for (int q = 0; q < G * RUN_N; ++q) {
             const int r = q % RUN_N;
             const size_t from = o.items.size();
             for (int j = at[q]; j < at[q + 1]; ++j) {
-                const Item& x = items[sorted[j]];
+                const SchedAdds::Item& x = sorted[j];
                 const unsigned idx = x.target & TGT_MASK, off = (unsigned)(x.t * S * (int)sizeof(double));
                 if (r == RUN_PROD || r == RUN_PROD_FIRST)
                     o.items.push_back(make_uint2(idx, off | (((unsigned)x.q & 0x7ffu) << 20)));
@@ -334,16 +337,16 @@ bool sched_build(const SchedInput& in, int slog, int warps, int rounds, int buf_
             }
             while ((o.items.size() - from) % kItemUnroll)
                 o.items.push_back(r == RUN_SLOT_FIRST ? o.items.back() : r == RUN_SLOT ? make_uint2(o.items.back().x, 0u)
-                                  : r == RUN_GENERAL ? make_uint2(unread | TGT_VEC | TGT_FIRST, 1u << 20) : make_uint2(unread, 0u));
+                                  : r == RUN_GENERAL ? make_uint2(in.unread | TGT_VEC | TGT_FIRST, 1u << 20) : make_uint2(in.unread, 0u));
             o.item_off.push_back((int)o.items.size());
         }
     }
-    o.items.insert(o.items.end(), kItemUnroll, make_uint2(unread, 0u));  // loaded ahead, not used
-    std::vector<int> post_count(n_slot + o.n_vec, 0), post_owner;
-    for (const PostItem& x : post) ++post_count[dense(x.target)];
-    deal(post_count, G, post_owner);
+    o.items.insert(o.items.end(), kItemUnroll, make_uint2(in.unread, 0u));  // loaded ahead, not used
+    std::vector<int> post_count(in.n_slot + in.n_vec, 0), post_owner;
+    for (const PostItem& x : in.post) ++post_count[in.dense(x.target)];
+    deal(post_count, longest_first(post_count), G, post_owner);
     std::vector<std::vector<PostItem>> of(G);
-    for (const PostItem& x : post) of[post_owner[dense(x.target)]].push_back(x);
+    for (const PostItem& x : in.post) of[post_owner[in.dense(x.target)]].push_back(x);
     o.post_off.assign(1, 0);
     for (const auto& l : of) {
         o.post.insert(o.post.end(), l.begin(), l.end());
