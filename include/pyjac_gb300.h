@@ -97,7 +97,11 @@ int pjg_jacobian_indices(const pjg_mech* mech, char order, int32_t* ptr, int32_t
  * Replace the generated species_rates / jacobian drivers.  Calls on one
  * mechanism share its device working buffer (grown on demand): calls that
  * can overlap on the GPU, on different streams, must be serialised by the
- * caller or use separate pjg_mech objects. */
+ * caller or use separate pjg_mech objects.  The first call of an entry point,
+ * order and format, and each call with more states than any before, makes
+ * tables or grows the buffer (device allocations); calls with fewer states only
+ * launch and can be captured in a graph.  Growing moves the buffer, so a graph
+ * captured before must not be replayed after. */
 int pjg_species_rates(pjg_mech* mech, int64_t n, char order, int conp, const double* param,
                       const double* phi, double* dphi, void* stream);
 int pjg_jacobian(pjg_mech* mech, int64_t n, char order, int conp, int jac_format,

@@ -556,7 +556,11 @@ struct Plan {
     size_t need = 0;  // bytes of working buffer
 };
 
-int make_plan(pjg_mech* m, int kind, bool F, bool sparse, const SlotTables* t, int64_t n, int64_t most_states, Plan* p)
+// With smaller, also makes the tables and counts the working buffer of every
+// smaller n, so that after one call all smaller ones only launch (they may then
+// be captured in a graph).
+int make_plan(pjg_mech* m, int kind, bool F, bool sparse, const SlotTables* t, int64_t n, int64_t most_states,
+              bool smaller, Plan* p)
 {
     const size_t per_state = eval_state_bytes(kind, F, t);
     const int layout = kind == PJG_JACOBIAN ? (F ? 2 : 0) + (sparse ? 1 : 0) : 0;
@@ -564,12 +568,22 @@ int make_plan(pjg_mech* m, int kind, bool F, bool sparse, const SlotTables* t, i
     const int64_t W = wave_states(m, kind);
     KindTables* kt = nullptr;
     p->n_wave = wave_sooner(m, kind, n % W) ? n : n / W * W;
+    if (smaller) {
+        // what a smaller batch leaves to the tiles is less than a wave
+        const int64_t most = p->n_wave > 0 ? std::min(n, W) : n;
+        const int top = p->n_wave > 0 ? 5 : choose_shape(m, kind, per_state ? chunk_states(per_state, n, W) : n);
+        if (int rc = make_tables(m, kind, layout, slot, 0, top, p->n_wave > 0, &kt)) return rc;
+        size_t slices = 0;
+        for (int q = 0; q <= top; ++q)
+            if (kt->tile[q].made) slices = std::max(slices, slice_bytes(kt->tile[q], most));
+        p->need = per_state * (size_t)(per_state ? chunk_states(per_state, most, W) : 0) + slices;
+    }
     if (p->n_wave > 0) {
         if (int rc = make_tables(m, kind, layout, slot, 0, -1, true, &kt)) return rc;
         p->wh = &kt->wave;
         const size_t each = per_state + wave_state_bytes(m, kind, p->wh->n_vec);
         p->ch_wave = std::min<int64_t>(most_states ? most_states : chunk_states(each, p->n_wave, W), p->n_wave);
-        p->need = each * (size_t)p->ch_wave;
+        p->need = std::max(p->need, each * (size_t)p->ch_wave);
     }
     if (p->n_wave < n) {
         // the accumulator's states, then the blocks' scratch slices
@@ -614,7 +628,7 @@ int run_eval(pjg_mech* m, int kind, int64_t n, char order, int conp, int jac_for
     }
     const size_t per_state = eval_state_bytes(kind, F, t);
     Plan pl;
-    if (int rc = make_plan(m, kind, F, jac_format == PJG_JAC_SPARSE, t, n, ext_work ? ext_states : 0, &pl)) return rc;
+    if (int rc = make_plan(m, kind, F, jac_format == PJG_JAC_SPARSE, t, n, ext_work ? ext_states : 0, !ext_work, &pl)) return rc;
     const size_t need = pl.need;
     const int64_t n_wave = pl.n_wave;
     WaveHold* wh = pl.wh;
@@ -1686,7 +1700,7 @@ int pjg_kernel_resize(pjg_kernel* k, size_t problem_size, size_t work_size)
     for (int64_t cnt : {chunk, (int64_t)(problem_size % (size_t)chunk)}) {
         if (cnt == 0) continue;
         Plan pl;
-        if (int rc = make_plan(m, k->kind, k->order == 'F', k->jac_format == PJG_JAC_SPARSE, t, cnt, chunk, &pl))
+        if (int rc = make_plan(m, k->kind, k->order == 'F', k->jac_format == PJG_JAC_SPARSE, t, cnt, chunk, false, &pl))
             return rc;
         work_bytes = std::max(work_bytes, pl.need);
     }
