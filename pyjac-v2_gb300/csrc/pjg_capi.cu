@@ -711,7 +711,7 @@ int run_eval(pjg_mech* m, int kind, int64_t n, char order, int conp, int jac_for
             cudaEventCreate(&e1);
             cudaEventRecord(e0, st);
         }
-        rc = wave ? pjg_launch_wave(a, kind, st)
+        rc = wave ? pjg_launch_wave(a, kind, sm_count(m), st)
                   : pjg_launch_tile(a, kind, (int)std::min<int64_t>(pl.grid, (cnt + (1 << sd->sc.slog) - 1) >> sd->sc.slog), st);
         if (rc) return fail(PJG_ERR_CUDA, "kernel launch failed: %s", pjg_launch_error_string());
         g_launches.fetch_add(1);

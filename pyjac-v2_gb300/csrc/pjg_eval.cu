@@ -45,6 +45,8 @@
 // 74 % for the rates.
 #include <cuda_runtime.h>
 
+#include <type_traits>
+
 #include "pjg_eval.cuh"
 #include "pjg_math.cuh"
 #include "pjg_rxn.cuh"
@@ -56,15 +58,34 @@ const char* pjg_launch_error_string() { return cudaGetErrorString(pjg_launch_err
 
 namespace {
 
-// per-state array view: element k at base[k * stride]
-struct SV {
+// One of the per-state arrays of ns entries.  The rates kernel keeps a pointer
+// for each of its 6; the other two keep one base and a 32-bit first entry each
+// (element k lies first + k strides of bytes from the state's place).  With
+// pointers the Jacobian kernel's 13 arrays spilled 636 bytes of stores and 1,260
+// of loads, now 396 and 528: GRI-Mech 3.0, dense F, 200,000 states 11.96 ->
+// 11.68 ms, H2/O2 155,648 states 875 -> 847 us.  The rates kernel lost by the
+// change (GRI, 200,000 states 3.88 -> 3.98 ms).
+struct PtrView {
     double* b;
-    int64_t st;
-    __device__ __forceinline__ double& operator[](int k) const { return b[(int64_t)k * st]; }
+    int64_t ld;
+    __device__ __forceinline__ PtrView(double* base, int64_t stride, int first) : b(base + first * stride), ld(stride) {}
+    __device__ __forceinline__ double& operator[](int k) const { return b[k * ld]; }
+};
+struct BaseView {
+    char* b;
+    uint32_t st, first;  // the stride fits 32 bits: the working buffer's budget
+    __device__ __forceinline__ BaseView(double* base, int64_t stride, int first_)
+        : b(reinterpret_cast<char*>(base)), st((uint32_t)stride * sizeof(double)), first(first_) {}
+    __device__ __forceinline__ double& operator[](int k) const
+    {
+        return *reinterpret_cast<double*>(b + (uint64_t)(first + k) * st);
+    }
 };
 
 // Registers against warps, 1M GRI states dense F: 3 blocks per SM 75.4 ms, 4
-// 63.0, 5 65.2.
+// 63.0, 5 65.2.  A launch that leaves at most two blocks to an SM has the
+// registers for no spills at all (H2/O2, 38,000 states: 293 -> 282 us), so the
+// Jacobian kernel comes in that form, too.
 #ifndef PJG_VJP_MINB
 #define PJG_VJP_MINB 3  // resident 128-thread blocks per SM requested for the J^T v kernel
 #endif
@@ -73,9 +94,13 @@ struct SV {
 #define PJG_JAC_MINB 4  // resident 128-thread blocks per SM requested for the Jacobian kernel
 #endif
 
+constexpr int kFewBlocks = 2;
+
 #ifndef PJG_RATES_MINB
 #define PJG_RATES_MINB 6  // resident 128-thread blocks per SM requested for the species-rate kernel
 #endif
+
+constexpr int min_blocks(int kind) { return kind == KIND_JAC ? PJG_JAC_MINB : kind == KIND_VJP ? PJG_VJP_MINB : PJG_RATES_MINB; }
 
 constexpr int kPostUnroll = 8;
 
@@ -88,9 +113,8 @@ struct E22Stoich {
 
 // One thread per state; the per-state arrays and accumulators live in global
 // scratch (state-innermost, so a warp's accesses are coalesced).
-template <int KIND>  // KIND_RATES, KIND_JAC, KIND_VJP
-__global__ void __launch_bounds__(PJG_BLOCK, KIND == KIND_JAC ? PJG_JAC_MINB : (KIND == KIND_VJP ? PJG_VJP_MINB : PJG_RATES_MINB))
-    wave_kernel(const EvalArgs a)
+template <int KIND, int MINB = min_blocks(KIND)>  // KIND_RATES, KIND_JAC, KIND_VJP
+__global__ void __launch_bounds__(PJG_BLOCK, MINB) wave_kernel(const EvalArgs a)
 {
     __shared__ double etab[PJG_EXP_TAB];
     fill_exp_table(etab);
@@ -102,8 +126,8 @@ __global__ void __launch_bounds__(PJG_BLOCK, KIND == KIND_JAC ? PJG_JAC_MINB : (
     constexpr bool DER = JAC || VJP;  // derivative terms needed
     constexpr int kArr = tile_arrays(KIND);
     const int ns = a.ns, last = ns - 1;
-    const int64_t ld = a.sc_ld;
-    auto arr = [&](int which) -> SV { return SV{a.scratch + (int64_t)which * ns * ld + s, ld}; };
+    using SV = std::conditional_t<DER, BaseView, PtrView>;
+    auto arr = [&](int which) -> SV { return SV(a.scratch + s, a.sc_ld, which * ns); };
     auto vec = [&](int v) -> SV { return arr(kArr + v); };
     const SV conc = arr(ARR_CONC), ep = arr(ARR_EP), em = arr(ARR_EM);
     const SV& bk = ep;  // b_k until the state's split is known (then exp(b_k) if it holds)
@@ -659,12 +683,13 @@ int pjg_wave_blocks_per_sm(int kind)
     return e == cudaSuccess && b > 0 ? b : 1;
 }
 
-int pjg_launch_wave(const EvalArgs& a, int kind, void* stream)
+int pjg_launch_wave(const EvalArgs& a, int kind, int sms, void* stream)
 {
     if (a.n <= 0) return 0;
     const cudaStream_t st = (cudaStream_t)stream;
     const unsigned grid = (unsigned)((a.n + PJG_BLOCK - 1) / PJG_BLOCK);
-    if (kind == KIND_JAC) wave_kernel<KIND_JAC><<<grid, PJG_BLOCK, 0, st>>>(a);
+    if (kind == KIND_JAC && grid <= (unsigned)(kFewBlocks * sms)) wave_kernel<KIND_JAC, kFewBlocks><<<grid, PJG_BLOCK, 0, st>>>(a);
+    else if (kind == KIND_JAC) wave_kernel<KIND_JAC><<<grid, PJG_BLOCK, 0, st>>>(a);
     else if (kind == KIND_VJP) wave_kernel<KIND_VJP><<<grid, PJG_BLOCK, 0, st>>>(a);
     else wave_kernel<KIND_RATES><<<grid, PJG_BLOCK, 0, st>>>(a);
     pjg_launch_err = cudaGetLastError();

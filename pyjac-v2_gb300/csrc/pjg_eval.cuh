@@ -228,7 +228,7 @@ int pjg_launch_tile(const EvalArgs& a, int kind, int grid, void* stream);
 int pjg_tile_blocks_per_sm(int kind, int warps, size_t smem);
 // pjg_eval.cu
 int pjg_wave_blocks_per_sm(int kind);
-int pjg_launch_wave(const EvalArgs& a, int kind, void* stream);
+int pjg_launch_wave(const EvalArgs& a, int kind, int sms, void* stream);
 extern thread_local cudaError_t pjg_launch_err;  // of this thread's last evaluation launch
 const char* pjg_launch_error_string();           // CUDA's description of it
 int pjg_fp64_probe(int blocks, int threads, int iters, double* out, void* stream);
