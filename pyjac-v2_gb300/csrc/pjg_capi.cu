@@ -140,6 +140,12 @@ struct pjg_mech {
     int4* m_lists = nullptr;
     std::vector<RxnRec> d_rxn;    // host copy of the device records
     int device = 0;
+    // of the device, and per kind: states of a wave of the thread-per-state kernel,
+    // and log2 of the largest tile's states (-1: none fits) with the states of a
+    // round of resident ones
+    int sms = 1;
+    int64_t wave[3] = {}, round[3] = {};
+    int top_slog[3] = {-1, -1, -1};
     RxnRec* rxn = nullptr;
     double* sp = nullptr;
     int* thd_spec = nullptr;
@@ -326,20 +332,6 @@ int64_t chunk_states(size_t per_state, int64_t n, int64_t wave)
     return std::min<int64_t>(c, n);
 }
 
-int sm_count(const pjg_mech* m)
-{
-    int sms = 1;
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, m->device);
-    return sms;
-}
-
-// States of one full wave of the thread-per-state kernel (a launch of a
-// fraction of a wave takes more than its share of a whole one).
-int64_t wave_states(const pjg_mech* m, int kind)
-{
-    return (int64_t)sm_count(m) * pjg_wave_blocks_per_sm(kind) * PJG_BLOCK;
-}
-
 constexpr int64_t kNoallocStates = 4096;
 constexpr int kListTerms = 8;  // entries of an unshared third-body list, at most
 
@@ -380,13 +372,12 @@ bool shape_fits(const pjg_mech* m, int kind, int slog, int warps, Shape* out)
 // The tile shape for n states (log2 of a tile's states), or -1.
 int choose_shape(const pjg_mech* m, int kind, int64_t n)
 {
-    const int sms = sm_count(m);
     int found = -1;
     for (int slog = 5; slog >= 0; --slog) {
         Shape s;
         if (!shape_fits(m, kind, slog, 8, &s)) continue;
         found = slog;
-        if ((n + (1 << slog) - 1) >> slog >= 2 * sms) break;
+        if ((n + (1 << slog) - 1) >> slog >= 2 * m->sms) break;
     }
     return found;
 }
@@ -416,7 +407,7 @@ int make_tables(pjg_mech* m, int kind, int layout, const std::vector<int>* slot,
         t.sc.buf_terms = sh.buf_terms;
         t.sc.n_vec = ad.n_vec;
         t.n_ns_post = (int)ad.ns_post.size();
-        t.resident = sm_count(m) * pjg_tile_blocks_per_sm(kind, sh.warps, pjg_tile_smem(kind, m->ns, m->n_m, slog, sh.warps, sh.buf_terms));
+        t.resident = m->sms * pjg_tile_blocks_per_sm(kind, sh.warps, pjg_tile_smem(kind, m->ns, m->n_m, slog, sh.warps, sh.buf_terms));
         pk.add(h.tasks, &t.sc.tasks);
         pk.add(h.term_off, &t.sc.term_off);
         pk.add(h.item_off, &t.sc.item_off);
@@ -456,28 +447,48 @@ size_t wave_state_bytes(const pjg_mech* m, int kind, int n_vec)
 }
 
 // Whether a thread per state evaluates `rest` states, less than a wave, sooner
-// than tiles do.  A launch of part of a wave takes a fixed share of the wave's
-// time (0.55 for the Jacobian, 0.5 for J^T v, 0.35 for the rates) and the rest
-// in proportion, tiles take 1.09 to 1.6 times a wave's time in proportion (2.4
-// where the mechanism's tiles are smaller than 32 states).  Measured on GB300,
-// thread per state / tiles, ms: GRI-Mech 3.0 dense Jacobian F 20,000 states
-// 3.11 / 1.69, 60,000 4.28 / 4.14, 77,824 (a wave) 4.63 / 5.03; H2/O2 30,000
-// 0.301 / 0.279, 77,824 0.455 / 0.598; GRI rates 40,000 1.25 / 1.16, 80,000
-// 1.82 / 2.17; GRI J^T v 20,000 1.71 / 1.59, 30,000 1.78 / 2.23; 500 species,
-// sparse Jacobian, 16,384 59 / 46, rates 8,192 12.2 / 5.8, 32,768 16.4 / 22.3.
+// than tiles do, by a model of both in units of a wave's time.  A thread per
+// state takes its time by the blocks of the fullest SM, tiles by rounds of
+// resident blocks, where a short last round costs two thirds of one and more.
+// Slopes from fits to four mechanisms at 27 sizes each on GB300; a mechanism
+// whose item lists are short (sum_parts draws that line) keeps its warps waiting
+// on barriers, and where tiles are smaller than 32 states they are slow.
+// Thread per state / tiles, us: Jacobian F GRI-Mech 3.0 59,000 states 4,194 /
+// 4,080, 72,000 4,248 / 4,809, H2/O2 29,000 280 / 256, 30,000 278 / 315; rates GRI
+// 38,800 998 / 1,083, 39,000 1,178 / 1,084, 50,000 1,221 / 1,332; J^T v GRI 29,000
+// 1,695 / 1,510, 30,000 1,693 / 1,812, H2/O2 26,000 208 / 234; 500 species, sparse
+// Jacobian, 16,384 59 / 46 ms, rates 8,192 12.2 / 5.8, 32,768 16.4 / 22.3.
 bool wave_sooner(const pjg_mech* m, int kind, int64_t rest)
 {
-    Shape s;
-    bool fits = false;
-    for (int slog = 5; slog >= 0 && !fits; --slog) fits = shape_fits(m, kind, slog, 8, &s);
-    if (!fits) return true;  // no tile of this mechanism fits in shared memory
-    // short item lists keep a tile's warps waiting on its barriers, so a small
-    // mechanism's tiles gain less; sum_parts draws the same line.  H2/O2 C, us,
-    // thread per state / tiles: Jacobian 32,000 states 300 / 318, 50,000 361 / 487;
-    // rates 27,000 114 / 100, 38,000 115 / 142, 50,000 146 / 180.
-    const bool small = sum_parts(m->ns) == 1;
-    const double share = s.slog < 5 ? 0.25 : kind == PJG_JACOBIAN ? (small ? 0.375 : 0.75) : kind == PJG_KIND_VJP ? 0.45 : small ? 0.25 : 0.45;
-    return rest >= (int64_t)(share * wave_states(m, kind));
+    struct Cost {
+        double first, block, tile, small, half;  // half: tiles below 32 states
+    };
+    static const Cost costs[3] = {{0.20, 0.133, 1.30, 1.70, 2.2}, {0.40, 0.15, 1.05, 1.55, 2.2}, {0.28, 0.24, 1.24, 1.60, 2.2}};
+    const Cost& c = costs[kind];
+    if (rest <= 0) return false;
+    if (m->top_slog[kind] < 0) return true;  // no tile of this mechanism fits in shared memory
+    const int64_t round = m->round[kind], per_block = (int64_t)m->sms * PJG_BLOCK;
+    double rounds = (double)(rest / round);
+    if (rest % round) rounds += 0.65 + 0.35 * (double)(rest % round) / (double)round;
+    const double slope = m->top_slog[kind] < 5 ? c.half : sum_parts(m->ns) == 1 ? c.small : c.tile;
+    return slope * rounds * (double)round / (double)m->wave[kind] >=
+           c.first + c.block * (double)((rest + per_block - 1) / per_block);
+}
+
+// what the mechanism's launches ask of the device (pjg_mech, once n_m is known)
+void device_shapes(pjg_mech* m)
+{
+    cudaDeviceGetAttribute(&m->sms, cudaDevAttrMultiProcessorCount, m->device);
+    for (int kind = 0; kind < 3; ++kind) {
+        m->wave[kind] = (int64_t)m->sms * pjg_wave_blocks_per_sm(kind) * PJG_BLOCK;
+        for (int slog = 5; slog >= 0 && m->top_slog[kind] < 0; --slog) {
+            Shape s;
+            if (!shape_fits(m, kind, slog, 8, &s)) continue;
+            m->top_slog[kind] = slog;
+            const size_t smem = pjg_tile_smem(kind, m->ns, m->n_m, slog, s.warps, s.buf_terms);
+            m->round[kind] = ((int64_t)m->sms * pjg_tile_blocks_per_sm(kind, s.warps, smem)) << slog;
+        }
+    }
 }
 
 // blocks of a launch over n states
@@ -547,9 +558,15 @@ size_t eval_state_bytes(int kind, bool F, const SlotTables* t)
 
 // How n states are evaluated: whole waves go to the thread-per-state kernel,
 // what is left to the sooner one, in launches of ch_wave and ch_tile states
-// (most_states at most, or by the budget of the shared working buffer).
+// (most_states at most, or by the budget of the shared working buffer).  A rest
+// that leaves an SM fewer blocks than it holds is a launch of its own (n_whole
+// states come before it), which spreads it evenly; in one launch with the waves
+// some SMs take a full load of it.  H2/O2 Jacobian F 110,000 states 755 -> 705
+// us; J^T v of a 40-species mechanism, 97,300 states, 5.08 -> 4.73 ms.  The rates
+// lost by it (GRI-Mech 3.0, 170,000 states 3.34 ms in one launch, 3.42 as the sum
+// of its parts).
 struct Plan {
-    int64_t n_wave = 0, ch_wave = 0, ch_tile = 0;
+    int64_t n_wave = 0, n_whole = 0, ch_wave = 0, ch_tile = 0;
     WaveHold* wh = nullptr;
     SchedTables* sd = nullptr;
     int grid = 0;
@@ -565,18 +582,29 @@ int make_plan(pjg_mech* m, int kind, bool F, bool sparse, const SlotTables* t, i
     const size_t per_state = eval_state_bytes(kind, F, t);
     const int layout = kind == PJG_JACOBIAN ? (F ? 2 : 0) + (sparse ? 1 : 0) : 0;
     const std::vector<int>* slot = t ? &t->slot : nullptr;
-    const int64_t W = wave_states(m, kind);
+    const int64_t W = m->wave[kind];
     KindTables* kt = nullptr;
-    p->n_wave = wave_sooner(m, kind, n % W) ? n : n / W * W;
+    const bool rest_wave = wave_sooner(m, kind, n % W);
+    p->n_wave = rest_wave ? n : n / W * W;
+    const int64_t per_block = (int64_t)m->sms * PJG_BLOCK;
+    p->n_whole = kind != PJG_SPECIES_RATES && n % W <= W - per_block ? n / W * W : p->n_wave;
     if (smaller) {
-        // what a smaller batch leaves to the tiles is less than a wave
-        const int64_t most = p->n_wave > 0 ? std::min(n, W) : n;
-        const int top = p->n_wave > 0 ? 5 : choose_shape(m, kind, per_state ? chunk_states(per_state, n, W) : n);
-        if (int rc = make_tables(m, kind, layout, slot, 0, top, p->n_wave > 0, &kt)) return rc;
+        // What a smaller batch leaves to the tiles is less than a wave.  The most
+        // of n or fewer states, less than a wave, that a thread per state takes
+        // fill their blocks: its time is the same with fewer.
+        const int64_t most = std::min(n, W);
+        int64_t wave = most == W ? W : rest_wave ? n : most / per_block * per_block;
+        while (wave > 0 && wave < W && !wave_sooner(m, kind, wave)) wave = (wave - 1) / per_block * per_block;
+        const int top = n >= W || wave > 0 ? 5 : choose_shape(m, kind, per_state ? chunk_states(per_state, n, W) : n);
+        if (int rc = make_tables(m, kind, layout, slot, 0, top, wave > 0, &kt)) return rc;
         size_t slices = 0;
         for (int q = 0; q <= top; ++q)
             if (kt->tile[q].made) slices = std::max(slices, slice_bytes(kt->tile[q], most));
         p->need = per_state * (size_t)(per_state ? chunk_states(per_state, most, W) : 0) + slices;
+        if (wave > 0) {
+            const size_t each = per_state + wave_state_bytes(m, kind, kt->wave.n_vec);
+            p->need = std::max(p->need, each * (size_t)chunk_states(each, wave, W));
+        }
     }
     if (p->n_wave > 0) {
         if (int rc = make_tables(m, kind, layout, slot, 0, -1, true, &kt)) return rc;
@@ -643,7 +671,7 @@ int run_eval(pjg_mech* m, int kind, int64_t n, char order, int conp, int jac_for
     for (int64_t off = 0, cnt = 0; off < n; off += cnt) {
         const bool wave = off < n_wave;
         const int64_t ch = wave ? pl.ch_wave : pl.ch_tile;
-        cnt = std::min<int64_t>(ch, (wave ? n_wave : n) - off);
+        cnt = std::min<int64_t>(ch, (off < pl.n_whole ? pl.n_whole : wave ? n_wave : n) - off);
         EvalArgs a;
         fill_common(m, a);
         a.n = cnt;
@@ -711,7 +739,7 @@ int run_eval(pjg_mech* m, int kind, int64_t n, char order, int conp, int jac_for
             cudaEventCreate(&e1);
             cudaEventRecord(e0, st);
         }
-        rc = wave ? pjg_launch_wave(a, kind, sm_count(m), st)
+        rc = wave ? pjg_launch_wave(a, kind, m->sms, st)
                   : pjg_launch_tile(a, kind, (int)std::min<int64_t>(pl.grid, (cnt + (1 << sd->sc.slog) - 1) >> sd->sc.slog), st);
         if (rc) return fail(PJG_ERR_CUDA, "kernel launch failed: %s", pjg_launch_error_string());
         g_launches.fetch_add(1);
@@ -1363,6 +1391,7 @@ int pjg_mech_create(const pjg_tables* tb, pjg_mech** out)
     }
     std::vector<int4> m_lists;
     device_records(m, tb->species, m_lists);
+    device_shapes(m);
     std::vector<double> sp(tb->species, tb->species + (size_t)tb->ns * PJG_SP_DOUBLES);
     std::vector<double> coef(tb->thd_coef, tb->thd_coef + std::max(tb->n_thd, 0));
     std::vector<double> aux(tb->aux ? tb->aux : (const double*)nullptr,
@@ -1492,7 +1521,7 @@ int pjg_eval_chunk(pjg_mech* m, int kind, int64_t n, char order, int jac_format,
     KindTables* kt = nullptr;
     if (int rc = make_tables(m, kind, layout, t ? &t->slot : nullptr, 0, -1, true, &kt)) return rc;
     const size_t per_state = eval_state_bytes(kind, order == 'F', t);
-    const int64_t W = wave_states(m, kind), n_wave = wave_sooner(m, kind, n % W) ? n : n / W * W;
+    const int64_t W = m->wave[kind], n_wave = wave_sooner(m, kind, n % W) ? n : n / W * W;
     *states = n_wave ? chunk_states(per_state + wave_state_bytes(m, kind, kt->wave.n_vec), n_wave, W)
                      : chunk_states(per_state, n, W);
     return 0;
@@ -1675,7 +1704,7 @@ int pjg_kernel_resize(pjg_kernel* k, size_t problem_size, size_t work_size)
     // (the evaluation's arrays a little above their size, which the tables give)
     const size_t arrays = (size_t)(tile_arrays(k->kind) + vec_arrays(k->kind) + 2) * m->ns * sizeof(double);
     const size_t ring_state = kRing * (1 + nn + k->out_per_state) * sizeof(double) + per_state + arrays;
-    const int64_t wave = wave_states(m, PJG_JACOBIAN);
+    const int64_t wave = m->wave[PJG_JACOBIAN];
     int64_t chunk = std::min<int64_t>((int64_t)problem_size, PJG_CHUNK_WAVES * wave);
     if ((size_t)chunk * ring_state > kKernelBudget) {
         int64_t c = (int64_t)(kKernelBudget / ring_state);
