@@ -148,8 +148,9 @@ __device__ __forceinline__ double fexp(double x, const double* tab)
 // an integer.  The nearest integer to xs comes from its bits on the integer
 // pipe, so that of fexp's eight FP64 instructions five remain: xs - n, two for
 // the polynomial (in units of the table step), and two for the result.  The
-// rest xs - n is exact.  Values whose exponent leaves the normal range, the
-// reference's clamp at exp(690.775...), infinities and NaN take fexp's way.
+// rest xs - n is exact.  Within 2 ulp (tests/test_scaled_exp.py).  Values from
+// 2^996 (the reference's clamp is at exp(690.775...)), values whose exponent
+// leaves the normal range, infinities and NaN take the library's exp.
 #if PJG_EXP_BITS < 10
 #error "fexp_s takes the degree-3 polynomial of the tables with 1,024 entries and more"
 #endif
