@@ -4,14 +4,10 @@
 For B table bits the kernels read 2^(j/2^B), j = 0 .. 2^B - 1, each the double
 nearest the exact value (computed here in 200-bit arithmetic).  The residual
 r of the argument reduction lies in |r| <= h = ln 2 / 2^(B+1), where exp(r) is
-a polynomial:
-
-* B = 8: the degree-4 Taylor polynomial (truncation below 4e-17 relative);
-* B = 10, 11: a degree-3 polynomial 1 + r + c2 r^2 + c3 r^3 whose c2, c3
-  minimise the largest relative error |p(r) / e^r - 1| over [-h, h] (a
-  linear program over 4,001 Chebyshev points of the interval, the discrete
-  form of the Remez minimax problem), 9.4e-17 for B = 10 and 5.9e-18 for
-  B = 11.
+the polynomial 1 + r + c2 r^2 + c3 r^3 whose c2, c3 minimise the largest relative
+error |p(r) / e^r - 1| over [-h, h] (a linear program over 4,001 Chebyshev points
+of the interval, the discrete form of the Remez minimax problem), 9.4e-17 for
+B = 10 and 5.9e-18 for B = 11.
 
 Run: python gen_exp_table.py  (needs mpmath and scipy; the output is committed)
 """
@@ -21,7 +17,7 @@ import mpmath as mp
 from scipy.optimize import linprog
 
 mp.mp.prec = 200
-BITS = (8, 10, 11)
+BITS = (10, 11)
 
 
 def minimax_deg3(B):
@@ -56,12 +52,10 @@ def main():
         n = 1 << B
         vals = [float(mp.mpf(2) ** (mp.mpf(j) / n)) for j in range(n)]
         out.append("#if PJG_EXP_BITS == %d" % B)
-        out.append("#define PJG_EXP_HAVE_TABLE 1")
-        if B >= 10:
-            c2, c3, worst = minimax_deg3(B)
-            out.append("// minimax on |r| <= ln 2 / 2^%d: largest relative error %.2e" % (B + 1, worst))
-            out.append("#define PJG_EXP_C2 %s" % float.hex(c2))
-            out.append("#define PJG_EXP_C3 %s" % float.hex(c3))
+        c2, c3, worst = minimax_deg3(B)
+        out.append("// minimax on |r| <= ln 2 / 2^%d: largest relative error %.2e" % (B + 1, worst))
+        out.append("#define PJG_EXP_C2 %s" % float.hex(c2))
+        out.append("#define PJG_EXP_C3 %s" % float.hex(c3))
         out.append("__device__ const double pjg_exp2_table[%d] = {" % n)
         for i in range(0, n, 4):
             out.append("    " + ", ".join(float.hex(v) for v in vals[i:i + 4]) + ",")

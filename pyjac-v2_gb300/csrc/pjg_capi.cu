@@ -335,16 +335,16 @@ int64_t chunk_states(size_t per_state, int64_t n, int64_t wave)
 constexpr int64_t kNoallocStates = 4096;
 constexpr int kListTerms = 8;  // entries of an unshared third-body list, at most
 
-// The tile shape for n states: the states of a tile and its warps.
+// A tile's shape: log2 of its states, tasks of a warp per batch, terms of a buffer.
 struct Shape {
-    int slog, warps, rounds, buf_terms;
+    int slog, rounds, buf_terms;
 };
 
 // Shared memory of a block: two blocks of 8 warps per SM where the tile's
 // arrays leave room for a batch's terms in half of it, else the whole.
 constexpr size_t kHalfSmem = ((228u << 10) / 2 - 1024) & ~size_t(127);
 
-bool shape_fits(const pjg_mech* m, int kind, int slog, int warps, Shape* out)
+bool shape_fits(const pjg_mech* m, int kind, int slog, Shape* out)
 {
     const int S = 1 << slog, wpw = 32 / S;
     // terms of a full batch (10 per reaction is more than most leave), at
@@ -353,17 +353,16 @@ bool shape_fits(const pjg_mech* m, int kind, int slog, int warps, Shape* out)
     const int rounds = kind == KIND_RATES ? 4 : 1;
     // the buffers also hold the sums over species: 11 and 6 x 8 partial ones,
     // and three per worker for J^T v
-    const int sums = (72 + (kind == KIND_VJP ? 96 * warps / S : 0) + 1) / 2;
-    const int want = std::max((kind == KIND_RATES ? 1 : 10) * rounds * warps * wpw + 1, sums);
+    const int sums = (72 + (kind == KIND_VJP ? 96 * kTileWarps / S : 0) + 1) / 2;
+    const int want = std::max((kind == KIND_RATES ? 1 : 10) * rounds * kTileWarps * wpw + 1, sums);
     const int least = std::max(per + 1, sums);
     for (size_t limit : {kHalfSmem, (size_t)kTileSmemMax}) {
-        if (warps > 8 && limit != (size_t)kTileSmemMax) continue;
-        const size_t fixed = pjg_tile_smem(kind, m->ns, m->n_m, slog, warps, 0);
+        const size_t fixed = pjg_tile_smem(kind, m->ns, m->n_m, slog, 0);
         if (fixed >= limit) continue;
         const int fit = (int)((limit - fixed) / (2 * S * sizeof(double)));
         const bool half = limit == kHalfSmem;
         if (fit < (half ? std::max(least, want / 2) : least)) continue;
-        *out = Shape{slog, warps, rounds, std::min(std::min(fit, want), 65000)};
+        *out = Shape{slog, rounds, std::min(std::min(fit, want), 65000)};
         return true;
     }
     return false;
@@ -375,7 +374,7 @@ int choose_shape(const pjg_mech* m, int kind, int64_t n)
     int found = -1;
     for (int slog = 5; slog >= 0; --slog) {
         Shape s;
-        if (!shape_fits(m, kind, slog, 8, &s)) continue;
+        if (!shape_fits(m, kind, slog, &s)) continue;
         found = slog;
         if ((n + (1 << slog) - 1) >> slog >= 2 * m->sms) break;
     }
@@ -396,18 +395,17 @@ int make_tables(pjg_mech* m, int kind, int layout, const std::vector<int>* slot,
     for (int slog = from; slog <= to; ++slog) {
         SchedTables& t = kt.tile[slog];
         Shape sh;
-        if (t.made || !shape_fits(m, kind, slog, 8, &sh)) continue;
+        if (t.made || !shape_fits(m, kind, slog, &sh)) continue;
         SchedHost h;
-        if (!sched_build(ad, slog, sh.warps, sh.rounds, sh.buf_terms, h))
+        if (!sched_build(ad, slog, sh.rounds, sh.buf_terms, h))
             return fail(PJG_ERR_UNSUPPORTED, "a reaction's terms pass the evaluation kernel's buffer");
         t.sc.slog = slog;
-        t.sc.warps = sh.warps;
         t.sc.rounds = sh.rounds;
         t.sc.n_batch = h.n_batch;
         t.sc.buf_terms = sh.buf_terms;
         t.sc.n_vec = ad.n_vec;
         t.n_ns_post = (int)ad.ns_post.size();
-        t.resident = m->sms * pjg_tile_blocks_per_sm(kind, sh.warps, pjg_tile_smem(kind, m->ns, m->n_m, slog, sh.warps, sh.buf_terms));
+        t.resident = m->sms * pjg_tile_blocks_per_sm(kind, pjg_tile_smem(kind, m->ns, m->n_m, slog, sh.buf_terms));
         pk.add(h.tasks, &t.sc.tasks);
         pk.add(h.term_off, &t.sc.term_off);
         pk.add(h.item_off, &t.sc.item_off);
@@ -483,10 +481,10 @@ void device_shapes(pjg_mech* m)
         m->wave[kind] = (int64_t)m->sms * pjg_wave_blocks_per_sm(kind) * PJG_BLOCK;
         for (int slog = 5; slog >= 0 && m->top_slog[kind] < 0; --slog) {
             Shape s;
-            if (!shape_fits(m, kind, slog, 8, &s)) continue;
+            if (!shape_fits(m, kind, slog, &s)) continue;
             m->top_slog[kind] = slog;
-            const size_t smem = pjg_tile_smem(kind, m->ns, m->n_m, slog, s.warps, s.buf_terms);
-            m->round[kind] = ((int64_t)m->sms * pjg_tile_blocks_per_sm(kind, s.warps, smem)) << slog;
+            const size_t smem = pjg_tile_smem(kind, m->ns, m->n_m, slog, s.buf_terms);
+            m->round[kind] = ((int64_t)m->sms * pjg_tile_blocks_per_sm(kind, smem)) << slog;
         }
     }
 }
@@ -879,9 +877,6 @@ int ma_pattern_of(const PjgRxn& R)
 struct Packing {
     std::vector<PjgRxn> rx;
     std::vector<int> orig, cls;
-    int nr_e22 = 0;
-    int ma_off[pjg::kMaPatterns + 1] = {};
-    int tp_off[pjg::kTpPatterns + 1] = {};
 };
 
 // Reactions with a third body whose [M] is the same function of the state
@@ -934,8 +929,9 @@ void pack_reactions(const std::vector<PjgRxn>& in, const int* thd_spec, const do
     }
     // third-body groups and the general group: the later reactions sharing
     // [M] with a reaction are moved up to follow it (every other reaction
-    // keeps its place in mechanism order), so that the kernels reuse [M] and
-    // ln [M]; identical lists share one stored copy
+    // keeps its place in mechanism order), so that the thread-per-state kernel
+    // keeps [M] and ln [M] from one to the next (MLast); identical lists share one
+    // stored copy
     std::vector<int> canon;
     const std::vector<int> key = third_body_keys(in, thd_spec, thd_coef, canon);
     for (int g = 1 + nma; g < (int)groups.size(); ++g) {
@@ -958,8 +954,6 @@ void pack_reactions(const std::vector<PjgRxn>& in, const int* thd_spec, const do
     pk.orig.clear();
     pk.cls.clear();
     for (int g = 0; g < (int)groups.size(); ++g) {
-        if (g >= 1 && g <= nma) pk.ma_off[g - 1] = (int)pk.rx.size();
-        if (g > nma && g <= nma + ntp) pk.tp_off[g - 1 - nma] = (int)pk.rx.size();
         for (int i : groups[g]) {
             const PjgRxn& R = in[i];
             PjgRxn c = R;
@@ -977,11 +971,9 @@ void pack_reactions(const std::vector<PjgRxn>& in, const int* thd_spec, const do
             pk.orig.push_back(i);
             pk.cls.push_back(g <= nma + ntp ? g : -1);
         }
-        if (g == 0) pk.nr_e22 = (int)pk.rx.size();
-        if (g == nma) pk.ma_off[nma] = (int)pk.rx.size();
-        if (g == nma + ntp) pk.tp_off[ntp] = (int)pk.rx.size();
     }
-    // RX_SAMEM: [M] equals the previous reaction's in the same group;
+    // Marks that pjg_reaction_order reports; the kernels know a list by its number
+    // (RxnRec).  RX_SAMEM: [M] equals the previous reaction's in the same group;
     // RX_SAMELNM: and an earlier reaction of that run formed ln [M] (a Troe or
     // SRI fall-off with both rate constants in exponential form, which forms
     // it whatever Pr)

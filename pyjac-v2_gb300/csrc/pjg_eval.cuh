@@ -16,9 +16,10 @@ enum { KIND_RATES = 0, KIND_JAC = 1, KIND_VJP = 2 };
 
 // A block evaluates a tile of S = 2^slog states with W warps: lane % S is the
 // state, and the 32 / S lane groups of a warp are workers (G = 32 W / S per
-// block) that take different reactions, species and additions.  Tile arrays
-// (ns doubles per state, in shared memory; in the thread-per-state kernel's
-// scratch before the vectors below):
+// block) that take different reactions, species and additions.
+constexpr int kTileWarps = 8;
+// Tile arrays (ns doubles per state, in shared memory; in the thread-per-state
+// kernel's scratch before the vectors below):
 enum {
     ARR_CONC = 0,  // concentrations c_k
     ARR_EP,        // exp(b_k), the reactant factor of 1 / Kc, where the state's
@@ -81,8 +82,10 @@ struct PostItem {  // target += coef * vec[src], after the reactions
     double coef;
 };
 
-struct Schedule {  // device tables of one (kind, output layout, S, W)
-    int slog = 5, warps = 8, rounds = 1, n_batch = 0, buf_terms = 0;
+struct Schedule {  // device tables of one (kind, output layout, S)
+    // warps: read by the kernel, whose code for a constant ran the 500-species
+    // Jacobian in 14.02 ms against 13.83
+    int slog = 5, warps = kTileWarps, rounds = 1, n_batch = 0, buf_terms = 0;
     int n_vec = 0;                 // entries of the scratch slice per state
     const int4* tasks = nullptr;         // n_batch * rounds * W: class, first reaction, count
     const int* term_off = nullptr;       // per reaction: its terms in the batch's buffer
@@ -216,16 +219,16 @@ struct SchedHost {  // one shape's tables before upload
 };
 void sched_adds(const SchedInput& in, SchedAdds& out);
 // false: a reaction's terms pass the buffer
-bool sched_build(const SchedAdds& in, int slog, int warps, int rounds, int buf_terms, SchedHost& out);
+bool sched_build(const SchedAdds& in, int slog, int rounds, int buf_terms, SchedHost& out);
 
 // host launchers: pjg_tile.cu
 constexpr size_t kTileStatic = 8192 + 256;  // exp table and flags, bytes
-inline size_t stage_bytes(int slog, int warps) { return (size_t)warps * (32 >> slog) * item_stage(slog) * 8; }
+inline size_t stage_bytes(int slog) { return (size_t)kTileWarps * (32 >> slog) * item_stage(slog) * 8; }
 constexpr int kTileSmemMax = 227 << 10;
-size_t pjg_tile_smem(int kind, int ns, int n_m, int slog, int warps, int buf_terms);
+size_t pjg_tile_smem(int kind, int ns, int n_m, int slog, int buf_terms);
 int pjg_launch_tile(const EvalArgs& a, int kind, int grid, void* stream);
 // resident blocks per SM of the kernels of `kind`
-int pjg_tile_blocks_per_sm(int kind, int warps, size_t smem);
+int pjg_tile_blocks_per_sm(int kind, size_t smem);
 // pjg_eval.cu
 int pjg_wave_blocks_per_sm(int kind);
 int pjg_launch_wave(const EvalArgs& a, int kind, int sms, void* stream);

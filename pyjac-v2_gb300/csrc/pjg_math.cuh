@@ -43,52 +43,40 @@ __device__ __forceinline__ double mulpow(double acc, double v, int p)
     return acc * powi(v, p);
 }
 
-// Table of 2^(j/2^B), j = 0 .. 2^B - 1, in shared memory (B = PJG_EXP_BITS):
-// every kernel that calls fexp fills one per block with fill_exp_table before
-// its first use, copied from the generated pjg_exp2_table (B = 8, 10, 11).
-// B = 10 (1,024 entries, 8 KB) is the default: its degree-3 minimax
-// polynomial has one FMA fewer than B = 8's degree-4 Taylor polynomial.  The
-// random lookups meet bank conflicts, which B = 4 (16 entries, one bank pair
-// each) avoids and B = 0 (no table) does without, both at the price of a
-// longer polynomial.  Measured on GB300 (1,048,576 GRI-Mech 3.0 states, F
-// order): B = 4 and B = 0 against B = 6, the Jacobian kernel 2.6 % and 8.3 %
-// slower, the species-rate kernel 13 % and 30 % slower; B = 8 against B = 6,
-// the Jacobian 73.5 against 74.3 ms and the species rates 29.0 against 30.1
-// ms; later B = 10 against B = 8, the Jacobian 70.4 against 70.9 ms and the
-// species rates 23.3 against 24.2 ms.  B = 11 (16 KB per block) equals B = 10
-// on GRI and slows the 500-species mechanism's Jacobian by 13 %.  The FP64
-// instruction count, not the shared-memory lookups, sets the time.
+// Table of 2^(j/2^B), j = 0 .. 2^B - 1, in shared memory (B = PJG_EXP_BITS, 10
+// or 11): every kernel that calls fexp fills one per block with fill_exp_table
+// before its first use, copied from the generated pjg_exp2_table.  B = 10 (1,024
+// entries, 8 KB) is the default.  A smaller table takes a longer polynomial:
+// measured on GB300 when the kernels still had them (1,048,576 GRI-Mech 3.0
+// states, F order), B = 10 against B = 8, the Jacobian 70.4 against 70.9 ms and
+// the species rates 23.3 against 24.2 ms; B = 8 against B = 6, 73.5 against 74.3
+// and 29.0 against 30.1.  B = 11 (16 KB per block) equals B = 10 on GRI and slows
+// the 500-species mechanism's Jacobian by 13 %.
 #ifndef PJG_EXP_BITS
 #define PJG_EXP_BITS 10
 #endif
+#if PJG_EXP_BITS < 10
+#error "the polynomial of degree 3 wants a table of 1,024 entries and more"
+#endif
 #define PJG_EXP_TAB (1 << PJG_EXP_BITS)
 }  // namespace pjg
-#include "pjg_exp_table.h"  // pjg_exp2_table for B = 8, 10, 11 (gen_exp_table.py)
+#include "pjg_exp_table.h"  // pjg_exp2_table for B = 10, 11 (gen_exp_table.py)
 namespace pjg {
 
 __device__ __forceinline__ void fill_exp_table(double* tab)
 {
-    for (int j = threadIdx.x; j < PJG_EXP_TAB; j += blockDim.x)
-#ifdef PJG_EXP_HAVE_TABLE
-        tab[j] = pjg_exp2_table[j];
-#else
-        tab[j] = exp2((double)j * (1.0 / PJG_EXP_TAB));
-#endif
+    for (int j = threadIdx.x; j < PJG_EXP_TAB; j += blockDim.x) tab[j] = pjg_exp2_table[j];
 }
 
 // exp(x) by the table-driven method of P. T. P. Tang ("Table-driven
 // implementation of the exponential function in IEEE floating-point
 // arithmetic", ACM TOMS 15(2), 1989): x = (2^B m + j) ln2 / 2^B + r with
 // |r| <= ln2 / 2^(B+1), so exp(x) = 2^m 2^(j/2^B) exp(r).  exp(r) is a
-// polynomial: of degree 3 for B = 10 and 11 with minimax coefficients
-// (gen_exp_table.py; |r| <= 3.4e-4, largest relative error 9.4e-17 for
-// B = 10), else the Taylor polynomial, of degree 4 for B = 8 (|r| <= 0.00136,
-// truncation below 4e-17 relative), 5 for B = 6 (|r| <= 0.0055, below
-// 4e-17), 7 for B = 4 (|r| <= 0.022, below 2e-18) and 13 for B = 0
-// (|r| <= 0.35, below 5e-18).  The reduction is Cody and Waite's with
-// ln2 split in two (the leading part is the double nearest ln 2, the trailing
-// part the rest), each product taken by one FMA.  The scale 2^m goes into the
-// exponent field with an integer add.  |x| >= 708, infinities and NaN take
+// polynomial of degree 3 with minimax coefficients (gen_exp_table.py; for B = 10
+// |r| <= 3.4e-4, largest relative error 9.4e-17).  The reduction is Cody and
+// Waite's with ln2 split in two (the leading part is the double nearest ln 2, the
+// trailing part the rest), each product taken by one FMA.  The scale 2^m goes into
+// the exponent field with an integer add.  |x| >= 708, infinities and NaN take
 // the library exp.  Tested against the CUDA library exp: within 3 ulp.
 __device__ __forceinline__ double fexp(double x, const double* tab)
 {
@@ -103,43 +91,11 @@ __device__ __forceinline__ double fexp(double x, const double* tab)
     const int n = __double2loint(t);               // the same integer
     double r = fma(-nd, l1, x);
     r = fma(-nd, l2, r);
-    // q = (exp(r) - 1) / r by Horner's rule on the Taylor coefficients 1/k!
-    // (B >= 10: on the minimax coefficients of gen_exp_table.py)
-#if PJG_EXP_BITS >= 10
+    // q = (exp(r) - 1) / r
     double q = fma(r, PJG_EXP_C3, PJG_EXP_C2);
     q = fma(q, r, 1.0);
-#elif PJG_EXP_BITS >= 8
-    double q = 1.0 / 24;
-#elif PJG_EXP_BITS >= 6
-    double q = fma(r, 1.0 / 120, 1.0 / 24);
-#elif PJG_EXP_BITS >= 4
-    double q = fma(r, 1.0 / 40320, 1.0 / 5040);
-    q = fma(q, r, 1.0 / 720);
-    q = fma(q, r, 1.0 / 120);
-    q = fma(q, r, 1.0 / 24);
-#else
-    double q = fma(r, 1.0 / 87178291200.0, 1.0 / 6227020800.0);
-    q = fma(q, r, 1.0 / 479001600.0);
-    q = fma(q, r, 1.0 / 39916800.0);
-    q = fma(q, r, 1.0 / 3628800.0);
-    q = fma(q, r, 1.0 / 362880.0);
-    q = fma(q, r, 1.0 / 40320);
-    q = fma(q, r, 1.0 / 5040);
-    q = fma(q, r, 1.0 / 720);
-    q = fma(q, r, 1.0 / 120);
-    q = fma(q, r, 1.0 / 24);
-#endif
-#if PJG_EXP_BITS < 10
-    q = fma(q, r, 1.0 / 6);
-    q = fma(q, r, 0.5);
-    q = fma(q, r, 1.0);
-#endif
-#if PJG_EXP_BITS > 0
     const double tj = tab[n & (PJG_EXP_TAB - 1)];
     const double y = fma(tj, r * q, tj);
-#else
-    const double y = fma(r, q, 1.0);
-#endif
     return __longlong_as_double(__double_as_longlong(y) + ((long long)(n >> PJG_EXP_BITS) << 52));
 }
 
@@ -151,9 +107,6 @@ __device__ __forceinline__ double fexp(double x, const double* tab)
 // rest xs - n is exact.  Within 2 ulp (tests/test_scaled_exp.py).  Values from
 // 2^996 (the reference's clamp is at exp(690.775...)), values whose exponent
 // leaves the normal range, infinities and NaN take the library's exp.
-#if PJG_EXP_BITS < 10
-#error "fexp_s takes the degree-3 polynomial of the tables with 1,024 entries and more"
-#endif
 constexpr double kExpStep = 0.6931471805599453 * (1.0 / PJG_EXP_TAB);    // ln 2 / 2^B
 constexpr double kExpScale = 1.4426950408889634 * PJG_EXP_TAB;           // 2^B / ln 2
 
@@ -224,18 +177,14 @@ __device__ __forceinline__ double gsmall(double x)
 
 // Arrhenius forms of rate_subs.py get_simple_arrhenius_rates (:2642-3023).  ls
 // is ln T and tis 1 / T, both times 2^B / ln 2; A and its integer n as RxnRec
-// holds them.  lns is the exponent's part besides n (has_ln false for the
-// forms A and A T^b).
+// holds them.
 __device__ __forceinline__ double arrhenius(int form, double A, int n, double b, double Ta, double Tc,
-                                            double Tinv, double ls, double tis, const double* tab,
-                                            double& lns, bool& has_ln)
+                                            double Tinv, double ls, double tis, const double* tab)
 {
-    has_ln = form > FORM_AT;
     if (form == FORM_A) return A;
     // fast_powi of a negative exponent inverts its base first
     if (form == FORM_AT) return __dmul_rn(A, n < 0 ? powi(Tinv, -n) : powi(Tc, n));
-    lns = fma(-Ta, tis, fma(b, ls, A));
-    return fexp_s(lns, n, tab);
+    return fexp_s(fma(-Ta, tis, fma(b, ls, A)), n, tab);
 }
 
 // PLOG: ln kf interpolated linearly in ln P between bracketing pressures,

@@ -257,11 +257,10 @@ __device__ __forceinline__ void rxn_terms(const RxnHead& h, const double* aux,
     const double* et = sv.etab;
 
     // forward rate constant and its log-derivatives (dl: T d ln kf / dT)
-    double kf, dl = 0.0, dlnkf_dlnP = 0.0, lnkf = 0.0;
-    bool has_lnkf = false;
+    double kf, dl = 0.0, dlnkf_dlnP = 0.0;
     if (form <= FORM_ARR) {
         kf = arrhenius(form, ldg(p + P_A), h.bint, ldg(p + P_B), ldg(p + P_TA), Tc, sv.Tinv, sv.ls, sv.tis,
-                       et, lnkf, has_lnkf);
+                       et);
         if (DER) dl = fma(ldg(p + P_TA), Tjinv, ldg(p + P_B));
     } else if (form == FORM_PLOG) {
         kf = gexp(plog_logk(aux + h.auxo, sv.logT, sv.Tinv, sv.logP, Tjinv, &dl, &dlnkf_dlnP), et);
@@ -340,10 +339,8 @@ __device__ __forceinline__ void rxn_terms(const RxnHead& h, const double* aux,
                 fs.kratio = fexp_s(lnr, h.fbint, et);
                 lnr = __dadd_rn(lnr, ldg(p + P_RN));
             } else {
-                double lnkfall = 0.0;
-                bool has_lnkfall = false;
                 const double kfall = arrhenius(RX_FFORM(flags), ldg(p + P_FA), h.fbint, ldg(p + P_FB),
-                                               ldg(p + P_FTA), Tc, sv.Tinv, sv.ls, sv.tis, et, lnkfall, has_lnkfall);
+                                               ldg(p + P_FTA), Tc, sv.Tinv, sv.ls, sv.tis, et);
                 fs.kratio = chem ? kf / kfall : kfall / kf;
             }
             fs.Pr = __dmul_rn(M, fs.kratio);
@@ -593,10 +590,8 @@ __device__ __forceinline__ void e22_terms(const E22Head& h, const E22Vals& v, in
 {
     const double* p = h.p;
     const double b = ldg(p + P_B), Ta = ldg(p + P_TA);
-    double lnk;
-    bool has_ln;
     const double kf = arrhenius(RX_FORM(h.flags), ldg(p + P_A), h.bint, b, Ta, sv.Tc, sv.Tinv, sv.ls, sv.tis,
-                                sv.etab, lnk, has_ln);
+                                sv.etab);
     double ikc;  // 1 / Kc = exp(-sum nu b)
     if (sv.split) {
         ikc = __dmul_rn(__dmul_rn(v.x[0], v.x[1]), __dmul_rn(v.x[2], v.x[3]));
@@ -705,10 +700,8 @@ __device__ __forceinline__ void ma_terms(const RxnHead& h, int last, const State
     constexpr int N = PT::n;
     const double* p = h.p;
     const double b = ldg(p + P_B), Ta = ldg(p + P_TA);
-    double lnk;
-    bool has_ln;
     const double kf = arrhenius(RX_FORM(h.flags), ldg(p + P_A), h.bint, b, Ta, sv.Tc, sv.Tinv, sv.ls, sv.tis,
-                                sv.etab, lnk, has_ln);
+                                sv.etab);
     int sp[N];
     double c[N];
 #pragma unroll

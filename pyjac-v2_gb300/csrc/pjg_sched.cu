@@ -260,9 +260,9 @@ void sched_adds(const SchedInput& in, SchedAdds& o)
     o.unread = (unsigned)o.n_vec++;  // the slice's last entry
 }
 
-bool sched_build(const SchedAdds& in, int slog, int warps, int rounds, int buf_terms, SchedHost& o)
+bool sched_build(const SchedAdds& in, int slog, int rounds, int buf_terms, SchedHost& o)
 {
-    const int S = 1 << slog, wpw = 32 / S, G = warps * wpw;
+    const int S = 1 << slog, wpw = 32 / S, G = kTileWarps * wpw;
     const int nr = (int)in.terms.size();
     o.n_batch = 0;
     // batches of tasks
@@ -270,7 +270,7 @@ bool sched_build(const SchedAdds& in, int slog, int warps, int rounds, int buf_t
     std::vector<int> batch_r = {0};  // first reactions of the batches
     for (int i = 0; i < nr;) {
         int terms = 1, n_tasks = 0;  // term 0 is zero
-        while (i < nr && n_tasks < warps * rounds) {
+        while (i < nr && n_tasks < kTileWarps * rounds) {
             const int cl = in.cls[i], i0 = i;
             while (i < nr && i - i0 < wpw && in.cls[i] == cl && terms + in.terms[i] <= buf_terms) {
                 o.term_off[i] = terms;
@@ -281,12 +281,12 @@ bool sched_build(const SchedAdds& in, int slog, int warps, int rounds, int buf_t
             ++n_tasks;
         }
         if (!n_tasks) return false;  // one reaction's terms pass the buffer
-        o.tasks.resize(o.tasks.size() + warps * rounds - n_tasks, make_int4(0, 0, 0, 0));
+        o.tasks.resize(o.tasks.size() + kTileWarps * rounds - n_tasks, make_int4(0, 0, 0, 0));
         ++o.n_batch;
         batch_r.push_back(i);
     }
     if (!nr) {  // one empty batch, for the zeros
-        o.tasks.assign(warps * rounds, make_int4(0, 0, 0, 0));
+        o.tasks.assign(kTileWarps * rounds, make_int4(0, 0, 0, 0));
         o.n_batch = 1;
         batch_r.push_back(0);
     }

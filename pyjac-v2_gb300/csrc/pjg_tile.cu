@@ -54,7 +54,7 @@ __device__ __forceinline__ void red_global(uint64_t p, double x)
 // 56 to 74 %): what is left are the phases between the reactions and the
 // reductions' rate, about 23 clocks per warp and SM.
 template <int KIND>  // KIND_RATES, KIND_JAC, KIND_VJP
-__global__ void __launch_bounds__(KIND == KIND_RATES ? 256 : 512, KIND == KIND_RATES ? 3 : 1)
+__global__ void __launch_bounds__(32 * kTileWarps, KIND == KIND_RATES ? 3 : 2)
     tile_kernel(const EvalArgs a)
 {
     constexpr bool JAC = KIND == KIND_JAC;
@@ -702,9 +702,9 @@ __global__ void __launch_bounds__(KIND == KIND_RATES ? 256 : 512, KIND == KIND_R
 
 }  // namespace
 
-size_t pjg_tile_smem(int kind, int ns, int n_m, int slog, int warps, int buf_terms)
+size_t pjg_tile_smem(int kind, int ns, int n_m, int slog, int buf_terms)
 {
-    return kTileStatic + stage_bytes(slog, warps) +
+    return kTileStatic + stage_bytes(slog) +
            (((size_t)tile_arrays(kind) * ns + 2 * (size_t)n_m + 2 * (size_t)buf_terms) << slog) * sizeof(double);
 }
 
@@ -719,12 +719,12 @@ const void* kernel_of(int kind)
 
 }  // namespace
 
-int pjg_tile_blocks_per_sm(int kind, int warps, size_t smem)
+int pjg_tile_blocks_per_sm(int kind, size_t smem)
 {
     int b = 0;
     const void* fn = kernel_of(kind);
     if (cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, kTileSmemMax) != cudaSuccess ||
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, fn, 32 * warps, smem) != cudaSuccess)
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, fn, 32 * kTileWarps, smem) != cudaSuccess)
         return 1;
     return b > 0 ? b : 1;
 }
@@ -733,8 +733,8 @@ int pjg_launch_tile(const EvalArgs& a, int kind, int grid, void* stream)
 {
     if (a.n <= 0) return 0;
     const cudaStream_t st = (cudaStream_t)stream;
-    const size_t smem = pjg_tile_smem(kind, a.ns, a.n_m, a.sc.slog, a.sc.warps, a.sc.buf_terms);
-    const int threads = 32 * a.sc.warps;
+    const size_t smem = pjg_tile_smem(kind, a.ns, a.n_m, a.sc.slog, a.sc.buf_terms);
+    const int threads = 32 * kTileWarps;
     pjg_launch_err = cudaFuncSetAttribute(kernel_of(kind), cudaFuncAttributeMaxDynamicSharedMemorySize, kTileSmemMax);
     if (pjg_launch_err != cudaSuccess) return -2;
     if (kind == KIND_JAC) tile_kernel<KIND_JAC><<<grid, threads, smem, st>>>(a);
