@@ -7,7 +7,11 @@ order, dense 54 x 54 Jacobian.  One step = one Jacobian evaluation of all
 states (pjg_jacobian).  Inputs (453 MB) and outputs (24.5 GB) are larger than
 L2, so no flush is needed between steps.
 
-The same JSON line carries, under ``configs``, the other benchmark
+Standard output is one JSON line.  It carries the headline whole and a value or
+two of each further block; the blocks themselves (rooflines, CPU baselines,
+parity, surrogate curves, implicit step) go to standard error, a JSON line each,
+so that the line stays short enough for a reader of the output's tail.  Under
+``configs`` are the other benchmark
 configurations, each timed on the device with its roofline, a CPU baseline on
 the same host and a sampled parity check against the oracle: H2/O2 dense
 Jacobian and species rates (65,536 states, C order), GRI-Mech 3.0 species
@@ -726,7 +730,7 @@ def implicit_bench(mech, ev, dev, n, order, steps, warmup, fp64_peak):
                       "fp64_frac": fl * f_rate / 1e12 / fp64_peak,
                       "fp64_peak_source": "measured DFMA probe (pjg_fp64_peak)",
                       "hbm_gbs": 2 * lu_bytes * f_rate / 1e9},
-           "solve": {"kernel": "lu_solve_kernel (one thread per state)", "ms": s_ms,
+           "solve": {"kernel": "lu_solve_kernel (32 states per block, rows shared by 8 warps)", "ms": s_ms,
                      "states_per_s": n / (s_ms * 1e-3), "launches": s_launch,
                      "alg_bytes_per_state": lu_bytes + 4 * nn + 16 * nn,
                      "hbm_gbs": (lu_bytes + 20 * nn) * n / (s_ms * 1e-3) / 1e9},
@@ -863,6 +867,45 @@ def run_reference(args):
                    "d2h_bytes_per_step": 0}}
     print(json.dumps(out))
     return 0
+
+
+def _pick(block, *keys):
+    return {k: block[k] for k in keys if k in block} if block else block
+
+
+def split_record(rec):
+    """(the line for standard output, the blocks for standard error)."""
+    line = dict(rec)
+    detail = {}
+    for key in ("roofline", "cpu_baseline", "e2e", "parity", "configs", "surrogate", "implicit_step"):
+        if rec.get(key):
+            detail[key] = rec[key]
+    r = rec.get("roofline") or {}
+    if r:
+        line["roofline"] = dict(_pick(r, "bound", "achieved", "peak", "unit", "frac", "traffic", "kernel",
+                                      "alg_bytes_per_state", "eval_ms_per_step", "eval_launches"),
+                                fp64=_pick(r.get("fp64"), "achieved", "peak", "unit", "frac", "exec_frac",
+                                           "pipe_frac"))
+    line["cpu_baseline"] = _pick(rec.get("cpu_baseline"), "value", "unit", "cores", "kind")
+    e = rec.get("e2e")
+    if e:
+        line["e2e"] = dict(_pick(e, "value", "unit", "h2d_bytes_per_step", "d2h_bytes_per_step", "steps",
+                                 "median_call_ms"), **_pick(e.get("link") or {}, "d2h_floor_ms_per_step"))
+    line["parity"] = {k: v for k, v in (rec.get("parity") or {}).items()
+                      if k == "n_checked" or k.endswith("_pass") or "max_r" in k}
+    c = rec.get("configs")
+    if c:
+        line["configs"] = {k: _pick(v, "value", "unit") for k, v in c.items()}
+    u = rec.get("surrogate")
+    if u:
+        line["surrogate"] = dict(_pick(u, "network_speedup_vs_fp64", "err_median"),
+                                 speedup_at_tol={str(x["tol"]): round(x["speedup_vs_fp64"], 3)
+                                                 for x in u.get("with_fallback", [])})
+    i = rec.get("implicit_step")
+    if i:
+        line["implicit_step_ms"] = {k: v["ms"] for k, v in i.items() if isinstance(v, dict) and "ms" in v}
+    line.pop("implicit_step", None)
+    return line, detail
 
 
 def run_gpu(args):
@@ -1055,15 +1098,19 @@ def run_gpu(args):
                               log=lambda h: print(json.dumps(h), file=sys.stderr))
 
     if rank == 0:
-        line = {"metric": metric, "value": value, "unit": unit, "n_gpus": world,
-                "steps": args.steps, "warmup": max(3, args.warmup), "ms_per_step": ms_step,
-                "higher_is_better": True, "scaling": "weak", "vs_baseline": None,
-                "dtype": "f64", "data": "synthetic",
-                "config": headline_config(args, mech),
-                "roofline": roofline, "cpu_baseline": cpu, "e2e": e2e,
-                "gpu_launches": launches, "clocks": clk, "parity": parity,
-                "configs": configs, "surrogate": sur, "implicit_step": implicit}
-        print(json.dumps(line))
+        rec = {"metric": metric, "value": value, "unit": unit, "n_gpus": world,
+               "steps": args.steps, "warmup": max(3, args.warmup), "ms_per_step": ms_step,
+               "higher_is_better": True, "scaling": "weak", "vs_baseline": None,
+               "dtype": "f64", "data": "synthetic",
+               "config": headline_config(args, mech),
+               "roofline": roofline, "cpu_baseline": cpu, "e2e": e2e,
+               "gpu_launches": launches, "clocks": clk, "parity": parity,
+               "configs": configs, "surrogate": sur, "implicit_step": implicit}
+        line, detail = split_record(rec)
+        for key_, block in detail.items():
+            print(json.dumps({key_: block}), file=sys.stderr)
+        sys.stderr.flush()
+        print(json.dumps(line), flush=True)
     sh.barrier()
     sh.destroy_process_group()
     return 0
