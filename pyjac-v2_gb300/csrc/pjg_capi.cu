@@ -3,7 +3,7 @@
 // Host responsibilities: validate and upload the mechanism tables, derive the
 // Jacobian slot tables for each output layout (dense/sparse x C/F), size the
 // per-state working arrays, chunk large problems, and launch the kernels of
-// pjg_eval.cu.  Mirrors the reference's generated Kernel class
+// pjg_wave.cuh and pjg_tile.cu.  Mirrors the reference's generated Kernel class
 // (pyjac/kernel_utils/common/kernel.hpp.in:86-335, kernel.cpp.in:539-633):
 // problems are evaluated in chunks (the reference's max_per_run) with a
 // per-kernel-object device working buffer (the reference's rwk).
@@ -454,21 +454,23 @@ size_t wave_state_bytes(const pjg_mech* m, int kind, int n_vec)
 // Thread per state / tiles, us: Jacobian F GRI-Mech 3.0 59,000 states 4,194 /
 // 4,080, 72,000 4,248 / 4,809, H2/O2 29,000 280 / 256, 30,000 278 / 315; rates GRI
 // 38,800 998 / 1,083, 39,000 1,178 / 1,084, 50,000 1,221 / 1,332; J^T v GRI 29,000
-// 1,695 / 1,510, 30,000 1,693 / 1,812, H2/O2 26,000 208 / 234; 500 species, sparse
-// Jacobian, 16,384 59 / 46 ms, rates 8,192 12.2 / 5.8, 32,768 16.4 / 22.3.
+// 1,695 / 1,510, 30,000 1,693 / 1,812, H2/O2 26,000 208 / 234; 500 species, ms:
+// sparse Jacobian F 16,384 50 / 50, 24,000 56 / 74, rates 19,456 13.8 / 10.1, 32,768
+// 16.5 / 17.2, J^T v 12,000 38 / 35, 16,384 38 / 48.
 bool wave_sooner(const pjg_mech* m, int kind, int64_t rest)
 {
     struct Cost {
-        double first, block, tile, small, half;  // half: tiles below 32 states
+        double first, block, tile, small;
     };
-    static const Cost costs[3] = {{0.20, 0.133, 1.30, 1.70, 2.2}, {0.40, 0.15, 1.05, 1.55, 2.2}, {0.28, 0.24, 1.24, 1.60, 2.2}};
-    const Cost& c = costs[kind];
+    static const Cost costs[3] = {{0.20, 0.133, 1.30, 1.70}, {0.40, 0.15, 1.05, 1.55}, {0.28, 0.24, 1.24, 1.60}};
+    static const Cost large[3] = {{0.33, 0.07, 1.75}, {0.60, 0.135, 2.54}, {0.63, 0.12, 3.31}};  // tiles below 32 states
+    const Cost& c = m->top_slog[kind] < 5 ? large[kind] : costs[kind];
     if (rest <= 0) return false;
     if (m->top_slog[kind] < 0) return true;  // no tile of this mechanism fits in shared memory
     const int64_t round = m->round[kind], per_block = (int64_t)m->sms * PJG_BLOCK;
     double rounds = (double)(rest / round);
     if (rest % round) rounds += 0.65 + 0.35 * (double)(rest % round) / (double)round;
-    const double slope = m->top_slog[kind] < 5 ? c.half : sum_parts(m->ns) == 1 ? c.small : c.tile;
+    const double slope = sum_parts(m->ns) == 1 ? c.small : c.tile;
     return slope * rounds * (double)round / (double)m->wave[kind] >=
            c.first + c.block * (double)((rest + per_block - 1) / per_block);
 }
@@ -478,7 +480,6 @@ void device_shapes(pjg_mech* m)
 {
     cudaDeviceGetAttribute(&m->sms, cudaDevAttrMultiProcessorCount, m->device);
     for (int kind = 0; kind < 3; ++kind) {
-        m->wave[kind] = (int64_t)m->sms * pjg_wave_blocks_per_sm(kind) * PJG_BLOCK;
         for (int slog = 5; slog >= 0 && m->top_slog[kind] < 0; --slog) {
             Shape s;
             if (!shape_fits(m, kind, slog, &s)) continue;
@@ -486,6 +487,7 @@ void device_shapes(pjg_mech* m)
             const size_t smem = pjg_tile_smem(kind, m->ns, m->n_m, slog, s.buf_terms);
             m->round[kind] = ((int64_t)m->sms * pjg_tile_blocks_per_sm(kind, smem)) << slog;
         }
+        m->wave[kind] = (int64_t)m->sms * pjg_wave_blocks_per_sm(kind, m->top_slog[kind] < 5) * PJG_BLOCK;
     }
 }
 
@@ -737,7 +739,7 @@ int run_eval(pjg_mech* m, int kind, int64_t n, char order, int conp, int jac_for
             cudaEventCreate(&e1);
             cudaEventRecord(e0, st);
         }
-        rc = wave ? pjg_launch_wave(a, kind, m->sms, st)
+        rc = wave ? pjg_launch_wave(a, kind, m->sms, m->top_slog[kind] < 5, st)
                   : pjg_launch_tile(a, kind, (int)std::min<int64_t>(pl.grid, (cnt + (1 << sd->sc.slog) - 1) >> sd->sc.slog), st);
         if (rc) return fail(PJG_ERR_CUDA, "kernel launch failed: %s", pjg_launch_error_string());
         g_launches.fetch_add(1);

@@ -1,5 +1,5 @@
 // Kernel argument block, work schedule and per-state array layout shared by
-// the evaluation kernels (pjg_eval.cu), the schedule builder (pjg_sched.cu)
+// the evaluation kernels (pjg_wave.cuh, pjg_tile.cu), the schedule builder (pjg_sched.cu)
 // and their host launcher (pjg_capi.cu).
 #pragma once
 #include <cuda_runtime.h>
@@ -10,7 +10,7 @@
 
 enum { KIND_RATES = 0, KIND_JAC = 1, KIND_VJP = 2 };
 
-// Two kernels: a thread per state (pjg_eval.cu), for batches of several waves of
+// Two kernels: a thread per state (pjg_wave.cuh), for batches of several waves of
 // resident blocks, and a block per tile of a few states (pjg_tile.cu).
 #define PJG_BLOCK 128  // threads of a block of the former
 
@@ -230,8 +230,9 @@ int pjg_launch_tile(const EvalArgs& a, int kind, int grid, void* stream);
 // resident blocks per SM of the kernels of `kind`
 int pjg_tile_blocks_per_sm(int kind, size_t smem);
 // pjg_eval.cu
-int pjg_wave_blocks_per_sm(int kind);
-int pjg_launch_wave(const EvalArgs& a, int kind, int sms, void* stream);
+int pjg_wave_blocks_per_sm(int kind, bool large);
+// large: of a mechanism whose tiles are smaller than 32 states
+int pjg_launch_wave(const EvalArgs& a, int kind, int sms, bool large, void* stream);
 extern thread_local cudaError_t pjg_launch_err;  // of this thread's last evaluation launch
 const char* pjg_launch_error_string();           // CUDA's description of it
 int pjg_fp64_probe(int blocks, int threads, int iters, double* out, void* stream);

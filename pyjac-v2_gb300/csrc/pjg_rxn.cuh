@@ -1,4 +1,4 @@
-// Per-reaction evaluation of the evaluation kernels (pjg_eval.cu).
+// Per-reaction evaluation of the evaluation kernels (pjg_wave.cuh, pjg_tile.cu).
 //
 // rxn_terms() evaluates one reaction at one state: forward rate constant
 // (get_simple_arrhenius_rates :2642, PLOG :2084, Chebyshev :1904 of

@@ -1,5 +1,5 @@
 // Species-rate, Jacobian and J^T v kernels for batches below a wave of the
-// thread-per-state kernels (pjg_eval.cu), whose results they give bit for bit:
+// thread-per-state kernels (pjg_wave.cuh), whose results they give bit for bit:
 // the same reaction code (pjg_rxn.cuh), every sum in the same order.
 #include <cuda_runtime.h>
 

@@ -127,6 +127,18 @@ def test_approximate_jacobian(cuda_device, name, order, fmt):
     check(mech, P, phi, order, True, fmt, cuda_device, wave(cuda_device), vjp=False)
 
 
+@pytest.mark.parametrize("blocks", [2, 3])
+def test_large_mechanism(cuda_device, blocks):
+    """The 500-species mechanism, whose Jacobian kernel holds three blocks per SM
+    (and two in the form for fewer blocks)."""
+    import torch
+    torch.cuda.empty_cache()
+    mech = load_mech("synthetic500")
+    P, phi = pkg("states").draw_states(mech.n_species, 6, seed=18)
+    check(mech, P, phi, "F", True, "sparse", cuda_device, blocks * wave(cuda_device) // 4, vjp=False)
+    torch.cuda.empty_cache()
+
+
 @pytest.mark.parametrize("waves", [0, 1])
 @pytest.mark.parametrize("conp", [True, False])
 def test_mechanism_that_does_not_conserve_mass(cuda_device, tmp_path, waves, conp):
