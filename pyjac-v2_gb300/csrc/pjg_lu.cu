@@ -1088,14 +1088,20 @@ extern "C" int pjg_internal_lu_solve(int32_t nn, int64_t n, char order, const do
         if (rc) return rc;
     } else {
         // A thread per state costs the latency of nn^2 entries in turn until its blocks
-        // fill the SMs; from there on it is the faster one in C order, where a column
-        // step of 32 states touches 32 sectors, and for short columns, which leave
-        // warps idle.  A whole ROS2 step on GB300, this kernel / a thread per state:
-        // GRI F 20,000 states 5.73 / 6.95 ms, F 70,000 17.4 / 18.7, C 70,000 19.2 /
-        // 17.8; h2o2 C 100 states 0.14 / 0.37, 38,000 0.79 / 0.70, 65,536 1.10 / 1.06.
+        // fill the SMs; from some number of states on it is the faster one.  Short
+        // columns leave the other kernel's warps idle.  In C order a column step of 32
+        // states touches a sector of each row, which the next columns find again only
+        // in L1, so it turns earlier, and earliest where the blocks' vectors leave L1
+        // 28 KB of the 256.  Solves on GB300, this kernel / a thread per state, us: C
+        // nn = 40 19,456 states 260 / 296, 54 17,000 500 / 510, 29,184 620 / 560, 60 9,728
+        // 0.77 of its time, 14,592 1.47, 80 9,728 0.60, 14,592 1.05, 100 7,000 0.82, 9,728
+        // 1.35; F 54 77,824 0.89, 97,280 1.03, 140 64,000 1.01, 77,824 1.12.
         int sms = 0;
         if (int rc = sm_count(&sms)) return rc;
-        if (nn < 32 ? n >= 128LL * sms : order == 'C' && n >= 256LL * sms) {
+        const size_t each = solve_smem(nn) + 1024, sm = size_t(228) << 10;
+        const bool tight = nn > 40 && sm / each * each > (size_t(196) << 10);
+        const long long per_sm = nn < 32 ? 128 : order == 'F' ? (nn < 104 ? 576 : 400) : tight ? 56 : nn < 72 ? 128 : 80;
+        if (n >= per_sm * sms) {
             const int grid = (int)((n + 127) / 128);
             if (order == 'F') lu_solve_lane_kernel<true><<<grid, 128, 0, st>>>(nn, n, lu, piv, b);
             else lu_solve_lane_kernel<false><<<grid, 128, 0, st>>>(nn, n, lu, piv, b);
