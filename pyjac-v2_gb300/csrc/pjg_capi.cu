@@ -332,7 +332,7 @@ int64_t chunk_states(size_t per_state, int64_t n, int64_t wave)
     return std::min<int64_t>(c, n);
 }
 
-constexpr int64_t kNoallocStates = 4096;
+constexpr int64_t kNoallocStates = 4096;  // pjg_vjp_noalloc's tiles are those of so many states
 constexpr int kListTerms = 8;  // entries of an unshared third-body list, at most
 
 // A tile's shape: log2 of its states, tasks of a warp per batch, terms of a buffer.
@@ -1109,15 +1109,29 @@ void device_records(pjg_mech* m, const double* species, std::vector<int4>& m_lis
 
 }  // namespace
 
+namespace {
+
+// The tile shape of pjg_vjp_noalloc.  A small mechanism's tile takes about as long
+// whatever its number of states, so more than a round of them goes to the
+// largest (H2/O2, us, tiles of 8 / of 32: 10,000 states 305 / 141, 200,000 5,067 /
+// 1,508; a thread per state in chunks had taken 160 and 1,928).
+int noalloc_shape(const pjg_mech* m, int64_t n)
+{
+    const int slog = choose_shape(m, PJG_KIND_VJP, kNoallocStates);
+    return slog >= 0 && sum_parts(m->ns) == 1 && n > (int64_t)2 * m->sms << slog ? m->top_slog[PJG_KIND_VJP] : slog;
+}
+
+}  // namespace
+
 // Internal accessors for other translation units of this library.
 int pjg_internal_fail(int code, const char* msg) { return fail(code, "%s", msg); }
-// The J^T v launch of n states with scratch_doubles of scratch, in tiles of the
-// shape for kNoallocStates states, whose schedule pjg_mech_create has made: the argument
-// block's mechanism and schedule, and the grid.
+// The J^T v launch of n states with scratch_doubles of scratch, in tiles whose
+// schedule pjg_mech_create has made (noalloc_shape): the argument block's mechanism
+// and schedule, and the grid.
 int pjg_internal_vjp_args(pjg_mech* m, int64_t n, size_t scratch_doubles, EvalArgs* a, int* grid)
 {
     KindTables* kt = nullptr;
-    const int slog = choose_shape(m, PJG_KIND_VJP, kNoallocStates);
+    const int slog = noalloc_shape(m, n);
     if (slog < 0) return fail(PJG_ERR_UNSUPPORTED, "mechanism too large for the evaluation kernels");
     if (int rc = make_tables(m, PJG_KIND_VJP, 0, nullptr, slog, slog, false, &kt)) return rc;
     const SchedTables& sd = kt->tile[slog];
@@ -1397,12 +1411,14 @@ int pjg_mech_create(const pjg_tables* tb, pjg_mech** out)
         pjg_mech_destroy(m);
         return rc;
     }
-    // pjg_vjp_noalloc may not allocate: its schedule now
+    // pjg_vjp_noalloc may not allocate: its schedules now
     KindTables* kt = nullptr;
-    const int slog = choose_shape(m, PJG_KIND_VJP, kNoallocStates);
-    if (slog >= 0 && (rc = make_tables(m, PJG_KIND_VJP, 0, nullptr, slog, slog, false, &kt))) {
-        pjg_mech_destroy(m);
-        return rc;
+    for (int64_t n : {(int64_t)1, INT64_MAX}) {
+        const int slog = noalloc_shape(m, n);
+        if (slog >= 0 && (rc = make_tables(m, PJG_KIND_VJP, 0, nullptr, slog, slog, false, &kt))) {
+            pjg_mech_destroy(m);
+            return rc;
+        }
     }
     *out = m;
     return 0;
