@@ -446,31 +446,37 @@ size_t wave_state_bytes(const pjg_mech* m, int kind, int n_vec)
 
 // Whether a thread per state evaluates `rest` states, less than a wave, sooner
 // than tiles do, by a model of both in units of a wave's time.  A thread per
-// state takes its time by the blocks of the fullest SM, tiles by rounds of
-// resident blocks, where a short last round costs two thirds of one and more.
-// Slopes from fits to four mechanisms at 27 sizes each on GB300; a mechanism
-// whose item lists are short (sum_parts draws that line) keeps its warps waiting
-// on barriers, and where tiles are smaller than 32 states they are slow.
-// Thread per state / tiles, us: Jacobian F GRI-Mech 3.0 59,000 states 4,194 /
-// 4,080, 72,000 4,248 / 4,809, H2/O2 29,000 280 / 256, 30,000 278 / 315; rates GRI
-// 38,800 998 / 1,083, 39,000 1,178 / 1,084, 50,000 1,221 / 1,332; J^T v GRI 29,000
-// 1,695 / 1,510, 30,000 1,693 / 1,812, H2/O2 26,000 208 / 234; 500 species, ms:
-// sparse Jacobian F 16,384 50 / 50, 24,000 56 / 74, rates 19,456 13.8 / 10.1, 32,768
-// 16.5 / 17.2, J^T v 12,000 38 / 35, 16,384 38 / 48.
+// state takes its time by the blocks of the fullest SM (first + block * blocks),
+// tiles theirs by rounds of resident blocks, where a short last round costs two
+// thirds of one and more; their slope grows where one block fills an SM's shared
+// memory and where less than 32 states fit.  A mechanism whose item lists are
+// short (sum_parts draws that line) keeps its warps waiting on barriers.  Fitted
+// to 15 mechanisms of 9 to 500 species at 14 to 27 sizes each on GB300.  Thread per
+// state / tiles, us: Jacobian F GRI-Mech 3.0 59,000 states 4,194 / 4,080, 72,000 4,248
+// / 4,809, H2/O2 29,000 280 / 256, 30,000 278 / 315; rates GRI 38,800 998 / 1,083, 39,000
+// 1,178 / 1,084, 50,000 1,221 / 1,332; J^T v GRI 29,000 1,695 / 1,510, 30,000 1,693 /
+// 1,812, H2/O2 26,000 208 / 234; ms: Jacobian F, 120 species 30,000 10.4 / 9.7, 38,912
+// 10.7 / 11.2, 220 species 25,000 21.9 / 20.3, 30,000 22.0 / 23.9, 500 species 16,384 50 /
+// 50, 24,000 56 / 74; rates 120 species 50,000 3.80 / 4.58; J^T v 80 species 19,456
+// 3.90 / 3.78, 25,000 4.73 / 5.18.
 bool wave_sooner(const pjg_mech* m, int kind, int64_t rest)
 {
     struct Cost {
-        double first, block, tile, small;
+        double first, block, tile;
     };
-    static const Cost costs[3] = {{0.20, 0.133, 1.30, 1.70}, {0.40, 0.15, 1.05, 1.55}, {0.28, 0.24, 1.24, 1.60}};
-    static const Cost large[3] = {{0.33, 0.07, 1.75}, {0.60, 0.135, 2.54}, {0.63, 0.12, 3.31}};  // tiles below 32 states
-    const Cost& c = m->top_slog[kind] < 5 ? large[kind] : costs[kind];
+    // tiles of 32 states, several blocks per SM and one; of 16; of fewer
+    static const Cost costs[3][4] = {{{0.25, 0.105, 1.30}, {0.25, 0.105, 1.46}, {0.33, 0.07, 1.75}, {0.33, 0.07, 2.20}},
+                                     {{0.40, 0.15, 1.05}, {0.43, 0.10, 1.32}, {0.62, 0.12, 1.73}, {0.60, 0.135, 2.54}},
+                                     {{0.28, 0.24, 1.24}, {0.45, 0.185, 1.78}, {0.63, 0.12, 2.25}, {0.63, 0.12, 3.31}}};
+    static const double small[3] = {1.70, 1.55, 1.60};
     if (rest <= 0) return false;
-    if (m->top_slog[kind] < 0) return true;  // no tile of this mechanism fits in shared memory
+    const int top = m->top_slog[kind];
+    if (top < 0) return true;  // no tile of this mechanism fits in shared memory
     const int64_t round = m->round[kind], per_block = (int64_t)m->sms * PJG_BLOCK;
+    const Cost& c = costs[kind][top == 5 ? (round >> 5 <= m->sms ? 1 : 0) : top == 4 ? 2 : 3];
     double rounds = (double)(rest / round);
     if (rest % round) rounds += 0.65 + 0.35 * (double)(rest % round) / (double)round;
-    const double slope = sum_parts(m->ns) == 1 ? c.small : c.tile;
+    const double slope = sum_parts(m->ns) == 1 ? small[kind] : c.tile;
     return slope * rounds * (double)round / (double)m->wave[kind] >=
            c.first + c.block * (double)((rest + per_block - 1) / per_block);
 }
@@ -566,7 +572,7 @@ size_t eval_state_bytes(int kind, bool F, const SlotTables* t)
 // lost by it (GRI-Mech 3.0, 170,000 states 3.34 ms in one launch, 3.42 as the sum
 // of its parts).
 struct Plan {
-    int64_t n_wave = 0, n_whole = 0, ch_wave = 0, ch_tile = 0;
+    int64_t n_wave = 0, n_whole = 0, ch_wave = 0, ch_whole = 0, ch_tile = 0;
     WaveHold* wh = nullptr;
     SchedTables* sd = nullptr;
     int grid = 0;
@@ -588,12 +594,17 @@ int make_plan(pjg_mech* m, int kind, bool F, bool sparse, const SlotTables* t, i
     p->n_wave = rest_wave ? n : n / W * W;
     const int64_t per_block = (int64_t)m->sms * PJG_BLOCK;
     p->n_whole = kind != PJG_SPECIES_RATES && n % W <= W - per_block ? n / W * W : p->n_wave;
+    // a large mechanism's waves are of three blocks; a rest of one goes with the last
+    // of them (as four, 320 species F 77,824 states 64 ms, in turn 72)
+    const bool threes = kind == PJG_JACOBIAN && m->top_slog[kind] < 5;
+    if (threes && rest_wave && n >= W && n % W <= per_block) p->n_whole -= W;
+    const int64_t unit = threes ? W + per_block : W;  // of a chunk
     if (smaller) {
         // What a smaller batch leaves to the tiles is less than a wave.  The most
         // of n or fewer states, less than a wave, that a thread per state takes
         // fill their blocks: its time is the same with fewer.
         const int64_t most = std::min(n, W);
-        int64_t wave = most == W ? W : rest_wave ? n : most / per_block * per_block;
+        int64_t wave = most == W ? std::min(n, unit) : rest_wave ? n : most / per_block * per_block;
         while (wave > 0 && wave < W && !wave_sooner(m, kind, wave)) wave = (wave - 1) / per_block * per_block;
         const int top = n >= W || wave > 0 ? 5 : choose_shape(m, kind, per_state ? chunk_states(per_state, n, W) : n);
         if (int rc = make_tables(m, kind, layout, slot, 0, top, wave > 0, &kt)) return rc;
@@ -603,14 +614,16 @@ int make_plan(pjg_mech* m, int kind, bool F, bool sparse, const SlotTables* t, i
         p->need = per_state * (size_t)(per_state ? chunk_states(per_state, most, W) : 0) + slices;
         if (wave > 0) {
             const size_t each = per_state + wave_state_bytes(m, kind, kt->wave.n_vec);
-            p->need = std::max(p->need, each * (size_t)chunk_states(each, wave, W));
+            p->need = std::max(p->need, each * (size_t)chunk_states(each, wave, unit));
         }
     }
     if (p->n_wave > 0) {
         if (int rc = make_tables(m, kind, layout, slot, 0, -1, true, &kt)) return rc;
         p->wh = &kt->wave;
         const size_t each = per_state + wave_state_bytes(m, kind, p->wh->n_vec);
-        p->ch_wave = std::min<int64_t>(most_states ? most_states : chunk_states(each, p->n_wave, W), p->n_wave);
+        p->ch_wave = std::min<int64_t>(most_states ? most_states : chunk_states(each, p->n_wave, unit), p->n_wave);
+        // whole waves a launch
+        p->ch_whole = p->ch_wave >= W ? p->ch_wave / W * W : p->ch_wave;
         p->need = std::max(p->need, each * (size_t)p->ch_wave);
     }
     if (p->n_wave < n) {
@@ -671,7 +684,7 @@ int run_eval(pjg_mech* m, int kind, int64_t n, char order, int conp, int jac_for
     for (int64_t off = 0, cnt = 0; off < n; off += cnt) {
         const bool wave = off < n_wave;
         const int64_t ch = wave ? pl.ch_wave : pl.ch_tile;
-        cnt = std::min<int64_t>(ch, (off < pl.n_whole ? pl.n_whole : wave ? n_wave : n) - off);
+        cnt = off < pl.n_whole ? std::min(pl.ch_whole, pl.n_whole - off) : std::min(ch, (wave ? n_wave : n) - off);
         EvalArgs a;
         fill_common(m, a);
         a.n = cnt;

@@ -79,7 +79,8 @@ int pjg_launch_wave(const EvalArgs& a, int kind, int sms, bool large, void* stre
     if (kind == KIND_VJP) wave_launch<KIND_VJP, PJG_VJP_MINB>(a, grid, st);
     else if (kind == KIND_RATES) wave_launch<KIND_RATES, PJG_RATES_MINB>(a, grid, st);
     else if (grid <= (unsigned)(kFewBlocks * sms)) wave_launch<KIND_JAC, kFewBlocks>(a, grid, st);
-    else if (large) wave_launch<KIND_JAC, kLargeBlocks>(a, grid, st);
+    else if (large && (grid <= (unsigned)(kLargeBlocks * sms) || grid > (unsigned)(PJG_JAC_MINB * sms)))
+        wave_launch<KIND_JAC, kLargeBlocks>(a, grid, st);
     else wave_launch<KIND_JAC, PJG_JAC_MINB>(a, grid, st);
     pjg_launch_err = cudaGetLastError();
     return pjg_launch_err == cudaSuccess ? 0 : -2;
