@@ -730,7 +730,7 @@ def implicit_bench(mech, ev, dev, n, order, steps, warmup, fp64_peak):
                       "fp64_frac": fl * f_rate / 1e12 / fp64_peak,
                       "fp64_peak_source": "measured DFMA probe (pjg_fp64_peak)",
                       "hbm_gbs": 2 * lu_bytes * f_rate / 1e9},
-           "solve": {"kernel": "lu_solve_kernel (32 states per block, rows shared by 8 warps)", "ms": s_ms,
+           "solve": {"kernel": "lu_solve_lane_kernel (a thread per state; smaller batches: lu_solve_kernel)", "ms": s_ms,
                      "states_per_s": n / (s_ms * 1e-3), "launches": s_launch,
                      "alg_bytes_per_state": lu_bytes + 4 * nn + 16 * nn,
                      "hbm_gbs": (lu_bytes + 20 * nn) * n / (s_ms * 1e-3) / 1e9},

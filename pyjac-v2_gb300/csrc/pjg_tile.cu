@@ -1,6 +1,9 @@
 // Species-rate, Jacobian and J^T v kernels for batches below a wave of the
-// thread-per-state kernels (pjg_wave.cuh), whose results they give bit for bit:
-// the same reaction code (pjg_rxn.cuh), every sum in the same order.
+// thread-per-state kernels (pjg_wave.cuh): the same reaction code (pjg_rxn.cuh),
+// the sums over reactions and species in the same order.  The rates are equal bit
+// for bit, the Jacobian but for the contraction of a few products; of J^T v, columns
+// T and E and the bath-gas term of every column are summed per worker first, so
+// their last bits depend on the tile's shape.
 #include <cuda_runtime.h>
 
 #include <type_traits>
@@ -38,8 +41,8 @@ __device__ __forceinline__ void red_global(uint64_t p, double x)
 // reactions come in batches, one per worker; a worker leaves its reaction's
 // terms in shared memory, and after a barrier the batch's additions to the
 // Jacobian and the rates are made from there, every target by one worker, in
-// the reactions' order.  So each sum has one fixed order, whatever S and W,
-// and the additions are fire-and-forget reductions (red.global.add.f64) that
+// the reactions' order.  So each of these sums has one fixed order, whatever S and
+// W, and the additions are fire-and-forget reductions (red.global.add.f64) that
 // take no FP64 instruction.
 //
 // The arrays that the reactions read (concentrations, 1 / Kc factors, weights)
@@ -50,9 +53,12 @@ __device__ __forceinline__ void red_global(uint64_t p, double x)
 // GRI-Mech 3.0 on GB300, before -> here: dense Jacobian C, 200 states 2,370 ->
 // 131 us; sparse F, 10,007 states 2,694 -> 1,031 us; rates C, 1,000 states 720 ->
 // 137 us; the 500-species mechanism's sparse Jacobian C, 4,096 states 60.9 ->
-// 14.0 ms.  Tiles of 32 states keep the FP64 pipe 62 % busy (a thread per state
-// 56 to 74 %): what is left are the phases between the reactions and the
-// reductions' rate, about 23 clocks per warp and SM.
+// 13.8 ms.  Tiles of 32 states keep the FP64 pipe 61 % busy where they fill the SMs
+// (37 % of the 10,007 states' time, nine of whose 313 tiles run a second round): what
+// is left are the phases between the reactions and waits on shared memory.  Tiles
+// of a few states wait on the barriers between a batch's reactions and its
+// additions (half to two thirds of the stalls), those of 500 species on instruction
+// fetch and barriers.
 template <int KIND>  // KIND_RATES, KIND_JAC, KIND_VJP
 __global__ void __launch_bounds__(32 * kTileWarps, KIND == KIND_RATES ? 3 : 2)
     tile_kernel(const EvalArgs a)

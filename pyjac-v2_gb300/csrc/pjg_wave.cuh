@@ -26,8 +26,11 @@
 // Numeric guards are the reference's (pyjac/core/instruction_creator.py:370-478):
 // T clamped to [100, 10000] K for rate evaluation, V >= 1e-30, moles and
 // concentrations in derivative products >= 1e-300, exp(min(x, 690.775527898)),
-// log(max(x, 1e-300)).  As in the reference, the explicit T, V, P factors of the
-// Jacobian blocks use the unclamped state values.
+// log(max(x, 1e-300)).  (The derivatives of A + B <=> C + D take the rates' own
+// products where no concentration is negative: moles there are >= 1e-300
+// already, and V > 1 or a vanishing bath gas may put a concentration below.)  As
+// in the reference, the explicit T, V, P factors of the Jacobian blocks use the
+// unclamped state values.
 //
 // FP64 instruction count is the cost that matters on GB300 (2 FP64 FMA per clock
 // per SM): quotients of the NASA polynomials come precomputed in the species
@@ -38,11 +41,12 @@
 // summed per reaction (d R_i / d c_j times the reaction's enthalpy, and times
 // sum nu) instead of over the species block, which is not read back; the
 // exponentials take their integer part on the integer pipe (fexp_s).  FP64
-// instructions per GRI state, ncu: Jacobian 27,817 -> 21,700, rates 11,255 ->
-// 9,830; 1M states dense F 68.5 -> 61.8 ms, rates 21.9 -> 19.0 ms.  What bounds
-// it now: loads of the per-state arrays (L1 hit rate 22 %, half of the warps'
-// stalls; DRAM moves 5.5x the output), at 56 % FP64 pipe for the Jacobian and
-// 74 % for the rates.
+// instructions per GRI state, ncu: Jacobian 27,817 -> 21,085, rates 11,255 ->
+// 9,619; 1M states dense F 68.5 -> 60.8 ms, rates 21.9 -> 19.0 ms.  The rates keep
+// the FP64 pipe 84 % busy.  The Jacobian keeps it 61 % busy and waits for its
+// per-state arrays, reductions and spilled registers (396 bytes of stores and 528
+// of loads): four blocks of 128 registers per SM, 28 % of the accesses that reach
+// L2 hit, DRAM moves 5.3x the output.  J^T v: 82 %.
 #pragma once
 #include <cuda_runtime.h>
 

@@ -127,10 +127,10 @@ def test_approximate_jacobian(cuda_device, name, order, fmt):
     check(mech, P, phi, order, True, fmt, cuda_device, wave(cuda_device), vjp=False)
 
 
-@pytest.mark.parametrize("blocks", [2, 3])
+@pytest.mark.parametrize("blocks", [2, 3, 4])
 def test_large_mechanism(cuda_device, blocks):
     """The 500-species mechanism, whose Jacobian kernel holds three blocks per SM
-    (and two in the form for fewer blocks)."""
+    (two in the form for fewer blocks, four where a rest of one joins the last wave)."""
     import torch
     torch.cuda.empty_cache()
     mech = load_mech("synthetic500")
