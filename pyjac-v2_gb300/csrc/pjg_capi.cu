@@ -622,7 +622,7 @@ int make_plan(pjg_mech* m, int kind, bool F, bool sparse, const SlotTables* t, i
         p->wh = &kt->wave;
         const size_t each = per_state + wave_state_bytes(m, kind, p->wh->n_vec);
         p->ch_wave = std::min<int64_t>(most_states ? most_states : chunk_states(each, p->n_wave, unit), p->n_wave);
-        // whole waves a launch
+        // where several launches are needed, each of whole waves
         p->ch_whole = p->ch_wave >= W ? p->ch_wave / W * W : p->ch_wave;
         p->need = std::max(p->need, each * (size_t)p->ch_wave);
     }
@@ -684,7 +684,8 @@ int run_eval(pjg_mech* m, int kind, int64_t n, char order, int conp, int jac_for
     for (int64_t off = 0, cnt = 0; off < n; off += cnt) {
         const bool wave = off < n_wave;
         const int64_t ch = wave ? pl.ch_wave : pl.ch_tile;
-        cnt = off < pl.n_whole ? std::min(pl.ch_whole, pl.n_whole - off) : std::min(ch, (wave ? n_wave : n) - off);
+        if (off < pl.n_whole) cnt = pl.n_whole - off <= ch ? pl.n_whole - off : pl.ch_whole;
+        else cnt = std::min(ch, (wave ? n_wave : n) - off);
         EvalArgs a;
         fill_common(m, a);
         a.n = cnt;
