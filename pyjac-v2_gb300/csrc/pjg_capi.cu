@@ -107,7 +107,6 @@ struct SchedTables {
     Schedule sc;
     const PostItem* ns_post = nullptr;
     int n_ns_post = 0;
-    int resident = 0;  // blocks that the device holds at a time
     bool made = false;
 };
 
@@ -140,12 +139,14 @@ struct pjg_mech {
     int4* m_lists = nullptr;
     std::vector<RxnRec> d_rxn;    // host copy of the device records
     int device = 0;
-    // of the device, and per kind: states of a wave of the thread-per-state kernel,
-    // and log2 of the largest tile's states (-1: none fits) with the states of a
-    // round of resident ones
+    // per kind: log2 of the largest tile's states (-1: none fits); of the device
+    // (device_shape): states of a wave of the thread-per-state kernel and of a round
+    // of resident largest tiles, resident tiles of each size
     int sms = 1;
-    int64_t wave[3] = {}, round[3] = {};
     int top_slog[3] = {-1, -1, -1};
+    std::once_flag shape_once[3];
+    int64_t wave[3] = {}, round[3] = {};
+    int resident[3][6] = {};
     RxnRec* rxn = nullptr;
     double* sp = nullptr;
     int* thd_spec = nullptr;
@@ -381,9 +382,10 @@ int choose_shape(const pjg_mech* m, int kind, int64_t n)
     return found;
 }
 
-// The tables of a kind and layout that are not there yet: the shapes from ..
-// to (those that fit), and with `wave` the thread-per-state kernel's.
-int make_tables(pjg_mech* m, int kind, int layout, const std::vector<int>* slot, int from, int to, bool wave,
+// The tables of a kind and layout that are not there yet: the tile shapes of a
+// mask (bit log2 of the states; those that fit), and with `wave` the
+// thread-per-state kernel's.
+int make_tables(pjg_mech* m, int kind, int layout, const std::vector<int>* slot, unsigned shapes, bool wave,
                 KindTables** out)
 {
     std::lock_guard<std::mutex> g(m->lock);
@@ -392,10 +394,10 @@ int make_tables(pjg_mech* m, int kind, int layout, const std::vector<int>* slot,
     *out = &kt;
     Pack pk;
     std::vector<bool*> made;
-    for (int slog = from; slog <= to; ++slog) {
+    for (int slog = 0; slog <= 5; ++slog) {
         SchedTables& t = kt.tile[slog];
         Shape sh;
-        if (t.made || !shape_fits(m, kind, slog, &sh)) continue;
+        if (!(shapes >> slog & 1u) || t.made || !shape_fits(m, kind, slog, &sh)) continue;
         SchedHost h;
         if (!sched_build(ad, slog, sh.rounds, sh.buf_terms, h))
             return fail(PJG_ERR_UNSUPPORTED, "a reaction's terms pass the evaluation kernel's buffer");
@@ -405,7 +407,6 @@ int make_tables(pjg_mech* m, int kind, int layout, const std::vector<int>* slot,
         t.sc.buf_terms = sh.buf_terms;
         t.sc.n_vec = ad.n_vec;
         t.n_ns_post = (int)ad.ns_post.size();
-        t.resident = m->sms * pjg_tile_blocks_per_sm(kind, pjg_tile_smem(kind, m->ns, m->n_m, slog, sh.buf_terms));
         pk.add(h.tasks, &t.sc.tasks);
         pk.add(h.term_off, &t.sc.term_off);
         pk.add(h.item_off, &t.sc.item_off);
@@ -481,32 +482,32 @@ bool wave_sooner(const pjg_mech* m, int kind, int64_t rest)
            c.first + c.block * (double)((rest + per_block - 1) / per_block);
 }
 
-// what the mechanism's launches ask of the device (pjg_mech, once n_m is known)
-void device_shapes(pjg_mech* m)
+// What the launches of a kind ask of the device, at its first use: the question
+// loads the kernels.
+void device_shape(pjg_mech* m, int kind)
 {
-    cudaDeviceGetAttribute(&m->sms, cudaDevAttrMultiProcessorCount, m->device);
-    for (int kind = 0; kind < 3; ++kind) {
-        for (int slog = 5; slog >= 0 && m->top_slog[kind] < 0; --slog) {
+    std::call_once(m->shape_once[kind], [&] {
+        const int top = m->top_slog[kind];
+        for (int slog = 0; slog <= top; ++slog) {
             Shape s;
-            if (!shape_fits(m, kind, slog, &s)) continue;
-            m->top_slog[kind] = slog;
-            const size_t smem = pjg_tile_smem(kind, m->ns, m->n_m, slog, s.buf_terms);
-            m->round[kind] = ((int64_t)m->sms * pjg_tile_blocks_per_sm(kind, smem)) << slog;
+            if (shape_fits(m, kind, slog, &s))
+                m->resident[kind][slog] = m->sms * pjg_tile_blocks_per_sm(kind, pjg_tile_smem(kind, m->ns, m->n_m, slog, s.buf_terms));
         }
-        m->wave[kind] = (int64_t)m->sms * pjg_wave_blocks_per_sm(kind, m->top_slog[kind] < 5) * PJG_BLOCK;
-    }
+        if (top >= 0) m->round[kind] = (int64_t)m->resident[kind][top] << top;
+        m->wave[kind] = (int64_t)m->sms * pjg_wave_blocks_per_sm(kind, top < 5) * PJG_BLOCK;
+    });
 }
 
 // blocks of a launch over n states
-int grid_of(const SchedTables& t, int64_t n)
+int grid_of(const pjg_mech* m, int kind, const SchedTables& t, int64_t n)
 {
-    return (int)std::min<int64_t>((n + (1 << t.sc.slog) - 1) >> t.sc.slog, t.resident);
+    return (int)std::min<int64_t>((n + (1 << t.sc.slog) - 1) >> t.sc.slog, m->resident[kind][t.sc.slog]);
 }
 
 // bytes of the blocks' scratch slices
-size_t slice_bytes(const SchedTables& t, int64_t n)
+size_t slice_bytes(const pjg_mech* m, int kind, const SchedTables& t, int64_t n)
 {
-    return ((size_t)grid_of(t, n) * t.sc.n_vec * sizeof(double)) << t.sc.slog;
+    return ((size_t)grid_of(m, kind, t, n) * t.sc.n_vec * sizeof(double)) << t.sc.slog;
 }
 
 int ensure_work(pjg_mech* m, size_t bytes)
@@ -585,6 +586,7 @@ struct Plan {
 int make_plan(pjg_mech* m, int kind, bool F, bool sparse, const SlotTables* t, int64_t n, int64_t most_states,
               bool smaller, Plan* p)
 {
+    device_shape(m, kind);
     const size_t per_state = eval_state_bytes(kind, F, t);
     const int layout = kind == PJG_JACOBIAN ? (F ? 2 : 0) + (sparse ? 1 : 0) : 0;
     const std::vector<int>* slot = t ? &t->slot : nullptr;
@@ -607,10 +609,10 @@ int make_plan(pjg_mech* m, int kind, bool F, bool sparse, const SlotTables* t, i
         int64_t wave = most == W ? std::min(n, unit) : rest_wave ? n : most / per_block * per_block;
         while (wave > 0 && wave < W && !wave_sooner(m, kind, wave)) wave = (wave - 1) / per_block * per_block;
         const int top = n >= W || wave > 0 ? 5 : choose_shape(m, kind, per_state ? chunk_states(per_state, n, W) : n);
-        if (int rc = make_tables(m, kind, layout, slot, 0, top, wave > 0, &kt)) return rc;
+        if (int rc = make_tables(m, kind, layout, slot, top < 0 ? 0u : (2u << top) - 1u, wave > 0, &kt)) return rc;
         size_t slices = 0;
         for (int q = 0; q <= top; ++q)
-            if (kt->tile[q].made) slices = std::max(slices, slice_bytes(kt->tile[q], most));
+            if (kt->tile[q].made) slices = std::max(slices, slice_bytes(m, kind, kt->tile[q], most));
         p->need = per_state * (size_t)(per_state ? chunk_states(per_state, most, W) : 0) + slices;
         if (wave > 0) {
             const size_t each = per_state + wave_state_bytes(m, kind, kt->wave.n_vec);
@@ -618,7 +620,7 @@ int make_plan(pjg_mech* m, int kind, bool F, bool sparse, const SlotTables* t, i
         }
     }
     if (p->n_wave > 0) {
-        if (int rc = make_tables(m, kind, layout, slot, 0, -1, true, &kt)) return rc;
+        if (int rc = make_tables(m, kind, layout, slot, 0u, true, &kt)) return rc;
         p->wh = &kt->wave;
         const size_t each = per_state + wave_state_bytes(m, kind, p->wh->n_vec);
         p->ch_wave = std::min<int64_t>(most_states ? most_states : chunk_states(each, p->n_wave, unit), p->n_wave);
@@ -633,10 +635,10 @@ int make_plan(pjg_mech* m, int kind, bool F, bool sparse, const SlotTables* t, i
             p->ch_tile = std::min<int64_t>(most_states ? most_states : chunk_states(per_state, p->ch_tile, W), p->ch_tile);
         const int slog = choose_shape(m, kind, p->ch_tile);
         if (slog < 0) return fail(PJG_ERR_UNSUPPORTED, "mechanism too large for the evaluation kernels");
-        if (int rc = make_tables(m, kind, layout, slot, slog, slog, false, &kt)) return rc;
+        if (int rc = make_tables(m, kind, layout, slot, 1u << slog, false, &kt)) return rc;
         p->sd = &kt->tile[slog];
-        p->grid = grid_of(*p->sd, p->ch_tile);
-        p->need = std::max(p->need, per_state * (size_t)p->ch_tile + slice_bytes(*p->sd, p->ch_tile));
+        p->grid = grid_of(m, kind, *p->sd, p->ch_tile);
+        p->need = std::max(p->need, per_state * (size_t)p->ch_tile + slice_bytes(m, kind, *p->sd, p->ch_tile));
     }
     return 0;
 }
@@ -1145,16 +1147,17 @@ int pjg_internal_fail(int code, const char* msg) { return fail(code, "%s", msg);
 int pjg_internal_vjp_args(pjg_mech* m, int64_t n, size_t scratch_doubles, EvalArgs* a, int* grid)
 {
     KindTables* kt = nullptr;
+    device_shape(m, PJG_KIND_VJP);
     const int slog = noalloc_shape(m, n);
     if (slog < 0) return fail(PJG_ERR_UNSUPPORTED, "mechanism too large for the evaluation kernels");
-    if (int rc = make_tables(m, PJG_KIND_VJP, 0, nullptr, slog, slog, false, &kt)) return rc;
+    if (int rc = make_tables(m, PJG_KIND_VJP, 0, nullptr, 1u << slog, false, &kt)) return rc;
     const SchedTables& sd = kt->tile[slog];
     fill_common(m, *a);
     a->sc = sd.sc;
     a->ns_post = sd.ns_post;
     a->n_ns_post = sd.n_ns_post;
     const size_t slice = (size_t)sd.sc.n_vec << slog;
-    *grid = (int)std::min<size_t>(grid_of(sd, n), scratch_doubles / slice);
+    *grid = (int)std::min<size_t>(grid_of(m, PJG_KIND_VJP, sd, n), scratch_doubles / slice);
     return *grid > 0 ? 0 : fail(PJG_ERR_ARG, "scratch too small for one tile");
 }
 int pjg_internal_mech_ns(const pjg_mech* m) { return m->ns; }
@@ -1413,7 +1416,12 @@ int pjg_mech_create(const pjg_tables* tb, pjg_mech** out)
     }
     std::vector<int4> m_lists;
     device_records(m, tb->species, m_lists);
-    device_shapes(m);
+    cudaDeviceGetAttribute(&m->sms, cudaDevAttrMultiProcessorCount, m->device);
+    for (int kind = 0; kind < 3; ++kind)
+        for (int slog = 0; slog <= 5; ++slog) {
+            Shape s;
+            if (shape_fits(m, kind, slog, &s)) m->top_slog[kind] = slog;
+        }
     std::vector<double> sp(tb->species, tb->species + (size_t)tb->ns * PJG_SP_DOUBLES);
     std::vector<double> coef(tb->thd_coef, tb->thd_coef + std::max(tb->n_thd, 0));
     std::vector<double> aux(tb->aux ? tb->aux : (const double*)nullptr,
@@ -1427,12 +1435,12 @@ int pjg_mech_create(const pjg_tables* tb, pjg_mech** out)
     }
     // pjg_vjp_noalloc may not allocate: its schedules now
     KindTables* kt = nullptr;
-    for (int64_t n : {(int64_t)1, INT64_MAX}) {
-        const int slog = noalloc_shape(m, n);
-        if (slog >= 0 && (rc = make_tables(m, PJG_KIND_VJP, 0, nullptr, slog, slog, false, &kt))) {
-            pjg_mech_destroy(m);
-            return rc;
-        }
+    unsigned shapes = 0;
+    for (int64_t n : {(int64_t)1, INT64_MAX})
+        if (noalloc_shape(m, n) >= 0) shapes |= 1u << noalloc_shape(m, n);
+    if ((rc = make_tables(m, PJG_KIND_VJP, 0, nullptr, shapes, false, &kt))) {
+        pjg_mech_destroy(m);
+        return rc;
     }
     *out = m;
     return 0;
@@ -1541,9 +1549,10 @@ int pjg_eval_chunk(pjg_mech* m, int kind, int64_t n, char order, int jac_format,
         int rc = build_slots(m, order == 'F', jac_format == PJG_JAC_SPARSE, &t);
         if (rc) return rc;
     }
+    device_shape(m, kind);
     const int layout = kind == PJG_JACOBIAN ? (order == 'F' ? 2 : 0) + (jac_format == PJG_JAC_SPARSE ? 1 : 0) : 0;
     KindTables* kt = nullptr;
-    if (int rc = make_tables(m, kind, layout, t ? &t->slot : nullptr, 0, -1, true, &kt)) return rc;
+    if (int rc = make_tables(m, kind, layout, t ? &t->slot : nullptr, 0u, true, &kt)) return rc;
     const size_t per_state = eval_state_bytes(kind, order == 'F', t);
     const int64_t W = m->wave[kind], n_wave = wave_sooner(m, kind, n % W) ? n : n / W * W;
     *states = n_wave ? chunk_states(per_state + wave_state_bytes(m, kind, kt->wave.n_vec), n_wave, W)
@@ -1728,6 +1737,7 @@ int pjg_kernel_resize(pjg_kernel* k, size_t problem_size, size_t work_size)
     // (the evaluation's arrays a little above their size, which the tables give)
     const size_t arrays = (size_t)(tile_arrays(k->kind) + vec_arrays(k->kind) + 2) * m->ns * sizeof(double);
     const size_t ring_state = kRing * (1 + nn + k->out_per_state) * sizeof(double) + per_state + arrays;
+    device_shape(m, PJG_JACOBIAN);
     const int64_t wave = m->wave[PJG_JACOBIAN];
     int64_t chunk = std::min<int64_t>((int64_t)problem_size, PJG_CHUNK_WAVES * wave);
     if ((size_t)chunk * ring_state > kKernelBudget) {
